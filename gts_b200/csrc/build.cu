@@ -7,8 +7,12 @@
 //   2. k_keys: every object of a split node gets the reference's double key
 //      dist/INFI_DIS + b*DIS_CODE (tree.cuh:155), distance in the
 //      F64-accumulated build arithmetic;
-//   3. a stable segmented sort of (key, id) inside each split node.  The
-//      reference sorts all N keys globally (tree.cuh:372); node codes keep
+//   3. a stable sort of (key, id) inside each split node: one radix sort of
+//      all keys, then (below the root) one by the node's first position, so
+//      every node's range keeps its place and an unsplit node its order (eight
+//      plus a few radix passes over the whole chip; a segmented sort gave each
+//      of the few huge segments near the root one CTA: 19.2 ms against 1.9 for
+//      the five levels of 1,000,000 objects).  The reference sorts all N keys globally (tree.cuh:372); node codes keep
 //      the segments apart and the sort is stable, so for every tree in which
 //      each level's objects all sit in split nodes the order is identical;
 //   4. k_split: O children per split node with the equal-count split, the
@@ -19,7 +23,7 @@
 //      run one thread per object instead of one block per node.
 // One 4-byte device->host read per level (the number of nodes still to
 // split) decides whether to continue, as the reference's reduce does.
-#include <cub/device/device_segmented_sort.cuh>
+#include <cub/device/device_radix_sort.cuh>
 #include <cstdio>
 #include <vector>
 #include "index.cuh"
@@ -94,8 +98,7 @@ __global__ void k_init(int n, int mnn, int *id_list, int *node_of_pos, int *node
 }
 
 __global__ void k_select_pivots(int start, int nb, const int *id_list, const int *node_size,
-                                const int *node_lid, const uint8_t *split, int *node_pivot,
-                                int *seg_begin, int *seg_end)
+                                const int *node_lid, const uint8_t *split, int *node_pivot)
 {
     int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nb) return;
@@ -104,26 +107,37 @@ __global__ void k_select_pivots(int start, int nb, const int *id_list, const int
         int lid = node_lid[nid], size = node_size[nid];
         int rid = lid + size - 1;
         node_pivot[nid] = id_list[(lid + rid) / 2];
-        seg_begin[b] = lid;
-        seg_end[b] = lid + size;
-    } else {
-        seg_begin[b] = 0;
-        seg_end[b] = 0;
     }
 }
 
 __global__ void k_keys(DevData d, int n, int start, int nb, int dis_code, int infi_dis,
                        const int *id_list, const int *node_of_pos, const uint8_t *split,
-                       const int *node_pivot, double *key)
+                       const int *node_pivot, double *key, int *posv)
 {
     size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t pos = (size_t)blockIdx.x * blockDim.x + threadIdx.x; pos < (size_t)n; pos += stride) {
         int nid = node_of_pos[pos];
         int b = nid - start;
+        posv[pos] = (int)pos;
+        key[pos] = 0.0;   // an unsplit node keeps its order
         if (b < 0 || b >= nb || !split[nid]) continue;
         double res = obj_dist(d, id_list[pos], node_pivot[nid], kAccF64);
         key[pos] = (double)(res / infi_dis + b * dis_code);
     }
+}
+
+// Sort key of the second pass: the first position of the node that holds
+// the object (node ranges partition the positions in order).
+__global__ void k_node_lids(int n, const int *posv, const int *node_of_pos, const int *node_lid, uint32_t *lid)
+{
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) lid[i] = (uint32_t)node_lid[node_of_pos[posv[i]]];
+}
+
+__global__ void k_apply_order(int n, const int *posv, const int *ids, int *out)
+{
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = ids[posv[i]];
 }
 
 __global__ void k_split(DevData d, int start, int nb, int order, int max_size, const int *id_list,
@@ -278,13 +292,13 @@ void free_data(gts_index *idx)
 namespace {
 // Build-time scratch, released on every exit path.
 struct BuildScratch {
-    int *node_of_pos = nullptr, *ids_alt = nullptr, *seg_b = nullptr, *seg_e = nullptr, *nsplit = nullptr;
+    int *node_of_pos = nullptr, *ids_alt = nullptr, *posv = nullptr, *posv_alt = nullptr, *nsplit = nullptr;
     double *key = nullptr, *key_alt = nullptr;
     uint8_t *split = nullptr;
     void *temp = nullptr;
     ~BuildScratch()
     {
-        void *ps[] = {node_of_pos, ids_alt, seg_b, seg_e, nsplit, key, key_alt, split, temp};
+        void *ps[] = {node_of_pos, ids_alt, posv, posv_alt, nsplit, key, key_alt, split, temp};
         for (void *p : ps)
             if (p) cudaFree(p);
     }
@@ -302,8 +316,6 @@ static int build_tree_impl(gts_index *idx, cudaStream_t s)
     }
     const int mnn = (int)mnn_d;
     idx->max_node_num = mnn;
-    int maxnb = 1;   // nodes at the deepest level that can split: O^(H-2)
-    for (int l = 0; l + 2 < H; l++) maxnb *= O;
 
     size_t acct = 0;
     int rc;
@@ -332,14 +344,18 @@ static int build_tree_impl(gts_index *idx, cudaStream_t s)
     ALLOC(sc.key, n);
     ALLOC(sc.key_alt, n);
     ALLOC(sc.split, mnn);
-    ALLOC(sc.seg_b, maxnb);
-    ALLOC(sc.seg_e, maxnb);
+    ALLOC(sc.posv, n);
+    ALLOC(sc.posv_alt, n);
     ALLOC(sc.nsplit, 1);
 #undef ALLOC
-    size_t temp_bytes = 0;
-    GTS_CUDA_TRY(cub::DeviceSegmentedSort::StableSortPairs(nullptr, temp_bytes, sc.key, sc.key_alt,
-                                                           idx->id_list, sc.ids_alt, n, maxnb,
-                                                           sc.seg_b, sc.seg_e, s));
+    int lid_bits = 1;
+    while (lid_bits < 31 && (1 << lid_bits) < n) lid_bits++;
+    size_t temp_bytes = 0, temp_lid = 0;
+    GTS_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, sc.key, sc.key_alt, sc.posv, sc.posv_alt, n, 0,
+                                                 64, s));
+    GTS_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, temp_lid, (uint32_t *)nullptr, (uint32_t *)nullptr,
+                                                 sc.posv_alt, sc.posv, n, 0, lid_bits, s));
+    temp_bytes = std::max(temp_bytes, temp_lid);
     if (cudaMalloc(&sc.temp, temp_bytes ? temp_bytes : 1) != cudaSuccess) {
         cudaGetLastError();
         gts_set_error("cudaMalloc of sort scratch (%zu bytes) failed", temp_bytes);
@@ -355,17 +371,23 @@ static int build_tree_impl(gts_index *idx, cudaStream_t s)
         int nb = 1;
         for (int l = 0; l < cur_level; l++) nb *= O;
         k_select_pivots<<<(nb + 255) / 256, 256, 0, s>>>(start, nb, idx->id_list, idx->node_size,
-                                                         idx->node_lid, sc.split, idx->node_pivot,
-                                                         sc.seg_b, sc.seg_e);
+                                                         idx->node_lid, sc.split, idx->node_pivot);
         k_keys<<<grid_for(n, 256), 256, 0, s>>>(dd, n, start, nb, p.dis_code, p.infi_dis,
                                                  idx->id_list, sc.node_of_pos, sc.split,
-                                                 idx->node_pivot, sc.key);
-        GTS_CUDA_TRY(cudaMemcpyAsync(sc.ids_alt, idx->id_list, sizeof(int) * (size_t)n,
-                                     cudaMemcpyDeviceToDevice, s));
+                                                 idx->node_pivot, sc.key, sc.posv);
         size_t tb = temp_bytes;
-        GTS_CUDA_TRY(cub::DeviceSegmentedSort::StableSortPairs(sc.temp, tb, sc.key, sc.key_alt,
-                                                               idx->id_list, sc.ids_alt, n, nb,
-                                                               sc.seg_b, sc.seg_e, s));
+        GTS_CUDA_TRY(cub::DeviceRadixSort::SortPairs(sc.temp, tb, sc.key, sc.key_alt, sc.posv, sc.posv_alt, n, 0, 64,
+                                                     s));
+        int *order = sc.posv_alt;
+        if (cur_level > 0) {   // the key buffers serve the second pass
+            uint32_t *lid = (uint32_t *)sc.key, *lid_alt = (uint32_t *)sc.key_alt;
+            k_node_lids<<<(n + 255) / 256, 256, 0, s>>>(n, sc.posv_alt, sc.node_of_pos, idx->node_lid, lid);
+            tb = temp_bytes;
+            GTS_CUDA_TRY(cub::DeviceRadixSort::SortPairs(sc.temp, tb, lid, lid_alt, sc.posv_alt, sc.posv, n, 0,
+                                                         lid_bits, s));
+            order = sc.posv;
+        }
+        k_apply_order<<<(n + 255) / 256, 256, 0, s>>>(n, order, idx->id_list, sc.ids_alt);
         std::swap(idx->id_list, sc.ids_alt);
         GTS_CUDA_TRY(cudaMemsetAsync(sc.nsplit, 0, sizeof(int), s));
         long nthreads = (long)nb * O;
