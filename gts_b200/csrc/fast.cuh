@@ -70,7 +70,7 @@ __host__ __device__ inline FastShape fast_shape(int dim)
     return s;
 }
 
-// Seeds per slot (fast.cu, k_fast_selfk): k = 2^j for j < kSelfKN
+// Seeds per slot (fast_seed.cu): k = 2^j for j < kSelfKN
 // (k = 1 .. 64) and one padding entry, 32 bytes per slot; made from the
 // object's own block and the kSeedNbr blocks with the nearest centres,
 // keeping the kSeedBest smallest distances per object.
@@ -159,6 +159,10 @@ inline FastSummary fast_summary(unsigned char *recs, const FastShape &fs, int nb
     s.scop = prune_cop_bytes(fs, nsb) ? recs + o.scop : nullptr;
     return s;
 }
+
+// The blocks' nearest centres (bs.nbr) and the seed table (bs.selfk) over
+// them, from the centres and the slot-ordered rows (fast_seed.cu).
+int seed_table_build(const FastSummary &bs, int nb, const FastShape &fs, cudaStream_t st);
 
 // The tiles' needed superblocks (mask words sb_mask[tile][nsbw]; cleared
 // first when `clear`) and then their needed blocks (blist[tile][..] in
