@@ -417,15 +417,19 @@ class Index:
     def range_ids(self, qids, r: float, capacity: int | None = None):
         """-> (counts, offsets, ids, dists); each query's hits in (distance, id) order."""
         q = np.ascontiguousarray(qids, dtype=np.int32)
-        counts = np.empty(len(q), np.int32)
+        counts = np.zeros(len(q), np.int32)
         offs = np.empty(len(q), np.int32)
-        if capacity is None:
-            capacity = int(self.range(q, r).sum())
-        ids = np.empty(max(capacity, 1), np.int32)
-        dis = np.empty(max(capacity, 1), np.float32)
-        _check(self._lib.gts_range_ids(self._h, _ip(q), len(q), C.c_float(r), _ip(counts),
-                                       _ip(offs), _ip(ids), _fp(dis), C.c_size_t(capacity)))
-        tot = int(counts.sum())
+        room = max(1024, 64 * len(q)) if capacity is None else capacity
+        while True:
+            ids = np.empty(max(room, 1), np.int32)
+            dis = np.empty(max(room, 1), np.float32)
+            rc = self._lib.gts_range_ids(self._h, _ip(q), len(q), C.c_float(r), _ip(counts),
+                                         _ip(offs), _ip(ids), _fp(dis), C.c_size_t(room))
+            tot = int(counts.sum(dtype=np.int64))
+            if rc == 0 or capacity is not None or tot <= room:
+                break
+            room = tot   # the first call counted them
+        _check(rc)
         return counts, offs, ids[:tot], dis[:tot]
 
     def learn_radius(self, n_train: int = 200_000, k_max: int = 64, epochs: int = 12,

@@ -382,6 +382,7 @@ extern "C" void gts_index_free(gts_index *idx)
     if (idx->scratch) cudaFree(idx->scratch);
     if (idx->split_buf) cudaFree(idx->split_buf);
     if (idx->io) cudaFree(idx->io);
+    if (idx->hits) cudaFree(idx->hits);
     for (int i = 0; i < gts_index::kGraphSlots; i++)
         if (idx->graph_exec[i]) cudaGraphExecDestroy(idx->graph_exec[i]);
     if (idx->graph_stream) cudaStreamDestroy(idx->graph_stream);
@@ -626,8 +627,30 @@ extern "C" int gts_range_ids(gts_index *idx, const int *qids, int qnum, float r,
         return GTS_ERR_INVALID;
     }
     if (qnum == 0) return GTS_OK;
-    int rc = gts_range(idx, qids, qnum, r, counts_out);
+    int rc = check_qids(idx, qids, qnum);
     if (rc) return rc;
+    {
+        // one sweep lists, evaluates and orders every hit on the device
+        IoCarve io;
+        io.add(sizeof(int) * (size_t)qnum);
+        io.add(sizeof(int) * (size_t)qnum);
+        void *buf[2];
+        if ((rc = io.get(idx, buf))) return rc;
+        GTS_CUDA_TRY(cudaMemcpyAsync(buf[0], qids, sizeof(int) * (size_t)qnum, cudaMemcpyHostToDevice, idx->stream));
+        size_t hits = 0;
+        int done = 0;
+        if ((rc = gts::sweep_range_ids(idx, (int *)buf[0], qnum, r, (int *)buf[1], counts_out, offsets_out, ids_out,
+                                       dists_out, capacity, &hits, &done, idx->stream)))
+            return rc;
+        if (done) {
+            if (hits > capacity || hits > 0x7fffffff) {
+                gts_set_error("range result needs %zu entries, capacity %zu", hits, capacity);
+                return GTS_ERR_NOMEM;
+            }
+            return GTS_OK;
+        }
+    }
+    if ((rc = gts_range(idx, qids, qnum, r, counts_out))) return rc;
     size_t total = 0;
     for (int i = 0; i < qnum; i++) {
         offsets_out[i] = (int)total;
@@ -785,7 +808,10 @@ extern "C" int gts_plain_split(gts_index *idx, int objects, long long *items_han
         gts_set_error("null index");
         return GTS_ERR_INVALID;
     }
-    if (objects >= 0) idx->plain_split = objects;
+    if (objects >= 0) {
+        idx->plain_split = objects;
+        idx->plain_split_set = true;
+    }
     if (items_handed) *items_handed = idx->last_split_items;
     return GTS_OK;
 }

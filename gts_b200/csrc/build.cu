@@ -219,6 +219,56 @@ __global__ void k_permute(int n, int dim, int metric, const int *id_list, const 
     }
 }
 
+// The batched sweep's cut nodes and their ancestors (index.cuh); a CTA
+// appends its nodes in order, so lists stay nearly in position order.
+__global__ void __launch_bounds__(256) k_cut_lists(int mnn, int order, const uint8_t *flags, const int *size,
+                                                   const int *pivot, int *cut, int *anc, int *anc_idx, int *counts)
+{
+    __shared__ int base[2], woff[2][8];
+    const int i = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    bool is[2] = {false, false};
+    if (i < mnn && (flags[i] & kExists) && size[i] > 0) {
+        is[1] = pivot[i] >= 0 && size[i] > kCutSize;
+        is[0] = !is[1] && (i == 0 || size[(i - 1) / order] > kCutSize);
+    }
+    unsigned m[2];
+    for (int u = 0; u < 2; u++) {
+        m[u] = __ballot_sync(0xffffffffu, is[u]);
+        if (lane == 0) woff[u][warp] = __popc(m[u]);
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        const int u = threadIdx.x;
+        int run = 0;
+        for (int w = 0; w < 8; w++) {
+            const int c = woff[u][w];
+            woff[u][w] = run;
+            run += c;
+        }
+        base[u] = run ? atomicAdd(&counts[u], run) : 0;
+    }
+    __syncthreads();
+    for (int u = 0; u < 2; u++)
+        if (is[u]) {
+            const int at = base[u] + woff[u][warp] + __popc(m[u] & ((1u << lane) - 1u));
+            (u == 0 ? cut : anc)[at] = i;
+            if (u == 1) anc_idx[i] = at;
+        }
+}
+
+// Norms of the rows in tree order, in the angle metric's own arithmetic
+// (dist_row_f64): FP32 fused sums in dimension order.
+__global__ void k_row_norms(int n, int dim, const float *trows, float *tnorm)
+{
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < (size_t)n; i += (size_t)gridDim.x * blockDim.x) {
+        const float *a = trows + i * dim;
+        float sa = 0.f;
+        for (int j = 0; j < dim; j++) sa = fmaf(a[j], a[j], sa);
+        sa = pow(sa, 0.5);
+        tnorm[i] = sa;
+    }
+}
+
 static inline unsigned grid_for(size_t n, int block, unsigned cap = 148u * 32u)
 {
     size_t g = (n + block - 1) / block;
@@ -259,6 +309,25 @@ int ensure_io(gts_index *idx, size_t bytes)
     return GTS_OK;
 }
 
+int ensure_hits(gts_index *idx, size_t bytes, void **out)
+{
+    if (bytes > idx->hits_bytes) {
+        if (idx->hits) cudaFree(idx->hits);
+        idx->hits = nullptr;
+        idx->hits_bytes = 0;
+        const size_t want = bytes + bytes / 4;
+        if (cudaMalloc(&idx->hits, want) != cudaSuccess) {
+            cudaGetLastError();
+            idx->hits = nullptr;
+            gts_set_error("cudaMalloc of %zu bytes for the hits failed", want);
+            return GTS_ERR_NOMEM;
+        }
+        idx->hits_bytes = want;
+    }
+    *out = idx->hits;
+    return GTS_OK;
+}
+
 void free_tree(gts_index *idx)
 {
     if (idx->fast_recs) cudaFree(idx->fast_recs);
@@ -271,13 +340,15 @@ void free_tree(gts_index *idx)
     idx->mlp_ready = false;   // its feature pivots belong to the old tree
     void *ps[] = {idx->trows, idx->tstrs, idx->tlens, idx->tsig, idx->id_list, idx->pos_of_id, idx->node_pid,
                   idx->node_size, idx->node_lid, idx->node_pivot, idx->node_min_dis,
-                  idx->node_flags};
+                  idx->node_flags, idx->cut_node, idx->cut_anc, idx->cut_anc_idx, idx->tnorm};
     for (void *p : ps)
         if (p) cudaFree(p);
     idx->trows = nullptr; idx->tstrs = nullptr; idx->tlens = nullptr; idx->tsig = nullptr;
     idx->id_list = nullptr; idx->pos_of_id = nullptr; idx->node_pid = nullptr;
     idx->node_size = nullptr; idx->node_lid = nullptr; idx->node_pivot = nullptr;
     idx->node_min_dis = nullptr; idx->node_flags = nullptr;
+    idx->cut_node = nullptr; idx->cut_anc = nullptr; idx->cut_anc_idx = nullptr; idx->tnorm = nullptr;
+    idx->ncut = idx->ncut_anc = 0;
 }
 
 void free_data(gts_index *idx)
@@ -329,6 +400,10 @@ static int build_tree_impl(gts_index *idx, cudaStream_t s)
     ALLOC(idx->node_pivot, mnn);
     ALLOC(idx->node_min_dis, mnn);
     ALLOC(idx->node_flags, mnn);
+    ALLOC(idx->cut_node, mnn);
+    ALLOC(idx->cut_anc, mnn);
+    ALLOC(idx->cut_anc_idx, mnn);
+    if (idx->metric == kAngle) ALLOC(idx->tnorm, n);
     if (idx->metric == kEdit) {
         ALLOC(idx->tstrs, (size_t)n * kStrStride);
         ALLOC(idx->tlens, n);
@@ -346,7 +421,7 @@ static int build_tree_impl(gts_index *idx, cudaStream_t s)
     ALLOC(sc.split, mnn);
     ALLOC(sc.posv, n);
     ALLOC(sc.posv_alt, n);
-    ALLOC(sc.nsplit, 1);
+    ALLOC(sc.nsplit, 3);   // nodes still to split; cut nodes, their ancestors
 #undef ALLOC
     int lid_bits = 1;
     while (lid_bits < 31 && (1 << lid_bits) < n) lid_bits++;
@@ -409,8 +484,16 @@ static int build_tree_impl(gts_index *idx, cudaStream_t s)
                                                   idx->trows, idx->strs, idx->tstrs, idx->lens,
                                                   idx->tlens, idx->pos_of_id);
     if (idx->metric == kEdit) k_str_sig<<<grid_for((size_t)n, 256), 256, 0, s>>>(n, idx->tstrs, idx->tlens, idx->tsig);
+    if (idx->metric == kAngle) k_row_norms<<<grid_for((size_t)n, 256), 256, 0, s>>>(n, idx->dim, idx->trows, idx->tnorm);
+    GTS_CUDA_TRY(cudaMemsetAsync(sc.nsplit + 1, 0, 2 * sizeof(int), s));
+    k_cut_lists<<<(mnn + 255) / 256, 256, 0, s>>>(mnn, O, idx->node_flags, idx->node_size, idx->node_pivot, idx->cut_node,
+                                                  idx->cut_anc, idx->cut_anc_idx, sc.nsplit + 1);
+    int ncuts[2] = {0, 0};
+    GTS_CUDA_TRY(cudaMemcpyAsync(ncuts, sc.nsplit + 1, sizeof(ncuts), cudaMemcpyDeviceToHost, s));
     GTS_CUDA_TRY(cudaStreamSynchronize(s));
     GTS_CUDA_TRY(cudaGetLastError());
+    idx->ncut = ncuts[0];
+    idx->ncut_anc = ncuts[1];
     return GTS_OK;
 }
 

@@ -19,6 +19,13 @@ struct gts_index {
     int *node_pid = nullptr, *node_size = nullptr, *node_lid = nullptr, *node_pivot = nullptr;
     float *node_min_dis = nullptr;
     uint8_t *node_flags = nullptr;
+    // the batched sweep's view of the tree (sweep.cu): its cut nodes (the
+    // topmost nodes of at most kCutSize objects, and larger childless ones),
+    // their ancestors with a node -> ancestor map, and for the angle metric
+    // the norms of the rows in tree order
+    int *cut_node = nullptr, *cut_anc = nullptr, *cut_anc_idx = nullptr;
+    int ncut = 0, ncut_anc = 0;
+    float *tnorm = nullptr;
 
     // per-call scratch owned by the handle
     int *d_counter = nullptr;   // persistent-kernel work counter
@@ -46,6 +53,10 @@ struct gts_index {
     // autotuned threads per query CTA of the plain traversal per search mode
     // (kNN, range count, range ids; search.cu), 0 = not tuned
     int plain_nt[3] = {};
+    // set by a caller: pinned threads or a hand-over threshold choose the
+    // traversal over the batched sweep
+    bool plain_pinned[3] = {};
+    bool plain_split_set = false;
     // range counts: objects a query verifies in one CTA before it hands its
     // older stack entries over as (query, node) items (0: never); the item
     // lists, and the items handed over since the last reset
@@ -61,6 +72,9 @@ struct gts_index {
     // grown on demand and kept, so those calls allocate nothing in steady state
     void *io = nullptr;
     size_t io_bytes = 0;
+    // hits of a range-ids run on their way to the host
+    void *hits = nullptr;
+    size_t hits_bytes = 0;
     // CUDA graph of the fast form's filter pass (fast.cu), launched on the
     // handle's own stream and replayed while the batch shape stays the same
     cudaStream_t graph_stream = nullptr;
@@ -99,6 +113,7 @@ namespace gts {
 //   [5] fast: candidates appended         [6] fast: filter passes
 //   [7] fast: (query tile, block) pairs tested by the block bound
 constexpr int kStatsN = 8;
+constexpr int kCutSize = 128;   // objects of a cut node at most, unless it has no children
 
 // Build the tree for the data already placed in idx->rows / strs / lens.
 int build_tree(gts_index *idx, cudaStream_t s);
@@ -126,6 +141,12 @@ int search_range_rows(gts_index *idx, const float *d_qrows, const char *d_qstrs,
                       float r, int *d_counts, cudaStream_t s);
 int search_range_ids(gts_index *idx, const int *d_qids, int qnum, float r, int *d_counts,
                      int *d_ids, float *d_dists, const int *d_offsets, cudaStream_t s);
+// Range counts and hits in one pass over the data (host outputs; hits only
+// up to `capacity`), ordered by (distance, id) per query.  *done = 0: not a
+// batch the sweep answers in full; *total: hits of all queries.
+int sweep_range_ids(gts_index *idx, const int *d_qids, int qnum, float r, int *d_counts, int *counts_out,
+                    int *offsets_out, int *ids_out, float *dists_out, size_t capacity, size_t *total, int *done,
+                    cudaStream_t s);
 
 template <typename T>
 int dev_alloc(T **p, size_t n, size_t *acct);
@@ -143,6 +164,8 @@ inline size_t search_budget(const gts_index *idx)
 int ensure_scratch(gts_index *idx, size_t bytes);
 // Grow idx->io to at least `bytes`.
 int ensure_io(gts_index *idx, size_t bytes);
+// idx->hits of at least `bytes`.
+int ensure_hits(gts_index *idx, size_t bytes, void **out);
 
 bool fast_supported(const gts_index *idx, int k);
 int mlp_seed(gts_index *idx, const int *d_qids, int qnum, int k, int *d_r2_bits, cudaStream_t st);

@@ -31,6 +31,22 @@ constexpr int kStrStride = 109;   // reference string row stride (file.cuh:15)
 // exact, reference operation order (one thread, sequential over the row)
 // ---------------------------------------------------------------------------
 
+// The angle in degrees from its cosine as the call sites evaluate it:
+// the F64 sites keep the float quotient in a double, the F32 sites in a float.
+__device__ __forceinline__ double angle_of_cos_f64(float c)
+{
+    double r = c;
+    if (r > 1) r = 0.99999999999999999;
+    return abs(acos(r) * 180 / 3.1415926);
+}
+__device__ __forceinline__ float angle_of_cos_f32(float c)
+{
+    float r = c;
+    if (r > 1) r = 0.99999999999999999;
+    r = abs(acos(r) * 180 / 3.1415926);
+    return r;
+}
+
 // Sequential F64-accumulated distance.  `pow(float_diff, 2)` in the
 // reference resolves to a double-returning overload that is not always the
 // exact square (measured on the device: ~6% of inputs differ in the last
@@ -62,9 +78,7 @@ __device__ __forceinline__ double dist_row_f64(const float *__restrict__ a,
         }
         sa1 = pow(sa1, 0.5);
         sa2 = pow(sa2, 0.5);
-        r = sa3 / (sa1 * sa2);
-        if (r > 1) r = 0.99999999999999999;
-        return abs(acos(r) * 180 / 3.1415926);
+        return angle_of_cos_f64(sa3 / (sa1 * sa2));
     }
 }
 
@@ -97,10 +111,7 @@ __device__ __forceinline__ float dist_row_f32(const float *__restrict__ a,
         }
         sa1 = pow(sa1, 0.5);
         sa2 = pow(sa2, 0.5);
-        r = sa3 / (sa1 * sa2);
-        if (r > 1) r = 0.99999999999999999;
-        r = abs(acos(r) * 180 / 3.1415926);
-        return r;
+        return angle_of_cos_f32(sa3 / (sa1 * sa2));
     }
 }
 

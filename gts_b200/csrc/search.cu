@@ -34,7 +34,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <cstdio>
-#include "index.cuh"
+#include "search.cuh"
 
 namespace gts {
 
@@ -44,69 +44,9 @@ constexpr int kBatch = 32;            // stack entries popped per step (one warp
 constexpr int kRows = 8;              // leaf rows per warp in flight
 constexpr int kStackCap = 2048;
 constexpr int kLeafObjCap = 1024;     // objects verified per step
-constexpr int kMaxK = 256;
 constexpr int kCandCap = kLeafObjCap + kMaxK;
 constexpr int kSortCap = 2048;        // next power of two >= kCandCap
 constexpr int kMaxDimSmem = 1024;
-constexpr int kLaneRowDim = 8;        // up to this dimension a lane filters a whole row
-
-enum SearchMode { kModeKnn = 0, kModeRangeCount = 1, kModeRangeIds = 2, kModeRangeTimed = 3 };
-
-struct SearchArgs {
-    DevTree t;
-    const int *qids;
-    int qnum;
-    int mode;
-    int k;
-    float r;
-    float *kth;
-    int *ids;
-    float *dists;
-    int *counts;
-    const int *offsets;
-    int *rids;
-    float *rdists;
-    const uint32_t *deleted;
-    int *counter;
-    int *status;
-    // kNN seeded by the learned radius (nullable): squared radius per query
-    // (float bits); a query with fewer than k objects inside is listed in
-    // fail / n_fail instead of answered
-    const int *seed_r2_bits;
-    int *fail, *n_fail;
-    unsigned long long *stats;   // [objects filtered, pivots evaluated, exact values, queries]
-    // kModeRangeTimed: the query's operation index; per object id its
-    // entries ents[ent_off[id] .. ent_off[id + 1]) as (tree_from, tree_to,
-    // cache_from, cache_to), live in the tree at t when tree_from < t <
-    // tree_to and in the cache list when cache_from < t < cache_to; counts
-    // receives the tree part, counts2 the cache part
-    const int *qtime;
-    const int *ent_off;
-    const int4 *ents;
-    int *counts2;
-    // queries given as data instead of ids (nullable): rows [qnum][dim], or
-    // strings [qnum][109] with lengths; such a query is no object of the
-    // index (no self match)
-    const float *qrows;
-    const char *qstrs;
-    const int *qlens;
-    // (query, node) work items, range counts only (count and timed modes):
-    // items_in (nullable) are (query, node, first unverified object, lower
-    // bound bits) handed over by an earlier launch; n_items_in of them are
-    // the work units instead of the queries.  A query that has verified more
-    // than split_objs objects in one CTA since its last hand-over gives all
-    // but its kBatch newest stack entries to items_out (capacity items_cap,
-    // count in *n_items_out; entries with query -1 are unused), so the next
-    // launch spreads its subtrees over every CTA.  With splitting on, counts
-    // are added atomically (the caller zeroes them first).
-    const int4 *items_in;
-    int4 *items_out;
-    int *n_items_out;
-    int items_cap;
-    int split_objs;   // 0: no hand-over
-    float rel_eps;   // relative pruning slack
-    float abs_eps;   // absolute pruning slack
-};
 
 struct __align__(16) SearchSmem {
     float qrow[kMaxDimSmem];
@@ -188,105 +128,6 @@ __device__ __forceinline__ double exact_id(const SearchArgs &a, const SearchSmem
                           : (double)dist_row_f32(row, q, t.dim, t.metric);
 }
 
-// Warp-cooperative FP32 partial value of a row against the query:
-// L2 -> sum of squares, L1 -> sum of |diff|, Linf -> max |diff| (exact).
-__device__ __forceinline__ float warp_row_value(const float *__restrict__ row,
-                                                const float *__restrict__ q, int dim, int metric,
-                                                int lane)
-{
-    float acc = 0.f;
-    if ((dim & 3) == 0) {
-        const float4 *r4 = reinterpret_cast<const float4 *>(row);
-        const float4 *q4 = reinterpret_cast<const float4 *>(q);
-        for (int j = lane; j < (dim >> 2); j += 32) {
-            float4 x = __ldg(r4 + j), y = q4[j];
-            float d0 = x.x - y.x, d1 = x.y - y.y, d2 = x.z - y.z, d3 = x.w - y.w;
-            if (metric == kL2) {
-                acc = fmaf(d0, d0, acc); acc = fmaf(d1, d1, acc);
-                acc = fmaf(d2, d2, acc); acc = fmaf(d3, d3, acc);
-            } else if (metric == kL1) {
-                acc += fabsf(d0) + fabsf(d1) + fabsf(d2) + fabsf(d3);
-            } else {
-                acc = fmaxf(acc, fmaxf(fmaxf(fabsf(d0), fabsf(d1)), fmaxf(fabsf(d2), fabsf(d3))));
-            }
-        }
-    } else {
-        for (int j = lane; j < dim; j += 32) {
-            float d0 = __ldg(row + j) - q[j];
-            if (metric == kL2) acc = fmaf(d0, d0, acc);
-            else if (metric == kL1) acc += fabsf(d0);
-            else acc = fmaxf(acc, fabsf(d0));
-        }
-    }
-    return metric == kLinf ? warp_max(acc) : warp_sum(acc);
-}
-
-// R rows at once (independent loads in flight): out[u] as warp_row_value.
-template <int R>
-__device__ __forceinline__ void warp_row_values(const float *const (&rows)[R], const float *__restrict__ q,
-                                                int dim, int metric, int lane, float (&out)[R])
-{
-    float acc[R];
-#pragma unroll
-    for (int u = 0; u < R; u++) acc[u] = 0.f;
-    if ((dim & 3) == 0) {
-        const float4 *q4 = reinterpret_cast<const float4 *>(q);
-        for (int j = lane; j < (dim >> 2); j += 32) {
-            float4 x[R];
-#pragma unroll
-            for (int u = 0; u < R; u++) x[u] = __ldg(reinterpret_cast<const float4 *>(rows[u]) + j);
-            const float4 y = q4[j];
-#pragma unroll
-            for (int u = 0; u < R; u++) {
-                float d0 = x[u].x - y.x, d1 = x[u].y - y.y, d2 = x[u].z - y.z, d3 = x[u].w - y.w;
-                if (metric == kL2) {
-                    acc[u] = fmaf(d0, d0, acc[u]); acc[u] = fmaf(d1, d1, acc[u]);
-                    acc[u] = fmaf(d2, d2, acc[u]); acc[u] = fmaf(d3, d3, acc[u]);
-                } else if (metric == kL1) {
-                    acc[u] += fabsf(d0) + fabsf(d1) + fabsf(d2) + fabsf(d3);
-                } else {
-                    acc[u] = fmaxf(acc[u], fmaxf(fmaxf(fabsf(d0), fabsf(d1)), fmaxf(fabsf(d2), fabsf(d3))));
-                }
-            }
-        }
-    } else {
-        for (int j = lane; j < dim; j += 32) {
-            float x[R];
-#pragma unroll
-            for (int u = 0; u < R; u++) x[u] = __ldg(rows[u] + j);
-            const float y = q[j];
-#pragma unroll
-            for (int u = 0; u < R; u++) {
-                float d0 = x[u] - y;
-                if (metric == kL2) acc[u] = fmaf(d0, d0, acc[u]);
-                else if (metric == kL1) acc[u] += fabsf(d0);
-                else acc[u] = fmaxf(acc[u], fabsf(d0));
-            }
-        }
-    }
-#pragma unroll
-    for (int u = 0; u < R; u++) out[u] = metric == kLinf ? warp_max(acc[u]) : warp_sum(acc[u]);
-}
-
-// Interval [lo, hi] that contains both exact leaf values (F32 and F64
-// sites) given the FP32 warp value v.
-__device__ __forceinline__ void value_bounds(int metric, int dim, float v, double &lo, double &hi)
-{
-    if (metric == kLinf) {   // max of exactly rounded |diff|: exact
-        lo = hi = (double)v;
-        return;
-    }
-    double g = 2.0 * (double)f32_sum_rel_bound(dim + 32) + 4.0 * 5.9604645e-8;
-    double vl = (double)v * (1.0 - g), vh = (double)v * (1.0 + g);
-    if (metric == kL2) {
-        lo = sqrt(vl > 0 ? vl : 0.0) * (1.0 - 1e-7);
-        hi = sqrt(vh) * (1.0 + 1e-7);
-    } else {
-        lo = vl;
-        hi = vh;
-    }
-}
-
 // Index of the leaf holding step object o: the last li < nleaf with
 // leaf_pre[li] <= o (leaf_pre ascending, at most kBatch + 1 entries).
 __device__ __forceinline__ int leaf_of(const int *leaf_pre, int nleaf, int o)
@@ -298,25 +139,6 @@ __device__ __forceinline__ int leaf_of(const int *leaf_pre, int nleaf, int o)
         else hi = mid - 1;
     }
     return lo;
-}
-
-// value_bounds in FP32: the products and square roots add at most a few
-// ulps, covered by the extra 4e-7 / 2e-7 relative margins.
-__device__ __forceinline__ void value_bounds_f(int metric, int dim, float v, float &lo, float &hi)
-{
-    if (metric == kLinf) {   // max of exactly rounded |diff|: exact
-        lo = hi = v;
-        return;
-    }
-    const float g = 2.f * f32_sum_rel_bound(dim + 32) + 4.f * 5.9604645e-8f;
-    const float vl = v * (1.f - g), vh = v * (1.f + g);
-    if (metric == kL2) {
-        lo = sqrtf(fmaxf(vl, 0.f)) * (1.f - 4e-7f);
-        hi = sqrtf(vh) * (1.f + 4e-7f);
-    } else {
-        lo = vl * (1.f - 2e-7f);
-        hi = vh * (1.f + 2e-7f);
-    }
 }
 
 // Bitonic sort of the candidate buffer by (distance, id), n entries padded
@@ -791,6 +613,12 @@ static int launch_search(gts_index *idx, const SearchArgs &a, int nt, cudaStream
     }
 }
 
+// Queries of a thread-count timing: four times the most CTAs resident at once.
+static int plain_tune_sample()
+{
+    return 4 * std::max(search_resident<128>(), std::max(search_resident<256>(), search_resident<512>()));
+}
+
 // Times 128 / 256 / 512 threads per query CTA on the batch's leading queries
 // (results identical; the full batch then runs with the fastest).  The
 // sample is four times the most CTAs any candidate keeps resident, so the
@@ -807,7 +635,7 @@ static int plain_autotune(gts_index *idx, const SearchArgs &a, cudaStream_t st, 
         *best_nt = idx->plain_nt[kModeRangeCount];
         return GTS_OK;
     }
-    const int sample = 4 * std::max(search_resident<128>(), std::max(search_resident<256>(), search_resident<512>()));
+    const int sample = plain_tune_sample();
     if (a.qnum < 2 * sample) return GTS_OK;
     SearchArgs t = a;
     t.seed_r2_bits = nullptr;
@@ -861,6 +689,7 @@ extern "C" int gts_plain_threads_set(gts_index *idx, int mode, int threads)
         return GTS_ERR_INVALID;
     }
     idx->plain_nt[mode] = threads;
+    idx->plain_pinned[mode] = threads != 0;
     return GTS_OK;
 }
 
@@ -917,9 +746,8 @@ static int run_split_phases(gts_index *idx, const SearchArgs &a0, int nt, cudaSt
     return GTS_OK;
 }
 
-static int run_search(gts_index *idx, SearchArgs &a, cudaStream_t st)
+void fill_search_args(gts_index *idx, SearchArgs &a)
 {
-    if (a.qnum <= 0) return GTS_OK;
     a.t = idx->dev();
     a.counter = idx->d_counter;
     a.stats = idx->d_stats;
@@ -938,20 +766,42 @@ static int run_search(gts_index *idx, SearchArgs &a, cudaStream_t st)
         double quantum = 4.0 * 2.220446e-16 * (kmax * idx->params.dis_code + 2.0) * idx->params.infi_dis;
         a.abs_eps = (float)(quantum + 1e-6);
     }
+}
+
+static int run_search(gts_index *idx, SearchArgs &a, cudaStream_t st)
+{
+    if (a.qnum <= 0) return GTS_OK;
+    fill_search_args(idx, a);
     GTS_CUDA_TRY(cudaMemsetAsync(idx->d_counter, 0, sizeof(int), st));
     GTS_CUDA_TRY(cudaMemsetAsync(idx->d_status, 0, sizeof(int), st));
     if (!idx->keep_stats) GTS_CUDA_TRY(cudaMemsetAsync(idx->d_stats, 0, kStatsN * sizeof(unsigned long long), st));
     // threads per query CTA: tuned per search mode on the first batch large
     // enough for plain_autotune's sample, else the tuned or default value
     const int slot = a.mode == kModeRangeTimed ? kModeRangeCount : a.mode;
+    // the batched sweep first (not nested in another search, which holds the
+    // scratch); the traversal answers the queries it leaves
+    int swept = 0;
+    if (!idx->keep_stats && a.mode != kModeRangeIds) {
+        const int4 *items = nullptr;
+        int n_left = 0;
+        int rc = run_sweep(idx, a, st, &swept, &items, &n_left);
+        if (rc) return rc;
+        if (swept) {
+            // where the sweep answers the large batches the traversal keeps its default
+            if (!idx->plain_nt[slot] && a.qnum >= 2 * plain_tune_sample()) idx->plain_nt[slot] = kPlainDefaultThreads;
+            if (n_left == 0) return GTS_OK;
+            a.items_in = items;
+            a.qnum = n_left;
+        }
+    }
     int nt = idx->plain_nt[slot];
-    if (!nt && !idx->keep_stats) {
+    if (!nt && !idx->keep_stats && !swept) {
         int rc = plain_autotune(idx, a, st, &nt);
         if (rc) return rc;
         if (a.mode != kModeRangeIds) idx->plain_nt[slot] = nt;
     }
     if (!nt) nt = kPlainDefaultThreads;
-    const bool split = (a.mode == kModeRangeCount || a.mode == kModeRangeTimed) && idx->plain_split > 0;
+    const bool split = (a.mode == kModeRangeCount || a.mode == kModeRangeTimed) && idx->plain_split > 0 && !swept;
     int rc = split ? run_split_phases(idx, a, nt, st) : launch_search(idx, a, nt, st);
     if (rc) return rc;
     int status = 0;
