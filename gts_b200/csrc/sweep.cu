@@ -46,6 +46,8 @@ constexpr int kSwList = 2048;          // pairs a tile may finish one by one
 constexpr int kSwWindow = 1024;        // objects around a query's place that bound its k-th distance
 constexpr int kSwMaxTiles = 32;        // query tiles per run
 constexpr int kSwCap = 2048;           // candidates listed per query
+constexpr int kSwSample = 16;          // the sample pass looks at every 16th row
+constexpr int kSwSampleMin = 1 << 16;  // objects from which on it pays
 constexpr int kSwRounds = 3;           // further passes over kNN queries whose lists overflowed
 constexpr int kSwHitCap = 16384;       // hits per query of a range-ids call at most
 constexpr float kSwTiny = 1e-36f;      // squares below this may have lost bits to underflow
@@ -73,6 +75,7 @@ struct SweepArgs {
     const int4 *again;                  // kNN, a later round: the run's queries and bounds come from
     const float *again_R;               //   again[q0 ..], again_R[q0 ..]
     int cap;                            // candidates listed per query
+    int sample;                         // look at every sample-th row only (1: all)
 };
 
 __device__ __forceinline__ void sw_cp16(void *dst, const void *src, int bytes)
@@ -299,6 +302,38 @@ __global__ void k_sw_iota(int n, int *v)
     if (i < n) v[i] = i;
 }
 
+// Thresholds on the filter value for radius R: above vthr (angle: below) no
+// bound admits the object, below vlow a range hit is certain.
+__device__ __forceinline__ void sw_thresholds(const DevTree &t, float R, bool ok, float &vthr, float &vlow)
+{
+    vlow = -1.f;
+    if (t.metric == kAngle) {
+        vthr = 3.f;   // nothing passes
+        if (ok) {
+            const double deg = (double)R * (1.0 + 1e-5) + 1e-3;
+            vthr = deg >= 180.0 ? -2.f : (float)(cos(deg * (3.14159265358979 / 180.0)) - 1e-6);
+        }
+        return;
+    }
+    vthr = -1.f;
+    if (!ok) return;
+    const double g = 2.0 * (double)f32_sum_rel_bound(t.dim + 32) + 4.0 * 5.9604645e-8;
+    double hi, lo;
+    if (t.metric == kL2) {
+        hi = (double)R * R * (1.0 + 4e-6) / (1.0 - g) + 4.0 * kSwTiny;
+        lo = (double)R * R * (1.0 - 4e-6) / (1.0 + g);
+        if (lo < 1e-30) lo = -1.0;
+    } else if (t.metric == kL1) {
+        hi = (double)R * (1.0 + 2e-6) / (1.0 - g);
+        lo = (double)R * (1.0 - 2e-6) / (1.0 + g);
+    } else {
+        hi = (double)R * (1.0 + 2e-6);
+        lo = (double)R * (1.0 - 2e-6);
+    }
+    vthr = hi < FLT_MAX ? __double2float_ru(hi) : FLT_MAX;
+    vlow = __double2float_rd(lo);
+}
+
 // One warp per sorted query slot: its row (zero padded), radius, thresholds
 // on the filter value, and an empty candidate list (the query object itself
 // first: its distance is 0 by definition, search_v2.cuh:338-340).
@@ -317,34 +352,14 @@ __global__ void __launch_bounds__(256) k_sw_query(SweepArgs s)
     if (lane == 0) {
         float R = -1.f;
         if (ok) R = s.a.mode != kModeKnn ? s.a.r : (s.again ? s.again_R[s.q0 + i] : s.seed[q - s.q0]);
-        float vthr = -1.f, vlow = -1.f, qn = 0.f;
-        if (t.metric == kAngle) {
-            vthr = 3.f;   // nothing passes
-            if (ok) {
-                float sa = 0.f;
-                for (int j = 0; j < t.dim; j++) sa = fmaf(src[j], src[j], sa);
-                sa = pow(sa, 0.5);
-                qn = sa;
-                const double deg = (double)R * (1.0 + 1e-5) + 1e-3;
-                vthr = deg >= 180.0 ? -2.f : (float)(cos(deg * (3.14159265358979 / 180.0)) - 1e-6);
-            }
-        } else if (ok) {
-            const double g = 2.0 * (double)f32_sum_rel_bound(t.dim + 32) + 4.0 * 5.9604645e-8;
-            double hi, lo;
-            if (t.metric == kL2) {
-                hi = (double)R * R * (1.0 + 4e-6) / (1.0 - g) + 4.0 * kSwTiny;
-                lo = (double)R * R * (1.0 - 4e-6) / (1.0 + g);
-                if (lo < 1e-30) lo = -1.0;
-            } else if (t.metric == kL1) {
-                hi = (double)R * (1.0 + 2e-6) / (1.0 - g);
-                lo = (double)R * (1.0 - 2e-6) / (1.0 + g);
-            } else {
-                hi = (double)R * (1.0 + 2e-6);
-                lo = (double)R * (1.0 - 2e-6);
-            }
-            vthr = hi < FLT_MAX ? __double2float_ru(hi) : FLT_MAX;
-            vlow = __double2float_rd(lo);
+        float vthr, vlow, qn = 0.f;
+        if (ok && t.metric == kAngle) {
+            float sa = 0.f;
+            for (int j = 0; j < t.dim; j++) sa = fmaf(src[j], src[j], sa);
+            sa = pow(sa, 0.5);
+            qn = sa;
         }
+        sw_thresholds(t, R, ok, vthr, vlow);
         s.R[i] = R;
         s.vthr[i] = vthr;
         s.vlow[i] = vlow;
@@ -437,6 +452,11 @@ __global__ void __launch_bounds__(256) k_sw_cut(SweepArgs s)
         }
         if (!(m[0] | m[1] | m[2] | m[3])) size = 0;
     }
+    if (s.sample > 1) {   // every sample-th position only
+        const int first = (lid + s.sample - 1) / s.sample * s.sample;
+        size = first < lid + size ? (lid + size - 1 - first) / s.sample + 1 : 0;
+        lid = first;
+    }
     int incl = size;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -461,7 +481,7 @@ __global__ void __launch_bounds__(256) k_sw_cut(SweepArgs s)
         const int from = __ffs(todo) - 1;
         const int n = __shfl_sync(0xffffffffu, size, from), l = __shfl_sync(0xffffffffu, lid, from);
         const int o = __shfl_sync(0xffffffffu, off, from);
-        for (int j = lane; j < n; j += 32) dst[o + j] = l + j;
+        for (int j = lane; j < n; j += 32) dst[o + j] = l + j * s.sample;
     }
 }
 
@@ -476,7 +496,7 @@ struct SweepSmem {
     int self[16 * QI];
     int cnt[16 * QI], cnt2[16 * QI];
     unsigned short list[kSwList];
-    int item[2], nalive[2], nlist;
+    int item[2], nlist[2];
 };
 
 // 16 QI query rows from qrow and 128 rows at rp, dimensions k0 .. k0 + 15,
@@ -667,8 +687,7 @@ __global__ void __launch_bounds__(kSwThreads, QI == 8 ? 2 : 3) k_sw_tile(SweepAr
             sm.self[tid] = s.self[q0 + tid];
         }
         if (tid == 0) {
-            sm.nalive[0] = sm.nalive[1] = 0;
-            sm.nlist = 0;
+            sm.nlist[0] = sm.nlist[1] = 0;
             pairs += (unsigned long long)nr * max(0, min(16 * QI, s.nq - q0));
         }
         __syncthreads();
@@ -680,6 +699,7 @@ __global__ void __launch_bounds__(kSwThreads, QI == 8 ? 2 : 3) k_sw_tile(SweepAr
             for (int c = 0; c < 8; c++) acc[i][c] = 0.f;
         sw_stage<QI>(sm, 0, qrow, s.ld, t.dim, 0);
         bool whole = true;   // the tile ran through all dimensions
+        int n = 0;           // else: pairs listed to be finished one by one
         for (int ch = 0; ch < nc; ch++) {
             // only the angle metric is sure to need the next stage
             if (M == kAngle && ch + 1 < nc) {
@@ -696,31 +716,31 @@ __global__ void __launch_bounds__(kSwThreads, QI == 8 ? 2 : 3) k_sw_tile(SweepAr
                 __syncthreads();
                 continue;
             }
-            int alive = 0;
+            // list the pairs still within their bounds; too many of them to
+            // finish one by one: drop the list and take the next stage
+            const int most = (int)min((long)kSwList, (long)(nc - 1 - ch) * stage_cost / alone);
+            int *nlist = &sm.nlist[ch & 1];
 #pragma unroll
             for (int i = 0; i < QI; i++) {
                 const float th = sm.vthr[tq + 16 * i];
+                float mn = acc[i][0];
 #pragma unroll
-                for (int c = 0; c < 8; c++) alive += acc[i][c] <= th && to + 16 * c < nr;
-            }
-            alive = __reduce_add_sync(0xffffffffu, alive);
-            if (lane == 0 && alive) atomicAdd(&sm.nalive[ch & 1], alive);
-            __syncthreads();
-            const int total = sm.nalive[ch & 1];
-            if (tid == 0) sm.nalive[(ch + 1) & 1] = 0;
-            if (total <= kSwList && (long)total * alone <= (long)(nc - 1 - ch) * stage_cost) {
-                whole = false;
-                asm volatile("cp.async.wait_group 0;" ::: "memory");
-                if (total == 0) break;
-#pragma unroll
-                for (int i = 0; i < QI; i++) {
-                    const float th = sm.vthr[tq + 16 * i];
+                for (int c = 1; c < 8; c++) mn = fminf(mn, acc[i][c]);
+                if (mn <= th && *(volatile int *)nlist <= most) {
 #pragma unroll
                     for (int c = 0; c < 8; c++)
-                        if (acc[i][c] <= th && to + 16 * c < nr)
-                            sm.list[atomicAdd(&sm.nlist, 1)] = (unsigned short)((tq + 16 * i) << 7 | (to + 16 * c));
+                        if (acc[i][c] <= th && to + 16 * c < nr) {
+                            const int at = atomicAdd(nlist, 1);
+                            if (at < kSwList) sm.list[at] = (unsigned short)((tq + 16 * i) << 7 | (to + 16 * c));
+                        }
                 }
-                __syncthreads();
+            }
+            __syncthreads();
+            n = *nlist;
+            if (tid == 0) sm.nlist[(ch + 1) & 1] = 0;
+            if (n <= most) {
+                whole = false;
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
                 break;
             }
             if (ch == 0 && nc > 1) sw_stage<QI>(sm, 1, qrow, s.ld, t.dim, kSwK);
@@ -746,7 +766,6 @@ __global__ void __launch_bounds__(kSwThreads, QI == 8 ? 2 : 3) k_sw_tile(SweepAr
             }
         } else {
             // the remaining pairs one by one: four in flight per warp
-            const int n = sm.nlist;
             constexpr int kP = 4;
             for (int p0 = warp * kP; p0 < n; p0 += (kSwThreads / 32) * kP) {
                 float v[kP];
@@ -1099,6 +1118,35 @@ inline int pow2_at_least(int n)
     return p;
 }
 
+// After a pass over a sample of the rows: the k-th smallest upper bound of the
+// listed candidates where that is tighter than the query's bound; empty lists
+// (the query object stays).
+__global__ void __launch_bounds__(128) k_sw_tighten(SweepArgs s)
+{
+    __shared__ uint32_t key[kSwCap];
+    __shared__ int hist[256];
+    const DevTree &t = s.a.t;
+    const int i = blockIdx.x, k = s.a.k, self = s.self[i];
+    const int m = min(s.ccnt[i], s.cap);
+    __syncthreads();
+    if (threadIdx.x == 0) s.ccnt[i] = self >= 0 ? 1 : 0;
+    if (m < k) return;
+    for (int c = threadIdx.x; c < m; c += 128) {
+        const int p = s.cpos[(size_t)i * s.cap + c];
+        const float v = s.cv[(size_t)i * s.cap + c];
+        const float hi = p == self ? 0.f : t.metric == kAngle ? (float)angle_of_cos_f64(v) * 1.00001f : sw_hi(t.metric, t.dim, v);
+        key[c] = __float_as_uint(hi < FLT_MAX ? hi : FLT_MAX);
+    }
+    __syncthreads();
+    const float R = __uint_as_float(cta_kth(key, m, k, hist));
+    if (threadIdx.x == 0 && R < s.R[i]) {
+        float vthr, vlow;
+        sw_thresholds(t, R, true, vthr, vlow);
+        s.R[i] = R;
+        s.vthr[i] = vthr;
+    }
+}
+
 // Buffers of a run of at most `tiles` query tiles; returns its bytes.
 size_t plan_sweep(const gts_index *idx, int tiles, int qnum, unsigned char *base, SweepArgs *s, void **cub, size_t *cub_bytes)
 {
@@ -1113,6 +1161,7 @@ size_t plan_sweep(const gts_index *idx, int tiles, int qnum, unsigned char *base
     r.left = (int4 *)take(sizeof(int4) * 2 * (size_t)qnum);   // two lists: this round's and the last one's
     r.left_R = (float *)take(4 * 2 * (size_t)qnum);
     r.cap = kSwCap;
+    r.sample = 1;
     r.ctr = (int *)take(64);
     r.nrows = (int *)take(4 * (size_t)tiles);
     r.key = (int *)take(4 * (size_t)Qp * 5);   // key, sorted key, identity, order, batch query
@@ -1140,7 +1189,7 @@ size_t plan_sweep(const gts_index *idx, int tiles, int qnum, unsigned char *base
 }
 
 template <int M, int QI>
-int launch_tiles(gts_index *idx, SweepArgs s, cudaStream_t st)
+int launch_tiles(gts_index *idx, SweepArgs s, bool sampled, cudaStream_t st)
 {
     const int smem = (int)sizeof(SweepSmem<QI>);
     int per_sm = 1, dev = 0, nsm = 148;
@@ -1152,21 +1201,32 @@ int launch_tiles(gts_index *idx, SweepArgs s, cudaStream_t st)
     const int tiles128 = s.ntiles;
     s.ntiles = (s.nq + 16 * QI - 1) / (16 * QI);
     if (s.nanc > 0) k_sw_pivots<M, QI><<<dim3((s.nanc + kSwRows - 1) / kSwRows, s.ntiles), kSwThreads, smem, st>>>(s);
-    k_sw_cut<<<dim3((s.ncut + 255) / 256, tiles128), 256, 0, st>>>(s);
-    k_sw_tile<M, QI><<<nsm * std::max(per_sm, 1), kSwThreads, smem, st>>>(s);
-    idx->kernel_launches += 2 + (s.nanc > 0);
+    idx->kernel_launches += s.nanc > 0;
+    // kNN seeds come from one neighbourhood of the tree order and are far off
+    // for a few queries, which would then keep every row in play: a pass over
+    // 1/16 of the rows first bounds every query by the whole data
+    for (s.sample = sampled ? kSwSample : 1;; s.sample = 1) {
+        k_sw_cut<<<dim3((s.ncut + 255) / 256, tiles128), 256, 0, st>>>(s);
+        k_sw_tile<M, QI><<<nsm * std::max(per_sm, 1), kSwThreads, smem, st>>>(s);
+        idx->kernel_launches += 2;
+        if (s.sample == 1) break;
+        k_sw_tighten<<<s.nq, 128, 0, st>>>(s);
+        idx->kernel_launches++;
+        GTS_CUDA_TRY(cudaMemsetAsync(s.ctr, 0, sizeof(int), st));
+        GTS_CUDA_TRY(cudaMemsetAsync(s.nrows, 0, sizeof(int) * tiles128, st));
+    }
     GTS_CUDA_TRY(cudaGetLastError());
     return GTS_OK;
 }
 
 template <int QI>
-int launch_metric(gts_index *idx, const SweepArgs &s, cudaStream_t st)
+int launch_metric(gts_index *idx, const SweepArgs &s, bool sampled, cudaStream_t st)
 {
     switch (idx->metric) {
-    case kL2: return launch_tiles<kL2, QI>(idx, s, st);
-    case kL1: return launch_tiles<kL1, QI>(idx, s, st);
-    case kLinf: return launch_tiles<kLinf, QI>(idx, s, st);
-    default: return launch_tiles<kAngle, QI>(idx, s, st);
+    case kL2: return launch_tiles<kL2, QI>(idx, s, sampled, st);
+    case kL1: return launch_tiles<kL1, QI>(idx, s, sampled, st);
+    case kLinf: return launch_tiles<kLinf, QI>(idx, s, sampled, st);
+    default: return launch_tiles<kAngle, QI>(idx, s, sampled, st);
     }
 }
 
@@ -1247,7 +1307,8 @@ int sweep_pass(gts_index *idx, SweepArgs &s, cudaStream_t st)
     k_sw_query<<<(s.Qp + 7) / 8, 256, 0, st>>>(s);
     // 32 queries per tile when there are no more of them: the 128-wide tile
     // would multiply padding
-    int rc = s.nq <= 32 ? launch_metric<2>(idx, s, st) : launch_metric<8>(idx, s, st);
+    const bool sampled = s.a.mode == kModeKnn && !s.again && idx->num >= kSwSampleMin;
+    int rc = s.nq <= 32 ? launch_metric<2>(idx, s, sampled, st) : launch_metric<8>(idx, s, sampled, st);
     if (rc) return rc;
     idx->kernel_launches++;
     return GTS_OK;
