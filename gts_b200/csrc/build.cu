@@ -188,11 +188,26 @@ __global__ void k_clear_level(int start, int nb, uint8_t *split)
 }
 
 // Tree-order copies of the data so that a leaf's objects are contiguous.
-// Character-class signatures of the strings in tree order (edit lower bounds).
-__global__ void k_str_sig(int n, const char *tstrs, const int *tlens, uint4 *tsig)
+// Character-class signatures of the strings in tree order (edit lower bounds)
+// and their first kPackChars characters (zeros past the end) as two 16-byte words.
+__global__ void k_str_sig(int n, const char *tstrs, const int *tlens, uint4 *tsig, uint4 *tpack)
 {
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < (size_t)n; i += (size_t)gridDim.x * blockDim.x)
-        tsig[i] = str_sig(tstrs + i * kStrStride, tlens[i]);
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < (size_t)n; i += (size_t)gridDim.x * blockDim.x) {
+        const char *s = tstrs + i * kStrStride;
+        const int len = tlens[i];
+        tsig[i] = str_sig(s, len);
+        uint32_t w[kPackChars / 4];
+#pragma unroll
+        for (int k = 0; k < kPackChars / 4; k++) {
+            uint32_t v = 0;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (4 * k + j < len) v |= (uint32_t)(unsigned char)s[4 * k + j] << (8 * j);
+            w[k] = v;
+        }
+        tpack[2 * i] = make_uint4(w[0], w[1], w[2], w[3]);
+        tpack[2 * i + 1] = make_uint4(w[4], w[5], w[6], w[7]);
+    }
 }
 
 __global__ void k_permute(int n, int dim, int metric, const int *id_list, const float *rows,
@@ -338,12 +353,12 @@ void free_tree(gts_index *idx)
     for (int &c : idx->plain_nt) c = 0;
     graph_invalidate(idx);
     idx->mlp_ready = false;   // its feature pivots belong to the old tree
-    void *ps[] = {idx->trows, idx->tstrs, idx->tlens, idx->tsig, idx->id_list, idx->pos_of_id, idx->node_pid,
+    void *ps[] = {idx->trows, idx->tstrs, idx->tlens, idx->tsig, idx->tpack, idx->id_list, idx->pos_of_id, idx->node_pid,
                   idx->node_size, idx->node_lid, idx->node_pivot, idx->node_min_dis,
                   idx->node_flags, idx->cut_node, idx->cut_anc, idx->cut_anc_idx, idx->tnorm};
     for (void *p : ps)
         if (p) cudaFree(p);
-    idx->trows = nullptr; idx->tstrs = nullptr; idx->tlens = nullptr; idx->tsig = nullptr;
+    idx->trows = nullptr; idx->tstrs = nullptr; idx->tlens = nullptr; idx->tsig = nullptr; idx->tpack = nullptr;
     idx->id_list = nullptr; idx->pos_of_id = nullptr; idx->node_pid = nullptr;
     idx->node_size = nullptr; idx->node_lid = nullptr; idx->node_pivot = nullptr;
     idx->node_min_dis = nullptr; idx->node_flags = nullptr;
@@ -408,6 +423,7 @@ static int build_tree_impl(gts_index *idx, cudaStream_t s)
         ALLOC(idx->tstrs, (size_t)n * kStrStride);
         ALLOC(idx->tlens, n);
         ALLOC(idx->tsig, n);
+        ALLOC(idx->tpack, 2 * (size_t)n);
     } else {
         ALLOC(idx->trows, (size_t)n * idx->dim);
     }
@@ -483,7 +499,8 @@ static int build_tree_impl(gts_index *idx, cudaStream_t s)
     k_permute<<<grid_for(work, 256), 256, 0, s>>>(n, idx->dim, idx->metric, idx->id_list, idx->rows,
                                                   idx->trows, idx->strs, idx->tstrs, idx->lens,
                                                   idx->tlens, idx->pos_of_id);
-    if (idx->metric == kEdit) k_str_sig<<<grid_for((size_t)n, 256), 256, 0, s>>>(n, idx->tstrs, idx->tlens, idx->tsig);
+    if (idx->metric == kEdit) k_str_sig<<<grid_for((size_t)n, 256), 256, 0, s>>>(n, idx->tstrs, idx->tlens, idx->tsig,
+                                                                             idx->tpack);
     if (idx->metric == kAngle) k_row_norms<<<grid_for((size_t)n, 256), 256, 0, s>>>(n, idx->dim, idx->trows, idx->tnorm);
     GTS_CUDA_TRY(cudaMemsetAsync(sc.nsplit + 1, 0, 2 * sizeof(int), s));
     k_cut_lists<<<(mnn + 255) / 256, 256, 0, s>>>(mnn, O, idx->node_flags, idx->node_size, idx->node_pivot, idx->cut_node,

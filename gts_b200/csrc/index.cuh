@@ -14,7 +14,7 @@ struct gts_index {
     float *rows = nullptr, *trows = nullptr;
     char *strs = nullptr, *tstrs = nullptr;
     int *lens = nullptr, *tlens = nullptr;
-    uint4 *tsig = nullptr;
+    uint4 *tsig = nullptr, *tpack = nullptr;   // strings in tree order: signatures, first kPackChars characters
     int *id_list = nullptr, *pos_of_id = nullptr;
     int *node_pid = nullptr, *node_size = nullptr, *node_lid = nullptr, *node_pivot = nullptr;
     float *node_min_dis = nullptr;
@@ -113,6 +113,7 @@ namespace gts {
 //   [5] fast: candidates appended         [6] fast: filter passes
 //   [7] fast: (query tile, block) pairs tested by the block bound
 constexpr int kStatsN = 8;
+constexpr int kPackChars = 32;
 constexpr int kCutSize = 128;   // objects of a cut node at most, unless it has no children
 
 // Build the tree for the data already placed in idx->rows / strs / lens.

@@ -32,7 +32,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <climits>
-#include "search.cuh"
+#include "sweep.cuh"
 
 namespace gts {
 
@@ -51,32 +51,6 @@ constexpr int kSwSampleMin = 1 << 16;  // objects from which on it pays
 constexpr int kSwRounds = 3;           // further passes over kNN queries whose lists overflowed
 constexpr int kSwHitCap = 16384;       // hits per query of a range-ids call at most
 constexpr float kSwTiny = 1e-36f;      // squares below this may have lost bits to underflow
-
-struct SweepArgs {
-    SearchArgs a;
-    int q0, nq, ntiles, Qp, ld;         // the run's queries a.qids[q0 ..], padded count, query row stride
-    int ncut, nanc;
-    const int *cut, *anc, *anc_idx;
-    const float *tnorm;                 // angle: norms of the rows in tree order
-    int *key, *order;                   // tree position of the query; sorted order -> query of the run
-    int *bq;                            // sorted slot -> query of the batch (-1: padding)
-    float *seed;                        // per query of the run: bound on the k-th distance (kNN)
-    float *qrow;                        // [Qp][ld] sorted query rows, zero padded
-    float *R, *vthr, *vlow, *qnorm;     // per sorted query: radius, value thresholds
-    int *self;                          // its tree position when it is an object (-1)
-    float *dlo, *dhi;                   // [nanc][Qp] pivot distance bounds
-    int *nrows, *rowpos;                // per tile: rows to look at, their positions [ntiles][num]
-    int *ccnt, *cpos;                   // candidate lists [Qp][cap]
-    float *cv;
-    int *cnt, *cnt2;                    // range: certain counts per sorted query
-    int *ctr;                           // [0] item counter, [1] queries left over
-    int4 *left;                         // queries whose list overflowed: (query, 0, 0, 0) for the traversal
-    float *left_R;                      // kNN: and a bound on their k-th distance, from the list
-    const int4 *again;                  // kNN, a later round: the run's queries and bounds come from
-    const float *again_R;               //   again[q0 ..], again_R[q0 ..]
-    int cap;                            // candidates listed per query
-    int sample;                         // look at every sample-th row only (1: all)
-};
 
 __device__ __forceinline__ void sw_cp16(void *dst, const void *src, int bytes)
 {
@@ -395,7 +369,7 @@ __global__ void __launch_bounds__(256) k_sw_query(SweepArgs s)
 // ---------------------------------------------------------------- ring bounds
 
 // The cut nodes that some query of tile blockIdx.y can reach: one thread per
-// cut node keeps a mask of the tile's 128 queries and walks its ancestors, as
+// cut node keeps a mask of the tile's (at most 128) queries and walks its ancestors, as
 // the traversal does from above.  The rows of the kept nodes of a CTA's 256
 // are appended to the tile's row list.
 __global__ void __launch_bounds__(256) k_sw_cut(SweepArgs s)
@@ -404,7 +378,7 @@ __global__ void __launch_bounds__(256) k_sw_cut(SweepArgs s)
     __shared__ int wsum[8], s_base;
     const DevTree &t = s.a.t;
     const int tile = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int q0 = tile * 128, nq = min(128, s.nq - q0);
+    const int q0 = tile * s.tq, nq = min(s.tq, s.nq - q0);
     if (tid < 128) sR[tid] = tid < nq ? s.R[q0 + tid] : 0.f;
     __syncthreads();
     const int i = blockIdx.x * 256 + tid;
@@ -1162,6 +1136,7 @@ size_t plan_sweep(const gts_index *idx, int tiles, int qnum, unsigned char *base
     r.left_R = (float *)take(4 * 2 * (size_t)qnum);
     r.cap = kSwCap;
     r.sample = 1;
+    r.tq = 128;
     r.ctr = (int *)take(64);
     r.nrows = (int *)take(4 * (size_t)tiles);
     r.key = (int *)take(4 * (size_t)Qp * 5);   // key, sorted key, identity, order, batch query
@@ -1206,7 +1181,7 @@ int launch_tiles(gts_index *idx, SweepArgs s, bool sampled, cudaStream_t st)
     // for a few queries, which would then keep every row in play: a pass over
     // 1/16 of the rows first bounds every query by the whole data
     for (s.sample = sampled ? kSwSample : 1;; s.sample = 1) {
-        k_sw_cut<<<dim3((s.ncut + 255) / 256, tiles128), 256, 0, st>>>(s);
+        sweep_cut_launch(s, tiles128, st);
         k_sw_tile<M, QI><<<nsm * std::max(per_sm, 1), kSwThreads, smem, st>>>(s);
         idx->kernel_launches += 2;
         if (s.sample == 1) break;
@@ -1243,6 +1218,11 @@ __global__ void k_sw_copy_hits(SweepArgs s, int base)
 }
 
 }  // namespace
+
+void sweep_cut_launch(const SweepArgs &s, int ntiles, cudaStream_t st)
+{
+    k_sw_cut<<<dim3((s.ncut + 255) / 256, ntiles), 256, 0, st>>>(s);
+}
 
 // Batches the sweep takes: row metrics of more dimensions than a lane filters
 // alone, without deletions, learned seeds, or a caller's choice of the
@@ -1360,6 +1340,7 @@ int run_sweep(gts_index *idx, const SearchArgs &a, cudaStream_t st, int *done, c
 {
     *done = 0;
     *n_left = 0;
+    if (idx->metric == kEdit) return run_sweep_edit(idx, a, st, done, items, n_left);
     SweepBatch b;
     if (!sweep_begin(idx, a, &b)) return GTS_OK;
     int rc;

@@ -62,6 +62,54 @@ def test_sweep_equals_traversal_and_brute_force(oracle, metric, n, dim, comps, s
             _same([x[:40] for x in got], (bk, bi, bd))
 
 
+def _words(n, seed, long_ones):
+    strs, lens = G.word_strings(n, seed)
+    rng = np.random.default_rng(seed)
+    for i, length in enumerate(long_ones):   # the pattern word and packed-text limits, and beyond
+        strs[i] = 0
+        strs[i, :length] = rng.integers(97, 123, length)
+        lens[i] = length
+    strs[60, :lens[60]] = 200                # bytes above 127
+    lens[61:64] = 0                          # empty strings
+    strs[61:64] = 0
+    return strs, lens
+
+
+@pytest.mark.parametrize("n,max_h,nq,k", [(20000, 4, 300, 16), (16501, 3, 1, 5), (40000, 5, 33, 128), (20000, 1, 31, 1)])
+def test_string_sweep_equals_traversal_and_brute_force(oracle, n, max_h, nq, k):
+    strs, lens = _words(n, n + 1, [31, 32, 33, 34, 63, 64, 65, 108])
+    ds = oracle.Dataset(6, strs=strs, lens=lens)
+    short = np.argsort(lens, kind="stable")[:20]   # heavy: thousands of close words
+    q = np.concatenate([np.arange(8), [60, 61], short, G.query_ids(n, nq, 9)])[-max(nq, 1):].astype(np.int32) \
+        if nq < 40 else np.concatenate([np.arange(8), [60, 61], short, G.query_ids(n, nq, 9)]).astype(np.int32)
+    qs, ql = strs[q].copy(), lens[q].copy()
+    qs[:, 0] = np.where(ql > 0, 113, qs[:, 0])     # new words: not in the index as such
+    a = gts.Index(None, 6, strs=strs, lens=lens, max_h=max_h)
+    b = gts.Index(None, 6, strs=strs, lens=lens, max_h=max_h)
+    for mode in (0, 1, 2):
+        b.set_plain_threads(mode, 256)
+    with a, b:
+        got = a.knn(q, k, return_ids=True)
+        _same(got, b.knn(q, k, return_ids=True))
+        _same([x[:40] for x in got], oracle.knn_brute(ds, q[:40], k))
+        _same(a.knn_rows((qs, ql), k, return_ids=True), b.knn_rows((qs, ql), k, return_ids=True))
+        for r in (0.0, 1.0, 2.5, 3.0, 40.0):
+            counts = a.range(q, r)
+            np.testing.assert_array_equal(counts, b.range(q, r))
+            np.testing.assert_array_equal(counts[:40], oracle.range_brute(ds, q[:40], r))
+            np.testing.assert_array_equal(a.range_rows((qs, ql), r), b.range_rows((qs, ql), r))
+
+
+def test_string_stream_counts():
+    strs, lens = G.word_strings(20000, 31)
+    flags, ids = G.update_stream(20000, 2000, 32, max_in_size=10)
+    a = gts.Index(None, 6, strs=strs, lens=lens, max_h=4)
+    b = gts.Index(None, 6, strs=strs, lens=lens, max_h=4)
+    b.set_plain_threads(1, 256)
+    with a, b:
+        np.testing.assert_array_equal(a.update_run(flags, ids, 2.0)[0], b.update_run(flags, ids, 2.0)[0])
+
+
 def test_overflowing_lists_and_long_hit_lists(oracle):
     """Thousands of equal distances overflow the candidate lists in every
     round; more hits than a list holds make range ids go over the rows again."""
