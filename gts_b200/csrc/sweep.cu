@@ -376,10 +376,12 @@ __global__ void __launch_bounds__(256) k_sw_cut(SweepArgs s)
 {
     __shared__ float sR[128];
     __shared__ int wsum[8], s_base;
+    __shared__ uint32_t lok[4];
     const DevTree &t = s.a.t;
     const int tile = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int q0 = tile * s.tq, nq = min(s.tq, s.nq - q0);
     if (tid < 128) sR[tid] = tid < nq ? s.R[q0 + tid] : 0.f;
+    if (s.lens_ok && tid < 4) lok[tid] = reinterpret_cast<const uint32_t *>(s.lens_ok + tile)[tid];
     __syncthreads();
     const int i = blockIdx.x * 256 + tid;
     int size = 0, lid = 0;
@@ -431,7 +433,35 @@ __global__ void __launch_bounds__(256) k_sw_cut(SweepArgs s)
         size = first < lid + size ? (lid + size - 1 - first) / s.sample + 1 : 0;
         lid = first;
     }
-    int incl = size;
+    // the warp goes over its kept nodes together; strings of lengths that no
+    // query of the tile can match are left out (strings are not sampled)
+    auto fits = [&](int pos) {
+        const int n = min(max(t.tlens[pos], 0), 127);
+        return (lok[n >> 5] >> (n & 31)) & 1u;
+    };
+    const unsigned mine = __ballot_sync(0xffffffffu, size > 0);
+    int kept = size;
+    unsigned kb[4] = {0, 0, 0, 0};   // the lane's node: which of its first 128 strings stay
+    if (s.lens_ok)
+        for (unsigned todo = mine; todo; todo &= todo - 1) {
+            const int from = __ffs(todo) - 1;
+            const int n = __shfl_sync(0xffffffffu, size, from), l = __shfl_sync(0xffffffffu, lid, from);
+            unsigned b[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) b[u] = __ballot_sync(0xffffffffu, u * 32 + lane < n && fits(l + u * 32 + lane));
+            int c = 0;
+            for (int j = 128 + lane; j < n; j += 32) c += fits(l + j) ? 1 : 0;
+            if (n > 128) c = __reduce_add_sync(0xffffffffu, c);
+            if (lane == from) {
+                kept = c;
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    kb[u] = b[u];
+                    kept += __popc(b[u]);
+                }
+            }
+        }
+    int incl = kept;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int y = __shfl_up_sync(0xffffffffu, incl, o);
@@ -449,13 +479,29 @@ __global__ void __launch_bounds__(256) k_sw_cut(SweepArgs s)
         s_base = run ? atomicAdd(&s.nrows[tile], run) : 0;
     }
     __syncthreads();
-    const int off = s_base + wsum[warp] + incl - size;
+    const int off = s_base + wsum[warp] + incl - kept;
     int *dst = s.rowpos + (size_t)tile * t.num;
-    for (unsigned todo = __ballot_sync(0xffffffffu, size > 0); todo; todo &= todo - 1) {
+    for (unsigned todo = mine; todo; todo &= todo - 1) {
         const int from = __ffs(todo) - 1;
         const int n = __shfl_sync(0xffffffffu, size, from), l = __shfl_sync(0xffffffffu, lid, from);
-        const int o = __shfl_sync(0xffffffffu, off, from);
-        for (int j = lane; j < n; j += 32) dst[o + j] = l + j * s.sample;
+        int o = __shfl_sync(0xffffffffu, off, from);
+        if (!s.lens_ok) {
+            for (int j = lane; j < n; j += 32) dst[o + j] = l + j * s.sample;
+            continue;
+        }
+        const unsigned below = (1u << lane) - 1u;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const unsigned b = __shfl_sync(0xffffffffu, kb[u], from);
+            if ((b >> lane) & 1u) dst[o + __popc(b & below)] = l + u * 32 + lane;
+            o += __popc(b);
+        }
+        for (int j0 = 128; j0 < n; j0 += 32) {
+            const bool ok = j0 + lane < n && fits(l + j0 + lane);
+            const unsigned b = __ballot_sync(0xffffffffu, ok);
+            if (ok) dst[o + __popc(b & below)] = l + j0 + lane;
+            o += __popc(b);
+        }
     }
 }
 

@@ -30,6 +30,7 @@ struct SweepArgs {
     const float *again_R;               //   again[q0 ..], again_R[q0 ..]
     int cap;                            // candidates listed per query
     int sample;                         // look at every sample-th row only (1: all)
+    const uint4 *lens_ok;               // strings: per tile a mask of the lengths some query can match (nullable)
 };
 
 // Ring bounds: the rows of the cut nodes that some query of each tile can

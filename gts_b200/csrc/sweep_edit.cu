@@ -18,8 +18,11 @@
 //
 // Distances are whole numbers, so kNN keeps a histogram of the distances found
 // per query: its k-th entry is the running bound, and after the sweep the
-// exact k-th distance.  Queries longer than 32 characters, and queries whose
-// list cannot hold their candidates, go to the traversal.
+// exact k-th distance.  Queries are taken in the order of their lengths, then
+// of their places in the tree: a tile then needs few lengths of strings, and
+// leaves out the rest when it lists its rows.  Queries of 33 to 64 characters
+// get a pass of their own in 64-bit words; longer ones, and queries whose list
+// cannot hold their candidates, go to the traversal.
 #include <cub/device/device_radix_sort.cuh>
 #include <algorithm>
 #include <climits>
@@ -37,52 +40,55 @@ constexpr int kSeChunk = 8;            // row tiles per work item
 constexpr int kSeWindow = 1024;        // objects around a query's place that bound its k-th distance
 constexpr int kSeCap = 2048;           // candidates listed per query
 constexpr int kSeHist = 128;           // distances are at most 108
-constexpr int kSeRounds = 1;           // further passes over kNN queries whose lists overflowed
+constexpr int kSeRounds = 1;           // further passes, in 64-bit words
 constexpr int kSeTextLd = kPackChars / 4 + 1;   // words per row's characters in shared memory (odd: no bank conflicts)
 
 struct EditArgs {
     SweepArgs s;
+    int wide;               // the pass takes patterns of up to 64 characters (else 32)
+    uint4 *lens_ok;         // per tile: lengths within some query's radius
     const uint4 *tpack;
     int *qlen;              // [Qp] pattern length; -1: not swept
-    uint32_t *qpack;        // [Qp][8] first 32 characters
+    uint32_t *qpack;        // [Qp][16] first 64 characters
     uint32_t *qsig;         // [Qp][8] low and high nibbles of the signature
     int *hist;              // kNN: [Qp][kSeHist] distances found
 };
 
 // One step of the bit-parallel column (Myers 1999, Hyyro's formulation) on a
-// 32-bit word, as edit_myers64.
-struct Myers32 {
-    uint32_t pv, mv, hi;
+// 32- or 64-bit word, as edit_myers64.
+template <typename W>
+struct Myers {
+    W pv, mv, hi;
     int score;
     __device__ __forceinline__ void start(int m)
     {
-        pv = 0xffffffffu;
+        pv = ~(W)0;
         mv = 0;
-        hi = 1u << (m - 1);
+        hi = (W)1 << (m - 1);
         score = m;
     }
-    __device__ __forceinline__ void step(uint32_t eq)
+    __device__ __forceinline__ void step(W eq)
     {
-        const uint32_t xv = eq | mv;
-        const uint32_t xh = (((eq & pv) + pv) ^ pv) | eq;
-        uint32_t ph = mv | ~(xh | pv), mh = pv & xh;
+        const W xv = eq | mv;
+        const W xh = (((eq & pv) + pv) ^ pv) | eq;
+        W ph = mv | ~(xh | pv), mh = pv & xh;
         score += (ph & hi) ? 1 : ((mh & hi) ? -1 : 0);
-        ph = (ph << 1) | 1u;
+        ph = (ph << 1) | (W)1;
         mh <<= 1;
         pv = mh | ~(xv | ph);
         mv = ph & xv;
     }
 };
 
-// Edit distance of the pattern behind peq (m <= 32 characters) to a text of n
-// characters, its first kPackChars from words, the rest from tail; some value
-// above limit where the distance is above limit.
-__device__ __forceinline__ int edit32(const uint32_t *peq, int m, const uint32_t *words, const char *tail, int n,
-                                      int limit)
+// Edit distance of the pattern behind peq (m characters, at most the word's
+// bits) to a text of n characters, its first kPackChars from words, the rest
+// from tail; some value above limit where the distance is above limit.
+template <typename W>
+__device__ __forceinline__ int edit_words(const W *peq, int m, const uint32_t *words, const char *tail, int n, int limit)
 {
     if (m == 0) return n;
     if (n == 0) return m;
-    Myers32 d;
+    Myers<W> d;
     d.start(m);
     for (int j0 = 0; j0 < n; j0 += 4) {
         uint32_t w;
@@ -104,56 +110,63 @@ __device__ __forceinline__ int edit32(const uint32_t *peq, int m, const uint32_t
 
 __device__ __forceinline__ int str_len(int n) { return min(max(n, 0), kStrStride); }
 
+__device__ __forceinline__ void set_bit(uint32_t *p, int i) { atomicOr(p, 1u << i); }
+__device__ __forceinline__ void set_bit(unsigned long long *p, int i) { atomicOr(p, 1ull << i); }
+
 // ---------------------------------------------------------------- seeds
 
 // The masks of one query's characters, made by the CTA.
-__device__ __forceinline__ void make_peq(uint32_t *peq, const char *src, int m)
+template <typename W>
+__device__ __forceinline__ void make_peq(W *peq, const char *src, int m)
 {
     for (int c = threadIdx.x; c < 256; c += blockDim.x) peq[c] = 0;
     __syncthreads();
-    if ((int)threadIdx.x < m) atomicOr(&peq[(unsigned char)src[threadIdx.x]], 1u << threadIdx.x);
+    if ((int)threadIdx.x < m) set_bit(&peq[(unsigned char)src[threadIdx.x]], threadIdx.x);
     __syncthreads();
 }
 
-__device__ __forceinline__ int edit_to_id(const DevTree &t, const uint32_t *peq, int m, int id)
+template <typename W>
+__device__ __forceinline__ int edit_to_id(const DevTree &t, const W *peq, int m, int id)
 {
     const char *txt = t.strs + (size_t)id * kStrStride;
     const int n = str_len(t.lens[id]);
     if (m == 0) return n;
     if (n == 0) return m;
-    Myers32 d;
+    Myers<W> d;
     d.start(m);
     for (int j = 0; j < n; j++) d.step(peq[(unsigned char)txt[j]]);
     return d.score;
 }
 
-// One CTA per query of the run: its place in the tree order, and for kNN the
-// k-th smallest distance over the kSeWindow objects around it.
-__global__ void __launch_bounds__(kSeThreads) k_se_seed(EditArgs e)
+// One CTA per query of the batch: its sort key (length, then its place in the
+// tree order), and for kNN the k-th smallest distance over the kSeWindow
+// objects around that place.
+__global__ void __launch_bounds__(kSeThreads) k_se_seed(EditArgs e, int pos_bits)
 {
-    __shared__ uint32_t peq[256];
+    __shared__ unsigned long long peq[256];
     __shared__ int hist[kSeHist];
     __shared__ int s_node;
     const SweepArgs &s = e.s;
     const DevTree &t = s.a.t;
-    const int q = s.q0 + blockIdx.x, tid = threadIdx.x;
+    const int q = blockIdx.x, tid = threadIdx.x;
     const bool by_data = s.a.qstrs != nullptr, knn = s.a.mode == kModeKnn;
     const int qid = by_data ? -1 : s.a.qids[q];
     if (!by_data && (qid < 0 || qid >= t.num)) {
         if (tid == 0) {
             atomicMax(s.a.status, (int)kKsBadQuery);
-            s.key[blockIdx.x] = 0;
-            s.seed[blockIdx.x] = -1.f;
+            s.key[q] = 0;
+            s.seed[q] = -1.f;
         }
         return;
     }
     const char *src = by_data ? s.a.qstrs + (size_t)q * kStrStride : t.strs + (size_t)qid * kStrStride;
     const int m = min(max(by_data ? s.a.qlens[q] : t.lens[qid], 0), kStrStride - 1);
     int pos = by_data ? 0 : t.pos_of_id[qid];
-    if ((!by_data && !knn) || m > 32) {
+    const int pos_shift = max(0, pos_bits - 24);   // 7 bits of length, up to 24 of position
+    if ((!by_data && !knn) || m > 64) {
         if (tid == 0) {
-            s.key[blockIdx.x] = pos;
-            s.seed[blockIdx.x] = -1.f;
+            s.key[q] = m << 24 | pos >> pos_shift;
+            s.seed[q] = -1.f;
         }
         return;
     }
@@ -179,7 +192,7 @@ __global__ void __launch_bounds__(kSeThreads) k_se_seed(EditArgs e)
         }
         pos = min(t.node_lid[node] + t.node_size[node] / 2, t.num - 1);
     }
-    if (tid == 0) s.key[blockIdx.x] = pos;
+    if (tid == 0) s.key[q] = m << 24 | pos >> pos_shift;
     if (!knn) return;
     for (int i = tid; i < kSeHist; i += kSeThreads) hist[i] = 0;
     __syncthreads();
@@ -188,7 +201,7 @@ __global__ void __launch_bounds__(kSeThreads) k_se_seed(EditArgs e)
         const int p = w0 + i;
         const uint4 a = e.tpack[2 * (size_t)p], b = e.tpack[2 * (size_t)p + 1];
         const uint32_t words[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        const int d = edit32(peq, m, words, t.tstrs + (size_t)p * kStrStride, str_len(t.tlens[p]), INT_MAX);
+        const int d = edit_words(peq, m, words, t.tstrs + (size_t)p * kStrStride, str_len(t.tlens[p]), INT_MAX);
         atomicAdd(&hist[min(d, kSeHist - 1)], 1);
     }
     __syncthreads();
@@ -201,7 +214,7 @@ __global__ void __launch_bounds__(kSeThreads) k_se_seed(EditArgs e)
                 break;
             }
         }
-        s.seed[blockIdx.x] = (float)R;
+        s.seed[q] = (float)R;
         if (s.a.stats) atomicAdd(&s.a.stats[0], (unsigned long long)w);
     }
 }
@@ -213,8 +226,9 @@ __global__ void k_se_iota(int n, int *v)
 }
 
 // One thread per sorted query slot: its pattern, signature and radius, empty
-// lists.  A query the sweep does not take (longer than 32 characters) goes to
-// the traversal's list.
+// lists.  A query the pass does not take goes to the next one's list, and
+// past the last pass to the traversal.  A warp is a tile: it also makes the
+// tile's mask of string lengths.
 __global__ void __launch_bounds__(128) k_se_query(EditArgs e)
 {
     const SweepArgs &s = e.s;
@@ -222,7 +236,7 @@ __global__ void __launch_bounds__(128) k_se_query(EditArgs e)
     const int i = blockIdx.x * 128 + threadIdx.x;
     if (i >= s.Qp) return;
     const bool have = i < s.nq;
-    const int q = !have ? -1 : (s.again ? s.again[s.q0 + i].x : s.q0 + s.order[i]);
+    const int q = !have ? -1 : (s.again ? s.again[s.q0 + i].x : s.order[s.q0 + i]);
     s.bq[i] = q;
     s.ccnt[i] = s.cnt[i] = s.cnt2[i] = 0;
     float R = -1.f;
@@ -231,16 +245,18 @@ __global__ void __launch_bounds__(128) k_se_query(EditArgs e)
     if (have && (s.a.qstrs || (qid >= 0 && qid < t.num))) {
         const char *src = s.a.qstrs ? s.a.qstrs + (size_t)q * kStrStride : t.strs + (size_t)qid * kStrStride;
         m = min(max(s.a.qstrs ? s.a.qlens[q] : t.lens[qid], 0), kStrStride - 1);
-        if (m > 32) {
+        if (m > (e.wide ? 64 : 32)) {
+            const int at = atomicAdd(&s.ctr[1], 1);
+            s.left[at] = make_int4(q, 0, 0, 0);
+            s.left_R[at] = s.seed[q];
             m = -1;
-            s.left[atomicAdd(&s.ctr[1], 1)] = make_int4(q, 0, 0, 0);
             if (s.a.mode != kModeKnn) {
                 s.a.counts[q] = 0;   // the traversal adds to it
                 if (s.a.mode == kModeRangeTimed) s.a.counts2[q] = 0;
             }
         } else {
             R = s.a.mode != kModeKnn ? floorf(fminf(s.a.r, (float)(kSeHist - 1)))
-                                     : (s.again ? s.again_R[s.q0 + i] : s.seed[q - s.q0]);
+                                     : (s.again ? s.again_R[s.q0 + i] : s.seed[q]);
             const uint4 g = str_sig(src, m);
             const uint32_t w[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
@@ -248,29 +264,36 @@ __global__ void __launch_bounds__(128) k_se_query(EditArgs e)
                 e.qsig[8 * (size_t)i + c] = w[c] & 0x0F0F0F0Fu;
                 e.qsig[8 * (size_t)i + 4 + c] = (w[c] >> 4) & 0x0F0F0F0Fu;
             }
-            for (int c = 0; c < 8; c++) {
+            for (int c = 0; c < 16; c++) {
                 uint32_t v = 0;
                 for (int u = 0; u < 4; u++)
                     if (4 * c + u < m) v |= (uint32_t)(unsigned char)src[4 * c + u] << (8 * u);
-                e.qpack[8 * (size_t)i + c] = v;
+                e.qpack[16 * (size_t)i + c] = v;
             }
         }
     }
     s.R[i] = R;
     e.qlen[i] = m;
+    uint32_t ok[4] = {0, 0, 0, 0};
+    if (m >= 0 && R >= 0.f)
+        for (int n = max(0, m - (int)R); n <= min(127, m + (int)R); n++) ok[n >> 5] |= 1u << (n & 31);
+#pragma unroll
+    for (int c = 0; c < 4; c++) ok[c] = __reduce_or_sync(0xffffffffu, ok[c]);
+    if ((i & 31) == 0) e.lens_ok[i / kSeTq] = make_uint4(ok[0], ok[1], ok[2], ok[3]);
     if (s.a.mode == kModeKnn)
         for (int d = 0; d < kSeHist; d++) e.hist[(size_t)i * kSeHist + d] = 0;
 }
 
 // Distances of one query per CTA to the cut nodes' ancestors' pivots.
+template <typename W>
 __global__ void __launch_bounds__(kSeThreads) k_se_pivots(EditArgs e)
 {
-    __shared__ uint32_t peq[256];
+    __shared__ W peq[256];
     const SweepArgs &s = e.s;
     const DevTree &t = s.a.t;
     const int i = blockIdx.x, m = e.qlen[i];
     if (m < 0) return;
-    make_peq(peq, reinterpret_cast<const char *>(e.qpack + 8 * (size_t)i), m);
+    make_peq(peq, reinterpret_cast<const char *>(e.qpack + 16 * (size_t)i), m);
     for (int a = blockIdx.y * kSeThreads + threadIdx.x; a < s.nanc; a += gridDim.y * kSeThreads) {
         const float d = (float)edit_to_id(t, peq, m, t.node_pivot[s.anc[a]]);
         s.dlo[(size_t)a * s.Qp + i] = d;
@@ -280,8 +303,9 @@ __global__ void __launch_bounds__(kSeThreads) k_se_pivots(EditArgs e)
 
 // ---------------------------------------------------------------- tiles
 
+template <typename W>
 struct EditSmem {
-    uint32_t peq[kSeTq][256];
+    W peq[kSeTq][256];
     uint32_t text[kSeRows * kSeTextLd];
     uint32_t sig[kSeTq][8];
     int pos[kSeRows], len[kSeRows];
@@ -293,10 +317,11 @@ struct EditSmem {
 
 // Persistent CTAs take (query tile, chunk of row tiles) items, query tiles
 // outermost: the tile's masks stay while the CTA goes over its rows.
-__global__ void __launch_bounds__(kSeThreads, 3) k_se_tile(EditArgs e)
+template <typename W>
+__global__ void __launch_bounds__(kSeThreads, sizeof(W) == 4 ? 3 : 2) k_se_tile(EditArgs e)
 {
     extern __shared__ __align__(16) unsigned char se_smem[];
-    EditSmem &sm = *reinterpret_cast<EditSmem *>(se_smem);
+    EditSmem<W> &sm = *reinterpret_cast<EditSmem<W> *>(se_smem);
     const SweepArgs &s = e.s;
     const DevTree &t = s.a.t;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -323,10 +348,11 @@ __global__ void __launch_bounds__(kSeThreads, 3) k_se_tile(EditArgs e)
                 sm.R[tid] = (int)s.R[q0 + tid];
             }
             __syncthreads();
-            for (int i = tid; i < kSeTq * 32; i += kSeThreads) {
-                const int q = i >> 5, j = i & 31;
+            constexpr int kBits = 8 * (int)sizeof(W);
+            for (int i = tid; i < kSeTq * kBits; i += kSeThreads) {
+                const int q = i / kBits, j = i % kBits;
                 if (j < sm.qlen[q])
-                    atomicOr(&sm.peq[q][(e.qpack[8 * (size_t)(q0 + q) + (j >> 2)] >> (8 * (j & 3))) & 255u], 1u << j);
+                    set_bit(&sm.peq[q][(e.qpack[16 * (size_t)(q0 + q) + (j >> 2)] >> (8 * (j & 3))) & 255u], j);
             }
             cur = tile;
         }
@@ -401,7 +427,7 @@ __global__ void __launch_bounds__(kSeThreads, 3) k_se_tile(EditArgs e)
             }
             for (int i = tid; i < total; i += kSeThreads) {
                 const int pr = sm.list[i], q = pr >> 8, r = pr & 255, R = sm.R[q];
-                const int d = edit32(sm.peq[q], sm.qlen[q], sm.text + r * kSeTextLd,
+                const int d = edit_words(sm.peq[q], sm.qlen[q], sm.text + r * kSeTextLd,
                                      t.tstrs + (size_t)sm.pos[r] * kStrStride, sm.len[r], R);
                 if (d > R) continue;
                 if (mode == kModeKnn) {
@@ -531,7 +557,7 @@ size_t plan_edit(const gts_index *idx, int tiles, int qnum, bool knn, unsigned c
     const int Qp = (tiles * kSeTq + 127) / 128 * 128;
     size_t off = 0, tb = 0;
     auto take = [&](size_t b) { size_t o = off; off += (b + 255) & ~(size_t)255; return base + o; };
-    cub::DeviceRadixSort::SortPairs(nullptr, tb, (int *)nullptr, (int *)nullptr, (int *)nullptr, (int *)nullptr, Qp, 0,
+    cub::DeviceRadixSort::SortPairs(nullptr, tb, (int *)nullptr, (int *)nullptr, (int *)nullptr, (int *)nullptr, qnum, 0,
                                     32, (cudaStream_t)0);
     EditArgs e{};
     SweepArgs &r = e.s;
@@ -543,16 +569,18 @@ size_t plan_edit(const gts_index *idx, int tiles, int qnum, bool knn, unsigned c
     r.left_R = (float *)take(4 * 2 * (size_t)qnum);
     r.ctr = (int *)take(64);
     r.nrows = (int *)take(4 * (size_t)tiles);
-    r.key = (int *)take(4 * (size_t)Qp * 5);
-    r.order = r.key + 3 * (size_t)Qp;
-    r.bq = r.order + Qp;
-    r.seed = (float *)take(4 * (size_t)Qp);
+    r.key = (int *)take(4 * (size_t)qnum * 4);   // key, sorted key, identity, order: of the whole batch
+    r.order = r.key + 3 * (size_t)qnum;
+    r.bq = (int *)take(4 * (size_t)Qp);
+    r.seed = (float *)take(4 * (size_t)qnum);
     r.R = (float *)take(4 * (size_t)Qp);
     r.ccnt = (int *)take(4 * (size_t)Qp * 3);
     r.cnt = r.ccnt + Qp;
     r.cnt2 = r.cnt + Qp;
     e.qlen = (int *)take(4 * (size_t)Qp);
-    e.qpack = (uint32_t *)take(32 * (size_t)Qp);
+    e.qpack = (uint32_t *)take(64 * (size_t)Qp);
+    e.lens_ok = (uint4 *)take(sizeof(uint4) * (size_t)(Qp / kSeTq));
+    r.lens_ok = e.lens_ok;
     e.qsig = (uint32_t *)take(32 * (size_t)Qp);
     r.dlo = (float *)take(4 * (size_t)std::max(idx->ncut_anc, 1) * Qp);
     r.dhi = (float *)take(4 * (size_t)std::max(idx->ncut_anc, 1) * Qp);
@@ -568,14 +596,15 @@ size_t plan_edit(const gts_index *idx, int tiles, int qnum, bool knn, unsigned c
     return off;
 }
 
-int edit_pass(gts_index *idx, EditArgs &e, cudaStream_t st)
+template <typename W>
+int edit_pass_words(gts_index *idx, EditArgs &e, cudaStream_t st)
 {
     SweepArgs &s = e.s;
     int dev = 0, nsm = 148, per_sm = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    GTS_CUDA_TRY(cudaFuncSetAttribute(k_se_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(EditSmem)));
-    GTS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_se_tile, kSeThreads, sizeof(EditSmem)));
+    GTS_CUDA_TRY(cudaFuncSetAttribute(k_se_tile<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(EditSmem<W>)));
+    GTS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_se_tile<W>, kSeThreads, sizeof(EditSmem<W>)));
     s.ntiles = (s.nq + kSeTq - 1) / kSeTq;
     GTS_CUDA_TRY(cudaMemsetAsync(s.ctr, 0, sizeof(int), st));
     GTS_CUDA_TRY(cudaMemsetAsync(s.nrows, 0, sizeof(int) * s.ntiles, st));
@@ -583,15 +612,20 @@ int edit_pass(gts_index *idx, EditArgs &e, cudaStream_t st)
     if (s.nanc > 0) {
         // a CTA per query leaves the chip idle for few of them: split the pivots
         const int split = std::max(1, std::min((s.nanc + kSeThreads - 1) / kSeThreads, 2 * nsm / s.nq));
-        k_se_pivots<<<dim3(s.nq, split), kSeThreads, 0, st>>>(e);
+        k_se_pivots<W><<<dim3(s.nq, split), kSeThreads, 0, st>>>(e);
     }
     sweep_cut_launch(s, s.ntiles, st);
-    k_se_tile<<<nsm * std::max(per_sm, 1), kSeThreads, sizeof(EditSmem), st>>>(e);
+    k_se_tile<W><<<nsm * std::max(per_sm, 1), kSeThreads, sizeof(EditSmem<W>), st>>>(e);
     if (s.a.mode == kModeKnn) k_se_knn<<<s.nq, 128, 0, st>>>(e);
     else k_se_counts<<<(s.nq + 127) / 128, 128, 0, st>>>(e);
     idx->kernel_launches += 4 + (s.nanc > 0);
     GTS_CUDA_TRY(cudaGetLastError());
     return GTS_OK;
+}
+
+int edit_pass(gts_index *idx, EditArgs &e, cudaStream_t st)
+{
+    return e.wide ? edit_pass_words<unsigned long long>(idx, e, st) : edit_pass_words<uint32_t>(idx, e, st);
 }
 
 }  // namespace
@@ -626,20 +660,19 @@ int run_sweep_edit(gts_index *idx, const SearchArgs &a, cudaStream_t st, int *do
     s.anc = idx->cut_anc;
     s.nanc = idx->ncut_anc;
     s.anc_idx = idx->cut_anc_idx;
-    int key_bits = 1, rc;
-    while (key_bits < 31 && (1 << key_bits) < idx->num) key_bits++;
+    int pos_bits = 1, rc;
+    while (pos_bits < 31 && (1 << pos_bits) < idx->num) pos_bits++;
     const int run = tiles * kSeTq;
     GTS_CUDA_TRY(cudaMemsetAsync(s.ctr, 0, 64, st));
+    int *skey = s.key + a.qnum, *iota = skey + a.qnum;
+    k_se_seed<<<a.qnum, kSeThreads, 0, st>>>(e, pos_bits);
+    k_se_iota<<<(a.qnum + 255) / 256, 256, 0, st>>>(a.qnum, a.qnum > kSeTq ? iota : s.order);
+    idx->kernel_launches += 2;
+    if (a.qnum > kSeTq)
+        GTS_CUDA_TRY(cub::DeviceRadixSort::SortPairs(cub, cub_bytes, s.key, skey, iota, s.order, a.qnum, 0, 31, st));
     for (int q0 = 0; q0 < a.qnum; q0 += run) {
         s.q0 = q0;
         s.nq = std::min(run, a.qnum - q0);
-        int *skey = s.key + s.Qp, *iota = skey + s.Qp;
-        k_se_seed<<<s.nq, kSeThreads, 0, st>>>(e);
-        k_se_iota<<<(s.nq + 255) / 256, 256, 0, st>>>(s.nq, s.nq > kSeTq ? iota : s.order);
-        idx->kernel_launches += 2;
-        if (s.nq > kSeTq)
-            GTS_CUDA_TRY(cub::DeviceRadixSort::SortPairs(cub, cub_bytes, s.key, skey, iota, s.order, s.nq, 0, key_bits,
-                                                         st));
         if ((rc = edit_pass(idx, e, st))) return rc;
     }
     auto outcome = [&](int *left, bool *ok) {
@@ -653,12 +686,13 @@ int run_sweep_edit(gts_index *idx, const SearchArgs &a, cudaStream_t st, int *do
     };
     bool ok = false;
     if ((rc = outcome(n_left, &ok))) return rc;
-    // kNN queries whose lists filled before their bound settled: once more from
-    // the exact k-th distance (long queries come along and are listed again)
+    // once more: queries of 33 to 64 characters, and kNN queries whose lists
+    // filled before their bound settled, from the exact k-th distance
     int4 *const lists[2] = {s.left, s.left + a.qnum};
     float *const bounds[2] = {s.left_R, s.left_R + a.qnum};
-    for (int round = 0; round < kSeRounds && ok && knn && *n_left > 0; round++) {
+    for (int round = 0; round < kSeRounds && ok && *n_left > 0; round++) {
         const int n = *n_left;
+        e.wide = 1;
         s.again = lists[round & 1];
         s.again_R = bounds[round & 1];
         s.left = lists[(round + 1) & 1];
