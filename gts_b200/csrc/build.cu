@@ -234,14 +234,18 @@ __global__ void k_permute(int n, int dim, int metric, const int *id_list, const 
     }
 }
 
-// The batched sweep's cut nodes and their ancestors (index.cuh); a CTA
+// The nodes as records, and the batched sweep's cut nodes and their ancestors
+// (index.cuh); a CTA
 // appends its nodes in order, so lists stay nearly in position order.
 __global__ void __launch_bounds__(256) k_cut_lists(int mnn, int order, const uint8_t *flags, const int *size,
-                                                   const int *pivot, int *cut, int *anc, int *anc_idx, int *counts)
+                                                   const int *pivot, const int *lid, const float *min_dis, int *cut,
+                                                   int *anc, int *anc_idx, int *counts, int4 *rec)
 {
     __shared__ int base[2], woff[2][8];
     const int i = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     bool is[2] = {false, false};
+    // a child that does not exist still bounds its neighbour's ring by its min_dis (0)
+    if (i < mnn) rec[i] = make_int4(__float_as_int(min_dis[i]), (flags[i] & kExists) ? size[i] : 0, lid[i], pivot[i]);
     if (i < mnn && (flags[i] & kExists) && size[i] > 0) {
         is[1] = pivot[i] >= 0 && size[i] > kCutSize;
         is[0] = !is[1] && (i == 0 || size[(i - 1) / order] > kCutSize);
@@ -355,7 +359,7 @@ void free_tree(gts_index *idx)
     idx->mlp_ready = false;   // its feature pivots belong to the old tree
     void *ps[] = {idx->trows, idx->tstrs, idx->tlens, idx->tsig, idx->tpack, idx->id_list, idx->pos_of_id, idx->node_pid,
                   idx->node_size, idx->node_lid, idx->node_pivot, idx->node_min_dis,
-                  idx->node_flags, idx->cut_node, idx->cut_anc, idx->cut_anc_idx, idx->tnorm};
+                  idx->node_flags, idx->cut_node, idx->cut_anc, idx->cut_anc_idx, idx->tnorm, idx->node_rec};
     for (void *p : ps)
         if (p) cudaFree(p);
     idx->trows = nullptr; idx->tstrs = nullptr; idx->tlens = nullptr; idx->tsig = nullptr; idx->tpack = nullptr;
@@ -363,6 +367,7 @@ void free_tree(gts_index *idx)
     idx->node_size = nullptr; idx->node_lid = nullptr; idx->node_pivot = nullptr;
     idx->node_min_dis = nullptr; idx->node_flags = nullptr;
     idx->cut_node = nullptr; idx->cut_anc = nullptr; idx->cut_anc_idx = nullptr; idx->tnorm = nullptr;
+    idx->node_rec = nullptr;
     idx->ncut = idx->ncut_anc = 0;
 }
 
@@ -418,6 +423,7 @@ static int build_tree_impl(gts_index *idx, cudaStream_t s)
     ALLOC(idx->cut_node, mnn);
     ALLOC(idx->cut_anc, mnn);
     ALLOC(idx->cut_anc_idx, mnn);
+    ALLOC(idx->node_rec, mnn);
     if (idx->metric == kAngle) ALLOC(idx->tnorm, n);
     if (idx->metric == kEdit) {
         ALLOC(idx->tstrs, (size_t)n * kStrStride);
@@ -503,8 +509,9 @@ static int build_tree_impl(gts_index *idx, cudaStream_t s)
                                                                              idx->tpack);
     if (idx->metric == kAngle) k_row_norms<<<grid_for((size_t)n, 256), 256, 0, s>>>(n, idx->dim, idx->trows, idx->tnorm);
     GTS_CUDA_TRY(cudaMemsetAsync(sc.nsplit + 1, 0, 2 * sizeof(int), s));
-    k_cut_lists<<<(mnn + 255) / 256, 256, 0, s>>>(mnn, O, idx->node_flags, idx->node_size, idx->node_pivot, idx->cut_node,
-                                                  idx->cut_anc, idx->cut_anc_idx, sc.nsplit + 1);
+    k_cut_lists<<<(mnn + 255) / 256, 256, 0, s>>>(mnn, O, idx->node_flags, idx->node_size, idx->node_pivot, idx->node_lid,
+                                                  idx->node_min_dis, idx->cut_node, idx->cut_anc, idx->cut_anc_idx,
+                                                  sc.nsplit + 1, idx->node_rec);
     int ncuts[2] = {0, 0};
     GTS_CUDA_TRY(cudaMemcpyAsync(ncuts, sc.nsplit + 1, sizeof(ncuts), cudaMemcpyDeviceToHost, s));
     GTS_CUDA_TRY(cudaStreamSynchronize(s));

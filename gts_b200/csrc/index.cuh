@@ -26,6 +26,7 @@ struct gts_index {
     int *cut_node = nullptr, *cut_anc = nullptr, *cut_anc_idx = nullptr;
     int ncut = 0, ncut_anc = 0;
     float *tnorm = nullptr;
+    int4 *node_rec = nullptr;   // per node: (min_dis bits, size, first position, pivot or -1), size 0 where none exists
 
     // per-call scratch owned by the handle
     int *d_counter = nullptr;   // persistent-kernel work counter

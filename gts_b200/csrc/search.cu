@@ -606,6 +606,7 @@ static int launch_search_nt(gts_index *idx, const SearchArgs &a, cudaStream_t st
 
 static int launch_search(gts_index *idx, const SearchArgs &a, int nt, cudaStream_t st)
 {
+    if (warp_search_takes(idx, a)) return launch_search_warp(idx, a, st);
     switch (nt) {
     case 128: return launch_search_nt<128>(idx, a, st);
     case 512: return launch_search_nt<512>(idx, a, st);
@@ -795,7 +796,9 @@ static int run_search(gts_index *idx, SearchArgs &a, cudaStream_t st)
         }
     }
     int nt = idx->plain_nt[slot];
-    if (!nt && !idx->keep_stats && !swept) {
+    const bool by_warp = warp_search_takes(idx, a);   // no threads to choose
+    if (by_warp && !nt && !idx->keep_stats && a.qnum >= 2 * plain_tune_sample()) idx->plain_nt[slot] = kPlainDefaultThreads;
+    if (!nt && !idx->keep_stats && !swept && !by_warp) {
         int rc = plain_autotune(idx, a, st, &nt);
         if (rc) return rc;
         if (a.mode != kModeRangeIds) idx->plain_nt[slot] = nt;

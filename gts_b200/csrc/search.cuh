@@ -69,6 +69,11 @@ struct SearchArgs {
 // The pruning slacks and the handle's device pointers of a search.
 void fill_search_args(gts_index *idx, SearchArgs &a);
 
+// Range counts of up to kLaneRowDim dimensions, a query per warp
+// (search_warp.cu).
+bool warp_search_takes(const gts_index *idx, const SearchArgs &a);
+int launch_search_warp(gts_index *idx, const SearchArgs &a, cudaStream_t st);
+
 // The batched sweep (sweep.cu).  *done = 1: it answered every query of the
 // batch except those it lists (query, 0, 0, 0) in items[0 .. *n_left), which
 // the traversal answers; *done = 0: the batch is not one it takes.
