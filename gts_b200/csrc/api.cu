@@ -376,21 +376,21 @@ extern "C" void gts_index_free(gts_index *idx)
     if (!idx) return;
     gts::free_tree(idx);
     gts::free_data(idx);
-    if (idx->d_counter) cudaFree(idx->d_counter);
-    if (idx->d_status) cudaFree(idx->d_status);
-    if (idx->d_stats) cudaFree(idx->d_stats);
-    if (idx->scratch) cudaFree(idx->scratch);
-    if (idx->split_buf) cudaFree(idx->split_buf);
-    if (idx->io) cudaFree(idx->io);
-    if (idx->hits) cudaFree(idx->hits);
+    if (idx->d_counter) gts::dev_free(idx->d_counter);
+    if (idx->d_status) gts::dev_free(idx->d_status);
+    if (idx->d_stats) gts::dev_free(idx->d_stats);
+    if (idx->scratch) gts::dev_free(idx->scratch);
+    if (idx->split_buf) gts::dev_free(idx->split_buf);
+    if (idx->io) gts::dev_free(idx->io);
+    if (idx->hits) gts::dev_free(idx->hits);
     for (int i = 0; i < gts_index::kGraphSlots; i++)
         if (idx->graph_exec[i]) cudaGraphExecDestroy(idx->graph_exec[i]);
     if (idx->graph_stream) cudaStreamDestroy(idx->graph_stream);
     for (int i = 0; i < 2; i++)
         if (idx->graph_ev[i]) cudaEventDestroy(idx->graph_ev[i]);
-    if (idx->mlp_P) cudaFree(idx->mlp_P);
-    if (idx->mlp_norm) cudaFree(idx->mlp_norm);
-    if (idx->mlp_piv) cudaFree(idx->mlp_piv);
+    if (idx->mlp_P) gts::dev_free(idx->mlp_P);
+    if (idx->mlp_norm) gts::dev_free(idx->mlp_norm);
+    if (idx->mlp_piv) gts::dev_free(idx->mlp_piv);
     for (int i = 0; i < 2; i++)
         if (idx->fev[i]) cudaEventDestroy(idx->fev[i]);
     delete idx;
@@ -462,10 +462,10 @@ namespace {
 // Device scratch for the host-buffer entry points, freed on scope exit.
 struct DevBuf {
     void *p = nullptr;
-    ~DevBuf() { if (p) cudaFree(p); }
+    ~DevBuf() { if (p) gts::dev_free(p); }
     int alloc(size_t bytes)
     {
-        if (cudaMalloc(&p, bytes ? bytes : 1) != cudaSuccess) {
+        if (gts::dev_malloc(&p, bytes ? bytes : 1) != cudaSuccess) {
             cudaGetLastError();
             p = nullptr;
             gts_set_error("cudaMalloc of %zu bytes failed", bytes);

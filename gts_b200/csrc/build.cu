@@ -35,7 +35,7 @@ int dev_alloc(T **p, size_t n, size_t *acct)
 {
     *p = nullptr;
     if (n == 0) n = 1;
-    cudaError_t e = cudaMalloc((void **)p, n * sizeof(T));
+    cudaError_t e = dev_malloc((void **)p, n * sizeof(T));
     if (e != cudaSuccess) {
         cudaGetLastError();
         gts_set_error("cudaMalloc of %zu bytes failed: %s", n * sizeof(T), cudaGetErrorString(e));
@@ -298,10 +298,10 @@ static inline unsigned grid_for(size_t n, int block, unsigned cap = 148u * 32u)
 int ensure_scratch(gts_index *idx, size_t bytes)
 {
     if (idx->scratch_bytes >= bytes) return GTS_OK;
-    if (idx->scratch) cudaFree(idx->scratch);
+    if (idx->scratch) dev_free(idx->scratch);
     idx->scratch = nullptr;
     idx->scratch_bytes = 0;
-    if (cudaMalloc(&idx->scratch, bytes) != cudaSuccess) {
+    if (dev_malloc(&idx->scratch, bytes) != cudaSuccess) {
         cudaGetLastError();
         idx->scratch = nullptr;
         gts_set_error("cudaMalloc of %zu bytes of search scratch failed", bytes);
@@ -314,11 +314,11 @@ int ensure_scratch(gts_index *idx, size_t bytes)
 int ensure_io(gts_index *idx, size_t bytes)
 {
     if (bytes <= idx->io_bytes) return GTS_OK;
-    if (idx->io) cudaFree(idx->io);
+    if (idx->io) dev_free(idx->io);
     idx->io = nullptr;
     idx->io_bytes = 0;
     size_t want = bytes + bytes / 4 + 4096;
-    if (cudaMalloc(&idx->io, want) != cudaSuccess) {
+    if (dev_malloc(&idx->io, want) != cudaSuccess) {
         cudaGetLastError();
         idx->io = nullptr;
         gts_set_error("cudaMalloc of %zu bytes of argument buffers failed", want);
@@ -331,11 +331,11 @@ int ensure_io(gts_index *idx, size_t bytes)
 int ensure_hits(gts_index *idx, size_t bytes, void **out)
 {
     if (bytes > idx->hits_bytes) {
-        if (idx->hits) cudaFree(idx->hits);
+        if (idx->hits) dev_free(idx->hits);
         idx->hits = nullptr;
         idx->hits_bytes = 0;
         const size_t want = bytes + bytes / 4;
-        if (cudaMalloc(&idx->hits, want) != cudaSuccess) {
+        if (dev_malloc(&idx->hits, want) != cudaSuccess) {
             cudaGetLastError();
             idx->hits = nullptr;
             gts_set_error("cudaMalloc of %zu bytes for the hits failed", want);
@@ -349,7 +349,7 @@ int ensure_hits(gts_index *idx, size_t bytes, void **out)
 
 void free_tree(gts_index *idx)
 {
-    if (idx->fast_recs) cudaFree(idx->fast_recs);
+    if (idx->fast_recs) dev_free(idx->fast_recs);
     idx->fast_recs = nullptr;
     idx->fast_nb = 0;
     idx->fast_nsb = 0;
@@ -361,7 +361,7 @@ void free_tree(gts_index *idx)
                   idx->node_size, idx->node_lid, idx->node_pivot, idx->node_min_dis,
                   idx->node_flags, idx->cut_node, idx->cut_anc, idx->cut_anc_idx, idx->tnorm, idx->node_rec};
     for (void *p : ps)
-        if (p) cudaFree(p);
+        if (p) dev_free(p);
     idx->trows = nullptr; idx->tstrs = nullptr; idx->tlens = nullptr; idx->tsig = nullptr; idx->tpack = nullptr;
     idx->id_list = nullptr; idx->pos_of_id = nullptr; idx->node_pid = nullptr;
     idx->node_size = nullptr; idx->node_lid = nullptr; idx->node_pivot = nullptr;
@@ -374,9 +374,9 @@ void free_tree(gts_index *idx)
 void free_data(gts_index *idx)
 {
     graph_invalidate(idx);   // the captured filter pass reads the rows
-    if (idx->rows) cudaFree(idx->rows);
-    if (idx->strs) cudaFree(idx->strs);
-    if (idx->lens) cudaFree(idx->lens);
+    if (idx->rows) dev_free(idx->rows);
+    if (idx->strs) dev_free(idx->strs);
+    if (idx->lens) dev_free(idx->lens);
     idx->rows = nullptr; idx->strs = nullptr; idx->lens = nullptr;
 }
 
@@ -391,7 +391,7 @@ struct BuildScratch {
     {
         void *ps[] = {node_of_pos, ids_alt, posv, posv_alt, nsplit, key, key_alt, split, temp};
         for (void *p : ps)
-            if (p) cudaFree(p);
+            if (p) dev_free(p);
     }
 };
 }  // namespace
@@ -453,7 +453,7 @@ static int build_tree_impl(gts_index *idx, cudaStream_t s)
     GTS_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, temp_lid, (uint32_t *)nullptr, (uint32_t *)nullptr,
                                                  sc.posv_alt, sc.posv, n, 0, lid_bits, s));
     temp_bytes = std::max(temp_bytes, temp_lid);
-    if (cudaMalloc(&sc.temp, temp_bytes ? temp_bytes : 1) != cudaSuccess) {
+    if (dev_malloc(&sc.temp, temp_bytes ? temp_bytes : 1) != cudaSuccess) {
         cudaGetLastError();
         gts_set_error("cudaMalloc of sort scratch (%zu bytes) failed", temp_bytes);
         return GTS_ERR_NOMEM;

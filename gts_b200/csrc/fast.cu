@@ -1894,7 +1894,7 @@ static int fast_prepare(gts_index *idx, cudaStream_t st)
         e = cudaErrorUnknown;
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
-        cudaFree(recs);
+        dev_free(recs);
         gts_set_error("filter records: %s", cudaGetErrorString(e));
         return GTS_ERR_CUDA;
     }
@@ -3022,14 +3022,14 @@ extern "C" int gts_fast_seeds(gts_index *idx, const int *qids, int qnum, int k, 
     int jk = 0;
     while ((1 << jk) < k) jk++;
     int *d = nullptr;
-    GTS_CUDA_TRY(cudaMalloc(&d, 2 * sizeof(int) * (size_t)qnum));
+    GTS_CUDA_TRY(gts::dev_malloc((void **)&d, 2 * sizeof(int) * (size_t)qnum));
     cudaError_t e = cudaMemcpy(d, qids, sizeof(int) * (size_t)qnum, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) {
         gts::k_fast_seed_get<<<(qnum + 255) / 256, 256>>>(d, qnum, bs.pos, bs.selfk, jk, d + qnum);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpy(seeds_out, d + qnum, sizeof(int) * (size_t)qnum, cudaMemcpyDeviceToHost);
-    cudaFree(d);
+    gts::dev_free(d);
     if (e != cudaSuccess) {
         gts_set_error("gts_fast_seeds: %s", cudaGetErrorString(e));
         return GTS_ERR_CUDA;

@@ -150,6 +150,11 @@ int sweep_range_ids(gts_index *idx, const int *d_qids, int qnum, float r, int *d
                     int *offsets_out, int *ids_out, float *dists_out, size_t capacity, size_t *total, int *done,
                     cudaStream_t s);
 
+// Device memory (memory.cu): as cudaMalloc / cudaFree, with freed blocks of
+// 1 MiB and more kept for the next request, up to a bound.
+cudaError_t dev_malloc(void **p, size_t bytes);
+void dev_free(void *p);
+
 template <typename T>
 int dev_alloc(T **p, size_t n, size_t *acct);
 
@@ -190,7 +195,7 @@ struct DevVec {
     ~DevVec()
     {
         for (int i = 0; i < n; i++)
-            if (ps[i]) cudaFree(ps[i]);
+            if (ps[i]) dev_free(ps[i]);
     }
     template <typename T>
     int alloc(T **p, size_t cnt)

@@ -709,10 +709,10 @@ static int run_split_phases(gts_index *idx, const SearchArgs &a0, int nt, cudaSt
     const size_t list_bytes = ((sizeof(int4) * (size_t)cap) + 255) & ~(size_t)255;
     const size_t need = 2 * list_bytes + 256;
     if (idx->split_bytes < need) {
-        if (idx->split_buf) cudaFree(idx->split_buf);
+        if (idx->split_buf) dev_free(idx->split_buf);
         idx->split_buf = nullptr;
         idx->split_bytes = 0;
-        if (cudaMalloc(&idx->split_buf, need) != cudaSuccess) {
+        if (dev_malloc(&idx->split_buf, need) != cudaSuccess) {
             cudaGetLastError();
             gts_set_error("cudaMalloc of %zu bytes for the work-item lists failed", need);
             return GTS_ERR_NOMEM;

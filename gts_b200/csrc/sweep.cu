@@ -1444,7 +1444,7 @@ int sweep_range_ids(gts_index *idx, const int *d_qids, int qnum, float r, int *d
     GTS_CUDA_TRY(cudaMemsetAsync(idx->d_stats, 0, kStatsN * sizeof(unsigned long long), st));
     struct Lists {   // longer lists than the run's own, freed on every way out
         void *p = nullptr;
-        ~Lists() { if (p) cudaFree(p); }
+        ~Lists() { if (p) dev_free(p); }
     } lists;
     int rc;
     GTS_CUDA_TRY(cudaMemsetAsync(b.s.ctr, 0, 64, st));
@@ -1462,9 +1462,9 @@ int sweep_range_ids(gts_index *idx, const int *d_qids, int qnum, float r, int *d
             const size_t list = sizeof(int) * (size_t)b.s.Qp * longest;
             if (b.bytes + 2 * list > search_budget(idx)) return GTS_OK;
             void *buf = nullptr;
-            if (lists.p) cudaFree(lists.p);
+            if (lists.p) dev_free(lists.p);
             lists.p = nullptr;
-            if (cudaMalloc(&buf, 2 * list) != cudaSuccess) {
+            if (dev_malloc(&buf, 2 * list) != cudaSuccess) {
                 cudaGetLastError();
                 return GTS_OK;
             }

@@ -111,7 +111,7 @@ struct DevScratch {
     ~DevScratch()
     {
         for (void *p : ps)
-            if (p) cudaFree(p);
+            if (p) dev_free(p);
     }
     template <typename T>
     int alloc(T **p, size_t n)
@@ -243,11 +243,11 @@ static int rebuild_on(gts_index *idx, const std::vector<int> &map, cudaStream_t 
         char *ns = nullptr;
         int *nl = nullptr;
         if ((rc = dev_alloc(&ns, (size_t)n_new * kStrStride, &acct))) return rc;
-        if ((rc = dev_alloc(&nl, (size_t)n_new, &acct))) { cudaFree(ns); return rc; }
+        if ((rc = dev_alloc(&nl, (size_t)n_new, &acct))) { dev_free(ns); return rc; }
         k_gather_strs<<<1184, 256, 0, s>>>(n_new, d_map, idx->strs, idx->lens, ns, nl);
         GTS_CUDA_TRY(cudaStreamSynchronize(s));
-        cudaFree(idx->strs);
-        cudaFree(idx->lens);
+        dev_free(idx->strs);
+        dev_free(idx->lens);
         idx->strs = ns;
         idx->lens = nl;
     } else {
@@ -255,7 +255,7 @@ static int rebuild_on(gts_index *idx, const std::vector<int> &map, cudaStream_t 
         if ((rc = dev_alloc(&nr, (size_t)n_new * idx->dim, &acct))) return rc;
         k_gather_rows<<<1184, 256, 0, s>>>(n_new, idx->dim, d_map, idx->rows, nr);
         GTS_CUDA_TRY(cudaStreamSynchronize(s));
-        cudaFree(idx->rows);
+        dev_free(idx->rows);
         idx->rows = nr;
     }
     free_tree(idx);
@@ -288,7 +288,7 @@ int update_run(gts_index *idx, const int *flags, const int *ids, int nops, float
         GTS_CUDA_TRY(cudaMemcpyAsync(all + (size_t)n_data * dim, new_rows, sizeof(float) * (size_t)n_new * dim,
                                      cudaMemcpyHostToDevice, s));
         GTS_CUDA_TRY(cudaStreamSynchronize(s));
-        cudaFree(idx->rows);
+        dev_free(idx->rows);
         idx->rows = all;
         free_tree(idx);
         idx->num = n_data + n_new;

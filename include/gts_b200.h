@@ -114,6 +114,14 @@ int gts_index_export(const gts_index *idx, int *id_list, int *pid, float *min_di
 
 void gts_index_free(gts_index *idx);
 
+/* No counterpart in the reference.  Blocks of device memory of 1 MiB and more
+ * that freed indexes (and grown work areas) no longer use are kept for the
+ * next index, up to 4 GiB per process, because the driver takes about a
+ * millisecond per block.  The library gives them back when one of its own
+ * allocations fails; this call gives them back now.  *bytes (nullable)
+ * receives how many there were. */
+int gts_memory_release(size_t *bytes);
+
 /* No counterpart in the reference (its only index is the tree).  Build
  * what a search form needs beyond the tree now, on `stream`, instead of in
  * the first search of that form: for GTS_FORM_FAST on an L2 index with
