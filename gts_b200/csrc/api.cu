@@ -383,6 +383,8 @@ extern "C" void gts_index_free(gts_index *idx)
     if (idx->split_buf) gts::dev_free(idx->split_buf);
     if (idx->io) gts::dev_free(idx->io);
     if (idx->hits) gts::dev_free(idx->hits);
+    if (idx->small_buf) gts::dev_free(idx->small_buf);
+    if (idx->small_result) cudaFreeHost(idx->small_result);
     for (int i = 0; i < gts_index::kGraphSlots; i++)
         if (idx->graph_exec[i]) cudaGraphExecDestroy(idx->graph_exec[i]);
     if (idx->graph_stream) cudaStreamDestroy(idx->graph_stream);
@@ -495,6 +497,9 @@ struct IoCarve {
     }
 };
 
+// Answers of at most this many bytes come back in one copy.
+constexpr long kCopyTogether = 32 << 10;
+
 int check_qids(const gts_index *idx, const int *qids, int qnum)
 {
     for (int i = 0; i < qnum; i++) {
@@ -539,6 +544,19 @@ extern "C" int gts_knn(gts_index *idx, const int *qids, int qnum, int k, int for
     GTS_CUDA_TRY(cudaMemcpyAsync(bq.p, qids, sizeof(int) * (size_t)qnum, cudaMemcpyHostToDevice, s));
     rc = gts::search_knn(idx, (int *)bq.p, qnum, k, form, (float *)bk.p, (int *)bi.p, (float *)bd.p, s);
     if (rc) return rc;
+    const size_t kk = sizeof(float) * (size_t)qnum * k;
+    const unsigned char *first = (const unsigned char *)bk.p;
+    const unsigned char *last = bd.p ? (unsigned char *)bd.p + kk : bi.p ? (unsigned char *)bi.p + kk : first;
+    if (last > first && last - first <= kCopyTogether) {
+        // small answers lie side by side: one copy, then apart
+        unsigned char tmp[kCopyTogether];
+        GTS_CUDA_TRY(cudaMemcpyAsync(tmp, first, (size_t)(last - first), cudaMemcpyDeviceToHost, s));
+        GTS_CUDA_TRY(cudaStreamSynchronize(s));
+        memcpy(kth_out, tmp, sizeof(float) * (size_t)qnum);
+        if (ids_out) memcpy(ids_out, tmp + ((unsigned char *)bi.p - first), kk);
+        if (dists_out) memcpy(dists_out, tmp + ((unsigned char *)bd.p - first), kk);
+        return GTS_OK;
+    }
     GTS_CUDA_TRY(cudaMemcpyAsync(kth_out, bk.p, sizeof(float) * (size_t)qnum, cudaMemcpyDeviceToHost, s));
     if (ids_out)
         GTS_CUDA_TRY(cudaMemcpyAsync(ids_out, bi.p, sizeof(int) * (size_t)qnum * k, cudaMemcpyDeviceToHost, s));

@@ -2324,8 +2324,18 @@ static int rerun_failed(gts_index *idx, FastCall &fc, const FastCfg &cfg, int st
         k_gather_i<<<(n + 255) / 256, 256, 0, st>>>(r2_prev, b.fail, n, b.sub_r2);
         idx->kernel_launches++;
     }
-    int rc;
-    if (stage < 2) {
+    int rc, n_small = n;
+    if (stage == 1 && fast_small_takes(idx, n)) {
+        // a few queries of a large batch: a tile pass of their own would cost
+        // as much as a fifth of the batch's
+        int *fail = nullptr;
+        if ((rc = fast_small_run(idx, b.sub_q, n, k, r2_prev ? b.sub_r2 : nullptr, b.sub_kth, sub_ids, sub_dis, &fail,
+                                 &n_small, false, st)))
+            return rc;
+    }
+    if (n_small == 0) {
+        // all answered
+    } else if (stage < 2) {
         int n2 = 0, *r2 = nullptr;
         // lists that overflowed (or pairs a block-stationary run could not
         // store) go through the tile filter, whose running bound tightens
@@ -2590,6 +2600,15 @@ int search_knn_fast(gts_index *idx, const int *d_qids, int qnum, int k, float *d
     int qc = 0;
     if ((rc = run_queries_for_budget(idx, qnum, [&](int q) { return rbytes_of(q) + 3 * bbytes_of(q); }, &qc)))
         return rc;
+    // a few queries do without tiles; those it leaves (rare) take the tiles
+    // with the rest
+    if (fast_small_takes(idx, qnum) && !idx->fast_pinned[k] && !idx->time_filter) {
+        int *fail = nullptr, n_fail = 0;
+        if ((rc = fast_small_run(idx, d_qids, qnum, k, nullptr, d_kth, d_ids, d_dists, &fail, &n_fail, true, st)))
+            return rc;
+        idx->last_fast_overflow = n_fail;
+        if (n_fail == 0) return GTS_OK;
+    }
     const size_t rbytes = rbytes_of(qc);
     const size_t bbytes = bbytes_of(qc);
     if ((rc = ensure_scratch(idx, rbytes + 3 * bbytes))) return rc;
@@ -2964,6 +2983,7 @@ extern "C" int gts_fast_config_set(gts_index *idx, int k, int learned, int col_g
         return GTS_ERR_INVALID;
     }
     idx->fast_cfg[k] = gts::cfg_pack(gts::FastCfg{learned != 0, col_groups, item_blocks, stream, blk});
+    idx->fast_pinned[k] = true;
     return GTS_OK;
 }
 
@@ -3044,5 +3064,6 @@ extern "C" int gts_fast_autotune_reset(gts_index *idx)
         return GTS_ERR_INVALID;
     }
     for (int &c : idx->fast_cfg) c = 0;
+    for (bool &b : idx->fast_pinned) b = false;
     return GTS_OK;
 }

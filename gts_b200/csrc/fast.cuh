@@ -181,6 +181,14 @@ int prune_blocks(const unsigned char *arec, const FastShape &fs, const FastSumma
                  int *bcnt, uint4 *bmask, int *bq_cnt, int item, int2 *fitems, int *fn_items, int fitems_cap,
                  unsigned long long *stats, int *status, cudaStream_t st);
 
+// kNN of at most kSmallMax queries without tiles (fast_small.cu): answers
+// those it can, lists the others' positions at *d_fail (valid until the next
+// call).  reset: clears the statistics first.
+constexpr int kSmallMax = 64;
+bool fast_small_takes(const gts_index *idx, int qnum);
+int fast_small_run(gts_index *idx, const int *d_qids, int qnum, int k, const int *d_carry, float *d_kth, int *d_ids,
+                   float *d_dists, int **d_fail, int *n_fail, bool reset, cudaStream_t st);
+
 // Result of the order construction, in the index's scratch: positions of
 // the final order (perm: position -> object id), the blocks as position
 // ranges, and the superblock starts (sb_start[pos] = 1 where a superblock

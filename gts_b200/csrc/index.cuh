@@ -73,6 +73,12 @@ struct gts_index {
     // grown on demand and kept, so those calls allocate nothing in steady state
     void *io = nullptr;
     size_t io_bytes = 0;
+    // the fast form's small batches (fast_small.cu): lists, and a result word
+    // in host memory; pinned configurations keep a k on the tiles
+    void *small_buf = nullptr;
+    size_t small_bytes = 0;
+    int *small_result = nullptr;
+    bool fast_pinned[65] = {};
     // hits of a range-ids run on their way to the host
     void *hits = nullptr;
     size_t hits_bytes = 0;

@@ -45,12 +45,10 @@ constexpr int kSwLd = kSwK + 4;        // row stride in shared memory (16-byte r
 constexpr int kSwList = 2048;          // pairs a tile may finish one by one
 constexpr int kSwWindow = 1024;        // objects around a query's place that bound its k-th distance
 constexpr int kSwMaxTiles = 32;        // query tiles per run
-constexpr int kSwCap = 2048;           // candidates listed per query
 constexpr int kSwSample = 16;          // the sample pass looks at every 16th row
 constexpr int kSwSampleMin = 1 << 16;  // objects from which on it pays
 constexpr int kSwRounds = 3;           // further passes over kNN queries whose lists overflowed
 constexpr int kSwHitCap = 16384;       // hits per query of a range-ids call at most
-constexpr float kSwTiny = 1e-36f;      // squares below this may have lost bits to underflow
 
 __device__ __forceinline__ void sw_cp16(void *dst, const void *src, int bytes)
 {
@@ -61,21 +59,6 @@ __device__ __forceinline__ void sw_cp4(void *dst, const void *src, int bytes)
 {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
-}
-
-// Upper / lower bound on the distance from a filter value, as value_bounds_f,
-// with the squares that underflow may have cut allowed for.
-__device__ __forceinline__ float sw_hi(int metric, int dim, float v)
-{
-    float lo, hi;
-    value_bounds_f(metric, dim, metric == kL2 ? v + kSwTiny : v, lo, hi);
-    return hi;
-}
-__device__ __forceinline__ float sw_lo(int metric, int dim, float v)
-{
-    float lo, hi;
-    value_bounds_f(metric, dim, metric == kL2 ? fmaxf(v - kSwTiny, 0.f) : v, lo, hi);
-    return lo;
 }
 
 // Sum over the CTA of a value per warp lane set (all threads get it).
@@ -92,50 +75,6 @@ __device__ __forceinline__ float cta_row_sum(float v, float *red, int metric)
 }
 
 // ---------------------------------------------------------------- seeds
-
-// k-th smallest (k >= 1) of n non-negative floats given as bits in keys: four
-// passes over their bytes.  All threads of the CTA call it and get the bits.
-__device__ __forceinline__ uint32_t cta_kth(const uint32_t *keys, int n, int k, int *hist)
-{
-    __shared__ uint32_t s_prefix;
-    __shared__ int s_rank;
-    uint32_t prefix = 0;
-    int rank = k;
-    for (int shift = 24; shift >= 0; shift -= 8) {
-        for (int i = threadIdx.x; i < 256; i += blockDim.x) hist[i] = 0;
-        __syncthreads();
-        const uint32_t mask = shift == 24 ? 0u : 0xffffffffu << (shift + 8);
-        for (int i = threadIdx.x; i < n; i += blockDim.x)
-            if ((keys[i] & mask) == prefix) atomicAdd(&hist[(keys[i] >> shift) & 255], 1);
-        __syncthreads();
-        if (threadIdx.x < 32) {
-            int c[8], sum = 0;
-#pragma unroll
-            for (int u = 0; u < 8; u++) sum += c[u] = hist[threadIdx.x * 8 + u];
-            int incl = sum;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                if ((int)threadIdx.x >= o) incl += y;
-            }
-            int run = incl - sum;
-            if (run < rank && rank <= incl)
-#pragma unroll
-                for (int u = 0; u < 8; u++) {
-                    if (run < rank && rank <= run + c[u]) {
-                        s_prefix = prefix | ((uint32_t)(threadIdx.x * 8 + u) << shift);
-                        s_rank = rank - run;
-                    }
-                    run += c[u];
-                }
-        }
-        __syncthreads();
-        prefix = s_prefix;
-        rank = s_rank;
-        __syncthreads();
-    }
-    return prefix;
-}
 
 __device__ __forceinline__ const float *sw_query_row(const SweepArgs &s, int q)
 {
@@ -843,88 +782,6 @@ __global__ void __launch_bounds__(kSwThreads, QI == 8 ? 2 : 3) k_sw_tile(SweepAr
 }
 
 // ---------------------------------------------------------------- exact values
-
-constexpr int kSwBatch = 8;   // candidates a warp evaluates side by side
-
-// The reference's value of up to kSwBatch rows against the query, row c's on
-// lane c: the lanes make the terms of 32 dimensions of each row (coalesced),
-// then lane c adds row c's in order.  F64 (kNN) or F32 (range) accumulation
-// as dist_row_f64 / dist_row_f32.
-template <bool F64>
-__device__ __forceinline__ double exact_batch(int metric, int dim, const float *const (&row)[kSwBatch], int n,
-                                              const float *q, double (*ts)[33], int lane)
-{
-    double r = 0.0;
-    float rf = 0.f;
-    for (int c0 = 0; c0 < dim; c0 += 32) {
-        const int j = c0 + lane;
-        const float y = j < dim ? q[j] : 0.f;
-        float x[kSwBatch];
-#pragma unroll
-        for (int c = 0; c < kSwBatch; c++) x[c] = c < n && j < dim ? __ldg(row[c] + j) : 0.f;
-#pragma unroll
-        for (int c = 0; c < kSwBatch; c++)
-            if (c < n) ts[c][lane] = metric == kL2 ? pow(x[c] - y, 2) : (double)fabsf(x[c] - y);
-        __syncwarp();
-        if (lane < n) {
-            const int m = min(32, dim - c0);
-            const double *e = ts[lane];
-            if (metric == kLinf) {
-                for (int u = 0; u < m; u++)
-                    if (e[u] > r) r = e[u];
-            } else if (F64) {
-                for (int u = 0; u < m; u++) r += e[u];
-            } else if (metric == kL2) {
-                for (int u = 0; u < m; u++) rf += e[u];
-            } else {
-                for (int u = 0; u < m; u++) rf += (float)e[u];
-            }
-        }
-        __syncwarp();
-    }
-    if (metric == kLinf) return r;
-    if (F64) return metric == kL2 ? pow(r, 0.5) : r;
-    if (metric == kL2) rf = pow(rf, 0.5);
-    return (double)rf;
-}
-
-struct FinalSmem {
-    double d[kSwCap];
-    int id[kSwCap];
-    uint32_t key[kSwCap];
-    int pos[kSwCap];
-    double ts[4][kSwBatch][33];
-    int hist[256];
-    int n;
-};
-
-// Ascending (distance, id) order of the first n entries.
-__device__ __forceinline__ void sort_hits(FinalSmem &s, int n)
-{
-    int p2 = 1;
-    while (p2 < n) p2 <<= 1;
-    for (int i = n + threadIdx.x; i < p2; i += blockDim.x) {
-        s.d[i] = DBL_MAX;
-        s.id[i] = INT_MAX;
-    }
-    __syncthreads();
-    for (int size = 2; size <= p2; size <<= 1)
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int i = threadIdx.x; i < p2 / 2; i += blockDim.x) {
-                const int lo = 2 * i - (i & (stride - 1)), hi = lo + stride;
-                const bool up = (lo & size) == 0;
-                const double dl = s.d[lo], dh = s.d[hi];
-                const int il = s.id[lo], ih = s.id[hi];
-                if (((dl > dh) || (dl == dh && il > ih)) == up) {
-                    s.d[lo] = dh;
-                    s.d[hi] = dl;
-                    s.id[lo] = ih;
-                    s.id[hi] = il;
-                }
-            }
-            __syncthreads();
-        }
-}
 
 // The answers of one query from its candidate list, one CTA of 128 threads
 // per sorted query.  kNN: candidates whose lower bound exceeds the k-th
