@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(128) k_small_final(SmallArgs a)
 {
     extern __shared__ __align__(16) unsigned char sm_smem[];
     FinalSmem &f = *reinterpret_cast<FinalSmem *>(sm_smem);
-    const int q = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, k = a.k;
+    const int q = blockIdx.x, tid = threadIdx.x, k = a.k;
     const int m = a.ccnt[q], nblk = a.nblk[q];
     const int qid = a.qids[q];
     const bool ok = qid >= 0 && qid < a.t.num;
@@ -180,20 +180,7 @@ __global__ void __launch_bounds__(128) k_small_final(SmallArgs a)
         __syncthreads();
         n = f.n;
         const float *qrow = a.t.rows + (size_t)qid * a.t.dim;
-        for (int b0 = warp * kSwBatch; b0 < n; b0 += 4 * kSwBatch) {
-            const int nb = min(kSwBatch, n - b0);
-            const float *row[kSwBatch];
-#pragma unroll
-            for (int c = 0; c < kSwBatch; c++) row[c] = a.bs.prow + (size_t)f.pos[b0 + min(c, nb - 1)] * a.kp;
-            const double d = exact_batch<true>(kL2, a.t.dim, row, nb, qrow, f.ts[warp], lane);
-            if (lane < nb) {
-                const int p = f.pos[b0 + lane];
-                f.d[b0 + lane] = p == self ? 0.0 : d;
-                f.id[b0 + lane] = a.bs.ids[p];
-            }
-        }
-        __syncthreads();
-        sort_hits(f, n);
+        exact_knn(f, kL2, a.t.dim, a.bs.prow, (size_t)a.kp, a.bs.ids, self, qrow, n, k);
         for (int j = tid; j < k; j += 128) {
             const bool have = j < n;
             if (a.ids) a.ids[(size_t)q * k + j] = have ? f.id[j] : -1;

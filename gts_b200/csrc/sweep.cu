@@ -849,22 +849,21 @@ __global__ void __launch_bounds__(128) k_sw_final(SweepArgs s)
     }
     __syncthreads();
     const int n = f.n;
-    if (t.metric != kAngle) {
+    if (mode == kModeKnn && t.metric != kAngle) {
+        exact_knn(f, t.metric, t.dim, t.trows, (size_t)t.dim, t.id_list, self, qrow, n, k);
+        if (tid == 0 && s.a.stats) atomicAdd(&s.a.stats[2], (unsigned long long)n);
+    } else if (mode != kModeKnn && t.metric != kAngle) {
         int wt = 0, wc = 0;
         for (int b0 = warp * kSwBatch; b0 < n; b0 += 4 * kSwBatch) {
             const int nb = min(kSwBatch, n - b0);
             const float *row[kSwBatch];
 #pragma unroll
             for (int c = 0; c < kSwBatch; c++) row[c] = t.trows + (size_t)f.pos[b0 + min(c, nb - 1)] * t.dim;
-            double d = mode == kModeKnn ? exact_batch<true>(t.metric, t.dim, row, nb, qrow, f.ts[warp], lane)
-                                        : exact_batch<false>(t.metric, t.dim, row, nb, qrow, f.ts[warp], lane);
+            double d = range_batch(t.metric, t.dim, row, nb, qrow, f.ts[warp], lane);
             if (lane < nb) {
                 const int p = f.pos[b0 + lane], id = t.id_list[p];
                 if (p == self) d = 0.0;
-                if (mode == kModeKnn) {
-                    f.d[b0 + lane] = d;
-                    f.id[b0 + lane] = id;
-                } else if ((float)d <= s.a.r) {
+                if ((float)d <= s.a.r) {
                     if (mode == kModeRangeCount) {
                         wt++;
                     } else {
@@ -879,13 +878,11 @@ __global__ void __launch_bounds__(128) k_sw_final(SweepArgs s)
             }
         }
         if (tid == 0 && s.a.stats) atomicAdd(&s.a.stats[2], (unsigned long long)n);
-        if (mode == kModeRangeCount || mode == kModeRangeTimed) {
-            wt = __reduce_add_sync(0xffffffffu, wt);
-            wc = __reduce_add_sync(0xffffffffu, wc);
-            if (lane == 0) {
-                if (wt) atomicAdd(&s.cnt[i], wt);
-                if (wc) atomicAdd(&s.cnt2[i], wc);
-            }
+        wt = __reduce_add_sync(0xffffffffu, wt);
+        wc = __reduce_add_sync(0xffffffffu, wc);
+        if (lane == 0) {
+            if (wt) atomicAdd(&s.cnt[i], wt);
+            if (wc) atomicAdd(&s.cnt2[i], wc);
         }
         __syncthreads();
     }
@@ -897,7 +894,7 @@ __global__ void __launch_bounds__(128) k_sw_final(SweepArgs s)
         }
         return;
     }
-    sort_hits(f, n);
+    if (t.metric == kAngle) sort_hits(f, n);
     for (int j = tid; j < k; j += 128) {
         const bool have = j < n;
         if (s.a.ids) s.a.ids[(size_t)q * k + j] = have ? f.id[j] : -1;
@@ -937,7 +934,7 @@ __global__ void __launch_bounds__(256) k_sw_hits(SweepArgs s)
             const float *row[kSwBatch];
 #pragma unroll
             for (int c = 0; c < kSwBatch; c++) row[c] = t.trows + (size_t)__shfl_sync(0xffffffffu, p, c) * t.dim;
-            d = exact_batch<false>(t.metric, t.dim, row, nb, qrow, f.ts[warp], lane);
+            d = range_batch(t.metric, t.dim, row, nb, qrow, f.ts[warp], lane);
         }
         if (lane < nb) {
             if (p == self) d = 0.0;

@@ -103,12 +103,20 @@ constexpr int kSwBatch = 8;   // candidates a warp evaluates side by side
 // lane c: the lanes make the terms of 32 dimensions of each row (coalesced),
 // then lane c adds row c's in order.  F64 (kNN) or F32 (range) accumulation
 // as dist_row_f64 / dist_row_f32.
-template <bool F64>
+//
+// L2 terms: the reference's pow(e, 2) is within 2 ulp of the square, which is
+// exact in FP64 for a float e and costs a multiplication (pow: 0.5 per clock
+// and SM, which made it most of these kernels' time).  POW = false adds the
+// squares.  F64: the caller checks that the sums are clear of everything they
+// decide (l2_margin).  F32: a step whose FP64 sum comes within the terms'
+// error of a float rounding midpoint sets *risky: that row wants POW = true.
+template <bool F64, bool POW>
 __device__ __forceinline__ double exact_batch(int metric, int dim, const float *const (&row)[kSwBatch], int n,
-                                              const float *q, double (*ts)[33], int lane)
+                                              const float *q, double (*ts)[33], int lane, bool *risky)
 {
     double r = 0.0;
     float rf = 0.f;
+    bool risk = false;
     for (int c0 = 0; c0 < dim; c0 += 32) {
         const int j = c0 + lane;
         const float y = j < dim ? q[j] : 0.f;
@@ -117,7 +125,10 @@ __device__ __forceinline__ double exact_batch(int metric, int dim, const float *
         for (int c = 0; c < kSwBatch; c++) x[c] = c < n && j < dim ? __ldg(row[c] + j) : 0.f;
 #pragma unroll
         for (int c = 0; c < kSwBatch; c++)
-            if (c < n) ts[c][lane] = metric == kL2 ? pow(x[c] - y, 2) : (double)fabsf(x[c] - y);
+            if (c < n) {
+                const float e = x[c] - y;
+                ts[c][lane] = metric != kL2 ? (double)fabsf(e) : (POW ? pow(e, 2) : (double)e * (double)e);
+            }
         __syncwarp();
         if (lane < n) {
             const int m = min(32, dim - c0);
@@ -126,19 +137,57 @@ __device__ __forceinline__ double exact_batch(int metric, int dim, const float *
                 for (int u = 0; u < m; u++)
                     if (e[u] > r) r = e[u];
             } else if (F64) {
+#pragma unroll 8
                 for (int u = 0; u < m; u++) r += e[u];
-            } else if (metric == kL2) {
+            } else if (metric == kL2 && POW) {
                 for (int u = 0; u < m; u++) rf += e[u];
+            } else if (metric == kL2) {
+#pragma unroll 4
+                for (int u = 0; u < m; u++) {
+                    const double s2 = (double)rf + e[u];
+                    const float f = __double2float_rn(s2);
+                    const double fd = f, up = (double)__int_as_float(__float_as_int(f) + (s2 > fd ? 1 : -1));
+                    if (s2 != fd && fabs(s2 - 0.5 * (fd + up)) <= e[u] * 8.9e-16 + s2 * 4.5e-16) risk = true;
+                    rf = f;
+                }
             } else {
                 for (int u = 0; u < m; u++) rf += (float)e[u];
             }
         }
         __syncwarp();
     }
+    *risky = risk;
     if (metric == kLinf) return r;
     if (F64) return metric == kL2 ? pow(r, 0.5) : r;
     if (metric == kL2) rf = pow(rf, 0.5);
     return (double)rf;
+}
+
+// The reference's range value of up to kSwBatch rows, row c's on lane c.
+__device__ __forceinline__ double range_batch(int metric, int dim, const float *const (&row)[kSwBatch], int n,
+                                              const float *q, double (*ts)[33], int lane)
+{
+    bool risky;
+    double d = exact_batch<false, false>(metric, dim, row, n, q, ts, lane, &risky);
+    if (__any_sync(0xffffffffu, risky)) d = exact_batch<false, true>(metric, dim, row, n, q, ts, lane, &risky);
+    return d;
+}
+
+// Relative distance within which two L2 values summed from exact squares may
+// differ from the reference's: 2 ulp per term and one rounding per addition,
+// halved by the root, with a factor above 2 to spare (1e-13 at dim 320).
+__device__ __forceinline__ double l2_margin(int dim) { return 3.2e-16 * (double)(dim + 8); }
+
+// Whether an L2 value d summed from exact squares may round to another float
+// than the reference's.
+__device__ __forceinline__ bool rounds_riskily(double d, double margin)
+{
+    if (d == 0.0) return false;   // all terms zero: exact
+    const float f = __double2float_rn(d);
+    const double fd = f, dl = d * margin;
+    const double hi = 0.5 * (fd + (double)__int_as_float(__float_as_int(f) + 1));
+    const double lo = 0.5 * (fd + (double)__int_as_float(__float_as_int(f) - 1));
+    return !(f > 0.f && d - dl > lo && d + dl < hi);
 }
 
 struct FinalSmem {
@@ -148,7 +197,7 @@ struct FinalSmem {
     int pos[kSwCap];
     double ts[4][kSwBatch][33];
     int hist[256];
-    int n;
+    int n, risk;
 };
 
 // Ascending (distance, id) order of the first n entries.
@@ -177,6 +226,49 @@ __device__ __forceinline__ void sort_hits(FinalSmem &s, int n)
             }
             __syncthreads();
         }
+}
+
+// kNN values of the n rows at f.pos (slots of `rows`, stride ld; ids of the
+// slots in ids; the query's own slot `self` at 0) into f.d / f.id, in
+// (distance, id) order.  128 threads.  L2 values come from exact squares
+// unless that could change a float or the order of the k nearest.
+__device__ __forceinline__ void exact_knn(FinalSmem &f, int metric, int dim, const float *rows, size_t ld,
+                                          const int *ids, int self, const float *q, int n, int k)
+{
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int per = min(kSwBatch, (n + 3) / 4);   // few rows: all four warps
+    const double margin = l2_margin(dim);
+    for (int pass = 0; pass < 2; pass++) {
+        if (tid == 0) f.risk = 0;
+        __syncthreads();
+        for (int b0 = warp * per; b0 < n; b0 += 4 * per) {
+            const int nb = min(per, n - b0);
+            const float *row[kSwBatch];
+#pragma unroll
+            for (int c = 0; c < kSwBatch; c++) row[c] = rows + (size_t)f.pos[b0 + min(c, nb - 1)] * ld;
+            bool risky;
+            double d = pass == 0 ? exact_batch<true, false>(metric, dim, row, nb, q, f.ts[warp], lane, &risky)
+                                 : exact_batch<true, true>(metric, dim, row, nb, q, f.ts[warp], lane, &risky);
+            if (lane < nb) {
+                const int p = f.pos[b0 + lane];
+                if (p == self) d = 0.0;
+                f.d[b0 + lane] = d;
+                f.id[b0 + lane] = ids[p];
+                if (pass == 0 && metric == kL2 && rounds_riskily(d, margin)) f.risk = 1;
+            }
+        }
+        __syncthreads();
+        sort_hits(f, n);
+        if (metric != kL2 || pass == 1) break;
+        for (int j = tid; j + 1 < n && j < k; j += 128) {
+            const double a = f.d[j], b = f.d[j + 1];
+            if (b != 0.0 && b - a <= (a + b) * margin) f.risk = 1;   // which comes first is open
+        }
+        __syncthreads();
+        const int again = f.risk;
+        __syncthreads();
+        if (!again) break;
+    }
 }
 
 // Ring bounds: the rows of the cut nodes that some query of each tile can
