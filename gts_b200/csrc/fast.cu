@@ -50,8 +50,8 @@
 #include <vector>
 #include "fast.cuh"
 #include "fast_blk.cuh"
-#include "search.cuh"
 #include "sm100.cuh"
+#include "sweep.cuh"
 
 namespace gts {
 
@@ -2715,6 +2715,7 @@ __global__ void __launch_bounds__(128) k_fast_range_final(const float *__restric
 {
     __shared__ int c;
     __shared__ __align__(16) float qs[kFMaxKp];
+    __shared__ double ts[4][kSwBatch][33];
     const int q = blockIdx.x, t = threadIdx.x;
     const int cnt = cand_cnt[q];
     if (cnt > kFCand) {
@@ -2727,6 +2728,12 @@ __global__ void __launch_bounds__(128) k_fast_range_final(const float *__restric
     __syncthreads();
     const int lane = t & 31, warp = t >> 5;
     constexpr int kR = 8;
+    static_assert(kR == kSwBatch, "the warp's rows are one exact batch");
+    // the reference's FP32 sum of dim terms is within (dim + 2) 2^-24 of the
+    // exact square, a warp-split sum (kp / 32 terms per lane, five levels)
+    // within (kp / 32 + 8) 2^-24; twice the second for the roots
+    const float g = ((float)(dim + 2) + 2.f * ((float)kp / 32.f + 8.f)) * 5.9604645e-8f;
+    const float vlow = r * r * (1.f - g) * (1.f - 6e-7f), vhigh = r * r * (1.f + g) * (1.f + 6e-7f);
     for (int i0 = warp * kR; i0 < cnt; i0 += 4 * kR) {
         int slot = 0, id = -1;
         if (lane < kR && i0 + lane < cnt) {
@@ -2743,16 +2750,23 @@ __global__ void __launch_bounds__(128) k_fast_range_final(const float *__restric
 #pragma unroll
         for (int u = 0; u < kR; u++)
             if (lane == u) mine = v[u];
+        bool in = false, open = false;
         if (lane < kR && id >= 0 && id < num) {
-            float lo, hi;
-            value_bounds_f(kL2, kp, mine, lo, hi);
-            bool in = false;
             if (id == qid) in = 0.f <= r;
-            else if (mine > 1e-30f && (double)hi < (double)r * (1.0 - 2.4e-7)) in = true;
-            else if (mine <= 1e-30f || !((double)lo > (double)r * (1.0 + 2.4e-7)))
-                in = dist_row_f32(prow + (size_t)slot * kp, qs, dim, kL2) <= r;
-            if (in) atomicAdd(&c, 1);
+            else if (mine > 1e-30f && mine < vlow) in = true;
+            else open = mine <= vhigh || mine <= 1e-30f;
         }
+        // the rows between the thresholds side by side, row c of them on lane c
+        const unsigned om = __ballot_sync(0xffffffffu, open);
+        if (om) {
+            const int n = __popc(om);
+            const float *row[kR];
+#pragma unroll
+            for (int u = 0; u < kR; u++) row[u] = prow + (size_t)__shfl_sync(0xffffffffu, slot, __fns(om, 0, min(u, n - 1) + 1)) * kp;
+            const float d = (float)range_batch(kL2, dim, row, n, qs, ts[warp], lane);
+            if (lane < n && d <= r) atomicAdd(&c, 1);
+        }
+        if (in) atomicAdd(&c, 1);
     }
     __syncthreads();
     if (t == 0) {

@@ -903,10 +903,35 @@ __global__ void __launch_bounds__(128) k_sw_final(SweepArgs s)
     if (tid == 0) s.a.kth[q] = n >= k ? (float)f.d[k - 1] : (float)t.infi_dis;
 }
 
-struct HitSmem {
-    double ts[8][kSwBatch][33];
-    int n, pad;
-};
+// Range ids: the reference's values of the listed objects, in place of the
+// filter's, eight rows per warp.  A query's batches are spread over
+// gridDim.x CTAs: hit numbers are uneven (58 on average, several hundred at
+// most on 50,000 x 300), and one CTA per query ended 0.3 ms after the rest.
+__global__ void __launch_bounds__(256) k_sw_hit_values(SweepArgs s)
+{
+    __shared__ double ts[8][kSwBatch][33];
+    const DevTree &t = s.a.t;
+    const int i = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int m = s.ccnt[i], self = s.self[i];
+    const int *cpos = s.cpos + (size_t)i * s.cap;
+    float *cv = s.cv + (size_t)i * s.cap;
+    const float *qrow = s.qrow + (size_t)i * s.ld;
+    for (int b0 = (blockIdx.x * 8 + warp) * kSwBatch; b0 < m; b0 += gridDim.x * 8 * kSwBatch) {
+        const int nb = min(kSwBatch, m - b0);
+        const int p = cpos[b0 + min(lane, nb - 1)];
+        float d;
+        if (t.metric == kAngle) {   // the value is exact already
+            d = angle_of_cos_f32(cv[b0 + min(lane, nb - 1)]);
+        } else {
+            const float *row[kSwBatch];
+#pragma unroll
+            for (int c = 0; c < kSwBatch; c++) row[c] = t.trows + (size_t)__shfl_sync(0xffffffffu, p, c) * t.dim;
+            d = (float)range_batch(t.metric, t.dim, row, nb, qrow, ts[warp], lane);
+        }
+        __syncwarp();
+        if (lane < nb) cv[b0 + lane] = p == self ? 0.f : d;
+    }
+}
 
 // Range ids: the listed objects within r, in (distance, id) order, back into
 // the query's list as (id, value); their number to counts.  The keys sort as
@@ -914,36 +939,20 @@ struct HitSmem {
 __global__ void __launch_bounds__(256) k_sw_hits(SweepArgs s)
 {
     extern __shared__ __align__(16) unsigned char sw_smem[];
-    HitSmem &f = *reinterpret_cast<HitSmem *>(sw_smem);
-    unsigned long long *key = reinterpret_cast<unsigned long long *>(sw_smem + sizeof(HitSmem));
+    __shared__ int hits;
+    unsigned long long *key = reinterpret_cast<unsigned long long *>(sw_smem);
     const DevTree &t = s.a.t;
-    const int i = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int m = s.ccnt[i], self = s.self[i];
+    const int i = blockIdx.x, tid = threadIdx.x;
+    const int m = s.ccnt[i];
     int *cpos = s.cpos + (size_t)i * s.cap;
     float *cv = s.cv + (size_t)i * s.cap;
-    const float *qrow = s.qrow + (size_t)i * s.ld;
-    if (tid == 0) f.n = 0;
+    if (tid == 0) hits = 0;
     __syncthreads();
-    for (int b0 = warp * kSwBatch; b0 < m; b0 += 8 * kSwBatch) {
-        const int nb = min(kSwBatch, m - b0);
-        const int p = cpos[b0 + min(lane, nb - 1)];
-        double d;
-        if (t.metric == kAngle) {   // the value is exact already
-            d = (double)angle_of_cos_f32(cv[b0 + min(lane, nb - 1)]);
-        } else {
-            const float *row[kSwBatch];
-#pragma unroll
-            for (int c = 0; c < kSwBatch; c++) row[c] = t.trows + (size_t)__shfl_sync(0xffffffffu, p, c) * t.dim;
-            d = range_batch(t.metric, t.dim, row, nb, qrow, f.ts[warp], lane);
-        }
-        if (lane < nb) {
-            if (p == self) d = 0.0;
-            if ((float)d <= s.a.r)
-                key[atomicAdd(&f.n, 1)] = ((unsigned long long)__float_as_uint((float)d) << 32) | (unsigned)t.id_list[p];
-        }
-    }
+    for (int c = tid; c < m; c += 256)
+        if (cv[c] <= s.a.r)
+            key[atomicAdd(&hits, 1)] = ((unsigned long long)__float_as_uint(cv[c]) << 32) | (unsigned)t.id_list[cpos[c]];
     __syncthreads();
-    const int n = f.n;
+    const int n = hits;
     int p2 = 1;
     while (p2 < n) p2 <<= 1;
     for (int c = n + tid; c < p2; c += 256) key[c] = ~0ull;
@@ -1328,10 +1337,11 @@ int sweep_range_ids(gts_index *idx, const int *d_qids, int qnum, float r, int *d
             b.s.cv = (float *)((unsigned char *)buf + list);
             if ((rc = sweep_pass(idx, b.s, st))) return rc;
         }
-        const size_t hsm = sizeof(HitSmem) + sizeof(unsigned long long) * (size_t)pow2_at_least(longest);
+        k_sw_hit_values<<<dim3(std::min(16, (longest + 63) / 64), nq), 256, 0, st>>>(b.s);
+        const size_t hsm = sizeof(unsigned long long) * (size_t)pow2_at_least(longest);
         GTS_CUDA_TRY(cudaFuncSetAttribute(k_sw_hits, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsm));
         k_sw_hits<<<nq, 256, hsm, st>>>(b.s);
-        idx->kernel_launches += 2;
+        idx->kernel_launches += 3;
         GTS_CUDA_TRY(cudaGetLastError());
         GTS_CUDA_TRY(cudaMemcpyAsync(counts_out + q0, d_counts + q0, sizeof(int) * nq, cudaMemcpyDeviceToHost, st));
         GTS_CUDA_TRY(cudaStreamSynchronize(st));

@@ -99,6 +99,32 @@ __device__ __forceinline__ uint32_t cta_kth(const uint32_t *keys, int n, int k, 
 
 constexpr int kSwBatch = 8;   // candidates a warp evaluates side by side
 
+// One step of the F32 sites' sum, r = (float)((double)r + pow(e, 2)), as one
+// fused multiply-add: both round r + e^2 once, except that the reference's
+// FP64 sum carries up to 2 ulp of the term and its own rounding, so the two
+// may part where r + e^2 lies within 2^-50 of a float rounding midpoint.  The
+// remainder e^2 + (r - f) is known to 2^-23 of itself when r >= f / 2 (the
+// difference is then exact), which tells all but about 2^-19 of the steps
+// apart; the few steps whose square is the larger part go through FP64.
+__device__ __forceinline__ float add_square(float r, float e, bool &risk)
+{
+    const float f = fmaf(e, e, r);
+    if (r < 0.5f * f) {
+        const double t = (double)e * (double)e, s2 = (double)r + t;
+        const float g = __double2float_rn(s2);
+        const double gd = g, up = (double)__int_as_float(__float_as_int(g) + (s2 > gd ? 1 : -1));
+        if (s2 != gd && fabs(s2 - 0.5 * (gd + up)) <= t * 8.9e-16 + s2 * 4.5e-16) risk = true;
+        return g;
+    }
+    const float rem = fabsf(fmaf(e, e, r - f));
+    const int bits = __float_as_int(f);
+    const float half = __int_as_float((bits & 0x7f800000) - (24 << 23));   // half an ulp of f
+    // below 2^-90 or past the floats the remainder is not reliable; at a power
+    // of two the spacing below is half as wide
+    if (fabsf(rem - half) <= half * 3e-6f || (e != 0.f && ((bits & 0x7fffff) == 0 || !(f > 1e-27f && f < 3e38f)))) risk = risk || e != 0.f;
+    return f;
+}
+
 // The reference's value of up to kSwBatch rows against the query, row c's on
 // lane c: the lanes make the terms of 32 dimensions of each row (coalesced),
 // then lane c adds row c's in order.  F64 (kNN) or F32 (range) accumulation
@@ -108,8 +134,8 @@ constexpr int kSwBatch = 8;   // candidates a warp evaluates side by side
 // exact in FP64 for a float e and costs a multiplication (pow: 0.5 per clock
 // and SM, which made it most of these kernels' time).  POW = false adds the
 // squares.  F64: the caller checks that the sums are clear of everything they
-// decide (l2_margin).  F32: a step whose FP64 sum comes within the terms'
-// error of a float rounding midpoint sets *risky: that row wants POW = true.
+// decide (l2_margin).  F32: see add_square; a step that may round differently
+// sets *risky: that row wants POW = true.
 template <bool F64, bool POW>
 __device__ __forceinline__ double exact_batch(int metric, int dim, const float *const (&row)[kSwBatch], int n,
                                               const float *q, double (*ts)[33], int lane, bool *risky)
@@ -117,41 +143,48 @@ __device__ __forceinline__ double exact_batch(int metric, int dim, const float *
     double r = 0.0;
     float rf = 0.f;
     bool risk = false;
-    for (int c0 = 0; c0 < dim; c0 += 32) {
-        const int j = c0 + lane;
-        const float y = j < dim ? q[j] : 0.f;
-        float x[kSwBatch];
+    float x[kSwBatch], y = lane < dim ? q[lane] : 0.f;
 #pragma unroll
-        for (int c = 0; c < kSwBatch; c++) x[c] = c < n && j < dim ? __ldg(row[c] + j) : 0.f;
+    for (int c = 0; c < kSwBatch; c++) x[c] = c < n && lane < dim ? __ldg(row[c] + lane) : 0.f;
+    for (int c0 = 0; c0 < dim; c0 += 32) {
 #pragma unroll
         for (int c = 0; c < kSwBatch; c++)
             if (c < n) {
                 const float e = x[c] - y;
-                ts[c][lane] = metric != kL2 ? (double)fabsf(e) : (POW ? pow(e, 2) : (double)e * (double)e);
+                if (!F64 && !POW) reinterpret_cast<float *>(ts[c])[lane] = metric == kL2 ? e : fabsf(e);
+                else ts[c][lane] = metric != kL2 ? (double)fabsf(e) : (POW ? pow(e, 2) : (double)e * (double)e);
             }
+        // the next 32 dimensions are on their way while lane c adds these
+        const int j = c0 + 32 + lane;
+        y = j < dim ? q[j] : 0.f;
+#pragma unroll
+        for (int c = 0; c < kSwBatch; c++) x[c] = c < n && j < dim ? __ldg(row[c] + j) : 0.f;
         __syncwarp();
         if (lane < n) {
             const int m = min(32, dim - c0);
-            const double *e = ts[lane];
-            if (metric == kLinf) {
-                for (int u = 0; u < m; u++)
-                    if (e[u] > r) r = e[u];
-            } else if (F64) {
-#pragma unroll 8
-                for (int u = 0; u < m; u++) r += e[u];
-            } else if (metric == kL2 && POW) {
-                for (int u = 0; u < m; u++) rf += e[u];
-            } else if (metric == kL2) {
+            if (!F64 && !POW) {
+                const float *e = reinterpret_cast<const float *>(ts[lane]);
+                if (metric == kL2) {
 #pragma unroll 4
-                for (int u = 0; u < m; u++) {
-                    const double s2 = (double)rf + e[u];
-                    const float f = __double2float_rn(s2);
-                    const double fd = f, up = (double)__int_as_float(__float_as_int(f) + (s2 > fd ? 1 : -1));
-                    if (s2 != fd && fabs(s2 - 0.5 * (fd + up)) <= e[u] * 8.9e-16 + s2 * 4.5e-16) risk = true;
-                    rf = f;
+                    for (int u = 0; u < m; u++) rf = add_square(rf, e[u], risk);
+                } else if (metric == kL1) {
+                    for (int u = 0; u < m; u++) rf += e[u];
+                } else {
+                    for (int u = 0; u < m; u++)
+                        if (e[u] > rf) rf = e[u];
                 }
+                r = rf;
             } else {
-                for (int u = 0; u < m; u++) rf += (float)e[u];
+                const double *e = ts[lane];
+                if (metric == kLinf) {
+                    for (int u = 0; u < m; u++)
+                        if (e[u] > r) r = e[u];
+                } else if (F64) {
+#pragma unroll 8
+                    for (int u = 0; u < m; u++) r += e[u];
+                } else {
+                    for (int u = 0; u < m; u++) rf += e[u];   // POW: L2
+                }
             }
         }
         __syncwarp();
