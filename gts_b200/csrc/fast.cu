@@ -2715,7 +2715,7 @@ __global__ void __launch_bounds__(128) k_fast_range_final(const float *__restric
 {
     __shared__ int c;
     __shared__ __align__(16) float qs[kFMaxKp];
-    __shared__ double ts[4][kSwBatch][33];
+    __shared__ float ts[4][8][33];
     const int q = blockIdx.x, t = threadIdx.x;
     const int cnt = cand_cnt[q];
     if (cnt > kFCand) {
@@ -2728,7 +2728,6 @@ __global__ void __launch_bounds__(128) k_fast_range_final(const float *__restric
     __syncthreads();
     const int lane = t & 31, warp = t >> 5;
     constexpr int kR = 8;
-    static_assert(kR == kSwBatch, "the warp's rows are one exact batch");
     // the reference's FP32 sum of dim terms is within (dim + 2) 2^-24 of the
     // exact square, a warp-split sum (kp / 32 terms per lane, five levels)
     // within (kp / 32 + 8) 2^-24; twice the second for the roots
@@ -2760,10 +2759,8 @@ __global__ void __launch_bounds__(128) k_fast_range_final(const float *__restric
         const unsigned om = __ballot_sync(0xffffffffu, open);
         if (om) {
             const int n = __popc(om);
-            const float *row[kR];
-#pragma unroll
-            for (int u = 0; u < kR; u++) row[u] = prow + (size_t)__shfl_sync(0xffffffffu, slot, __fns(om, 0, min(u, n - 1) + 1)) * kp;
-            const float d = (float)range_batch(kL2, dim, row, n, qs, ts[warp], lane);
+            const int at = __shfl_sync(0xffffffffu, slot, __fns(om, 0, min(lane, n - 1) + 1));
+            const float d = range_batch<kR>(kL2, dim, prow, (size_t)kp, at, n, qs, ts[warp], lane);
             if (lane < n && d <= r) atomicAdd(&c, 1);
         }
         if (in) atomicAdd(&c, 1);

@@ -854,16 +854,15 @@ __global__ void __launch_bounds__(128) k_sw_final(SweepArgs s)
         if (tid == 0 && s.a.stats) atomicAdd(&s.a.stats[2], (unsigned long long)n);
     } else if (mode != kModeKnn && t.metric != kAngle) {
         int wt = 0, wc = 0;
+        // the staged terms lie over the warp's part of ts
+        float(*ts)[33] = reinterpret_cast<float(*)[33]>(f.ts[warp]);
         for (int b0 = warp * kSwBatch; b0 < n; b0 += 4 * kSwBatch) {
-            const int nb = min(kSwBatch, n - b0);
-            const float *row[kSwBatch];
-#pragma unroll
-            for (int c = 0; c < kSwBatch; c++) row[c] = t.trows + (size_t)f.pos[b0 + min(c, nb - 1)] * t.dim;
-            double d = range_batch(t.metric, t.dim, row, nb, qrow, f.ts[warp], lane);
+            const int nb = min(kSwBatch, n - b0), p0 = f.pos[b0 + min(lane, nb - 1)];
+            float d = range_batch<kSwBatch>(t.metric, t.dim, t.trows, (size_t)t.dim, p0, nb, qrow, ts, lane);
             if (lane < nb) {
-                const int p = f.pos[b0 + lane], id = t.id_list[p];
-                if (p == self) d = 0.0;
-                if ((float)d <= s.a.r) {
+                const int p = p0, id = t.id_list[p];
+                if (p == self) d = 0.f;
+                if (d <= s.a.r) {
                     if (mode == kModeRangeCount) {
                         wt++;
                     } else {
@@ -904,30 +903,26 @@ __global__ void __launch_bounds__(128) k_sw_final(SweepArgs s)
 }
 
 // Range ids: the reference's values of the listed objects, in place of the
-// filter's, eight rows per warp.  A query's batches are spread over
-// gridDim.x CTAs: hit numbers are uneven (58 on average, several hundred at
-// most on 50,000 x 300), and one CTA per query ended 0.3 ms after the rest.
-__global__ void __launch_bounds__(256) k_sw_hit_values(SweepArgs s)
+// filter's, kHitBatch rows per warp and one warp per CTA: hit numbers are
+// uneven (58 on average, several hundred at most on 50,000 x 300), and idle
+// warps of a larger CTA would hold registers that other queries' batches want
+// (0.35 ms with eight warps, 0.37 with one CTA per query).
+constexpr int kHitBatch = 16;
+__global__ void __launch_bounds__(32) k_sw_hit_values(SweepArgs s)
 {
-    __shared__ double ts[8][kSwBatch][33];
+    __shared__ float ts[kHitBatch][33];
     const DevTree &t = s.a.t;
-    const int i = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = blockIdx.y, lane = threadIdx.x;
     const int m = s.ccnt[i], self = s.self[i];
     const int *cpos = s.cpos + (size_t)i * s.cap;
     float *cv = s.cv + (size_t)i * s.cap;
     const float *qrow = s.qrow + (size_t)i * s.ld;
-    for (int b0 = (blockIdx.x * 8 + warp) * kSwBatch; b0 < m; b0 += gridDim.x * 8 * kSwBatch) {
-        const int nb = min(kSwBatch, m - b0);
+    for (int b0 = blockIdx.x * kHitBatch; b0 < m; b0 += gridDim.x * kHitBatch) {
+        const int nb = min(kHitBatch, m - b0);
         const int p = cpos[b0 + min(lane, nb - 1)];
         float d;
-        if (t.metric == kAngle) {   // the value is exact already
-            d = angle_of_cos_f32(cv[b0 + min(lane, nb - 1)]);
-        } else {
-            const float *row[kSwBatch];
-#pragma unroll
-            for (int c = 0; c < kSwBatch; c++) row[c] = t.trows + (size_t)__shfl_sync(0xffffffffu, p, c) * t.dim;
-            d = (float)range_batch(t.metric, t.dim, row, nb, qrow, ts[warp], lane);
-        }
+        if (t.metric == kAngle) d = angle_of_cos_f32(cv[b0 + min(lane, nb - 1)]);   // the value is exact already
+        else d = range_batch<kHitBatch>(t.metric, t.dim, t.trows, (size_t)t.dim, p, nb, qrow, ts, lane);
         __syncwarp();
         if (lane < nb) cv[b0 + lane] = p == self ? 0.f : d;
     }
@@ -1337,7 +1332,7 @@ int sweep_range_ids(gts_index *idx, const int *d_qids, int qnum, float r, int *d
             b.s.cv = (float *)((unsigned char *)buf + list);
             if ((rc = sweep_pass(idx, b.s, st))) return rc;
         }
-        k_sw_hit_values<<<dim3(std::min(16, (longest + 63) / 64), nq), 256, 0, st>>>(b.s);
+        k_sw_hit_values<<<dim3(std::min(64, (longest + kHitBatch - 1) / kHitBatch), nq), 32, 0, st>>>(b.s);
         const size_t hsm = sizeof(unsigned long long) * (size_t)pow2_at_least(longest);
         GTS_CUDA_TRY(cudaFuncSetAttribute(k_sw_hits, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsm));
         k_sw_hits<<<nq, 256, hsm, st>>>(b.s);

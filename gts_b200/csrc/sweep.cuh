@@ -99,50 +99,47 @@ __device__ __forceinline__ uint32_t cta_kth(const uint32_t *keys, int n, int k, 
 
 constexpr int kSwBatch = 8;   // candidates a warp evaluates side by side
 
-// One step of the F32 sites' sum, r = (float)((double)r + pow(e, 2)), as one
-// fused multiply-add: both round r + e^2 once, except that the reference's
-// FP64 sum carries up to 2 ulp of the term and its own rounding, so the two
-// may part where r + e^2 lies within 2^-50 of a float rounding midpoint.  The
-// remainder e^2 + (r - f) is known to 2^-23 of itself when r >= f / 2 (the
-// difference is then exact), which tells all but about 2^-19 of the steps
-// apart; the few steps whose square is the larger part go through FP64.
-__device__ __forceinline__ float add_square(float r, float e, bool &risk)
+// One step of the F32 sites' sum, r = (float)((double)r + pow(e, 2)).  pow is
+// within 2 ulp of the square, so this is one fused multiply-add unless the
+// exact sum lies next to a float rounding midpoint (the reference's FP64 sum
+// is within 2^-26 of half an ulp of the exact one).  The remainder r + e^2 - f
+// tells, in FP32: the difference of f and the larger of r and e^2 is exact, so
+// it is known to 2^-23 of itself.  Steps that come close (one in 10^5, mostly
+// squares of short differences) are done as written; an FP64 step's dependent
+// instructions take some 1,000 cycles.
+__device__ __forceinline__ float add_square(float r, float e)
 {
     const float f = fmaf(e, e, r);
+    float rem = fmaf(e, e, r - f);
     if (r < 0.5f * f) {
-        const double t = (double)e * (double)e, s2 = (double)r + t;
-        const float g = __double2float_rn(s2);
-        const double gd = g, up = (double)__int_as_float(__float_as_int(g) + (s2 > gd ? 1 : -1));
-        if (s2 != gd && fabs(s2 - 0.5 * (gd + up)) <= t * 8.9e-16 + s2 * 4.5e-16) risk = true;
-        return g;
+        const float p = e * e;
+        rem = ((p - f) + r) + fmaf(e, e, -p);
     }
-    const float rem = fabsf(fmaf(e, e, r - f));
     const int bits = __float_as_int(f);
     const float half = __int_as_float((bits & 0x7f800000) - (24 << 23));   // half an ulp of f
-    // below 2^-90 or past the floats the remainder is not reliable; at a power
+    // below 2^-60 or past the floats the remainder is not reliable; at a power
     // of two the spacing below is half as wide
-    if (fabsf(rem - half) <= half * 3e-6f || (e != 0.f && ((bits & 0x7fffff) == 0 || !(f > 1e-27f && f < 3e38f)))) risk = risk || e != 0.f;
+    if (fabsf(fabsf(rem) - half) <= half * 4e-7f || (bits & 0x7fffff) == 0 || !(f > 1e-18f && f < 3e38f)) {
+        if (e != 0.f || !(r == r)) r += pow(e, 2);
+        return r;
+    }
     return f;
 }
 
-// The reference's value of up to kSwBatch rows against the query, row c's on
-// lane c: the lanes make the terms of 32 dimensions of each row (coalesced),
-// then lane c adds row c's in order.  F64 (kNN) or F32 (range) accumulation
-// as dist_row_f64 / dist_row_f32.
+// The reference's kNN value (F64 accumulation, dist_row_f64) of up to
+// kSwBatch rows against the query, row c's on lane c: the lanes make the terms
+// of 32 dimensions of each row (coalesced), then lane c adds row c's in order.
 //
 // L2 terms: the reference's pow(e, 2) is within 2 ulp of the square, which is
 // exact in FP64 for a float e and costs a multiplication (pow: 0.5 per clock
 // and SM, which made it most of these kernels' time).  POW = false adds the
-// squares.  F64: the caller checks that the sums are clear of everything they
-// decide (l2_margin).  F32: see add_square; a step that may round differently
-// sets *risky: that row wants POW = true.
-template <bool F64, bool POW>
+// squares, and the caller checks that the sums are clear of everything they
+// decide (l2_margin).
+template <bool POW>
 __device__ __forceinline__ double exact_batch(int metric, int dim, const float *const (&row)[kSwBatch], int n,
-                                              const float *q, double (*ts)[33], int lane, bool *risky)
+                                              const float *q, double (*ts)[33], int lane)
 {
     double r = 0.0;
-    float rf = 0.f;
-    bool risk = false;
     float x[kSwBatch], y = lane < dim ? q[lane] : 0.f;
 #pragma unroll
     for (int c = 0; c < kSwBatch; c++) x[c] = c < n && lane < dim ? __ldg(row[c] + lane) : 0.f;
@@ -151,8 +148,7 @@ __device__ __forceinline__ double exact_batch(int metric, int dim, const float *
         for (int c = 0; c < kSwBatch; c++)
             if (c < n) {
                 const float e = x[c] - y;
-                if (!F64 && !POW) reinterpret_cast<float *>(ts[c])[lane] = metric == kL2 ? e : fabsf(e);
-                else ts[c][lane] = metric != kL2 ? (double)fabsf(e) : (POW ? pow(e, 2) : (double)e * (double)e);
+                ts[c][lane] = metric != kL2 ? (double)fabsf(e) : (POW ? pow(e, 2) : (double)e * (double)e);
             }
         // the next 32 dimensions are on their way while lane c adds these
         const int j = c0 + 32 + lane;
@@ -162,48 +158,67 @@ __device__ __forceinline__ double exact_batch(int metric, int dim, const float *
         __syncwarp();
         if (lane < n) {
             const int m = min(32, dim - c0);
-            if (!F64 && !POW) {
-                const float *e = reinterpret_cast<const float *>(ts[lane]);
-                if (metric == kL2) {
-#pragma unroll 4
-                    for (int u = 0; u < m; u++) rf = add_square(rf, e[u], risk);
-                } else if (metric == kL1) {
-                    for (int u = 0; u < m; u++) rf += e[u];
-                } else {
-                    for (int u = 0; u < m; u++)
-                        if (e[u] > rf) rf = e[u];
-                }
-                r = rf;
+            const double *e = ts[lane];
+            if (metric == kLinf) {
+                for (int u = 0; u < m; u++)
+                    if (e[u] > r) r = e[u];
             } else {
-                const double *e = ts[lane];
-                if (metric == kLinf) {
-                    for (int u = 0; u < m; u++)
-                        if (e[u] > r) r = e[u];
-                } else if (F64) {
 #pragma unroll 8
-                    for (int u = 0; u < m; u++) r += e[u];
-                } else {
-                    for (int u = 0; u < m; u++) rf += e[u];   // POW: L2
+                for (int u = 0; u < m; u++) r += e[u];
+            }
+        }
+        __syncwarp();
+    }
+    return metric == kL2 ? pow(r, 0.5) : r;
+}
+
+// The reference's range value (F32 accumulation, dist_row_f32) of up to NB
+// rows at positions pos (lane c's row: rows + pos * ld) against the query, on
+// lane c.  The sum is a chain of some 25 instructions a term, so as many
+// lanes as there are rows walk theirs side by side.
+template <int NB>
+__device__ __forceinline__ float range_batch(int metric, int dim, const float *rows, size_t ld, int pos, int n,
+                                             const float *q, float (*ts)[33], int lane)
+{
+    float r = 0.f, x[NB], y = lane < dim ? q[lane] : 0.f;
+    const float *row = rows + (size_t)pos * ld;
+    auto load = [&](int c0) {
+#pragma unroll
+        for (int c = 0; c < NB; c++) {
+            const float *p = reinterpret_cast<const float *>(
+                __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(row), c < n ? c : n - 1));
+            x[c] = c0 + lane < dim ? __ldg(p + c0 + lane) : 0.f;
+        }
+    };
+    load(0);
+    for (int c0 = 0; c0 < dim; c0 += 32) {
+#pragma unroll
+        for (int c = 0; c < NB; c++) ts[c][lane] = x[c] - y;
+        // the next 32 dimensions are on their way while the lanes add these
+        if (c0 + 32 < dim) {
+            y = c0 + 32 + lane < dim ? q[c0 + 32 + lane] : 0.f;
+            load(c0 + 32);
+        }
+        __syncwarp();
+        if (lane < n) {
+            const int m = min(32, dim - c0);
+            const float *e = ts[lane];
+            if (metric == kL2) {
+#pragma unroll 4
+                for (int u = 0; u < m; u++) r = add_square(r, e[u]);
+            } else if (metric == kL1) {
+                for (int u = 0; u < m; u++) r += fabsf(e[u]);
+            } else {
+                for (int u = 0; u < m; u++) {
+                    const float v = fabsf(e[u]);
+                    if (v > r) r = v;
                 }
             }
         }
         __syncwarp();
     }
-    *risky = risk;
-    if (metric == kLinf) return r;
-    if (F64) return metric == kL2 ? pow(r, 0.5) : r;
-    if (metric == kL2) rf = pow(rf, 0.5);
-    return (double)rf;
-}
-
-// The reference's range value of up to kSwBatch rows, row c's on lane c.
-__device__ __forceinline__ double range_batch(int metric, int dim, const float *const (&row)[kSwBatch], int n,
-                                              const float *q, double (*ts)[33], int lane)
-{
-    bool risky;
-    double d = exact_batch<false, false>(metric, dim, row, n, q, ts, lane, &risky);
-    if (__any_sync(0xffffffffu, risky)) d = exact_batch<false, true>(metric, dim, row, n, q, ts, lane, &risky);
-    return d;
+    if (metric == kL2) r = pow(r, 0.5);
+    return r;
 }
 
 // Relative distance within which two L2 values summed from exact squares may
@@ -279,9 +294,8 @@ __device__ __forceinline__ void exact_knn(FinalSmem &f, int metric, int dim, con
             const float *row[kSwBatch];
 #pragma unroll
             for (int c = 0; c < kSwBatch; c++) row[c] = rows + (size_t)f.pos[b0 + min(c, nb - 1)] * ld;
-            bool risky;
-            double d = pass == 0 ? exact_batch<true, false>(metric, dim, row, nb, q, f.ts[warp], lane, &risky)
-                                 : exact_batch<true, true>(metric, dim, row, nb, q, f.ts[warp], lane, &risky);
+            double d = pass == 0 ? exact_batch<false>(metric, dim, row, nb, q, f.ts[warp], lane)
+                                 : exact_batch<true>(metric, dim, row, nb, q, f.ts[warp], lane);
             if (lane < nb) {
                 const int p = f.pos[b0 + lane];
                 if (p == self) d = 0.0;
