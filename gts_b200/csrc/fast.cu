@@ -1577,15 +1577,6 @@ __global__ void __launch_bounds__(32 * kFinWarps) k_fast_final_warp(
     if (threadIdx.x == 0 && stats && nrechk) atomicAdd(&stats[2], nrechk);
 }
 
-__global__ void k_fast_keys(const int *qids, int qnum, const int *pos_of, int *keys, int *vals)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < qnum) {
-        keys[i] = pos_of[qids[i]] / kFB;
-        vals[i] = i;
-    }
-}
-
 // Query order of a filter run in one CTA (nb <= kOrderMaxNb): the queries
 // sorted by the block of their slot (keys), ties by query index -- the order
 // a stable sort gives.  A counting sort in shared memory: per-block counts,
@@ -1657,21 +1648,22 @@ __global__ void __launch_bounds__(kOrderThreads) k_fast_order(const int *__restr
     }
 }
 
-// The start of a kNN filter run in one launch.  Per query i: an empty
-// candidate list, the starting bound (carry, else FLT_MAX; with selfk, the
+// The start of a filter run in one launch.  Per query i: an empty
+// candidate list, the starting bound (carry, else start; with selfk, the
 // smaller of that and the seed table's bound for the k at column jk) and the
 // sort key (the block of the query's slot) with its index; over the grid:
 // the run's counters, the tiles' block counts and the superblock mask words
-// cleared, and the run counted in stats[6].
+// cleared, a range run's counts (rcnt) cleared, and the run counted in stats[6].
 __global__ void k_fast_begin(int qnum, const int *__restrict__ qids, const int *__restrict__ pos_of,
                              const int *__restrict__ selfk, int jk, const int *__restrict__ carry, int *cand_cnt,
                              int *r2_bits, int *keys, int *vals, int *ctr, int nctr, int *bcnt, int ntiles,
-                             uint32_t *sb_mask, int nmask, unsigned long long *stats)
+                             uint32_t *sb_mask, int nmask, int start, int *rcnt, unsigned long long *stats)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     if (i < qnum) {
         const int pos = pos_of[qids[i]];
-        int r2 = carry ? carry[i] : __float_as_int(FLT_MAX);
+        if (rcnt) rcnt[i] = 0;
+        int r2 = carry ? carry[i] : start;
         if (selfk) r2 = min(r2, selfk[(size_t)pos * kSelfK + jk]);   // non-negative floats order as ints
         cand_cnt[i] = 0;
         r2_bits[i] = r2;
@@ -1990,17 +1982,16 @@ static size_t plan_run(const gts_index *idx, int qnum, unsigned char *base, RunB
 
 // The tiles' needed superblocks, then their needed blocks (blist, bcnt;
 // bmask and bq_cnt for the block-stationary filter): on the tensor cores up
-// to kFResKp (fast_prune.cu), else with the FP32 pruning kernels.  cleared:
-// the superblock masks are zero already.  item > 0: the tensor-core path
-// also makes the tile filter's work items of `item` blocks (*listed = true);
+// to kFResKp (fast_prune.cu), else with the FP32 pruning kernels.  The
+// superblock masks are zero already.  item > 0: the tensor-core path also makes the tile filter's work items of `item` blocks (*listed = true);
 // otherwise the caller runs k_items.
 static int prune_enqueue(gts_index *idx, const FastShape &fs, const FastSummary &bs, const RunBufs &r, int ntiles,
-                         bool blk, bool cleared, int item, bool *listed, cudaStream_t st)
+                         bool blk, int item, bool *listed, cudaStream_t st)
 {
     const int nb = idx->fast_nb, nsb = idx->fast_nsb, nsbw = (nsb + 31) / 32;
     *listed = false;
     if (bs.cop && bs.scop && r.pbufs) {
-        int rc = prune_superblocks(r.arec, fs, bs, nsb, ntiles, r.r2, r.sb_mask, nsbw, !cleared, idx->d_status, st);
+        int rc = prune_superblocks(r.arec, fs, bs, nsb, ntiles, r.r2, r.sb_mask, nsbw, idx->d_status, st);
         if (!rc)
             rc = prune_blocks(r.arec, fs, bs, nb, ntiles, r.r2, r.sb_mask, nsbw, r.pbufs, r.ctr + 5, r.blist, r.bcnt,
                               blk ? r.bmask : nullptr, blk ? r.bq_cnt : nullptr, item, item > 0 ? r.items : nullptr,
@@ -2027,6 +2018,28 @@ static int prune_enqueue(gts_index *idx, const FastShape &fs, const FastSummary 
     GTS_CUDA_TRY(cudaGetLastError());
     return GTS_OK;
 }
+
+// The run's queries in the order of their blocks (r.keys -> r.order).
+static int order_enqueue(gts_index *idx, const RunBufs &r, int qnum, cudaStream_t st)
+{
+    const int nb = idx->fast_nb;
+    if (nb <= kOrderMaxNb) {
+        const size_t osmem = 2 * sizeof(int) * (size_t)nb;
+        GTS_CUDA_TRY(cudaFuncSetAttribute(k_fast_order, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)osmem));
+        k_fast_order<<<1, kOrderThreads, osmem, st>>>(r.keys, qnum, nb, r.order);
+        idx->kernel_launches++;
+    } else {
+        // block ids are below nb: sort only the bits they use
+        int key_bits = 1;
+        while (key_bits < 32 && (1ll << key_bits) < (long long)nb) key_bits++;
+        size_t cb = r.cub_bytes;
+        GTS_CUDA_TRY(cub::DeviceRadixSort::SortPairs(r.cub, cb, r.keys, r.skeys, r.vals, r.order, qnum, 0, key_bits,
+                                                     st));
+    }
+    return GTS_OK;
+}
+
+static constexpr int kFltMaxBits = 0x7f7fffff;
 
 // One filter run over a query batch.  learned: also seed each query's bound
 // from the learned radius model.  carry (nullable): certified starting bounds
@@ -2063,26 +2076,14 @@ static int fast_run_enqueue(gts_index *idx, const RunBufs &r, const int *d_qids,
     const int nsbw = (idx->fast_nsb + 31) / 32;
     k_fast_begin<<<(qnum + 255) / 256, 256, 0, st>>>(qnum, d_qids, bs.pos, learned ? nullptr : bs.selfk, jk, carry,
                                                      r.ccnt, r.r2, r.keys, r.vals, r.ctr, 8, r.bcnt, ntiles, r.sb_mask,
-                                                     ntiles * nsbw, idx->d_stats);
+                                                     ntiles * nsbw, kFltMaxBits, nullptr, idx->d_stats);
     idx->kernel_launches++;
     if (learned) {
         if ((rc = mlp_seed(idx, d_qids, qnum, k, r.r2, st))) return rc;
         k_fast_seed_tab<<<(qnum + 255) / 256, 256, 0, st>>>(d_qids, qnum, bs.pos, bs.selfk, jk, r.r2);
         idx->kernel_launches++;
     }
-    if (nb <= kOrderMaxNb) {
-        const size_t osmem = 2 * sizeof(int) * (size_t)nb;
-        GTS_CUDA_TRY(cudaFuncSetAttribute(k_fast_order, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)osmem));
-        k_fast_order<<<1, kOrderThreads, osmem, st>>>(r.keys, qnum, nb, r.order);
-        idx->kernel_launches++;
-    } else {
-        // block ids are below nb: sort only the bits they use
-        int key_bits = 1;
-        while (key_bits < 32 && (1ll << key_bits) < (long long)nb) key_bits++;
-        size_t cb = r.cub_bytes;
-        GTS_CUDA_TRY(cub::DeviceRadixSort::SortPairs(r.cub, cb, r.keys, r.skeys, r.vals, r.order, qnum, 0, key_bits,
-                                                     st));
-    }
+    if ((rc = order_enqueue(idx, r, qnum, st))) return rc;
     const bool blk = cfg.blk && r.bmask && fast_blk_stages(fs) >= 2;
     if (blk) {
         GTS_CUDA_TRY(cudaMemsetAsync(r.bq_cnt, 0, sizeof(int) * nb, st));
@@ -2091,7 +2092,7 @@ static int fast_run_enqueue(gts_index *idx, const RunBufs &r, const int *d_qids,
     k_fast_arec<<<ntiles, 128, 0, st>>>(idx->rows, d_qids, r.order, qnum, idx->dim, fs, r.arec, r.qt);
     idx->kernel_launches++;
     bool listed = false;   // the filter's work items already made by the pruning
-    if ((rc = prune_enqueue(idx, fs, bs, r, ntiles, blk, true, blk ? 0 : cfg.item, &listed, st))) return rc;
+    if ((rc = prune_enqueue(idx, fs, bs, r, ntiles, blk, blk ? 0 : cfg.item, &listed, st))) return rc;
     if (!blk && !listed) {
         k_items<<<(ntiles + 127) / 128, 128, 0, st>>>(ntiles, r.bcnt, nb, cfg.item, r.items, r.ctr + 2,
                                                       (int)plan_items_cap(ntiles, nb));
@@ -2389,7 +2390,7 @@ static int fast_search_graph(gts_index *idx, FastCall &fc, const FastCfg &cfg, c
     RunBufs r;
     plan_run(idx, qnum, fc.region, &r, cfg.blk);
     const long long key[8] = {qnum, k,
-                              cfg_pack(cfg) | (learned ? 1 << 16 : 0) | (timed ? 1 << 19 : 0),
+                              cfg_pack(cfg) | (learned ? 1 << 17 : 0) | (timed ? 1 << 19 : 0),
                               (long long)(uintptr_t)fc.region, (long long)(uintptr_t)idx->fast_recs,
                               (long long)(uintptr_t)d_qids, (long long)(uintptr_t)d_kth,
                               (long long)(uintptr_t)d_ids ^ ((long long)(uintptr_t)d_dists << 1)};
@@ -2682,16 +2683,6 @@ int search_knn_fast_fixed(gts_index *idx, const int *d_qids, int qnum, int k, fl
 
 // ---------------------------------------------------------------- range counts
 
-__global__ void k_fast_range_init(int qnum, int *cand_cnt, int *r2_bits, int *rcnt, int r2hi_bits)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < qnum) {
-        cand_cnt[i] = 0;
-        r2_bits[i] = r2hi_bits;
-        rcnt[i] = 0;
-    }
-}
-
 // One CTA per query: the listed (uncertain) objects count when the reference's
 // range value (searchIndexRnnV2's leaf: FP32 accumulation of pow terms, then
 // pow(., 0.5); the query itself at 0) is within r; the count adds to the
@@ -2813,31 +2804,29 @@ int search_range_fast(gts_index *idx, const int *d_qids, int qnum, float r, int 
     const FastSummary bs = fast_summary(idx->fast_recs, fs, nb, nsb, idx->num);
     GTS_CUDA_TRY(cudaMemsetAsync(idx->d_status, 0, sizeof(int), st));
     if (!idx->keep_stats) GTS_CUDA_TRY(cudaMemsetAsync(idx->d_stats, 0, kStatsN * sizeof(unsigned long long), st));
-    int key_bits = 1;
-    while (key_bits < 32 && (1ll << key_bits) < (long long)nb) key_bits++;
     for (int q0 = 0; q0 < qnum; q0 += qc) {
         const int n = std::min(qc, qnum - q0);
         const int *dq = d_qids + q0;
         const int ntiles = (n + kFT - 1) / kFT;
         RunBufs rb;
         plan_run(idx, n, region, &rb, blk);
-        k_fast_keys<<<(n + 255) / 256, 256, 0, st>>>(dq, n, bs.pos, rb.keys, rb.vals);
-        size_t cb = rb.cub_bytes;
-        GTS_CUDA_TRY(cub::DeviceRadixSort::SortPairs(rb.cub, cb, rb.keys, rb.skeys, rb.vals, rb.order, n, 0,
-                                                     key_bits, st));
-        k_fast_range_init<<<(n + 255) / 256, 256, 0, st>>>(n, rb.ccnt, rb.r2, rcnt, r2hi_bits);
-        GTS_CUDA_TRY(cudaMemsetAsync(rb.ctr, 0, 8 * sizeof(int), st));
-        GTS_CUDA_TRY(cudaMemsetAsync(rb.bcnt, 0, sizeof(int) * ntiles, st));
+        const int nsbw = (nsb + 31) / 32;
+        k_fast_begin<<<(n + 255) / 256, 256, 0, st>>>(n, dq, bs.pos, nullptr, 0, nullptr, rb.ccnt, rb.r2, rb.keys,
+                                                      rb.vals, rb.ctr, 8, rb.bcnt, ntiles, rb.sb_mask, ntiles * nsbw,
+                                                      r2hi_bits, rcnt, idx->d_stats);
+        if ((rc = order_enqueue(idx, rb, n, st))) return rc;
         if (blk) {
             GTS_CUDA_TRY(cudaMemsetAsync(rb.bq_cnt, 0, sizeof(int) * nb, st));
             GTS_CUDA_TRY(cudaMemsetAsync(rb.bq_fill, 0, sizeof(int) * nb, st));
         }
         k_fast_arec<<<ntiles, 128, 0, st>>>(idx->rows, dq, rb.order, n, idx->dim, fs, rb.arec, rb.qt);
         bool listed = false;
-        if ((rc = prune_enqueue(idx, fs, bs, rb, ntiles, blk, false, blk ? 0 : 16, &listed, st))) return rc;
-        if (!blk && !listed)
+        if ((rc = prune_enqueue(idx, fs, bs, rb, ntiles, blk, blk ? 0 : 16, &listed, st))) return rc;
+        if (!blk && !listed) {
             k_items<<<(ntiles + 127) / 128, 128, 0, st>>>(ntiles, rb.bcnt, nb, 16, rb.items, rb.ctr + 2,
                                                           (int)plan_items_cap(ntiles, nb));
+            idx->kernel_launches++;
+        }
         GTS_CUDA_TRY(cudaGetLastError());
         FastTileArgs a;
         a.recs = idx->fast_recs;
@@ -2901,14 +2890,13 @@ int search_range_fast(gts_index *idx, const int *d_qids, int qnum, float r, int 
             br.timed_end = timed ? idx->fev[1] : nullptr;
             br.capturing = false;
             if ((rc = fast_blk_enqueue(br, st, &idx->kernel_launches))) return rc;
-            idx->kernel_launches += 7;   // keys, init, arec, need_sb, need_blk, stat, final
         } else {
             if (timed) GTS_CUDA_TRY(cudaEventRecord(idx->fev[0], st));
             if ((rc = launch_fast_tile_ks<4, 8, true>(a, nsm, st))) return rc;
             if (timed) GTS_CUDA_TRY(cudaEventRecord(idx->fev[1], st));
-            idx->kernel_launches += 9;   // keys, init, arec, need_sb, need_blk, items, tile, stat, final
+            idx->kernel_launches++;
         }
-        k_add_stat<<<1, 1, 0, st>>>(idx->d_stats + 6, 1ull);
+        idx->kernel_launches += 3;   // begin, arec, final
         k_fast_range_final<<<n, 128, 0, st>>>(idx->rows, idx->dim, idx->num, bs.prow, fs.kp, bs.ids, nb * kFB, dq, r,
                                               rb.cpos, rb.ccnt, rcnt, d_counts + q0, fail, rb.ctr, idx->d_stats);
         GTS_CUDA_TRY(cudaGetLastError());

@@ -518,7 +518,7 @@ static int prune_grid(int total)
 }
 
 int prune_superblocks(const unsigned char *arec, const FastShape &fs, const FastSummary &bs, int nsb, int ntiles,
-                      const int *r2_bits, uint32_t *sb_mask, int nsbw, bool clear, int *status, cudaStream_t st)
+                      const int *r2_bits, uint32_t *sb_mask, int nsbw, int *status, cudaStream_t st)
 {
     PruneArgs a{};
     a.arec = arec;
@@ -534,8 +534,6 @@ int prune_superblocks(const unsigned char *arec, const FastShape &fs, const Fast
     a.sb_mask = sb_mask;
     a.nsbw = nsbw;
     a.status = status;
-    // the epilogue warps OR their balls into the mask words
-    if (clear) GTS_CUDA_TRY(cudaMemsetAsync(sb_mask, 0, sizeof(uint32_t) * (size_t)ntiles * nsbw, st));
     const size_t smem = prune_smem(fs);
     GTS_CUDA_TRY(cudaFuncSetAttribute(k_prune<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_prune<false><<<prune_grid(ntiles * a.ngroups), kPThreads, smem, st>>>(a);
