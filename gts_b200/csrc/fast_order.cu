@@ -22,8 +22,8 @@
 // ball lets the filter drop all of them with one test.
 //
 // Per level: plan (k-means or halving), centroid seeds at evenly spread
-// positions of the segment, kOrdIters Lloyd passes (one warp per object,
-// per-CTA shared-memory sums when a CTA's objects share a segment), a final
+// positions of the segment, kOrdIters Lloyd passes (one thread per object,
+// sums per CTA, segment and child), a final
 // pass that writes the sort key (segment, child) or (segment, projection),
 // a stable radix sort, and the child segments.
 #include <cub/device/device_radix_sort.cuh>
@@ -36,7 +36,9 @@ namespace gts {
 
 namespace {
 
-constexpr int kOAsgPos = 256;   // positions per assignment CTA (8 warps)
+constexpr int kOAsgPos = 256;         // positions (and threads) per assignment CTA
+constexpr int kOAsgK = 16;            // dimensions per stage
+constexpr int kOAsgLd = kOAsgK + 4;   // row stride in shared memory
 
 __device__ __forceinline__ uint32_t order_bits(float f)
 {
@@ -98,103 +100,192 @@ __global__ void k_o_seed(int nseg, int dim, const float *__restrict__ rows, cons
     }
 }
 
-// One warp per position.  Pass 0 (Lloyd): nearest centroid of the segment,
-// its sum and count.  Pass 1 (final): the sort key (segment << 32 | child)
-// for k-means segments, (segment << 32 | projection on c1 - c0) for halving
-// segments, (segment << 32) for leaves; counts of the k-means children.
-template <int NX>
-__global__ void __launch_bounds__(256) k_o_assign(int n, int dim, const float *__restrict__ rows,
-                                                  const int *__restrict__ perm, const int *__restrict__ sid,
-                                                  const int *__restrict__ kind, const int *__restrict__ kk,
-                                                  const int *__restrict__ cbase, const float *__restrict__ cent,
-                                                  float *__restrict__ csum, int *__restrict__ ccnt, int final_pass,
-                                                  unsigned long long *__restrict__ keys)
+// Copies of 16 or 4 bytes to shared memory, zeros where !live.
+__device__ __forceinline__ void cp_async16z(float *dst, const float *src, bool live)
 {
-    __shared__ float ssum[kOrdBranch * NX * 32];
-    __shared__ int scnt[kOrdBranch];
-    const int p0 = blockIdx.x * kOAsgPos, p1 = min(n, p0 + kOAsgPos);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int s0 = sid[p0];
-    const bool uni = !final_pass && sid[p1 - 1] == s0 && kind[s0] != 0;
-    const int K0 = uni ? kk[s0] : 0;
-    if (uni) {
-        for (int i = threadIdx.x; i < K0 * dim; i += blockDim.x) ssum[i] = 0.f;
-        if (threadIdx.x < K0) scnt[threadIdx.x] = 0;
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(live ? 16 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async4z(float *dst, const float *src, bool live)
+{
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(live ? 4 : 0) : "memory");
+}
+
+struct alignas(16) AsgSmem {   // the centroids behind it are read 16 bytes at a time
+    float x[2][kOAsgPos * kOAsgLd];   // staged dimensions of the positions' rows
+    int row[kOAsgPos];                // their rows, later ordered by child
+    int cnt[kOrdBranch], base[kOrdBranch + 1];
+    // followed by the centroids, [dimensions rounded up to kOAsgK / 4][kOrdBranch][4]
+};
+static_assert(sizeof(AsgSmem) % 16 == 0, "centroids on a 16-byte boundary");
+
+// acc[j] += squared differences of x and the KK centroids at c over the
+// staged dimensions; the constant layout leaves no address arithmetic.
+template <int KK>
+__device__ __forceinline__ void dist_add(const float *x, const float *c, float (&acc)[kOrdBranch])
+{
+#pragma unroll
+    for (int k = 0; k < kOAsgK; k += 4) {
+        const float4 a = *reinterpret_cast<const float4 *>(x + k);
+#pragma unroll
+        for (int j = 0; j < KK; j++) {
+            const float4 o = *reinterpret_cast<const float4 *>(c + k * kOrdBranch + 4 * j);
+            const float e0 = a.x - o.x, e1 = a.y - o.y, e2 = a.z - o.z, e3 = a.w - o.w;
+            acc[j] = fmaf(e3, e3, fmaf(e2, e2, fmaf(e1, e1, fmaf(e0, e0, acc[j]))));
+        }
     }
-    __syncthreads();
-    for (int pos = p0 + warp; pos < p1; pos += 8) {
-        const int s = sid[pos], kd = kind[s];
+}
+
+// kOAsgPos consecutive positions per CTA, segment by segment.  Pass 0
+// (Lloyd): nearest centroid of the segment, its sum and count.  Pass 1
+// (final): the sort key (segment << 32 | child) for k-means segments,
+// (segment << 32 | projection on c1 - c0) for halving segments, (segment
+// << 32) for leaves; counts of the k-means children.
+//
+// A thread holds one position's distances to all centroids: the rows come 16
+// dimensions at a time through shared memory (two stages, stride 20 floats,
+// free of bank conflicts; the first 64 bytes bring 256 to L2), the centroids'
+// reads are broadcasts.  The sums then read the rows again (from L2), ordered
+// by child: a warp adds 32 dimensions of a child's rows in registers, one
+// atomic addition each.  The rows' two reads (1 GB a pass at 1,000,000 x 128)
+// and their latency bound it; four CTAs an SM hide more of it than three with
+// more registers (11.1 against 11.8 ms over the 63 passes).  A pass there
+// with 16 children takes 320 us and one with 2 200, the whole order 11.1 ms
+// instead of 25.6 with a warp per position, bounded by 5 shuffles per position
+// and child, and atomic additions per position in segments below 512.
+// VEC: rows on 16-byte boundaries.
+template <bool VEC>
+__global__ void __launch_bounds__(kOAsgPos, 4) k_o_assign(int n, int dim, const float *__restrict__ rows,
+                                                          const int *__restrict__ perm, const int *__restrict__ sid,
+                                                          const int *__restrict__ sr, const int *__restrict__ kind,
+                                                          const int *__restrict__ kk, const int *__restrict__ cbase,
+                                                          const float *__restrict__ cent, float *__restrict__ csum,
+                                                          int *__restrict__ ccnt, int final_pass,
+                                                          unsigned long long *__restrict__ keys)
+{
+    extern __shared__ __align__(16) unsigned char asg_smem[];
+    AsgSmem &sm = *reinterpret_cast<AsgSmem *>(asg_smem);
+    const int nc = (dim + kOAsgK - 1) / kOAsgK, ldc = nc * kOAsgK;
+    float *cs = reinterpret_cast<float *>(asg_smem + sizeof(AsgSmem));
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int p1 = min(n, (int)(blockIdx.x + 1) * kOAsgPos);
+    for (int p = blockIdx.x * kOAsgPos, e; p < p1; p = e) {
+        const int s = sid[p], kd = kind[s];
+        e = min(p1, sr[s]);
+        const int m = e - p;
         if (kd == 0) {
-            if (final_pass && lane == 0) keys[pos] = (unsigned long long)s << 32;
+            if (final_pass && t < m) keys[p + t] = (unsigned long long)s << 32;
             continue;
         }
-        const float *xr = rows + (size_t)perm[pos] * dim;
-        float x[NX];
-#pragma unroll
-        for (int i = 0; i < NX; i++) {
-            const int d = lane + 32 * i;
-            x[i] = d < dim ? xr[d] : 0.f;
-        }
         const int K = kk[s], cb = cbase[s];
-        float best = FLT_MAX;
-        int bj = 0;
-        for (int j = 0; j < K; j++) {
-            const float *c = cent + (size_t)(cb + j) * dim;
-            float acc = 0.f;
+        const bool proj = final_pass && kd == 2;
+        __syncthreads();   // the previous segment's reads are done
+        if (t < m) sm.row[t] = perm[p + t];
+        if (t < kOrdBranch) sm.cnt[t] = 0;
+        for (int i = t; i < kOrdBranch * ldc; i += kOAsgPos) {
+            const int j = i / ldc, d = i - j * ldc;
+            float v = 0.f;
+            if (d < dim && j < K) {
+                v = cent[(size_t)(cb + j) * dim + d];
+                if (proj && j == 0) v = cent[(size_t)(cb + 1) * dim + d] - v;
+            }
+            cs[(d >> 2) * (4 * kOrdBranch) + 4 * j + (d & 3)] = v;
+        }
+        __syncthreads();
+        auto issue = [&](int ch) {
+            float *dst = sm.x[ch & 1];
+            const int k0 = ch * kOAsgK;
+            if (VEC) {
 #pragma unroll
-            for (int i = 0; i < NX; i++) {
-                const int d = lane + 32 * i;
-                if (d < dim) {
-                    const float e = x[i] - c[d];
-                    acc = fmaf(e, e, acc);
+                for (int u = 0; u < kOAsgK / 4; u++) {
+                    const int i = t + u * kOAsgPos, r = i / (kOAsgK / 4), d = k0 + 4 * (i % (kOAsgK / 4));
+                    if (r < m) {
+                        const bool live = d < dim;
+                        cp_async16z(dst + r * kOAsgLd + d - k0, rows + (size_t)sm.row[r] * dim + (live ? d : 0), live);
+                    }
+                }
+            } else {
+#pragma unroll 4
+                for (int u = 0; u < kOAsgK; u++) {
+                    const int i = t + u * kOAsgPos, r = i / kOAsgK, d = k0 + i % kOAsgK;
+                    if (r < m) {
+                        const bool live = d < dim;
+                        cp_async4z(dst + r * kOAsgLd + d - k0, rows + (size_t)sm.row[r] * dim + (live ? d : 0), live);
+                    }
                 }
             }
-            acc = warp_sum(acc);
-            if (acc < best) {
-                best = acc;
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        float acc[kOrdBranch];
+#pragma unroll
+        for (int j = 0; j < kOrdBranch; j++) acc[j] = 0.f;
+        issue(0);
+        for (int ch = 0; ch < nc; ch++) {
+            // the stage has come, and everyone is done with the other one
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            if (ch + 1 < nc) issue(ch + 1);
+            if (warp * 32 >= m) continue;
+            const float *x = sm.x[ch & 1] + t * kOAsgLd, *c = cs + ch * (kOAsgK * kOrdBranch);
+            if (proj) {
+#pragma unroll
+                for (int k = 0; k < kOAsgK; k += 4) {
+                    const float4 a = *reinterpret_cast<const float4 *>(x + k);
+                    const float4 o = *reinterpret_cast<const float4 *>(c + k * kOrdBranch);
+                    acc[0] = fmaf(a.w, o.w, fmaf(a.z, o.z, fmaf(a.y, o.y, fmaf(a.x, o.x, acc[0]))));
+                }
+            } else if (K <= 2) {
+                dist_add<2>(x, c, acc);
+            } else if (K <= 4) {
+                dist_add<4>(x, c, acc);
+            } else if (K <= 8) {
+                dist_add<8>(x, c, acc);
+            } else {
+                dist_add<kOrdBranch>(x, c, acc);
+            }
+        }
+        if (proj) {
+            if (t < m) keys[p + t] = ((unsigned long long)s << 32) | order_bits(acc[0]);
+            continue;
+        }
+        int bj = 0, at = 0;
+        float best = FLT_MAX;
+#pragma unroll
+        for (int j = 0; j < kOrdBranch; j++)
+            if (j < K && acc[j] < best) {
+                best = acc[j];
                 bj = j;
             }
+        const int row = t < m ? sm.row[t] : 0;
+        if (t < m) at = atomicAdd(&sm.cnt[bj], 1);
+        __syncthreads();
+        if (t < K && sm.cnt[t]) atomicAdd(&ccnt[cb + t], sm.cnt[t]);
+        if (final_pass) {
+            if (t < m) keys[p + t] = ((unsigned long long)s << 32) | (uint32_t)bj;
+            continue;
         }
-        if (!final_pass) {
-            if (uni) {
-#pragma unroll
-                for (int i = 0; i < NX; i++) {
-                    const int d = lane + 32 * i;
-                    if (d < dim) atomicAdd(&ssum[bj * dim + d], x[i]);
-                }
-                if (lane == 0) atomicAdd(&scnt[bj], 1);
-            } else {
-#pragma unroll
-                for (int i = 0; i < NX; i++) {
-                    const int d = lane + 32 * i;
-                    if (d < dim) atomicAdd(&csum[(size_t)(cb + bj) * dim + d], x[i]);
-                }
-                if (lane == 0) atomicAdd(&ccnt[cb + bj], 1);
-            }
-        } else {
-            uint32_t lo;
-            if (kd == 1) {
-                lo = (uint32_t)bj;
-                if (lane == 0) atomicAdd(&ccnt[cb + bj], 1);
-            } else {
-                const float *c0 = cent + (size_t)cb * dim, *c1 = c0 + dim;
-                float p = 0.f;
-#pragma unroll
-                for (int i = 0; i < NX; i++) {
-                    const int d = lane + 32 * i;
-                    if (d < dim) p = fmaf(x[i], c1[d] - c0[d], p);
-                }
-                lo = order_bits(warp_sum(p));
-            }
-            if (lane == 0) keys[pos] = ((unsigned long long)s << 32) | lo;
+        if (t <= kOrdBranch) {
+            int b = 0;
+            for (int j = 0; j < t; j++) b += sm.cnt[j];
+            sm.base[t] = b;
         }
-    }
-    __syncthreads();
-    if (uni) {
-        const int cb = cbase[s0];
-        for (int i = threadIdx.x; i < K0 * dim; i += blockDim.x)
-            if (scnt[i / dim]) atomicAdd(&csum[(size_t)cb * dim + i], ssum[i]);
-        if (threadIdx.x < K0 && scnt[threadIdx.x]) atomicAdd(&ccnt[cb + threadIdx.x], scnt[threadIdx.x]);
+        __syncthreads();
+        if (t < m) sm.row[sm.base[bj] + at] = row;
+        __syncthreads();
+        const int ng = (dim + 31) / 32;
+        for (int task = warp; task < 2 * ng; task += kOAsgPos / 32) {
+            const int d = (task >> 1) * 32 + lane, i0 = task & 1 ? m / 2 : 0, i1 = task & 1 ? m : m / 2;
+            for (int j = 0; j < K; j++) {
+                const int lo = max(sm.base[j], i0), hi = min(sm.base[j + 1], i1);
+                if (lo >= hi || d >= dim) continue;
+                float v = 0.f;
+#pragma unroll 8
+                for (int i = lo; i < hi; i++) v += rows[(size_t)sm.row[i] * dim + d];
+                atomicAdd(&csum[(size_t)(cb + j) * dim + d], v);
+            }
+        }
     }
 }
 
@@ -349,6 +440,16 @@ int fast_block_order(gts_index *idx, FastOrder *out, cudaStream_t st)
     if (n <= kOrdSbMax) GTS_CUDA_TRY(cudaMemsetAsync(sb_start, 1, 1, st));
     int nseg = 1, level = 0;
     const int agrid = (n + kOAsgPos - 1) / kOAsgPos;
+    const bool vec = dim % 4 == 0 && (uintptr_t)idx->rows % 16 == 0;
+    const size_t asmem = sizeof(AsgSmem) + sizeof(float) * kOrdBranch * ((dim + kOAsgK - 1) / kOAsgK * kOAsgK);
+    auto assign_fn = vec ? k_o_assign<true> : k_o_assign<false>;
+    GTS_CUDA_TRY(cudaFuncSetAttribute(assign_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)asmem));
+    auto assign = [&](int final_pass) {
+        assign_fn<<<agrid, kOAsgPos, asmem, st>>>(n, dim, idx->rows, perm, sid, sr, kind, kk, cbase, cent, csum, ccnt,
+                                                  final_pass, keys);
+        GTS_CUDA_TRY(cudaGetLastError());
+        return (int)GTS_OK;
+    };
     for (; level < kOrdMaxLevels; level++) {
         GTS_CUDA_TRY(cudaMemsetAsync(misc, 0, 2 * sizeof(int), st));
         k_o_plan<<<(nseg + 255) / 256, 256, 0, st>>>(nseg, sl, sr, force, kind, kk, misc);
@@ -369,21 +470,11 @@ int fast_block_order(gts_index *idx, FastOrder *out, cudaStream_t st)
         for (int it = 0; it < kOrdIters; it++) {
             GTS_CUDA_TRY(cudaMemsetAsync(csum, 0, sizeof(float) * (size_t)C * dim, st));
             GTS_CUDA_TRY(cudaMemsetAsync(ccnt, 0, sizeof(int) * (size_t)C, st));
-            if (dim <= kFResKp)
-                k_o_assign<kFResKp / 32><<<agrid, 256, 0, st>>>(n, dim, idx->rows, perm, sid, kind, kk, cbase, cent,
-                                                               csum, ccnt, 0, keys);
-            else
-                k_o_assign<kFMaxKp / 32><<<agrid, 256, 0, st>>>(n, dim, idx->rows, perm, sid, kind, kk, cbase, cent,
-                                                               csum, ccnt, 0, keys);
+            if ((rc = assign(0))) return rc;
             k_o_update<<<ugrid, 256, 0, st>>>(C, dim, csum, ccnt, cent);
         }
         GTS_CUDA_TRY(cudaMemsetAsync(ccnt, 0, sizeof(int) * (size_t)C, st));
-        if (dim <= kFResKp)
-            k_o_assign<kFResKp / 32><<<agrid, 256, 0, st>>>(n, dim, idx->rows, perm, sid, kind, kk, cbase, cent, csum,
-                                                           ccnt, 1, keys);
-        else
-            k_o_assign<kFMaxKp / 32><<<agrid, 256, 0, st>>>(n, dim, idx->rows, perm, sid, kind, kk, cbase, cent, csum,
-                                                           ccnt, 1, keys);
+        if ((rc = assign(1))) return rc;
         int sbits = 1;
         while ((1 << sbits) < nseg) sbits++;
         size_t tb3 = cub_bytes;

@@ -62,7 +62,7 @@ __device__ __forceinline__ void stage_rows(float *dst, const float *rows, int n,
 // the staged dimensions.
 __device__ __forceinline__ void tile_add(const float *a, const float *b, int tq, int to, float (&acc)[8][8])
 {
-#pragma unroll
+#pragma unroll 2   // fully unrolled the loop misses the instruction cache: 54.4 ms of seeds instead of 51.0
     for (int k = 0; k < kSdK; k += 4) {
         float4 o[8];
 #pragma unroll
@@ -143,8 +143,9 @@ struct SelfkSmem {
 // row's waiting values (a 64-value bitonic sort and merge) when 32 have come
 // or a value found no room, and the values without room try again.
 // Two CTAs fit an SM, so one merges while the other multiplies.  At
-// 1,000,000 x 128: 165 ms before (a warp per object, 4 pairs per lane, a
-// rank-by-counting merge at every block).
+// 1,000,000 x 128: 51 ms, of which the FP32 pipe needs 31 and the merges 5
+// (165 ms with a warp per object, 4 pairs per lane, a rank-by-counting merge
+// at every block).
 __global__ void __launch_bounds__(kSdThreads, 2) k_fast_selfk(FastSummary bs, int kp, const int *__restrict__ nbr)
 {
     extern __shared__ __align__(16) unsigned char sd_smem[];
@@ -183,15 +184,11 @@ __global__ void __launch_bounds__(kSdThreads, 2) k_fast_selfk(FastSummary bs, in
 #pragma unroll
             for (int c = 0; c < 8; c++) acc[q][c] = 0.f;
         for (int ch = 0; ch < nc; ch++, step++) {
-            if (step + 1 < steps) {
-                issue(step + 1);
-                asm volatile("cp.async.wait_group 1;" ::: "memory");
-            } else {
-                asm volatile("cp.async.wait_group 0;" ::: "memory");
-            }
+            // the stage has come, and everyone is done with the other one
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
             __syncthreads();
+            if (step + 1 < steps) issue(step + 1);
             tile_add(s.t.a[step & 1], s.t.b[step & 1], tq, to, acc);
-            __syncthreads();
         }
         // values that may rank: valid rows, below the row's 64th so far
         unsigned valid = 0;
@@ -293,15 +290,11 @@ __global__ void __launch_bounds__(kSdThreads, 1) k_fast_nbrs(FastSummary bs, int
 #pragma unroll
             for (int c = 0; c < 8; c++) acc[q][c] = 0.f;
         for (int ch = 0; ch < nc; ch++, step++) {
-            if (step + 1 < steps) {
-                issue(step + 1);
-                asm volatile("cp.async.wait_group 1;" ::: "memory");
-            } else {
-                asm volatile("cp.async.wait_group 0;" ::: "memory");
-            }
+            // the stage has come, and everyone is done with the other one
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
             __syncthreads();
+            if (step + 1 < steps) issue(step + 1);
             tile_add(s.t.a[step & 1], s.t.b[step & 1], tq, to, acc);
-            __syncthreads();
         }
         unsigned long long todo = 0;
 #pragma unroll
