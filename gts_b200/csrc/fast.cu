@@ -1881,7 +1881,8 @@ static int fast_prepare(gts_index *idx, cudaStream_t st)
     k_fast_sbprep<<<nsb, 256, 0, st>>>(idx->dim, idx->rows, fs, bs);
     // the seed table: neighbour blocks by centre, then per object the k-th
     // distances over its block and those
-    rc = seed_table_build(bs, nb, fs, st);
+    rc = ensure_scratch(idx, seed_table_scratch(nb, idx->num));   // the order's scratch is read and done
+    if (!rc) rc = seed_table_build(bs, nb, idx->num, fs, (int *)idx->scratch, st);
     cudaError_t e = rc ? cudaErrorUnknown : cudaSuccess;
     if (e == cudaSuccess && (prune_cop_build(bs.cen, nb, fs, bs.cop, st) || prune_cop_build(bs.sb_cen, nsb, fs, bs.scop, st)))
         e = cudaErrorUnknown;

@@ -161,8 +161,10 @@ inline FastSummary fast_summary(unsigned char *recs, const FastShape &fs, int nb
 }
 
 // The blocks' nearest centres (bs.nbr) and the seed table (bs.selfk) over
-// them, from the centres and the slot-ordered rows (fast_seed.cu).
-int seed_table_build(const FastSummary &bs, int nb, const FastShape &fs, cudaStream_t st);
+// them, from the centres and the slot-ordered rows (fast_seed.cu); scratch of
+// seed_table_scratch bytes.
+size_t seed_table_scratch(int nb, int num);
+int seed_table_build(const FastSummary &bs, int nb, int num, const FastShape &fs, int *scratch, cudaStream_t st);
 
 // The tiles' needed superblocks (zeroed mask words sb_mask[tile][nsbw]) and
 // then their needed blocks (blist[tile][..] in ascending order, counts in

@@ -35,6 +35,13 @@ constexpr int kSdPend = 64;            // values of one row waiting to be merged
 constexpr int kSdMergeAt = 32;         // merge a row's waiting values from this many on
 constexpr int kNbrKeep = 32;           // nearest centres kept per block (kSeedNbr of them used)
 constexpr int kNbrPend = 64;
+// Weak seeds: k = 2^kWkFirst on, more than 1.5 times (squared) the smallest of
+// the neighbourhood; at most one object in kWkShare is looked at again, over
+// its kWkBlocks nearest blocks.
+constexpr int kWkFirst = 3, kWkCols = kSelfKN - kWkFirst;
+constexpr float kWkRatio = 2.25f;
+constexpr int kWkShare = 64;
+constexpr int kWkBlocks = 8;
 
 static_assert(kSeedBest == 64 && kSdPend == 64 && kSeedNbr <= kNbrKeep, "list sizes");
 
@@ -362,9 +369,151 @@ __global__ void __launch_bounds__(256) k_fast_nbrs_merge(int nb, int slices, con
     if (lane < kSeedNbr) nbr[(size_t)b * kSeedNbr + lane] = best[lane] == ~0ull ? -1 : (int)(uint32_t)best[lane];
 }
 
+// Smallest seed of each block for k = 8 .. 64 (float bits).
+__global__ void __launch_bounds__(kFB) k_fast_seed_min(FastSummary bs, int *__restrict__ bmin)
+{
+    __shared__ int part[kFB / 32][kWkCols];
+    const int b = blockIdx.x, t = threadIdx.x, slot = b * kFB + t;
+    const bool live = bs.ids[slot] >= 0;
+#pragma unroll
+    for (int c = 0; c < kWkCols; c++) {
+        const int v = __reduce_min_sync(0xffffffffu, live ? bs.selfk[(size_t)slot * kSelfK + kWkFirst + c] : INT_MAX);
+        if ((t & 31) == 0) part[t >> 5][c] = v;
+    }
+    __syncthreads();
+    if (t < kWkCols) bmin[b * kWkCols + t] = min(min(part[0][t], part[1][t]), min(part[2][t], part[3][t]));
+}
+
+// Objects whose seed is far above the smallest of their block and its
+// neighbours (cnt counts them, the first cap are listed by slot).
+__global__ void __launch_bounds__(kFB) k_fast_weak_list(FastSummary bs, const int *__restrict__ bmin, int cap,
+                                                        int *__restrict__ list, int *__restrict__ cnt)
+{
+    __shared__ float ref[kWkCols];
+    const int b = blockIdx.x, t = threadIdx.x, lane = t & 31, slot = b * kFB + t;
+    static_assert(kSeedNbr == 31 && kWkCols == kFB / 32, "a warp per column, a lane per block");
+    const int j = lane < kSeedNbr ? bs.nbr[(size_t)b * kSeedNbr + lane] : b;
+    const int m = __reduce_min_sync(0xffffffffu, j >= 0 ? bmin[j * kWkCols + (t >> 5)] : INT_MAX);
+    if (lane == 0) ref[t >> 5] = __int_as_float(m);
+    __syncthreads();
+    if (bs.ids[slot] < 0) return;
+    bool weak = false;
+#pragma unroll
+    for (int c = 0; c < kWkCols; c++)
+        weak |= __int_as_float(bs.selfk[(size_t)slot * kSelfK + kWkFirst + c]) > kWkRatio * ref[c];
+    if (!weak) return;
+    const int at = atomicAdd(cnt, 1);
+    if (at < cap) list[at] = slot;
+}
+
+// Squared distance of x (shared, kp floats) to the rows at p and the next
+// three, ld apart, in every lane.
+__device__ __forceinline__ void dist4(const float *x, const float *p, size_t ld, int n, int kp, int lane, float (&s)[4])
+{
+#pragma unroll
+    for (int u = 0; u < 4; u++) s[u] = 0.f;
+    for (int d = 4 * lane; d < kp; d += 128) {
+        const float4 a = *reinterpret_cast<const float4 *>(x + d);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const float4 o = *reinterpret_cast<const float4 *>(p + (size_t)min(u, n - 1) * ld + d);
+            const float e0 = o.x - a.x, e1 = o.y - a.y, e2 = o.z - a.z, e3 = o.w - a.w;
+            s[u] = fmaf(e3, e3, fmaf(e2, e2, fmaf(e1, e1, fmaf(e0, e0, s[u]))));
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+#pragma unroll
+        for (int m = 16; m > 0; m >>= 1) s[u] += __shfl_xor_sync(0xffffffffu, s[u], m);
+}
+
+// Better seeds for the listed objects, one CTA each: the k-th distances over
+// the objects of the kWkBlocks blocks whose centres lie nearest to the object
+// itself.  A block that halving left across two groups has its neighbours
+// around its centre, so the few objects of the smaller group get seeds that
+// reach over half of the data: 2 of 10,000 queries at 1,000,000 x 128 made
+// 16,000 of the 33,500 (tile, block) entries of their filter run and 260 of
+// its 780 us.  The centres are read once per object (4.4 MB there, from L2),
+// a pass of about 20 us; 200 objects of that data are listed.
+__global__ void __launch_bounds__(kSdThreads) k_fast_weak(FastSummary bs, int nb, int kp, int cap,
+                                                          const int *__restrict__ list, const int *__restrict__ cnt)
+{
+    __shared__ __align__(16) float x[kFMaxKp];
+    __shared__ __align__(16) float d[kWkBlocks * kFB];
+    __shared__ unsigned long long key[8 * kWkBlocks];
+    __shared__ int sel[kWkBlocks];
+    static_assert(kSdThreads == 32 * 8 && kWkBlocks == 8, "a warp per chosen block");
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31, n = min(*cnt, cap);
+    for (int e = blockIdx.x; e < n; e += gridDim.x) {
+        const int slot = list[e];
+        __syncthreads();
+        for (int i = t; i < kp; i += kSdThreads) x[i] = bs.prow[(size_t)slot * kp + i];
+        __syncthreads();
+        // the warp's nearest centres, ascending over the lanes
+        unsigned long long mine = ~0ull;
+        for (int j0 = 4 * warp; j0 < nb; j0 += 32) {
+            float s[4];
+            dist4(x, bs.cen + (size_t)j0 * kp, kp, nb - j0, kp, lane, s);
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const unsigned long long v = ((unsigned long long)__float_as_uint(s[u]) << 32) | (unsigned)(j0 + u);
+                if (j0 + u >= nb || v >= __shfl_sync(0xffffffffu, mine, kWkBlocks - 1)) continue;
+                const int at = __popc(__ballot_sync(0xffffffffu, mine < v));
+                const unsigned long long up = __shfl_up_sync(0xffffffffu, mine, 1);
+                if (lane >= at) mine = lane == at ? v : up;
+            }
+        }
+        if (lane < kWkBlocks) key[warp * kWkBlocks + lane] = mine;
+        if (t < kWkBlocks) sel[t] = -1;
+        __syncthreads();
+        if (t < 8 * kWkBlocks && key[t] != ~0ull) {
+            int r = 0;
+            for (int i = 0; i < 8 * kWkBlocks; i++) r += key[i] < key[t];
+            if (r < kWkBlocks) sel[r] = (int)(uint32_t)key[t];
+        }
+        __syncthreads();
+        const int b = sel[warp];
+        for (int r = 0; r < kFB; r += 4) {
+            float s[4] = {FLT_MAX, FLT_MAX, FLT_MAX, FLT_MAX};
+            if (b >= 0) dist4(x, bs.prow + ((size_t)b * kFB + r) * kp, kp, 4, kp, lane, s);
+            if (lane < 4)
+                d[warp * kFB + r + lane] = b >= 0 && bs.ids[b * kFB + r + lane] >= 0
+                                               ? (lane == 0 ? s[0] : lane == 1 ? s[1] : lane == 2 ? s[2] : s[3])
+                                               : FLT_MAX;
+        }
+        __syncthreads();
+        // ranks, ties by position
+        float v[4];
+        int rk[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = d[t + u * kSdThreads];
+        for (int i = 0; i < kWkBlocks * kFB; i += 4) {
+            const float4 o = *reinterpret_cast<const float4 *>(d + i);
+            const float oo[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+            for (int w = 0; w < 4; w++)
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    rk[u] += oo[w] < v[u] || (oo[w] == v[u] && i + w < t + u * kSdThreads);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int k = rk[u] + 1;
+            if (k > kSeedBest || (k & (k - 1)) || !(v[u] < FLT_MAX)) continue;
+            int *out = bs.selfk + (size_t)slot * kSelfK + (31 - __clz(k));
+            *out = min(*out, __float_as_int(v[u] * (1.f + 4e-5f)));   // widened like every seed
+        }
+    }
+}
+
 }  // namespace
 
-int seed_table_build(const FastSummary &bs, int nb, const FastShape &fs, cudaStream_t st)
+size_t seed_table_scratch(int nb, int num)
+{
+    return sizeof(int) * ((size_t)nb * kWkCols + 1 + num / kWkShare + 1);
+}
+
+int seed_table_build(const FastSummary &bs, int nb, int num, const FastShape &fs, int *scratch, cudaStream_t st)
 {
     // slices of the centre tiles: enough CTAs for every SM; a slice writes
     // kNbrKeep keys per block into the seed table's own bytes (not made yet)
@@ -378,6 +527,12 @@ int seed_table_build(const FastSummary &bs, int nb, const FastShape &fs, cudaStr
     k_fast_nbrs<<<dim3(nt, slices), kSdThreads, sizeof(NbrSmem), st>>>(bs, nb, fs.kp, part);
     k_fast_nbrs_merge<<<(nb + 7) / 8, 256, 0, st>>>(nb, slices, part, bs.nbr);
     k_fast_selfk<<<nb, kSdThreads, sizeof(SelfkSmem), st>>>(bs, fs.kp, bs.nbr);
+    int *bmin = scratch, *cnt = bmin + (size_t)nb * kWkCols, *list = cnt + 1;
+    const int cap = num / kWkShare + 1;
+    GTS_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int), st));
+    k_fast_seed_min<<<nb, kFB, 0, st>>>(bs, bmin);
+    k_fast_weak_list<<<nb, kFB, 0, st>>>(bs, bmin, cap, list, cnt);
+    k_fast_weak<<<std::min(cap, 148 * 8), kSdThreads, 0, st>>>(bs, nb, fs.kp, cap, list, cnt);
     GTS_CUDA_TRY(cudaGetLastError());
     return GTS_OK;
 }
