@@ -645,6 +645,11 @@ constexpr size_t kStagedBytes = sizeof(int) + sizeof(float) + sizeof(unsigned sh
 // as a binary max-heap in shared memory, k per thread, each bound stored as
 // the upper 16 bits of its float rounded up (a bound again, 2 bytes).
 //
+// KH < 0: none; the query keeps the bound it came with (its seed).  Seeds that
+// lie next to the answer leave the kept bounds nothing to tighten: a thread
+// sees k objects below the seed only where a block holds most of the answer.
+// The autotuner measures both.  @@
+//
 // RANGE: range counts instead of kNN.  The bound stays the query's (r^2 with
 // the reference-arithmetic margin); objects certainly inside are counted per
 // thread, only the uncertain ones are listed; no bound heap.
@@ -662,6 +667,7 @@ __global__ void __launch_bounds__(128 * CG + 32, 1) k_fast_tile(FastTileArgs a)
     constexpr int NT = 128 * CG;   // epilogue threads
     constexpr int NEW = NT / 32;   // epilogue warps
     constexpr int CW = 128 / CG;   // object columns per thread
+    constexpr bool FLAT = RANGE || KH < 0;
     extern __shared__ __align__(1024) unsigned char fsm[];
     // 1024-byte aligned start (the swizzled operand layout needs it), as an
     // offset from the shared array so every access stays a shared-memory one
@@ -673,7 +679,7 @@ __global__ void __launch_bounds__(128 * CG + 32, 1) k_fast_tile(FastTileArgs a)
     // KS: chunk stages at B0 (1024-aligned), then the tail buffers
     unsigned char *T0 = B0 + (KS ? (size_t)a.nsc * kFChunkBytes : 0);
     unsigned short *heap = reinterpret_cast<unsigned short *>(KS ? T0 + kFS * kFTailPad : B0 + kFS * rec_pad);
-    FastCtl &ctl = *reinterpret_cast<FastCtl *>(heap + (KH > 0 ? 0 : NT * a.k));
+    FastCtl &ctl = *reinterpret_cast<FastCtl *>(heap + (KH != 0 ? 0 : NT * a.k));
     // staging area: a.st_cap entries (slot, lower bound, margin), pcap per
     // epilogue thread
     const int st_cap = a.st_cap, pcap = st_cap / NT;
@@ -919,7 +925,7 @@ __global__ void __launch_bounds__(128 * CG + 32, 1) k_fast_tile(FastTileArgs a)
             if constexpr (KH > 0) {
 #pragma unroll
                 for (int h = 0; h < KH; h++) hreg[h] = h < k ? FLT_MAX : -FLT_MAX;
-            } else {
+            } else if constexpr (KH == 0) {
                 for (int i = 0; i < k; i++) heap[i * NT + t] = 0x7f80u;   // +inf
             }
             // the query's bound as published so far (its seed, tightened by
@@ -943,7 +949,8 @@ __global__ void __launch_bounds__(128 * CG + 32, 1) k_fast_tile(FastTileArgs a)
                 // record tail visible here (KS: in the accumulator's tail buffer)
                 mbar_wait(KS ? &ctl.tfull[s] : &ctl.full[s], (uint32_t)((gi / kFS) & 1), kFWait);
                 // the bound the query's other column groups have reached
-                R2 = fminf(R2, __int_as_float(*(volatile const int *)&ctl.r2s[lq]));
+                if constexpr (!FLAT) R2 = fminf(R2, __int_as_float(*(volatile const int *)&ctl.r2s[lq]));
+                const float s2 = sqrtf(fmaxf(R2, 0.f)) * 1.000001f;
                 const float *tail = reinterpret_cast<const float *>(
                     KS ? T0 + (size_t)s * kFTailPad : B0 + (size_t)s * rec_pad + fs.btile_bytes);
                 const float *wv = tail + kTailW, *dn = tail + kTailDn;
@@ -962,25 +969,25 @@ __global__ void __launch_bounds__(128 * CG + 32, 1) k_fast_tile(FastTileArgs a)
                 const float ec = 2.f * kEpsC * eps_scale(fs.kp) * qn * cn + 1e-6f;
                 const float c2 = cn * cn;
                 const float qmc2 = q2 - 2.f * qc + c2;
-                const float A = 2.000004f * sqrtf(fmaxf(qmc2 + ec + 4e-6f * (q2 + c2), 0.f)) + 2e-6f * cn;
-                const float eb = ec + 2e-6f * q2 + cr * rb + 2e-6f * wb;
-                const float T = q2 - 2.f * qc - eb;
                 // ball test: |q - o| >= |q - c| - radius for every object, so a
                 // block entirely beyond the bound is skipped for this query (and
                 // by the whole warp when no lane of it needs the block)
-                const float dlo = sqrtf(fmaxf(qmc2 - ec - 4e-6f * (q2 + c2), 0.f)) * 0.999999f - brad;
-                const bool skip = qi < 0 || (dlo > 0.f && dlo * dlo * 0.999999f > R2);
+                const float reach = brad + s2;
+                const bool skip = qi < 0 || (qmc2 - ec - 4e-6f * (q2 + c2)) * 0.999998f > reach * reach;
                 const bool warp_skip = __all_sync(0xffffffffu, skip);
+                const float A = 2.000004f * sqrtf(fmaxf(qmc2 + ec + 4e-6f * (q2 + c2), 0.f)) + 2e-6f * cn;
+                const float eb = ec + 2e-6f * q2 + cr * rb + 2e-6f * wb;
+                const float T = q2 - 2.f * qc - eb;
 #pragma unroll 1
                 for (int c = g * CW; c < (g + 1) * CW && !warp_skip; c += 16) {
                     uint32_t r[16];
                     __syncwarp();   // tcgen05.ld is warp-collective: reconverge after the appends
                     tmem_ld16_nowait(taddr + (uint32_t)c, r);
                     tmem_wait_ld(r);
-                    uint32_t pass = 0, inside = 0;
-                    const float RT = R2 - T;
-                    // range: ub < r2lo, with the comparison's own rounding covered
-                    const float RLT = a.r2lo - T - 2e-6f * q2;
+                    // lb - T of every object (padding objects have w = +inf
+                    // and never pass); most batches end at the smallest
+                    const float RT = skip ? -FLT_MAX : R2 - T;
+                    float x[16], mn = FLT_MAX;
 #pragma unroll
                     for (int u4 = 0; u4 < 4; u4++) {
                         const float4 w4 = *reinterpret_cast<const float4 *>(wv + c + 4 * u4);
@@ -989,21 +996,29 @@ __global__ void __launch_bounds__(128 * CG + 32, 1) k_fast_tile(FastTileArgs a)
 #pragma unroll
                         for (int e = 0; e < 4; e++) {
                             const int u = 4 * u4 + e;
-                            // lb - T; padding objects have w = +inf and never pass
-                            const float x = fmaf(-2.f, __uint_as_float(r[u]), fmaf(-A, dq[e], wq[e]));
-                            pass |= (x <= RT ? 1u : 0u) << u;
-                            if constexpr (RANGE) inside |= (x + 2.f * fmaf(A, dq[e], eb) < RLT ? 1u : 0u) << u;
+                            x[u] = fmaf(-2.f, __uint_as_float(r[u]), fmaf(-A, dq[e], wq[e]));
+                            mn = fminf(mn, x[u]);
                         }
                     }
-                    if (skip) pass = inside = 0;
+                    if (!__any_sync(0xffffffffu, mn <= RT)) continue;
+                    uint32_t pass = 0;
+#pragma unroll
+                    for (int u = 0; u < 16; u++) pass |= (x[u] <= RT ? 1u : 0u) << u;
+                    if (skip) pass = 0;
                     if constexpr (RANGE) {
+                        // ub < r2lo, with the comparison's own rounding covered
+                        const float RLT = a.r2lo - T - 2e-6f * q2;
+                        uint32_t inside = 0;
+#pragma unroll
+                        for (int u = 0; u < 16; u++)
+                            inside |= (x[u] + 2.f * fmaf(A, dn[c + u], eb) < RLT ? 1u : 0u) << u;
+                        inside &= pass;
                         pass &= ~inside;
                         certain += __popc(inside);
                     }
                     // staging: each thread appends to its own slice of the
                     // staging area (entry e of thread t at e * NT + t), no
                     // atomics; past its slice, straight to the query's list
-                    if (!__any_sync(0xffffffffu, pass != 0)) continue;
                     if (!pass) continue;
                     appended += __popc(pass);
 #pragma unroll
@@ -1011,7 +1026,7 @@ __global__ void __launch_bounds__(128 * CG + 32, 1) k_fast_tile(FastTileArgs a)
                         if (!((pass >> u) & 1u)) continue;
                         const int jj = c + u;
                         const float dj = dn[jj];
-                        const float lb = T + fmaf(-2.f, __uint_as_float(r[u]), fmaf(-A, dj, wv[jj]));
+                        const float lb = T + x[u];
                         const float ub = lb + 2.f * fmaf(A, dj, eb);
                         const int slot = blk * kFB + jj;
                         if (nst < pcap) {
@@ -1028,7 +1043,7 @@ __global__ void __launch_bounds__(128 * CG + 32, 1) k_fast_tile(FastTileArgs a)
                                 a.cand_ub[(size_t)qi * kFCand + gsl] = ub;
                             }
                         }
-                        if (!RANGE && ub < R2) {   // replace the largest of the k kept bounds
+                        if (!FLAT && ub < R2) {   // replace the largest of the k kept bounds
                             float mx = -FLT_MAX;
                             if constexpr (KH > 0) {
                                 int mi = 0;
@@ -1069,7 +1084,7 @@ __global__ void __launch_bounds__(128 * CG + 32, 1) k_fast_tile(FastTileArgs a)
                     }
                 }
                 // k distinct objects' upper bounds bound the query's k-th d^2
-                if (!RANGE && qi >= 0 && hmx < pub) {
+                if (!FLAT && qi >= 0 && hmx < pub) {
                     atomicMin(a.r2_bits + qi, __float_as_int(fmaxf(hmx, 0.f)));
                     if (CG > 1) atomicMin(&ctl.r2s[lq], __float_as_int(fmaxf(hmx, 0.f)));
                     pub = hmx;
@@ -1715,24 +1730,26 @@ static int fast_cg(int k) { return k <= 32 ? 4 : 2; }
 // records streamed in K chunks (forced above kp = kFResKp) or resident --
 // or the block-stationary filter (blk; fast_blk.cu), which has no column
 // groups or items.  wfin: the light recheck one warp per query
-// (k_fast_final_warp, k <= kFinWarpK) instead of one CTA per query.
+// (k_fast_final_warp, k <= kFinWarpK) instead of one CTA per query.  flat: the
+// tile filter keeps the bound each query starts with.
 struct FastCfg {
     bool learned;
     int cg, item;
     bool stream;
     bool blk;
     bool wfin;
+    bool flat;
 };
 
 static int cfg_pack(const FastCfg &c)
 {
     return 1 | (c.learned ? 2 : 0) | (c.cg << 2) | (c.item << 8) | (c.stream ? 1 << 14 : 0) | (c.blk ? 1 << 15 : 0) |
-           (c.wfin ? 1 << 16 : 0);
+           (c.wfin ? 1 << 16 : 0) | (c.flat ? 1 << 17 : 0);
 }
 static FastCfg cfg_unpack(int v)
 {
     return FastCfg{(v & 2) != 0, (v >> 2) & 7, (v >> 8) & 63, (v & (1 << 14)) != 0, (v & (1 << 15)) != 0,
-                   (v & (1 << 16)) != 0};
+                   (v & (1 << 16)) != 0, (v & (1 << 17)) != 0};
 }
 
 // Filter variant of a configuration as the ABI reports it.
@@ -1828,8 +1845,9 @@ static int launch_fast_tile_ks(const FastTileArgs &a, int grid, cudaStream_t st)
                                            : launch_fast_tile_cg<CG, KH, RANGE, false>(a, grid, st);
 }
 
-static int launch_fast_tile(const FastTileArgs &a, int cg, int grid, cudaStream_t st)
+static int launch_fast_tile(const FastTileArgs &a, int cg, bool flat, int grid, cudaStream_t st)
 {
+    if (flat) return launch_fast_tile_ks<4, -1>(a, grid, st);
     // k <= 16: the k kept bounds live in registers
     if (a.k <= 8) {
         switch (cg) {
@@ -2167,7 +2185,7 @@ static int fast_run_enqueue(gts_index *idx, const RunBufs &r, const int *d_qids,
     } else {
         if (timed)
             GTS_CUDA_TRY(cudaEventRecordWithFlags(idx->fev[0], st, capturing ? cudaEventRecordExternal : 0));
-        if ((rc = launch_fast_tile(a, cfg.cg, nsm, st))) return rc;
+        if ((rc = launch_fast_tile(a, cfg.cg, cfg.flat, nsm, st))) return rc;
         idx->kernel_launches++;
         if (timed)
             GTS_CUDA_TRY(cudaEventRecordWithFlags(idx->fev[1], st, capturing ? cudaEventRecordExternal : 0));
@@ -2343,7 +2361,10 @@ static int rerun_failed(gts_index *idx, FastCall &fc, const FastCfg &cfg, int st
         // lists that overflowed (or pairs a block-stationary run could not
         // store) go through the tile filter, whose running bound tightens
         FastCfg c = cfg;
-        if (stage == 1) c.blk = false;
+        if (stage == 1) {
+            c.blk = c.flat = false;
+            c.cg = fast_default_cfg(idx, k).cg;
+        }
         if ((rc = fast_run(idx, fc.region, fc.region_bytes, b.sub_q, n, k, c, false,
                            stage == 1 && r2_prev ? b.sub_r2 : nullptr, b.sub_kth, sub_ids, sub_dis,
                            fc.book[stage + 1].fail, &n2, &r2, st)))
@@ -2391,7 +2412,7 @@ static int fast_search_graph(gts_index *idx, FastCall &fc, const FastCfg &cfg, c
     RunBufs r;
     plan_run(idx, qnum, fc.region, &r, cfg.blk);
     const long long key[8] = {qnum, k,
-                              cfg_pack(cfg) | (learned ? 1 << 17 : 0) | (timed ? 1 << 19 : 0),
+                              cfg_pack(cfg) | (learned ? 1 << 18 : 0) | (timed ? 1 << 19 : 0),
                               (long long)(uintptr_t)fc.region, (long long)(uintptr_t)idx->fast_recs,
                               (long long)(uintptr_t)d_qids, (long long)(uintptr_t)d_kth,
                               (long long)(uintptr_t)d_ids ^ ((long long)(uintptr_t)d_dists << 1)};
@@ -2521,6 +2542,10 @@ static int fast_autotune(gts_index *idx, FastCall &fc, int qc, const int *d_qids
     std::vector<FastCfg> cands;
     for (int learned = 0; learned <= (idx->mlp_ready ? 1 : 0); learned++) {
         if (fast_blk_stages(fs) >= 2) cands.push_back(FastCfg{learned != 0, fast_cg(k), 16, false, true});
+        for (int item = 8; item <= kFItemMax; item *= 2)
+            for (int stream = fs.kp > kFResKp ? 1 : 0; stream <= 1; stream++)
+                if (fast_tile_fits(fs, 4, 1, stream != 0))   // no heaps: k does not count
+                    cands.push_back(FastCfg{learned != 0, 4, item, stream != 0, false, false, true});
         for (int cg = 4; cg >= 1; cg >>= 1) {
             if (k > 16 && cg * k > 128) continue;   // heaps: 128 cg threads x k x 2 bytes <= 32 KB
             for (int item = 8; item <= kFItemMax; item *= 2)
@@ -2893,7 +2918,7 @@ int search_range_fast(gts_index *idx, const int *d_qids, int qnum, float r, int 
             if ((rc = fast_blk_enqueue(br, st, &idx->kernel_launches))) return rc;
         } else {
             if (timed) GTS_CUDA_TRY(cudaEventRecord(idx->fev[0], st));
-            if ((rc = launch_fast_tile_ks<4, 8, true>(a, nsm, st))) return rc;
+            if ((rc = launch_fast_tile_ks<4, -1, true>(a, nsm, st))) return rc;
             if (timed) GTS_CUDA_TRY(cudaEventRecord(idx->fev[1], st));
             idx->kernel_launches++;
         }
