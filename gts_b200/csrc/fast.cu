@@ -25,14 +25,14 @@
 //    reach within its seed are never copied or multiplied (GTS's pivot
 //    pruning, done with balls instead of rings).  The needed blocks of a
 //    tile become work items of up to 8-32 blocks (autotuned).
-//  * filter: a persistent CTA per SM takes work items.  One producer warp
+//  * filter: a persistent CTA per SM takes work items.  A copy warp
 //    streams the tile's query operand and the item's block records with
-//    bulk copies and issues a 128 x 144 x K MMA chain per block into one of
-//    two TMEM accumulators; 4 x CG epilogue warps turn each TMEM row into
+//    bulk copies, an MMA warp issues a 128 x 144 x K chain per block into one
+//    of three TMEM accumulators; 4 x CG epilogue warps turn each TMEM row into
 //    certified bounds lb <= d^2 <= ub for the 128 objects, keep the k
 //    smallest ub (a running k-th bound shared through global memory) and
 //    append every object with lb <= bound to the query's candidate list.
-//    Producer and epilogue meet only on mbarriers.
+//    They meet only on mbarriers.
 //  * recheck: the final bound is the k-th smallest candidate ub; candidates
 //    with lb <= bound get their reference-arithmetic distance (one warp per
 //    candidate) and the k best (distance, id) are the answer.
@@ -590,10 +590,10 @@ struct FastTileArgs {
     int stream;                  // streamed form also at kp <= kFResKp (autotuned)
 };
 
-constexpr int kFS = 3;         // block stages, each with its own TMEM accumulator
+constexpr int kFS = 3;         // TMEM accumulators, and stages of whole blocks
 constexpr int kFAccCols = 160; // TMEM columns between accumulators (kFN = 144 used)
 // Streamed form (kp > kFResKp): K-chunk stages (a.nsc of them, at most
-// kFSCMax) and, per accumulator, the block's record tail in its own buffer.
+// kFSCMax).  Per accumulator, the block's record tail has its own buffer.
 constexpr int kFSCMax = 6;
 constexpr uint32_t kFTailBytes = 1024u + 32u;   // w, dn, block scalars
 constexpr uint32_t kFTailPad = 1088u;
@@ -603,42 +603,64 @@ constexpr uint32_t kFTailPad = 1088u;
 constexpr int kFStageMax = 8192;
 
 struct __align__(16) FastCtl {
-    uint64_t full[kFS];    // block copy landed
-    uint64_t efree[kFS];   // epilogue of the block in this stage done (one arrive per epilogue warp)
-    uint64_t mmad[kFS];    // MMA chain into TMEM accumulator s (one per stage) done
-    uint64_t tfull[kFS];   // streamed form: the block's record tail landed in tail buffer s
-    uint64_t cfull[kFSCMax];   // streamed form: K chunk landed in chunk stage c
-    uint64_t cfree[kFSCMax];   // streamed form: the MMAs reading chunk stage c done
+    uint64_t efree[kFS];   // epilogue of the block in accumulator s done (one arrive per warp that takes it)
+    uint64_t mmad[kFS];    // MMA chain into TMEM accumulator s done
+    uint64_t tfull[kFS];   // the block's record tail landed in the accumulator's buffer
+    uint64_t cfull[kFSCMax];   // operand unit landed in stage c
+    uint64_t cfree[kFSCMax];   // the MMAs reading stage c done
     uint64_t afull;        // query tile copy landed
+    uint64_t ifull[2];     // item descriptor i (slot i & 1) written
+    uint64_t ifree[2];     // every warp is done with the item in the slot
+    uint64_t icopied;      // all copies of an item issued
     uint32_t tmem;
-    int tile, nblk;
     int err;
-    int blk[kFItemMax];    // the item's blocks
-    int th_cnt[4 * kFT];   // at the flush: staged candidates per epilogue thread
-    int qbase[kFT];        // at the flush: list offset per query lane
-    int r2s[kFT];          // per query lane: the smallest bound its column groups reached (float bits)
+    int tile[2], nblk[2];
+    int blk[2][kFItemMax]; // the items' blocks
+    int r2s[2][kFT];       // per query lane: the smallest bound its column groups reached in the item (float bits)
 };
 
 // A staged candidate: its slot, its lower bound and the margin ub - lb as a
 // half rounded up (so lb + margin >= ub), in three arrays.
 constexpr size_t kStagedBytes = sizeof(int) + sizeof(float) + sizeof(unsigned short);
 
-// Persistent filter kernel, one CTA per SM, 4 x CG epilogue warps + one
-// producer warp.  CG column groups: warps w, w+4, ... share TMEM lanes
+// A bounded wait that also gives up once the CTA's error flag (nullable) is set.
+__device__ __forceinline__ bool fast_wait(uint64_t *bar, uint32_t parity, const volatile int *err)
+{
+    for (long long i = 0; i < kFWait; i++) {
+        if (mbar_try_wait_sleep(bar, parity, 1000u)) return true;
+        if (err && *err) return false;
+    }
+    return false;
+}
+
+// Persistent filter kernel, one CTA per SM, 4 x CG epilogue warps, a copy warp,
+// an MMA warp and a scheduling warp.  CG column groups: warps w, w+4, ... share TMEM lanes
 // 32*(w%4)..+31 (the same 32 queries) and split the 128 object columns.
 //
 // Per item (a tile and up to a.item of its needed blocks), with gi counting
 // blocks over the CTA's life (barrier phases follow it):
-//   producer:  copy A (unless this CTA's previous item had the same tile);
-//              copy blocks 0..2 into stages gi%3; for each block:
-//              wait its copy, wait the epilogue of block gi-2 (frees TMEM
-//              accumulator gi%2 and stage (gi-2)%3 = (gi+1)%3), MMA chain into
-//              accumulator gi%2, commit, copy block gi+1 into the freed stage.
+//   copies:    A (unless this CTA's previous item had the same tile); each
+//              block's operand rows into a stage as soon as the MMAs that
+//              read it are done (tcgen05.commit on cfree), its tail (w, dn,
+//              scalars) into the buffer of its accumulator once the epilogue
+//              of block gi-3 has freed both.
+//   MMAs:      wait the operand and the accumulator gi%3, MMA chain, commit.
 //   epilogue:  wait the MMA of block gi, bound the 128 x 128 pairs, arrive
 //              on efree[gi%3].  Passing objects are staged in shared memory
 //              (shared-memory atomics only) and written to the queries'
-//              candidate lists once per item, one global atomic per query.
-// The CTA synchronises only between items.
+//              candidate lists once per item, one global atomic per thread.
+// The warps meet only on mbarriers, across items too: the scheduling warp
+// writes an item's blocks while the one before is in work.
+//
+// The filter of 10,000 queries at 1,000,000 x 128, k = 8 (17,000 blocks through
+// 148 CTAs) takes 190 us: 81 of MMAs at full rate, the rest the epilogue's
+// dependent steps per block (about 1.2 us a warp).  With one thread issuing
+// copies and MMAs from a branch on its index, a CTA-wide barrier between items
+// and every warp in every block it took 230, 60 % of it MMA issue at half rate
+// (see elect_one), 12 % claims and flushes; of these steps the loop without
+// barriers gave 30, the others 10 together (each alone moved the bound).  A
+// deeper prefetch of the records, or all TMEM columns loaded before the ball
+// test, gave nothing or lost 10 %.
 //
 // KH > 0 (k <= KH): each epilogue thread keeps its k smallest upper bounds in
 // registers (slots k..KH-1 hold -FLT_MAX and are never the largest); KH = 0:
@@ -648,25 +670,23 @@ constexpr size_t kStagedBytes = sizeof(int) + sizeof(float) + sizeof(unsigned sh
 // KH < 0: none; the query keeps the bound it came with (its seed).  Seeds that
 // lie next to the answer leave the kept bounds nothing to tighten: a thread
 // sees k objects below the seed only where a block holds most of the answer.
-// The autotuner measures both.  @@
+// The autotuner measures both: 2,500 queries at 1,000,000 x 128, k = 64, take
+// 165 us without, 540 with (heaps of 64 in shared memory).
 //
 // RANGE: range counts instead of kNN.  The bound stays the query's (r^2 with
 // the reference-arithmetic margin); objects certainly inside are counted per
 // thread, only the uncertain ones are listed; no bound heap.
 //
-// KS (kp > kFResKp, where a whole record does not fit a stage beside the
-// query tile; below it an autotuner choice): the producer streams each block's operand rows in 64-wide K
-// chunks through a.nsc chunk stages -- a stage is refilled as soon as the
-// MMAs reading it are done (tcgen05.commit on cfree), one unit behind the
-// MMA issue -- and copies the block's record tail (w, dn, scalars) into the
-// tail buffer of its accumulator once the epilogue of the block three back
-// has freed both.  The epilogue is the same, reading the tail buffer.
+// KS (kp > kFResKp, where three whole blocks do not fit beside the query
+// tile; below it an autotuner choice): the operand rows come in 64-wide K
+// chunks through a.nsc stages instead of whole blocks through three.
 template <int CG, int KH, bool RANGE, bool KS>
-__global__ void __launch_bounds__(128 * CG + 32, 1) k_fast_tile(FastTileArgs a)
+__global__ void __launch_bounds__(128 * CG + 96, 1) k_fast_tile(FastTileArgs a)
 {
     constexpr int NT = 128 * CG;   // epilogue threads
     constexpr int NEW = NT / 32;   // epilogue warps
-    constexpr int CW = 128 / CG;   // object columns per thread
+    constexpr int BG = CG == 4 ? 2 : 1;   // block groups: warps of group b take the blocks gi % BG == b
+    constexpr int CW = 128 * BG / CG;     // object columns per thread
     constexpr bool FLAT = RANGE || KH < 0;
     extern __shared__ __align__(1024) unsigned char fsm[];
     // 1024-byte aligned start (the swizzled operand layout needs it), as an
@@ -674,11 +694,13 @@ __global__ void __launch_bounds__(128 * CG + 32, 1) k_fast_tile(FastTileArgs a)
     unsigned char *base = fsm + ((1024u - (smem_u32(fsm) & 1023u)) & 1023u);
     const FastShape fs = a.fs;
     const uint32_t arec_pad = (fs.arec_bytes + 1023u) & ~1023u;
-    const uint32_t rec_pad = (fs.rec_bytes + 1023u) & ~1023u;
+    // operand units: a block's K chunks one by one (KS) or all at once
+    const int cpu = KS ? 1 : fs.nk, upb = KS ? fs.nk : 1, SC = KS ? a.nsc : kFS;
+    const uint32_t ubytes = (uint32_t)cpu * kFChunkBytes;
     unsigned char *B0 = base + arec_pad;
-    // KS: chunk stages at B0 (1024-aligned), then the tail buffers
-    unsigned char *T0 = B0 + (KS ? (size_t)a.nsc * kFChunkBytes : 0);
-    unsigned short *heap = reinterpret_cast<unsigned short *>(KS ? T0 + kFS * kFTailPad : B0 + kFS * rec_pad);
+    // unit stages at B0 (1024-aligned), then the accumulators' tail buffers
+    unsigned char *T0 = B0 + (size_t)SC * ubytes;
+    unsigned short *heap = reinterpret_cast<unsigned short *>(T0 + kFS * kFTailPad);
     FastCtl &ctl = *reinterpret_cast<FastCtl *>(heap + (KH != 0 ? 0 : NT * a.k));
     // staging area: a.st_cap entries (slot, lower bound, margin), pcap per
     // epilogue thread
@@ -688,15 +710,11 @@ __global__ void __launch_bounds__(128 * CG + 32, 1) k_fast_tile(FastTileArgs a)
     unsigned short *stg_m = reinterpret_cast<unsigned short *>(stg_lb + st_cap);
 
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    const bool producer = warp == NEW;
     const int lq = t & 127, g = t >> 7;
     const int k = a.k;
 
     if (t == 0) {
-        for (int s = 0; s < kFS; s++) {
-            mbar_init(&ctl.full[s], 1);
-            mbar_init(&ctl.efree[s], NEW);
-        }
+        for (int s = 0; s < kFS; s++) mbar_init(&ctl.efree[s], NEW / BG);
         for (int s = 0; s < kFS; s++) mbar_init(&ctl.mmad[s], 1);
         for (int s = 0; s < kFS; s++) mbar_init(&ctl.tfull[s], 1);
         for (int s = 0; s < kFSCMax; s++) {
@@ -704,6 +722,11 @@ __global__ void __launch_bounds__(128 * CG + 32, 1) k_fast_tile(FastTileArgs a)
             mbar_init(&ctl.cfree[s], 1);
         }
         mbar_init(&ctl.afull, 1);
+        for (int s = 0; s < 2; s++) {
+            mbar_init(&ctl.ifull[s], 1);
+            mbar_init(&ctl.ifree[s], NEW + 2);
+        }
+        mbar_init(&ctl.icopied, 1);
         ctl.err = 0;
         fence_mbar_init();
     }
@@ -718,199 +741,152 @@ __global__ void __launch_bounds__(128 * CG + 32, 1) k_fast_tile(FastTileArgs a)
     const uint32_t idesc = idesc_bf16_f32(kFT, kFN);
     const uint32_t a_hi_s = smem_u32(base), a_lo_s = smem_u32(base + fs.atile_bytes);
     long long gblk = 0;   // blocks this CTA has run through the pipeline
-    // producer bookkeeping (lane 0 of the producer warp), for the bounded
-    // drain on error: last block whose copy was issued / waited, last block
-    // whose MMA chain was committed, tile copies issued / waited
-    long long c_iss = -1, c_wait = -1, m_iss = -1;
-    int a_iss = 0, a_wait = 0;
-    // streamed form: K-chunk units run through the pipeline, last chunk copy
-    // issued / waited, last unit whose MMAs were committed, last tail issued
-    long long gunit = 0, u_iss = -1, u_wait = -1, u_mma = -1, t_iss = -1;
+    long long gunit = 0;  // operand units
+    // copy and MMA lanes: the last unit and block issued (for the bounded
+    // drain on error), the tile in shared memory and the copies of one so far
+    long long unit_last = -1, blk_last = -1;
+    int a_tile = -1, a_use = 0;
     unsigned long long blocks_done = 0, appended = 0;
 
-    // guided self-scheduling (thread 0): a CTA claims a run of consecutive
-    // items, about half the remaining items over twice the CTAs (one item at
-    // the end); consecutive items mostly belong to one tile, whose query
-    // operand then stays in shared memory
-    int c_next = 0, c_end = 0;
-    // producer lane 0: the tile whose query operand is in shared memory
-    int a_tile = -1;
-    for (;;) {
-        if (t == 0) {
-            const int nfull = a.n_items[0], total = nfull + a.n_items[1];
-            if (c_next >= c_end) {
-                const int done = *(volatile const int *)a.item_counter;
-                const int chunk = max(1, (total - done) / (2 * (int)gridDim.x));
-                c_next = atomicAdd(a.item_counter, chunk);
-                c_end = min(c_next + chunk, total);
+    volatile int *cerr = &ctl.err;
+    if (warp == NEW + 2) {
+        // ---- items, each written while the one before is in work: guided
+        // self-scheduling, a CTA claims a run of consecutive items, about half
+        // the remaining items over twice the CTAs (one item at the end);
+        // consecutive items mostly belong to one tile, whose query operand
+        // then stays in shared memory.  The claim waits until the copies of
+        // the item before are issued, so that no CTA holds more than it works on.
+        int c_next = 0, c_end = 0;
+        for (int it = 0;; it++) {
+            const int b = it & 1;
+            bool ok = it < 1 || fast_wait(&ctl.icopied, (uint32_t)((it - 1) & 1), nullptr);
+            ok &= it < 2 || fast_wait(&ctl.ifree[b], (uint32_t)((it / 2 - 1) & 1), nullptr);
+            ok = __all_sync(0xffffffffu, ok && !*cerr);
+            for (int i = lane; i < kFT; i += 32) ctl.r2s[b][i] = __float_as_int(FLT_MAX);
+            int tile = -1, nblk = 0, first = 0;
+            if (lane == 0) {
+                const int nfull = a.n_items[0], total = nfull + a.n_items[1];
+                if (c_next >= c_end) {
+                    const int done = *(volatile const int *)a.item_counter;
+                    const int chunk = max(1, (total - done) / (2 * (int)gridDim.x));
+                    c_next = ok ? atomicAdd(a.item_counter, chunk) : total;
+                    c_end = min(c_next + chunk, total);
+                }
+                const int i = c_next++;
+                if (ok && i < total) {
+                    const int2 e = i < nfull ? a.items[i] : a.items[a.items_cap - 1 - (i - nfull)];
+                    tile = e.x;
+                    first = e.y;
+                    nblk = min(a.item, min(a.bcnt[tile], a.nbcap) - e.y);
+                }
+                if (!ok) atomicMax(&ctl.err, 6);
+                ctl.tile[b] = tile;
+                ctl.nblk[b] = nblk;
             }
-            const int it = c_next++;
-            int tile = -1, nblk = 0;
-            if (it < total) {
-                const int2 e = it < nfull ? a.items[it] : a.items[a.items_cap - 1 - (it - nfull)];
-                tile = e.x;
-                nblk = min(a.item, min(a.bcnt[tile], a.nbcap) - e.y);
-                for (int j = 0; j < nblk; j++) ctl.blk[j] = a.blist[(size_t)tile * a.nbcap + e.y + j];
-            }
-            ctl.tile = tile;
-            ctl.nblk = nblk;
+            tile = __shfl_sync(0xffffffffu, tile, 0);
+            nblk = __shfl_sync(0xffffffffu, nblk, 0);
+            first = __shfl_sync(0xffffffffu, first, 0);
+            if (lane < nblk) ctl.blk[b][lane] = a.blist[(size_t)tile * a.nbcap + first + lane];
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ctl.ifull[b]);
+            if (tile < 0) break;
         }
-        if (t < kFT) ctl.r2s[t] = __float_as_int(FLT_MAX);
-        __syncthreads();
-        const int tile = ctl.tile, nblk = ctl.nblk;
+    } else
+    for (int it = 0;; it++) {
+        // the scheduling warp gives up on its own waits in bounded time and
+        // then writes the last item, so this one ends
+        const int ib = it & 1;
+        const bool got = __all_sync(0xffffffffu, mbar_wait(&ctl.ifull[ib], (uint32_t)((it / 2) & 1), 4 * kFWait));
+        const int tile = got ? ctl.tile[ib] : -1, nblk = ctl.nblk[ib];
+        if (tile < 0) break;
+        const int *blks = ctl.blk[ib];
         int nst = 0;   // candidates this (epilogue) thread staged in this item
-        if (tile < 0 || ctl.err) break;
         const int4 *tinfo = reinterpret_cast<const int4 *>(a.arec + (size_t)tile * fs.arec_bytes + 2 * fs.atile_bytes);
 
-        if (producer && KS) {
+        if (warp == NEW) {
+            // ---- copies: operand units into the stages whose MMAs are done,
+            // each block's tail behind its last unit
             if (lane == 0) {
-                const int nk = fs.nk, SC = a.nsc, total = nblk * nk;
-                auto issue_chunk = [&](int u) {   // unit u: chunk u % nk of the item's block u / nk
-                    const long long gu = gunit + u;
-                    const int s = (int)(gu % SC);
-                    const int blk = ctl.blk[u / nk];
-                    mbar_arrive_expect_tx(&ctl.cfull[s], (uint32_t)kFChunkBytes);
-                    bulk_g2s(B0 + (size_t)s * kFChunkBytes,
-                             a.recs + (size_t)blk * fs.rec_bytes + (size_t)(u % nk) * kFChunkBytes,
-                             (uint32_t)kFChunkBytes, &ctl.cfull[s]);
-                    u_iss = gu;
-                };
-                // the query operand, unless this tile's is in shared memory already
-                const bool need_a = tile != a_tile;
-                if (need_a) {
+                const int total = nblk * upb;
+                int err = 0;
+                if (tile != a_tile) {
+                    // the query operand, unless this tile's is in shared memory
+                    // already; every MMA that reads the one there is done
+                    if (gblk > 0 && !fast_wait(&ctl.mmad[(gblk - 1) % kFS], (uint32_t)(((gblk - 1) / kFS) & 1), cerr))
+                        err = 1;
                     mbar_arrive_expect_tx(&ctl.afull, fs.arec_bytes);
                     bulk_g2s(base, a.arec + (size_t)tile * fs.arec_bytes, fs.arec_bytes, &ctl.afull);
-                    a_iss++;
+                    a_tile = tile;
+                    a_use++;
                 }
-                // chunk stages are free at an item start (the CTA synchronised
-                // after every MMA of the last item was consumed)
-                for (int u = 0; u < SC && u < total; u++) issue_chunk(u);
-                int err = 0;
-                if (need_a) {
-                    if (!mbar_wait(&ctl.afull, (uint32_t)(a_wait & 1), kFWait)) err = 1;
-                    else {
-                        a_wait++;
-                        a_tile = tile;
-                    }
-                }
-                const uint64_t dah = smem_desc_sw128(a_hi_s, 1024), dal = smem_desc_sw128(a_lo_s, 1024);
-                for (int j = 0; j < nblk && !err; j++) {
+                for (int u = 0; u < total && !err; u++) {
+                    const long long gu = gunit + u;
+                    const int s = (int)(gu % SC), j = u / upb, c = u - j * upb;
+                    const unsigned char *rec = a.recs + (size_t)blks[j] * fs.rec_bytes;
+                    if (gu >= SC && !fast_wait(&ctl.cfree[s], (uint32_t)((gu / SC - 1) & 1), cerr)) { err = 5; break; }
+                    mbar_arrive_expect_tx(&ctl.cfull[s], ubytes);
+                    bulk_g2s(B0 + (size_t)s * ubytes, rec + (size_t)c * ubytes, ubytes, &ctl.cfull[s]);
+                    unit_last = gu;
+                    if (c + 1 < upb) continue;
                     const long long gi = gblk + j;
                     const int acc = (int)(gi % kFS);
-                    const int blk = ctl.blk[j];
-                    // accumulator and tail buffer acc: free once the epilogue of
-                    // block gi - 3 is done
-                    if (gi >= kFS) {
-                        const long long gp = gi - kFS;
-                        if (!mbar_wait(&ctl.efree[acc], (uint32_t)((gp / kFS) & 1), kFWait)) { err = 3; break; }
-                    }
+                    if (gi >= kFS && !fast_wait(&ctl.efree[acc], (uint32_t)((gi / kFS - 1) & 1), cerr)) { err = 3; break; }
                     mbar_arrive_expect_tx(&ctl.tfull[acc], kFTailBytes);
-                    bulk_g2s(T0 + (size_t)acc * kFTailPad, a.recs + (size_t)blk * fs.rec_bytes + fs.btile_bytes,
-                             kFTailBytes, &ctl.tfull[acc]);
-                    t_iss = gi;
-                    const uint32_t dt = tmem + (uint32_t)(acc * kFAccCols);
-                    for (int c = 0; c < nk; c++) {
-                        const int u = j * nk + c;
-                        const long long gu = gunit + u;
-                        const int s = (int)(gu % SC);
-                        if (!mbar_wait(&ctl.cfull[s], (uint32_t)((gu / SC) & 1), kFWait)) { err = 2; break; }
-                        u_wait = gu;
-                        tc_fence_after();
-                        const uint64_t db = smem_desc_sw128(smem_u32(B0 + (size_t)s * kFChunkBytes), 1024);
-#pragma unroll
-                        for (int kk = 0; kk < 4; kk++) {
-                            const uint64_t ao = ((uint64_t)c * (kFT * 128u) + (uint64_t)kk * 32u) >> 4;
-                            mma_bf16(dt, dah + ao, db + (((uint64_t)kk * 32u) >> 4), idesc, (c | kk) ? 1u : 0u);
-                        }
-#pragma unroll
-                        for (int kk = 0; kk < 4; kk++) {
-                            const uint64_t ao = ((uint64_t)c * (kFT * 128u) + (uint64_t)kk * 32u) >> 4;
-                            mma_bf16(dt, dal + ao, db + (((uint64_t)kk * 32u) >> 4), idesc, 1u);
-                        }
-                        mma_commit(&ctl.cfree[s]);
-                        u_mma = gu;
-                        // refill the previous unit's stage (its MMAs retire first)
-                        if (u >= 1 && u - 1 + SC < total) {
-                            const long long gp = gu - 1;
-                            if (!mbar_wait(&ctl.cfree[gp % SC], (uint32_t)((gp / SC) & 1), kFWait)) {
-                                err = 5;
-                                break;
-                            }
-                            issue_chunk(u - 1 + SC);
-                        }
-                    }
-                    if (err) break;
-                    mma_commit(&ctl.mmad[acc]);
-                    m_iss = gi;
+                    bulk_g2s(T0 + (size_t)acc * kFTailPad, rec + fs.btile_bytes, kFTailBytes, &ctl.tfull[acc]);
+                    blk_last = gi;
                 }
                 if (err) atomicMax(&ctl.err, err);
-                blocks_done += nblk;
+                mbar_arrive(&ctl.icopied);
             }
             __syncwarp();
-        } else if (producer) {
-            if (lane == 0) {
-                // block gi uses stage gi % 3 and TMEM accumulator gi % 3; its
-                // copy waits for the epilogue of block gi - 3 (which frees both)
-                auto issue_copy = [&](long long gi) {
-                    const int s = (int)(gi % kFS);
-                    const int blk = ctl.blk[(int)(gi - gblk)];
-                    mbar_arrive_expect_tx(&ctl.full[s], fs.rec_bytes);
-                    bulk_g2s(B0 + (size_t)s * rec_pad, a.recs + (size_t)blk * fs.rec_bytes, fs.rec_bytes,
-                             &ctl.full[s]);
-                    c_iss = gi;
-                };
-                const bool need_a = tile != a_tile;
-                if (need_a) {
-                    mbar_arrive_expect_tx(&ctl.afull, fs.arec_bytes);
-                    bulk_g2s(base, a.arec + (size_t)tile * fs.arec_bytes, fs.arec_bytes, &ctl.afull);
-                    a_iss++;
-                }
-                // stages are free at an item start (the CTA synchronised)
-                for (int j = 0; j < 2 && j < nblk; j++) issue_copy(gblk + j);
-                int err = 0;
-                if (need_a) {
-                    if (!mbar_wait(&ctl.afull, (uint32_t)(a_wait & 1), kFWait)) err = 1;
-                    else {
-                        a_wait++;
-                        a_tile = tile;
-                    }
-                }
-                // operand descriptors: the start-address field (address >> 4,
-                // 14 bits; shared memory is below 256 KB) advances by adding
-                const uint64_t dah = smem_desc_sw128(a_hi_s, 1024), dal = smem_desc_sw128(a_lo_s, 1024);
-                const int ksteps = fs.kp / 16;
-                for (int j = 0; j < nblk && !err; j++) {
-                    const long long gi = gblk + j;
-                    const int s = (int)(gi % kFS);
-                    if (!mbar_wait(&ctl.full[s], (uint32_t)((gi / kFS) & 1), kFWait)) { err = 2; break; }
-                    c_wait = gi;
+        } else if (warp == NEW + 1) {
+            // ---- MMAs: block gi into accumulator gi % 3, free once the
+            // epilogue of block gi - 3 is done (the whole warp, see elect_one)
+            int err = 0;
+            auto wait = [&](uint64_t *bar, long long phase) {
+                return __all_sync(0xffffffffu, fast_wait(bar, (uint32_t)(phase & 1), cerr));
+            };
+            if (tile != a_tile) {
+                if (!wait(&ctl.afull, a_use)) err = 1;
+                a_tile = tile;
+                a_use++;
+            }
+            // operand descriptors: the start-address field (address >> 4,
+            // 14 bits; shared memory is below 256 KB) advances by adding
+            const uint64_t dah = smem_desc_sw128(a_hi_s, 1024), dal = smem_desc_sw128(a_lo_s, 1024);
+            for (int j = 0; j < nblk && !err; j++) {
+                const long long gi = gblk + j;
+                const int acc = (int)(gi % kFS);
+                if (gi >= kFS && !wait(&ctl.efree[acc], gi / kFS - 1)) { err = 3; break; }
+                const uint32_t dt = __shfl_sync(0xffffffffu, tmem + (uint32_t)(acc * kFAccCols), 0);
+                for (int c = 0; c < upb; c++) {
+                    const long long gu = gunit + (long long)j * upb + c;
+                    const int s = (int)(gu % SC);
+                    if (!wait(&ctl.cfull[s], gu / SC)) { err = 2; break; }
                     tc_fence_after();
-                    const uint64_t db = smem_desc_sw128(smem_u32(B0 + (size_t)s * rec_pad), 1024);
-                    const uint32_t dt = tmem + (uint32_t)(s * kFAccCols);
-                    for (int kk = 0; kk < ksteps; kk++) {
-                        const uint64_t ao = ((uint64_t)(kk >> 2) * (kFT * 128u) + (uint64_t)(kk & 3) * 32u) >> 4;
-                        const uint64_t bo = ((uint64_t)(kk >> 2) * (kFN * 128u) + (uint64_t)(kk & 3) * 32u) >> 4;
-                        mma_bf16(dt, dah + ao, db + bo, idesc, kk > 0 ? 1u : 0u);
-                    }
-                    for (int kk = 0; kk < ksteps; kk++) {
-                        const uint64_t ao = ((uint64_t)(kk >> 2) * (kFT * 128u) + (uint64_t)(kk & 3) * 32u) >> 4;
-                        const uint64_t bo = ((uint64_t)(kk >> 2) * (kFN * 128u) + (uint64_t)(kk & 3) * 32u) >> 4;
-                        mma_bf16(dt, dal + ao, db + bo, idesc, 1u);
-                    }
-                    mma_commit(&ctl.mmad[s]);
-                    m_iss = gi;
-                    if (j + 2 < nblk) {
-                        // stage (gi + 2) % 3 was last used by block gi - 1
-                        if (j >= 1) {
-                            const long long gp = gi - 1;
-                            if (!mbar_wait(&ctl.efree[gp % kFS], (uint32_t)((gp / kFS) & 1), kFWait)) {
-                                err = 3;
-                                break;
+                    const uint64_t db = smem_desc_sw128(
+                        __shfl_sync(0xffffffffu, smem_u32(B0) + (uint32_t)s * ubytes, 0), 1024);
+                    if (elect_one()) {
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            const uint64_t da = (h ? dal : dah) + (((uint64_t)(c * cpu) * (kFT * 128u)) >> 4);
+                            for (int cc = 0; cc < cpu; cc++) {
+                                const uint64_t ao = ((uint64_t)cc * (kFT * 128u)) >> 4;
+                                const uint64_t bo = ((uint64_t)cc * kFChunkBytes) >> 4;
+#pragma unroll
+                                for (int kk = 0; kk < 4; kk++)
+                                    mma_bf16(dt, da + ao + 2 * kk, db + bo + 2 * kk, idesc, (h | c | cc | kk) ? 1u : 0u);
                             }
                         }
-                        issue_copy(gi + 2);
+                        mma_commit(&ctl.cfree[s]);
+                        if (c + 1 == upb) mma_commit(&ctl.mmad[acc]);
                     }
+                    __syncwarp();
+                    unit_last = gu;
                 }
+                if (!err) blk_last = gi;
+            }
+            if (lane == 0) {
                 if (err) atomicMax(&ctl.err, err);
                 blocks_done += nblk;
             }
@@ -938,21 +914,21 @@ __global__ void __launch_bounds__(128 * CG + 32, 1) k_fast_tile(FastTileArgs a)
             const uint32_t trow = (uint32_t)(warp & 3) * 32u << 16;
             for (int j = 0; j < nblk; j++) {
                 const long long gi = gblk + j;
+                if (BG > 1 && (int)(gi % BG) != g % BG) continue;
                 const int s = (int)(gi % kFS);
-                const int blk = ctl.blk[j];
+                const int blk = blks[j];
                 // one verdict per warp: the TMEM loads below are warp-collective
-                if (!__all_sync(0xffffffffu, mbar_wait(&ctl.mmad[s], (uint32_t)((gi / kFS) & 1), kFWait))) {
+                if (!__all_sync(0xffffffffu, fast_wait(&ctl.mmad[s], (uint32_t)((gi / kFS) & 1), cerr))) {
                     atomicMax(&ctl.err, 4);
                     break;
                 }
                 tc_fence_after();
-                // record tail visible here (KS: in the accumulator's tail buffer)
-                mbar_wait(KS ? &ctl.tfull[s] : &ctl.full[s], (uint32_t)((gi / kFS) & 1), kFWait);
+                // record tail visible here
+                fast_wait(&ctl.tfull[s], (uint32_t)((gi / kFS) & 1), cerr);
                 // the bound the query's other column groups have reached
-                if constexpr (!FLAT) R2 = fminf(R2, __int_as_float(*(volatile const int *)&ctl.r2s[lq]));
+                if constexpr (!FLAT) R2 = fminf(R2, __int_as_float(*(volatile const int *)&ctl.r2s[ib][lq]));
                 const float s2 = sqrtf(fmaxf(R2, 0.f)) * 1.000001f;
-                const float *tail = reinterpret_cast<const float *>(
-                    KS ? T0 + (size_t)s * kFTailPad : B0 + (size_t)s * rec_pad + fs.btile_bytes);
+                const float *tail = reinterpret_cast<const float *>(T0 + (size_t)s * kFTailPad);
                 const float *wv = tail + kTailW, *dn = tail + kTailDn;
                 const float cn = tail[kTailC], rb = tail[kTailRb], wb = tail[kTailWb], brad = tail[kTailRad];
                 const uint32_t taddr = tmem + trow + (uint32_t)(s * kFAccCols);
@@ -979,7 +955,7 @@ __global__ void __launch_bounds__(128 * CG + 32, 1) k_fast_tile(FastTileArgs a)
                 const float eb = ec + 2e-6f * q2 + cr * rb + 2e-6f * wb;
                 const float T = q2 - 2.f * qc - eb;
 #pragma unroll 1
-                for (int c = g * CW; c < (g + 1) * CW && !warp_skip; c += 16) {
+                for (int c = g / BG * CW; c < (g / BG + 1) * CW && !warp_skip; c += 16) {
                     uint32_t r[16];
                     __syncwarp();   // tcgen05.ld is warp-collective: reconverge after the appends
                     tmem_ld16_nowait(taddr + (uint32_t)c, r);
@@ -1086,7 +1062,7 @@ __global__ void __launch_bounds__(128 * CG + 32, 1) k_fast_tile(FastTileArgs a)
                 // k distinct objects' upper bounds bound the query's k-th d^2
                 if (!FLAT && qi >= 0 && hmx < pub) {
                     atomicMin(a.r2_bits + qi, __float_as_int(fmaxf(hmx, 0.f)));
-                    if (CG > 1) atomicMin(&ctl.r2s[lq], __float_as_int(fmaxf(hmx, 0.f)));
+                    if (CG > 1) atomicMin(&ctl.r2s[ib][lq], __float_as_int(fmaxf(hmx, 0.f)));
                     pub = hmx;
                 }
                 tc_fence_before();
@@ -1094,57 +1070,37 @@ __global__ void __launch_bounds__(128 * CG + 32, 1) k_fast_tile(FastTileArgs a)
                 if (lane == 0) mbar_arrive(&ctl.efree[s]);
             }
             if (RANGE && qi >= 0 && certain) atomicAdd(a.rcnt + qi, certain);
-        }
-        gblk += nblk;
-        if (KS) gunit += (long long)nblk * fs.nk;
-        tc_fence_before();
-        __syncthreads();   // item done: every MMA consumed, stages and A free
-        tc_fence_after();
-        // flush the staged candidates: one list reservation per query lane,
-        // then each thread writes its own slice after its lane's earlier
-        // column groups
-        if (t < NT) ctl.th_cnt[t] = nst;
-        __syncthreads();
-        if (t < kFT) {
-            int c = 0;
-#pragma unroll
-            for (int g2 = 0; g2 < CG; g2++) c += ctl.th_cnt[t + kFT * g2];
-            const int qi = tinfo[t].x;
-            ctl.qbase[t] = (c > 0 && qi >= 0) ? atomicAdd(&a.cand_cnt[qi], c) : 0;
-        }
-        __syncthreads();
-        if (t < NT && nst > 0) {
-            const int qi = tinfo[lq].x;
-            int at = ctl.qbase[lq];
-            for (int g2 = 0; g2 < g; g2++) at += ctl.th_cnt[lq + kFT * g2];
-            for (int e = 0; e < nst && at < kFCand; e++, at++) {
-                const int x = e * NT + t;
-                const float lb = stg_lb[x];
-                const float margin = __half2float(__ushort_as_half(stg_m[x]));
-                a.cand_pos[(size_t)qi * kFCand + at] = stg_slot[x];
-                a.cand_lb[(size_t)qi * kFCand + at] = lb;
-                a.cand_ub[(size_t)qi * kFCand + at] = __fadd_ru(lb, margin);
+            // the staged candidates: one list reservation per thread, its own slice
+            if (nst > 0) {
+                int at = atomicAdd(&a.cand_cnt[qi], nst);
+                for (int e = 0; e < nst && at < kFCand; e++, at++) {
+                    const int x = e * NT + t;
+                    const float lb = stg_lb[x];
+                    const float margin = __half2float(__ushort_as_half(stg_m[x]));
+                    a.cand_pos[(size_t)qi * kFCand + at] = stg_slot[x];
+                    a.cand_lb[(size_t)qi * kFCand + at] = lb;
+                    a.cand_ub[(size_t)qi * kFCand + at] = __fadd_ru(lb, margin);
+                }
             }
         }
-        __syncthreads();
+        gblk += nblk;
+        gunit += (long long)nblk * upb;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ctl.ifree[ib]);
     }
-    if (producer && lane == 0 && ctl.err) {
-        // let copies and MMAs still in flight finish before the CTA leaves (bounded)
-        for (long long gi = c_wait + 1; gi <= c_iss; gi++)
-            mbar_wait(&ctl.full[gi % kFS], (uint32_t)((gi / kFS) & 1), kFWait);
-        if (a_wait < a_iss) mbar_wait(&ctl.afull, (uint32_t)((a_iss - 1) & 1), kFWait);
-        if (m_iss >= 0) mbar_wait(&ctl.mmad[m_iss % kFS], (uint32_t)((m_iss / kFS) & 1), kFWait);
-        if (KS) {
-            const int SC = a.nsc;
-            for (long long gu = u_wait + 1; gu <= u_iss; gu++)
-                mbar_wait(&ctl.cfull[gu % SC], (uint32_t)((gu / SC) & 1), kFWait);
-            if (u_mma >= 0) mbar_wait(&ctl.cfree[u_mma % SC], (uint32_t)((u_mma / SC) & 1), kFWait);
-            for (long long gi = t_iss - kFS + 1 > 0 ? t_iss - kFS + 1 : 0; gi <= t_iss; gi++)
-                mbar_wait(&ctl.tfull[gi % kFS], (uint32_t)((gi / kFS) & 1), kFWait);
-        }
+    __syncthreads();
+    if (warp >= NEW && lane == 0 && ctl.err) {
+        // let copies and MMAs still in flight finish before the CTA leaves
+        // (bounded): the last of every stage, which the earlier ones precede
+        const bool cp = warp == NEW;
+        for (long long gu = max(unit_last - SC + 1, 0ll); gu <= unit_last; gu++)
+            mbar_wait(cp ? &ctl.cfull[gu % SC] : &ctl.cfree[gu % SC], (uint32_t)((gu / SC) & 1), kFWait);
+        for (long long gi = max(blk_last - kFS + 1, 0ll); gi <= blk_last; gi++)
+            mbar_wait(cp ? &ctl.tfull[gi % kFS] : &ctl.mmad[gi % kFS], (uint32_t)((gi / kFS) & 1), kFWait);
+        if (cp && a_use) mbar_wait(&ctl.afull, (uint32_t)((a_use - 1) & 1), kFWait);
     }
     if (a.stats && appended) atomicAdd(&a.stats[5], appended);
-    if (a.stats && producer && lane == 0 && blocks_done) {
+    if (a.stats && blocks_done) {
         atomicAdd(&a.stats[0], blocks_done);
         atomicAdd(&a.stats[1], (unsigned long long)fs.rec_bytes * blocks_done);
     }
@@ -1770,16 +1726,15 @@ static FastCfg fast_default_cfg(const gts_index *idx, int k)
 }
 
 // Shared memory of the filter kernel before candidate staging: the query
-// tile, the block stages (whole records, or for kp > kFResKp nsc K-chunk
-// stages and three tail buffers), the bound heaps (k > 16) and the control
+// tile, the operand stages (whole blocks, or for kp > kFResKp nsc K-chunk
+// stages), three tail buffers, the bound heaps (k > 16) and the control
 // block.  nsc = 0 for the resident form.
 static size_t fast_tile_fixed_smem(const FastShape &fs, int cg, int k, bool heap_in_smem, int nsc, bool stream)
 {
     const uint32_t arec_pad = (fs.arec_bytes + 1023u) & ~1023u;
-    const uint32_t rec_pad = (fs.rec_bytes + 1023u) & ~1023u;
     const size_t heap = heap_in_smem ? sizeof(unsigned short) * 128 * cg * (size_t)k : 0;
-    const size_t stages = (fs.kp > kFResKp || stream) ? (size_t)nsc * kFChunkBytes + kFS * (size_t)kFTailPad
-                                                      : kFS * (size_t)rec_pad;
+    const size_t stages = ((fs.kp > kFResKp || stream) ? (size_t)nsc * kFChunkBytes : kFS * (size_t)fs.btile_bytes) +
+                          kFS * (size_t)kFTailPad;
     return 1024 + (size_t)arec_pad + stages + heap + sizeof(FastCtl) + 64;
 }
 
@@ -1833,7 +1788,7 @@ static int launch_fast_tile_cg(const FastTileArgs &a, int grid, cudaStream_t st)
     const size_t smem = fixed + kStagedBytes * (size_t)b.st_cap;
     GTS_CUDA_TRY(cudaFuncSetAttribute(k_fast_tile<CG, KH, RANGE, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
-    k_fast_tile<CG, KH, RANGE, KS><<<grid, 128 * CG + 32, smem, st>>>(b);
+    k_fast_tile<CG, KH, RANGE, KS><<<grid, 128 * CG + 96, smem, st>>>(b);
     GTS_CUDA_TRY(cudaGetLastError());
     return GTS_OK;
 }

@@ -262,64 +262,69 @@ __global__ void __launch_bounds__(kPThreads, 1) k_prune(PruneArgs a)
         }
         __syncwarp();
     } else if (warp == kEW + 1) {
-        // ---------------- MMAs
-        if (lane == 0) {
-            const uint32_t idesc = idesc_bf16_f32(kFT, kPN);
-            const int ksteps = fs.kp / 16;
-            int m_iss = -1;   // last item whose MMA pair is committed
-            int a_tile = -1, a_iss = 0;
-            bool a_pending = false;
-            for (int j = 0; j < n && !*err; j++) {
-                int tile, grp;
-                uint32_t elig;
-                prune_item<BLK>(a, i0 + j, tile, grp, elig);
-                if (tile != a_tile) {
-                    // every MMA reading the old tile's operand is done (the
-                    // commit of the last one covers all before it)
-                    if (m_iss >= 0 &&
-                        !prune_wait(&ctl.mmad[m_iss % kPS], (uint32_t)((m_iss / kPS) & 1), err)) {
-                        *err = 1;
-                        break;
-                    }
-                    mbar_arrive_expect_tx(&ctl.afull, fs.arec_bytes);
-                    bulk_g2s(base, a.arec + (size_t)tile * fs.arec_bytes, fs.arec_bytes, &ctl.afull);
-                    a_iss++;
-                    a_pending = true;
-                    if (!prune_wait(&ctl.afull, (uint32_t)((a_iss - 1) & 1), err)) {
-                        *err = 1;
-                        break;
-                    }
-                    a_pending = false;
-                    a_tile = tile;
-                }
-                const int s = j % kPS;
-                if (!prune_wait(&ctl.bfull[s], (uint32_t)((j / kPS) & 1), err)) {
+        // ---------------- MMAs (the whole warp, see elect_one)
+        const uint32_t idesc = idesc_bf16_f32(kFT, kPN);
+        auto wait = [&](uint64_t *bar, int phase) {
+            return __all_sync(0xffffffffu, prune_wait(bar, (uint32_t)(phase & 1), err));
+        };
+        int m_iss = -1;   // last item whose MMA pair is committed
+        int a_tile = -1, a_iss = 0;
+        bool a_pending = false;
+        for (int j = 0; j < n && !__any_sync(0xffffffffu, *err); j++) {
+            int tile, grp;
+            uint32_t elig;
+            prune_item<BLK>(a, i0 + j, tile, grp, elig);
+            if (tile != a_tile) {
+                // every MMA reading the old tile's operand is done (the
+                // commit of the last one covers all before it)
+                if (m_iss >= 0 && !wait(&ctl.mmad[m_iss % kPS], m_iss / kPS)) {
                     *err = 1;
                     break;
                 }
-                tc_fence_after();
-                const uint64_t dah = smem_desc_sw128(smem_u32(base), 1024);
-                const uint64_t dal = smem_desc_sw128(smem_u32(base + fs.atile_bytes), 1024);
-                const uint64_t db = smem_desc_sw128(smem_u32(B + (size_t)s * bstage), 1024);
-                const uint32_t dt = tmem + (uint32_t)s * kPAccCols;
-                for (int kk = 0; kk < ksteps; kk++) {
-                    const uint64_t ao = ((uint64_t)(kk >> 2) * (kFT * 128u) + (uint64_t)(kk & 3) * 32u) >> 4;
-                    const uint64_t bo = ((uint64_t)(kk >> 2) * kPlane + (uint64_t)(kk & 3) * 32u) >> 4;
-                    mma_bf16(dt, dah + ao, db + bo, idesc, kk > 0 ? 1u : 0u);
+                if (lane == 0) {
+                    mbar_arrive_expect_tx(&ctl.afull, fs.arec_bytes);
+                    bulk_g2s(base, a.arec + (size_t)tile * fs.arec_bytes, fs.arec_bytes, &ctl.afull);
                 }
-                for (int kk = 0; kk < ksteps; kk++) {
-                    const uint64_t ao = ((uint64_t)(kk >> 2) * (kFT * 128u) + (uint64_t)(kk & 3) * 32u) >> 4;
-                    const uint64_t bo = ((uint64_t)(kk >> 2) * kPlane + (uint64_t)(kk & 3) * 32u) >> 4;
-                    mma_bf16(dt, dal + ao, db + bo, idesc, 1u);
+                __syncwarp();
+                a_iss++;
+                a_pending = true;
+                if (!wait(&ctl.afull, a_iss - 1)) {
+                    *err = 1;
+                    break;
                 }
+                a_pending = false;
+                a_tile = tile;
+            }
+            const int s = j % kPS;
+            if (!wait(&ctl.bfull[s], j / kPS)) {
+                *err = 1;
+                break;
+            }
+            tc_fence_after();
+            const uint64_t dah = smem_desc_sw128(smem_u32(base), 1024);
+            const uint64_t dal = smem_desc_sw128(smem_u32(base + fs.atile_bytes), 1024);
+            const uint64_t db = smem_desc_sw128(
+                __shfl_sync(0xffffffffu, smem_u32(B) + (uint32_t)s * (uint32_t)bstage, 0), 1024);
+            const uint32_t dt = __shfl_sync(0xffffffffu, tmem + (uint32_t)s * kPAccCols, 0);
+            if (elect_one()) {
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                    for (int c = 0; c < fs.nk; c++) {
+                        const uint64_t ao = ((uint64_t)c * (kFT * 128u)) >> 4, bo = ((uint64_t)c * kPlane) >> 4;
+#pragma unroll
+                        for (int kk = 0; kk < 4; kk++)
+                            mma_bf16(dt, (h ? dal : dah) + ao + 2 * kk, db + bo + 2 * kk, idesc,
+                                     (h | c | kk) ? 1u : 0u);
+                    }
                 mma_commit(&ctl.mmad[s]);
-                m_iss = j;
             }
-            if (*err) {
-                // a tile copy or MMAs still in flight finish before the CTA leaves (bounded)
-                if (a_pending) mbar_wait(&ctl.afull, (uint32_t)((a_iss - 1) & 1), kFWait);
-                if (m_iss >= 0) mbar_wait(&ctl.mmad[m_iss % kPS], (uint32_t)((m_iss / kPS) & 1), kFWait);
-            }
+            __syncwarp();
+            m_iss = j;
+        }
+        if (lane == 0 && *err) {
+            // a tile copy or MMAs still in flight finish before the CTA leaves (bounded)
+            if (a_pending) mbar_wait(&ctl.afull, (uint32_t)((a_iss - 1) & 1), kFWait);
+            if (m_iss >= 0) mbar_wait(&ctl.mmad[m_iss % kPS], (uint32_t)((m_iss / kPS) & 1), kFWait);
         }
         __syncwarp();
     } else {

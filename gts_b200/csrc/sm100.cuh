@@ -190,6 +190,22 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int m, int n)
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
+// One lane of a converged warp, the same at every call.  MMAs are issued from
+// warp-uniform control flow under it: the compiler then keeps the operands in
+// uniform registers.  In a branch on the thread's index it moves each of them
+// there at every MMA: 107-135 cycles between 128 x 144 x 16 products that take
+// the tensor core 72.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(r));
+    return r != 0;
+}
+
 // D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread.
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                          uint32_t accumulate)
