@@ -82,6 +82,33 @@ __device__ __forceinline__ double dist_row_f64(const float *__restrict__ a,
     }
 }
 
+// One step of the F32 sites' sum, r = (float)((double)r + pow(e, 2)).  pow is
+// within 2 ulp of the square, so this is one fused multiply-add unless the
+// exact sum lies next to a float rounding midpoint (the reference's FP64 sum
+// is within 2^-26 of half an ulp of the exact one).  The remainder r + e^2 - f
+// tells, in FP32: the difference of f and the larger of r and e^2 is exact, so
+// it is known to 2^-23 of itself.  Steps that come close (one in 10^5, mostly
+// squares of short differences) are done as written; an FP64 step's dependent
+// instructions take some 1,000 cycles.
+__device__ __forceinline__ float add_square(float r, float e)
+{
+    const float f = fmaf(e, e, r);
+    float rem = fmaf(e, e, r - f);
+    if (r < 0.5f * f) {
+        const float p = e * e;
+        rem = ((p - f) + r) + fmaf(e, e, -p);
+    }
+    const int bits = __float_as_int(f);
+    const float half = __int_as_float((bits & 0x7f800000) - (24 << 23));   // half an ulp of f
+    // below 2^-60 or past the floats the remainder is not reliable; at a power
+    // of two the spacing below is half as wide
+    if (fabsf(fabsf(rem) - half) <= half * 4e-7f || (bits & 0x7fffff) == 0 || !(f > 1e-18f && f < 3e38f)) {
+        if (e != 0.f || !(r == r)) r += pow(e, 2);
+        return r;
+    }
+    return f;
+}
+
 // Sequential F32-accumulated distance (`float result += pow(..)` adds in
 // double and rounds to float at every step), same literal calls.
 __device__ __forceinline__ float dist_row_f32(const float *__restrict__ a,
