@@ -772,20 +772,27 @@ def make_roofline(args, w, groups, stats, per_step_ms, total_ms, filter_ms, filt
     step_ms = statistics.mean(per_step_ms)
     if not fast:
         # every leaf row and pivot row a query reads, plus its own row and
-        # result; a string row is its 109 bytes plus its 4-byte length
+        # result; a string row is its 109 bytes plus its 4-byte length.  The
+        # sweep counts (query, kept row) pairs and reads a row once per tile
+        # of 128 queries (strings: 32)
         row = 4 * d if w["metric"] != 6 else 113
-        alg_bytes = row * (stats["objects"] + stats["pivots"]) + sum(
+        swept = args.form == "plain" and (w["metric"] == 6 or d > 8)
+        share = (32 if w["metric"] == 6 else 128) if swept else 1
+        ranges = all(g["op"] == "range" for g in groups)
+        kernel = ("k_se_tile" if w["metric"] == 6 else "k_sw_tile") if swept else (
+            "k_search_warp" if args.form == "plain" and ranges else "k_search")
+        alg_bytes = row * (stats["objects"] / share + stats["pivots"]) + sum(
             len(g["sel"]) * (row + (4 if g["op"] == "range" else 8 * int(g["p"]))) for g in groups)
         achieved = alg_bytes / (step_ms / 1e3) / 1e9
         traffic = None
-        if "k_search" in per_unit and w["metric"] == 2:
+        if "k_search" in per_unit and w["metric"] == 2 and kernel == "k_search":
             traffic = per_unit["k_search"]["dram_bytes_per_object"] * stats["objects"] * d / 128
         Q = sum(len(g["sel"]) for g in groups)
         return {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"], "traffic": traffic, "peak_kind": peaks["kind"],
-                "kernel": "k_search (the plain traversal; the step's launches of it, one per batch)",
+                "kernel": f"{kernel} (the plain form; the step's launches of it, one per batch)",
                 "alg_bytes_per_step": alg_bytes,
-                "per_query": {"leaf_objects": stats["objects"] / Q, "pivots": stats["pivots"] / Q,
+                "per_query": {"pairs" if swept else "leaf_objects": stats["objects"] / Q, "pivots": stats["pivots"] / Q,
                               "exact_rechecks": stats["exact"] / Q}}
     Q = sum(len(g["sel"]) for g in groups)
     kp = (d + 63) // 64 * 64

@@ -3,8 +3,8 @@
 // As sweep.cu, with 32 queries per tile: the ring bounds keep the cut nodes
 // that some query of the tile can reach, and every object of those is tested
 // against the tile's queries.  The traversal spent 166 ms on 10,000 range-2
-// queries over 1,000,000 words: a leaf of ten strings keeps few of a CTA's
-// threads busy and every query reads the signatures and strings it reaches
+// queries over 1,000,000 words (8.8 here): a leaf of ten strings keeps few of a
+// CTA's threads busy and every query reads the signatures and strings it reaches
 // for itself.  Here
 //
 //   * a thread holds one object's character counts (metric.cuh, str_sig) in

@@ -37,7 +37,8 @@ extern "C" {
 #define GTS_METRIC_EDIT 6
 
 /* Search forms. */
-#define GTS_FORM_PLAIN 0     /* traversal + FP32 filter + exact recheck */
+#define GTS_FORM_PLAIN 0     /* ring bounds + FP32 filter + exact recheck, batched over row tiles
+                                (the pivot-tree traversal below its sizes and for what it leaves) */
 #define GTS_FORM_FAST 1      /* learned radius + BF16 tensor-core filter + exact recheck (L2) */
 #define GTS_FORM_PLAIN_LEARNED 2  /* plain traversal seeded by the learned radius (L2, after
                                      gts_learn_radius; otherwise the plain form) */
@@ -58,8 +59,10 @@ typedef struct {
                             form runs its queries in runs whose scratch fits (at most 32,768
                             queries, halved in 128-query tiles), the seeded plain form in
                             chunks, the update path its queries in batches; a call that cannot
-                            fit one tile / query returns GTS_ERR_NOMEM.  The plain traversal
-                            itself holds no per-query device memory.  Negative: invalid. */
+                            fit one tile / query returns GTS_ERR_NOMEM.  The plain form's
+                            sweep sizes its runs to it and leaves a batch of which not one
+                            tile fits to the traversal, which holds no per-query device
+                            memory.  Negative: invalid. */
 } gts_params;
 
 typedef struct {
@@ -136,8 +139,9 @@ int gts_index_set_stream(gts_index *idx, void *stream);
 
 /* Work counters of the last search call on this handle (no reference
  * counterpart; the reference prints only wall-clock times, main.cu:106-109).
- * out8[0] plain form: leaf objects read; fast form: operand blocks streamed
- * out8[1] plain form: pivots evaluated;  fast form: bytes streamed
+ * out8[0] plain form: leaf objects read (the sweep: (query, row) pairs of its
+ *         tiles); fast form: operand blocks streamed
+ * out8[1] traversal: pivots evaluated;  fast form: bytes streamed
  * out8[2] exact (reference-order) recomputations
  * out8[3] queries finished by the plain traversal
  * out8[4] fast form: queries answered again on the plain path
@@ -203,7 +207,9 @@ int gts_fast_autotune_reset(gts_index *idx);
  * once, about 1,800 on a B200) times 128 / 256 / 512 on its leading sample
  * and keeps the fastest (the answers do not depend on it); range ids take
  * the range-count choice.  *threads = 0 means not tuned yet (256 is used).
- * _set pins it (128, 256, 512; 0 = tune again). */
+ * Batches that the sweep or the warp-per-query range counts answer tune
+ * nothing.  _set pins it (128, 256, 512; 0 = tune again) and with it the
+ * traversal, for that mode. */
 int gts_plain_threads(const gts_index *idx, int mode, int *threads);
 int gts_plain_threads_set(gts_index *idx, int mode, int threads);
 
@@ -213,7 +219,8 @@ int gts_plain_threads_set(gts_index *idx, int mode, int threads);
  * objects in its CTA; then its older pending subtrees are handed over as
  * (query, node) work items, which the next launch spreads over every CTA
  * (their counts add up), so a few heavy queries do not leave the GPU idle
- * behind them.  objects = 0 turns this off, < 0 leaves it (default 32768).
+ * behind them.  objects = 0 turns this off, < 0 leaves it (default 32768);
+ * setting it pins range counts and ids to the traversal.
  * *items_handed (nullable): items handed over since the index was built. */
 int gts_plain_split(gts_index *idx, int objects, long long *items_handed);
 
