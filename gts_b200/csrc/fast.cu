@@ -2317,8 +2317,8 @@ static int rerun_failed(gts_index *idx, FastCall &fc, const FastCfg &cfg, int st
         // store) go through the tile filter, whose running bound tightens
         FastCfg c = cfg;
         if (stage == 1) {
+            if (c.flat) c.cg = fast_default_cfg(idx, k).cg;   // as many as the heaps allow
             c.blk = c.flat = false;
-            c.cg = fast_default_cfg(idx, k).cg;
         }
         if ((rc = fast_run(idx, fc.region, fc.region_bytes, b.sub_q, n, k, c, false,
                            stage == 1 && r2_prev ? b.sub_r2 : nullptr, b.sub_kth, sub_ids, sub_dis,
