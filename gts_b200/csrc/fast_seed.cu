@@ -36,11 +36,12 @@ constexpr int kSdMergeAt = 32;         // merge a row's waiting values from this
 constexpr int kNbrKeep = 32;           // nearest centres kept per block (kSeedNbr of them used)
 constexpr int kNbrPend = 64;
 // Weak seeds: k = 2^kWkFirst on, more than 1.5 times (squared) the smallest of
-// the neighbourhood; at most one object in kWkShare is looked at again, over
-// its kWkBlocks nearest blocks.
+// the neighbourhood; at most one object in kWkShare, and kWkMax in all, is
+// looked at again, over its kWkBlocks nearest blocks.  Each reads every centre:
+// kWkMax of them cost a few per cent of the seed table at any size.
 constexpr int kWkFirst = 3, kWkCols = kSelfKN - kWkFirst;
 constexpr float kWkRatio = 2.25f;
-constexpr int kWkShare = 64;
+constexpr int kWkShare = 64, kWkMax = 4096;
 constexpr int kWkBlocks = 8;
 
 static_assert(kSeedBest == 64 && kSdPend == 64 && kSeedNbr <= kNbrKeep, "list sizes");
@@ -432,9 +433,9 @@ __device__ __forceinline__ void dist4(const float *x, const float *p, size_t ld,
 // itself.  A block that halving left across two groups has its neighbours
 // around its centre, so the few objects of the smaller group get seeds that
 // reach over half of the data: 2 of 10,000 queries at 1,000,000 x 128 made
-// 16,000 of the 33,500 (tile, block) entries of their filter run and 260 of
-// its 780 us.  The centres are read once per object (4.4 MB there, from L2),
-// a pass of about 20 us; 200 objects of that data are listed.
+// 16,000 of the 33,500 (tile, block) entries of their filter run and 280 of
+// its 780 us.  The centres are read once per listed object (4.4 MB there, from
+// L2), which is why their number is bounded.
 __global__ void __launch_bounds__(kSdThreads) k_fast_weak(FastSummary bs, int nb, int kp, int cap,
                                                           const int *__restrict__ list, const int *__restrict__ cnt)
 {
@@ -528,7 +529,7 @@ int seed_table_build(const FastSummary &bs, int nb, int num, const FastShape &fs
     k_fast_nbrs_merge<<<(nb + 7) / 8, 256, 0, st>>>(nb, slices, part, bs.nbr);
     k_fast_selfk<<<nb, kSdThreads, sizeof(SelfkSmem), st>>>(bs, fs.kp, bs.nbr);
     int *bmin = scratch, *cnt = bmin + (size_t)nb * kWkCols, *list = cnt + 1;
-    const int cap = num / kWkShare + 1;
+    const int cap = std::min(num / kWkShare, kWkMax) + 1;
     GTS_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int), st));
     k_fast_seed_min<<<nb, kFB, 0, st>>>(bs, bmin);
     k_fast_weak_list<<<nb, kFB, 0, st>>>(bs, bmin, cap, list, cnt);
