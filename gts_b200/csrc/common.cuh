@@ -52,7 +52,12 @@ enum KernelStatus : int {
     kKsStackOverflow = 1,
     kKsBadNode = 2,
     kKsBadQuery = 3,
+    kKsBadFastQuery = 1 << 12,   // the fast form met an id out of range (above every filter error)
 };
+
+// An id given in device memory, kept inside the index: kernels that cannot
+// leave a query out work on object 0 in its place, and the call reports it.
+__device__ __forceinline__ int known_id(int id, int num) { return id >= 0 && id < num ? id : 0; }
 
 }  // namespace gts
 

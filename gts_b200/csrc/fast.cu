@@ -240,8 +240,9 @@ __global__ void __launch_bounds__(256) k_fast_sbprep(int dim, const float *__res
 // the CTA reads them coalesced (a warp reads 32 consecutive values of one
 // row, all of a thread's loads in flight at once), then each thread converts
 // its own query's row; |q|^2 is summed in column order as before.
-__global__ void __launch_bounds__(128) k_fast_arec(const float *__restrict__ rows, const int *__restrict__ qids,
-                                                   const int *__restrict__ order, int qnum, int dim, FastShape fs,
+__global__ void __launch_bounds__(128) k_fast_arec(const float *__restrict__ rows, int num,
+                                                   const int *__restrict__ qids, const int *__restrict__ order,
+                                                   int qnum, int dim, FastShape fs,
                                                    unsigned char *__restrict__ arec, float *__restrict__ qt)
 {
     __shared__ float sx[kFT][64 + 1];
@@ -252,7 +253,7 @@ __global__ void __launch_bounds__(128) k_fast_arec(const float *__restrict__ row
     int4 *info = reinterpret_cast<int4 *>(A_lo + fs.atile_bytes);
     const int slot = tile * kFT + lq;
     const int qi = slot < qnum ? order[slot] : -1;
-    rid[lq] = qi >= 0 ? qids[qi] : -1;
+    rid[lq] = qi >= 0 ? known_id(qids[qi], num) : -1;
     __syncthreads();
     double acc = 0.0;
     for (int c0 = 0; c0 < fs.kp; c0 += 64) {
@@ -295,11 +296,11 @@ __global__ void __launch_bounds__(128) k_fast_arec(const float *__restrict__ row
 
 // Seeds from the table: one thread per query (jk: the smallest power of two
 // 2^jk >= k).
-__global__ void k_fast_seed_tab(const int *__restrict__ qids, int qnum, const int *__restrict__ pos_of,
+__global__ void k_fast_seed_tab(const int *__restrict__ qids, int qnum, int num, const int *__restrict__ pos_of,
                                 const int *__restrict__ selfk, int jk, int *__restrict__ r2_bits)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < qnum) atomicMin(&r2_bits[i], selfk[(size_t)pos_of[qids[i]] * kSelfK + jk]);
+    if (i < qnum) atomicMin(&r2_bits[i], selfk[(size_t)pos_of[known_id(qids[i], num)] * kSelfK + jk]);
 }
 
 // ---------------------------------------------------------------- pruning
@@ -1165,7 +1166,7 @@ __global__ void __launch_bounds__(128) k_fast_final(const float *__restrict__ ro
     for (int wi = blockIdx.x; wi < nwork; wi += gridDim.x) {
     __syncthreads();   // the previous query's shared state is consumed
     const int q = only ? only[wi] : wi;
-    const int qid = qids[q];
+    const int qid = known_id(qids[q], num);
     const int cnt = cand_cnt[q];
     if (cnt > CAP) {
         if (t == 0) {
@@ -1418,7 +1419,7 @@ __global__ void __launch_bounds__(32 * kFinWarps) k_fast_final_warp(
             else overflow[atomicAdd(n_overflow, 1)] = q;
         }
     } else if (q < qnum) {
-        const int qid = qids[q];
+        const int qid = known_id(qids[q], num);
         float R2 = __int_as_float(r2_bits[q]);
         const bool have = lane < cnt;
         const size_t cb = (size_t)q * kFCand + lane;
@@ -1625,14 +1626,18 @@ __global__ void __launch_bounds__(kOrderThreads) k_fast_order(const int *__restr
 // sort key (the block of the query's slot) with its index; over the grid:
 // the run's counters, the tiles' block counts and the superblock mask words
 // cleared, a range run's counts (rcnt) cleared, and the run counted in stats[6].
-__global__ void k_fast_begin(int qnum, const int *__restrict__ qids, const int *__restrict__ pos_of,
+// An id out of range raises the status; the run then works on object 0.
+__global__ void k_fast_begin(int qnum, const int *__restrict__ qids, int num, const int *__restrict__ pos_of,
                              const int *__restrict__ selfk, int jk, const int *__restrict__ carry, int *cand_cnt,
                              int *r2_bits, int *keys, int *vals, int *ctr, int nctr, int *bcnt, int ntiles,
-                             uint32_t *sb_mask, int nmask, int start, int *rcnt, unsigned long long *stats)
+                             uint32_t *sb_mask, int nmask, int start, int *rcnt, int *status,
+                             unsigned long long *stats)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     if (i < qnum) {
-        const int pos = pos_of[qids[i]];
+        const int qid = qids[i], id = known_id(qid, num);
+        if (id != qid) atomicMax(status, (int)kKsBadFastQuery);
+        const int pos = pos_of[id];
         if (rcnt) rcnt[i] = 0;
         int r2 = carry ? carry[i] : start;
         if (selfk) r2 = min(r2, selfk[(size_t)pos * kSelfK + jk]);   // non-negative floats order as ints
@@ -2048,13 +2053,14 @@ static int fast_run_enqueue(gts_index *idx, const RunBufs &r, const int *d_qids,
     // bound is applied after it (the smaller of the two is used, and queries
     // it under-predicts are answered again)
     const int nsbw = (idx->fast_nsb + 31) / 32;
-    k_fast_begin<<<(qnum + 255) / 256, 256, 0, st>>>(qnum, d_qids, bs.pos, learned ? nullptr : bs.selfk, jk, carry,
-                                                     r.ccnt, r.r2, r.keys, r.vals, r.ctr, 8, r.bcnt, ntiles, r.sb_mask,
-                                                     ntiles * nsbw, kFltMaxBits, nullptr, idx->d_stats);
+    k_fast_begin<<<(qnum + 255) / 256, 256, 0, st>>>(qnum, d_qids, idx->num, bs.pos, learned ? nullptr : bs.selfk,
+                                                     jk, carry, r.ccnt, r.r2, r.keys, r.vals, r.ctr, 8, r.bcnt, ntiles,
+                                                     r.sb_mask, ntiles * nsbw, kFltMaxBits, nullptr, idx->d_status,
+                                                     idx->d_stats);
     idx->kernel_launches++;
     if (learned) {
         if ((rc = mlp_seed(idx, d_qids, qnum, k, r.r2, st))) return rc;
-        k_fast_seed_tab<<<(qnum + 255) / 256, 256, 0, st>>>(d_qids, qnum, bs.pos, bs.selfk, jk, r.r2);
+        k_fast_seed_tab<<<(qnum + 255) / 256, 256, 0, st>>>(d_qids, qnum, idx->num, bs.pos, bs.selfk, jk, r.r2);
         idx->kernel_launches++;
     }
     if ((rc = order_enqueue(idx, r, qnum, st))) return rc;
@@ -2063,7 +2069,7 @@ static int fast_run_enqueue(gts_index *idx, const RunBufs &r, const int *d_qids,
         GTS_CUDA_TRY(cudaMemsetAsync(r.bq_cnt, 0, sizeof(int) * nb, st));
         GTS_CUDA_TRY(cudaMemsetAsync(r.bq_fill, 0, sizeof(int) * nb, st));
     }
-    k_fast_arec<<<ntiles, 128, 0, st>>>(idx->rows, d_qids, r.order, qnum, idx->dim, fs, r.arec, r.qt);
+    k_fast_arec<<<ntiles, 128, 0, st>>>(idx->rows, idx->num, d_qids, r.order, qnum, idx->dim, fs, r.arec, r.qt);
     idx->kernel_launches++;
     bool listed = false;   // the filter's work items already made by the pruning
     if ((rc = prune_enqueue(idx, fs, bs, r, ntiles, blk, blk ? 0 : cfg.item, &listed, st))) return rc;
@@ -2204,6 +2210,11 @@ static int fast_run_enqueue(gts_index *idx, const RunBufs &r, const int *d_qids,
     return GTS_OK;
 }
 
+// A run met a query id out of range (device ids are not seen on the host
+// before): the callers answer the batch by the plain traversal, which leaves
+// such a query out, marks its answer and reports it.
+constexpr int kRcBadId = -100;
+
 // After a run: kernel status and failure count back on the host.
 static int fast_run_finish(gts_index *idx, const RunBufs &r, int *n_fail, int **r2_out, bool timed, cudaStream_t st)
 {
@@ -2211,6 +2222,7 @@ static int fast_run_finish(gts_index *idx, const RunBufs &r, int *n_fail, int **
     GTS_CUDA_TRY(cudaMemcpyAsync(&status, idx->d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     GTS_CUDA_TRY(cudaMemcpyAsync(n_fail, r.ctr, sizeof(int), cudaMemcpyDeviceToHost, st));
     GTS_CUDA_TRY(cudaStreamSynchronize(st));
+    if (status >= kKsBadFastQuery) return kRcBadId;
     if (status != 0) {
         gts_set_error("tensor-core filter kernel reported status %d (barrier wait gave up)", status);
         return GTS_ERR_KERNEL;
@@ -2570,8 +2582,17 @@ static int run_queries_for_budget(const gts_index *idx, int qnum, F per_run, int
     return GTS_OK;
 }
 
-int search_knn_fast(gts_index *idx, const int *d_qids, int qnum, int k, float *d_kth, int *d_ids,
-                    float *d_dists, cudaStream_t st)
+static int search_knn_by_traversal(gts_index *idx, const int *d_qids, int qnum, int k, float *d_kth, int *d_ids,
+                                   float *d_dists, cudaStream_t st)
+{
+    idx->keep_stats = true;   // not the sweep, which may want more scratch
+    const int rc = search_knn(idx, d_qids, qnum, k, 0, d_kth, d_ids, d_dists, st);
+    idx->keep_stats = false;
+    return rc;
+}
+
+static int search_knn_tiles(gts_index *idx, const int *d_qids, int qnum, int k, float *d_kth, int *d_ids,
+                            float *d_dists, cudaStream_t st)
 {
     int rc = fast_prepare(idx, st);
     if (rc) return rc;
@@ -2611,6 +2632,13 @@ int search_knn_fast(gts_index *idx, const int *d_qids, int qnum, int k, float *d
     return fast_search_cfg(idx, fc, qc, cfg, d_qids, qnum, k, d_kth, d_ids, d_dists, st);
 }
 
+int search_knn_fast(gts_index *idx, const int *d_qids, int qnum, int k, float *d_kth, int *d_ids,
+                    float *d_dists, cudaStream_t st)
+{
+    const int rc = search_knn_tiles(idx, d_qids, qnum, k, d_kth, d_ids, d_dists, st);
+    return rc == kRcBadId ? search_knn_by_traversal(idx, d_qids, qnum, k, d_kth, d_ids, d_dists, st) : rc;
+}
+
 // The filter without the learned seed, with every buffer carved out of
 // `scratch` (bytes long, 256-byte aligned): no device allocation on any
 // path.  The filter records must already exist.  Queries the run could not
@@ -2641,7 +2669,7 @@ int search_knn_fast_fixed(gts_index *idx, const int *d_qids, int qnum, int k, fl
     const FastCfg cfg{false, fast_cg(k), 16};
     if ((rc = fast_run(idx, scratch + bbytes, bytes - bbytes, d_qids, qnum, k, cfg, false, nullptr, d_kth, d_ids, d_dists,
                        b.fail, &n_fail, nullptr, st)))
-        return rc;
+        return rc == kRcBadId ? search_knn_by_traversal(idx, d_qids, qnum, k, d_kth, d_ids, d_dists, st) : rc;
     idx->last_fast_overflow = n_fail;
     if (n_fail == 0) return GTS_OK;
     int *sub_ids = d_ids ? b.sub_ids : nullptr;
@@ -2694,7 +2722,7 @@ __global__ void __launch_bounds__(128) k_fast_range_final(const float *__restric
         if (t == 0) overflow[atomicAdd(n_overflow, 1)] = q;
         return;
     }
-    const int qid = qids[q];
+    const int qid = known_id(qids[q], num);
     if (t == 0) c = 0;
     for (int j = t; j < kp; j += 128) qs[j] = j < dim ? rows[(size_t)qid * dim + j] : 0.f;
     __syncthreads();
@@ -2792,15 +2820,15 @@ int search_range_fast(gts_index *idx, const int *d_qids, int qnum, float r, int 
         RunBufs rb;
         plan_run(idx, n, region, &rb, blk);
         const int nsbw = (nsb + 31) / 32;
-        k_fast_begin<<<(n + 255) / 256, 256, 0, st>>>(n, dq, bs.pos, nullptr, 0, nullptr, rb.ccnt, rb.r2, rb.keys,
-                                                      rb.vals, rb.ctr, 8, rb.bcnt, ntiles, rb.sb_mask, ntiles * nsbw,
-                                                      r2hi_bits, rcnt, idx->d_stats);
+        k_fast_begin<<<(n + 255) / 256, 256, 0, st>>>(n, dq, idx->num, bs.pos, nullptr, 0, nullptr, rb.ccnt, rb.r2,
+                                                      rb.keys, rb.vals, rb.ctr, 8, rb.bcnt, ntiles, rb.sb_mask,
+                                                      ntiles * nsbw, r2hi_bits, rcnt, idx->d_status, idx->d_stats);
         if ((rc = order_enqueue(idx, rb, n, st))) return rc;
         if (blk) {
             GTS_CUDA_TRY(cudaMemsetAsync(rb.bq_cnt, 0, sizeof(int) * nb, st));
             GTS_CUDA_TRY(cudaMemsetAsync(rb.bq_fill, 0, sizeof(int) * nb, st));
         }
-        k_fast_arec<<<ntiles, 128, 0, st>>>(idx->rows, dq, rb.order, n, idx->dim, fs, rb.arec, rb.qt);
+        k_fast_arec<<<ntiles, 128, 0, st>>>(idx->rows, idx->num, dq, rb.order, n, idx->dim, fs, rb.arec, rb.qt);
         bool listed = false;
         if ((rc = prune_enqueue(idx, fs, bs, rb, ntiles, blk, blk ? 0 : 16, &listed, st))) return rc;
         if (!blk && !listed) {
@@ -2885,6 +2913,12 @@ int search_range_fast(gts_index *idx, const int *d_qids, int qnum, float r, int 
         GTS_CUDA_TRY(cudaMemcpyAsync(&status, idx->d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
         GTS_CUDA_TRY(cudaMemcpyAsync(&n_fail, rb.ctr, sizeof(int), cudaMemcpyDeviceToHost, st));
         GTS_CUDA_TRY(cudaStreamSynchronize(st));
+        if (status >= kKsBadFastQuery) {
+            idx->keep_stats = true;
+            rc = search_range(idx, d_qids, qnum, r, d_counts, nullptr, st);
+            idx->keep_stats = false;
+            return rc;
+        }
         if (status != 0) {
             gts_set_error("tensor-core filter kernel reported status %d (barrier wait gave up)", status);
             return GTS_ERR_KERNEL;

@@ -174,7 +174,7 @@ __global__ void k_mlp_adam(float *__restrict__ P, const float *__restrict__ G, f
 // by all its queries.
 constexpr int kInferQ = 32;
 
-__global__ void __launch_bounds__(kMH) k_mlp_infer(const float *__restrict__ rows, int dim,
+__global__ void __launch_bounds__(kMH) k_mlp_infer(const float *__restrict__ rows, int dim, int num,
                                                    const int *__restrict__ qids, int qnum,
                                                    const int *__restrict__ piv, int npiv, int k,
                                                    const float *__restrict__ P, const float *__restrict__ xmu,
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(kMH) k_mlp_infer(const float *__restrict__ row
     {
         const int ql = j >> 2;
         if (ql < nq) {
-            const float *a = rows + (size_t)qids[q0 + ql] * dim;
+            const float *a = rows + (size_t)known_id(qids[q0 + ql], num) * dim;   // the search reports a bad id
             for (int f = j & 3; f < kMFeatPivots; f += 4) {
                 float v = 0.f;
                 if (f < npiv) {
@@ -314,7 +314,7 @@ int mlp_seed(gts_index *idx, const int *d_qids, int qnum, int k, int *d_r2_bits,
 {
     if (qnum <= 0) return GTS_OK;
     k_mlp_infer<<<(qnum + kInferQ - 1) / kInferQ, kMH, 0, st>>>(
-        idx->rows, idx->dim, d_qids, qnum, idx->mlp_piv, idx->mlp_npiv, k, idx->mlp_P, idx->mlp_norm,
+        idx->rows, idx->dim, idx->num, d_qids, qnum, idx->mlp_piv, idx->mlp_npiv, k, idx->mlp_P, idx->mlp_norm,
         idx->mlp_norm + kMIn, idx->mlp_ymu, idx->mlp_ysig, widen_for(idx, k), d_r2_bits);
     idx->kernel_launches++;
     GTS_CUDA_TRY(cudaGetLastError());
