@@ -47,11 +47,14 @@ Pool &pool()
     return *p;
 }
 
-// Device and id of the current context (0 when it cannot be told: no reuse then).
+// Device and id of the current context (0 when it cannot be told: no reuse
+// then).  A thread that has made no CUDA call yet has none: cudaFree(nullptr)
+// makes the device's current in it, as a call of the runtime would.
 void where(int *dev, unsigned long long *ctx)
 {
     *dev = 0;
     *ctx = 0;
+    cudaFree(nullptr);
     cudaGetDevice(dev);
     using GetId = CUresult (*)(CUcontext, unsigned long long *);
     static const GetId get_id = [] {
@@ -99,7 +102,6 @@ cudaError_t dev_malloc(void **p, size_t bytes)
     if (bytes < kPoolMin) return cudaMalloc(p, bytes ? bytes : 1);
     const size_t want = (bytes + kPoolRound - 1) / kPoolRound * kPoolRound;
     Block b{nullptr, want, 0, 0};
-    cudaFree(nullptr);   // a context must be current
     where(&b.dev, &b.ctx);
     Pool &P = pool();
     {

@@ -63,3 +63,21 @@ def test_two_threads_build_and_ask():
     for t in threads:
         t.join()
     assert not bad
+
+
+def test_an_index_freed_by_another_thread_gives_its_blocks_back():
+    """The freeing thread has made no CUDA call before."""
+    import torch
+    rows = G.gmm_rows(300_000, 64, 16, 0.3, seed=6)   # 77 MB a copy
+    gts.Index(rows[:1000], 2, max_h=2).close()
+    _release()
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    for _ in range(3):
+        idx = gts.Index(rows, 2, max_h=5)
+        idx.prepare()
+        t = threading.Thread(target=idx.close)
+        t.start()
+        t.join()
+    _release()
+    assert free0 - torch.cuda.mem_get_info()[0] < 32e6
