@@ -245,7 +245,8 @@ __global__ void k_permute(int n, int dim, int metric, const int *id_list, const 
 
 // The nodes as records, and the batched sweep's cut nodes and their ancestors
 // (index.cuh); a CTA
-// appends its nodes in order, so lists stay nearly in position order.
+// appends its nodes in order, so lists stay nearly in position order.  Also
+// the number of childless nodes, counts[2].
 __global__ void __launch_bounds__(256) k_cut_lists(int mnn, int order, const uint8_t *flags, const int *size,
                                                    const int *pivot, const int *lid, const float *min_dis, int *cut,
                                                    int *anc, int *anc_idx, int *counts, int4 *rec)
@@ -253,6 +254,8 @@ __global__ void __launch_bounds__(256) k_cut_lists(int mnn, int order, const uin
     __shared__ int base[2], woff[2][8];
     const int i = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     bool is[2] = {false, false};
+    const int leaves = __syncthreads_count(i < mnn && (flags[i] & kExists) && size[i] > 0 && pivot[i] < 0);
+    if (threadIdx.x == 0 && leaves) atomicAdd(&counts[2], leaves);
     // a child that does not exist still bounds its neighbour's ring by its min_dis (0)
     if (i < mnn) rec[i] = make_int4(__float_as_int(min_dis[i]), (flags[i] & kExists) ? size[i] : 0, lid[i], pivot[i]);
     if (i < mnn && (flags[i] & kExists) && size[i] > 0) {
@@ -378,7 +381,7 @@ void free_tree(gts_index *idx)
     idx->node_min_dis = nullptr; idx->node_flags = nullptr;
     idx->cut_node = nullptr; idx->cut_anc = nullptr; idx->cut_anc_idx = nullptr; idx->tnorm = nullptr;
     idx->node_rec = nullptr;
-    idx->ncut = idx->ncut_anc = 0;
+    idx->ncut = idx->ncut_anc = idx->nleaf = 0;
 }
 
 void free_data(gts_index *idx)
@@ -453,7 +456,7 @@ static int build_tree_impl(gts_index *idx, cudaStream_t s)
     ALLOC(sc.split, mnn);
     ALLOC(sc.posv, n);
     ALLOC(sc.posv_alt, n);
-    ALLOC(sc.nsplit, 3);   // nodes still to split; cut nodes, their ancestors
+    ALLOC(sc.nsplit, 4);   // nodes still to split; cut nodes, their ancestors, childless nodes
 #undef ALLOC
     int lid_bits = 1;
     while (lid_bits < 31 && (1 << lid_bits) < n) lid_bits++;
@@ -518,16 +521,17 @@ static int build_tree_impl(gts_index *idx, cudaStream_t s)
     if (idx->metric == kEdit) k_str_sig<<<grid_for((size_t)n, 256), 256, 0, s>>>(n, idx->tstrs, idx->tlens, idx->tsig,
                                                                              idx->tpack);
     if (idx->metric == kAngle) k_row_norms<<<grid_for((size_t)n, 256), 256, 0, s>>>(n, idx->dim, idx->trows, idx->tnorm);
-    GTS_CUDA_TRY(cudaMemsetAsync(sc.nsplit + 1, 0, 2 * sizeof(int), s));
+    GTS_CUDA_TRY(cudaMemsetAsync(sc.nsplit + 1, 0, 3 * sizeof(int), s));
     k_cut_lists<<<(mnn + 255) / 256, 256, 0, s>>>(mnn, O, idx->node_flags, idx->node_size, idx->node_pivot, idx->node_lid,
                                                   idx->node_min_dis, idx->cut_node, idx->cut_anc, idx->cut_anc_idx,
                                                   sc.nsplit + 1, idx->node_rec);
-    int ncuts[2] = {0, 0};
+    int ncuts[3] = {0, 0, 0};
     GTS_CUDA_TRY(cudaMemcpyAsync(ncuts, sc.nsplit + 1, sizeof(ncuts), cudaMemcpyDeviceToHost, s));
     GTS_CUDA_TRY(cudaStreamSynchronize(s));
     GTS_CUDA_TRY(cudaGetLastError());
     idx->ncut = ncuts[0];
     idx->ncut_anc = ncuts[1];
+    idx->nleaf = ncuts[2];
     return GTS_OK;
 }
 

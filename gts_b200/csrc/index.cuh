@@ -25,6 +25,7 @@ struct gts_index {
     // the norms of the rows in tree order
     int *cut_node = nullptr, *cut_anc = nullptr, *cut_anc_idx = nullptr;
     int ncut = 0, ncut_anc = 0;
+    int nleaf = 0;              // childless nodes with objects
     float *tnorm = nullptr;
     int4 *node_rec = nullptr;   // per node: (min_dis bits, size, first position, pivot or -1), size 0 where none exists
 
@@ -54,6 +55,8 @@ struct gts_index {
     // autotuned threads per query CTA of the plain traversal per search mode
     // (kNN, range count, range ids; search.cu), 0 = not tuned
     int plain_nt[3] = {};
+    // its query CTAs of 128 / 256 / 512 threads resident at once (0: not asked yet)
+    int cta_resident[3] = {};
     // set by a caller: pinned threads or a hand-over threshold choose the
     // traversal over the batched sweep
     bool plain_pinned[3] = {};

@@ -596,7 +596,7 @@ static int launch_search_nt(gts_index *idx, const SearchArgs &a, cudaStream_t st
 {
     const size_t smem = sizeof(SearchSmem);
     GTS_CUDA_TRY(cudaFuncSetAttribute(k_search<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int grid = search_resident<NT>();
+    int grid = idx->cta_resident[NT == 128 ? 0 : NT == 256 ? 1 : 2];
     if (grid > a.qnum) grid = a.qnum;
     k_search<NT><<<grid, NT, smem, st>>>(a);
     idx->kernel_launches++;
@@ -615,9 +615,9 @@ static int launch_search(gts_index *idx, const SearchArgs &a, int nt, cudaStream
 }
 
 // Queries of a thread-count timing: four times the most CTAs resident at once.
-static int plain_tune_sample()
+static int plain_tune_sample(const gts_index *idx)
 {
-    return 4 * std::max(search_resident<128>(), std::max(search_resident<256>(), search_resident<512>()));
+    return 4 * std::max(idx->cta_resident[0], std::max(idx->cta_resident[1], idx->cta_resident[2]));
 }
 
 // Times 128 / 256 / 512 threads per query CTA on the batch's leading queries
@@ -636,7 +636,7 @@ static int plain_autotune(gts_index *idx, const SearchArgs &a, cudaStream_t st, 
         *best_nt = idx->plain_nt[kModeRangeCount];
         return GTS_OK;
     }
-    const int sample = plain_tune_sample();
+    const int sample = plain_tune_sample(idx);
     if (a.qnum < 2 * sample) return GTS_OK;
     SearchArgs t = a;
     t.seed_r2_bits = nullptr;
@@ -753,6 +753,11 @@ void fill_search_args(gts_index *idx, SearchArgs &a)
     a.counter = idx->d_counter;
     a.stats = idx->d_stats;
     a.status = idx->d_status;
+    if (!idx->cta_resident[0]) {
+        idx->cta_resident[0] = search_resident<128>();
+        idx->cta_resident[1] = search_resident<256>();
+        idx->cta_resident[2] = search_resident<512>();
+    }
     if (idx->metric == kAngle) {
         a.rel_eps = 1e-5f;
         a.abs_eps = 0.05f;
@@ -789,7 +794,7 @@ static int run_search(gts_index *idx, SearchArgs &a, cudaStream_t st)
         if (rc) return rc;
         if (swept) {
             // where the sweep answers the large batches the traversal keeps its default
-            if (!idx->plain_nt[slot] && a.qnum >= 2 * plain_tune_sample()) idx->plain_nt[slot] = kPlainDefaultThreads;
+            if (!idx->plain_nt[slot] && a.qnum >= 2 * plain_tune_sample(idx)) idx->plain_nt[slot] = kPlainDefaultThreads;
             if (n_left == 0) return GTS_OK;
             a.items_in = items;
             a.qnum = n_left;
@@ -797,7 +802,7 @@ static int run_search(gts_index *idx, SearchArgs &a, cudaStream_t st)
     }
     int nt = idx->plain_nt[slot];
     const bool by_warp = warp_search_takes(idx, a);   // no threads to choose
-    if (by_warp && !nt && !idx->keep_stats && a.qnum >= 2 * plain_tune_sample()) idx->plain_nt[slot] = kPlainDefaultThreads;
+    if (by_warp && !nt && !idx->keep_stats && a.qnum >= 2 * plain_tune_sample(idx)) idx->plain_nt[slot] = kPlainDefaultThreads;
     if (!nt && !idx->keep_stats && !swept && !by_warp) {
         int rc = plain_autotune(idx, a, st, &nt);
         if (rc) return rc;

@@ -253,9 +253,22 @@ int launch_warp(gts_index *idx, const SearchArgs &a, cudaStream_t st)
 
 }  // namespace
 
+// While most queries of a batch (or items of a hand-over) have a CTA of their
+// own, 256 threads finish them sooner than a warp each: one query that reaches
+// all of 4,000,000 points of the plane takes 0.84 ms there and 20.1 here, one
+// of 0.1 % of 1,000,000 x 8 0.41 against 1.95.  Once they queue for the CTAs
+// (296 resident on a B200) warps win: on small leaves from about half as many
+// again (444 queries of 0.1 % over 1,000,000 x 8: 1.20 ms by CTAs, 1.26 by
+// warps; 600: 1.40 and 1.30; of 10 %: 15.5 and 4.4), on leaves of more than a
+// warp's rows, which keep a CTA's threads busy, from four times as many (888
+// queries: 3.1 and 4.0, 1,200: 4.3 and 4.0).
+constexpr int kWsLeafRows = 32;
+
 bool warp_search_takes(const gts_index *idx, const SearchArgs &a)
 {
     if (a.mode != kModeRangeCount && a.mode != kModeRangeTimed) return false;
+    const bool wide_leaves = idx->num > (long long)kWsLeafRows * std::max(idx->nleaf, 1);
+    if (2 * a.qnum < (wide_leaves ? 8 : 3) * idx->cta_resident[1]) return false;
     const bool metric = idx->metric == kL2 || idx->metric == kL1 || idx->metric == kLinf;
     // radii whose square leaves FP32's range, or negative ones, stay with the CTA traversal
     return metric && idx->dim <= kLaneRowDim && idx->params.tree_order <= kWsOrder && !a.deleted &&

@@ -1,0 +1,43 @@
+"""Which of the plain form's searches answers a batch: the one that is chosen
+is not slower than the per-query traversal (pinned threads), for few and many
+queries, selective and wide radii, small and large leaves; and the answers are
+the traversal's on both sides of each line the rules draw."""
+import time
+
+import numpy as np
+import pytest
+
+import gts_b200 as gts
+from gts_b200 import datagen as G
+
+pytestmark = pytest.mark.gpu
+
+
+def _median_s(call, reps=7):
+    call()
+    t = []
+    for _ in range(reps):
+        t0 = time.perf_counter()
+        call()
+        t.append(time.perf_counter() - t0)
+    return float(np.median(t))
+
+
+def _not_slower(auto, pinned):
+    """Up to 1.5 times and 40 us more pass: launches are a few us each, and
+    the faults this looks for were 2 to 20 times."""
+    assert auto <= 1.5 * pinned + 40e-6, f"{auto * 1e6:.0f} us against {pinned * 1e6:.0f} us"
+
+
+@pytest.mark.parametrize("n,dim,max_h", [(400_000, 2, 4), (400_000, 8, 4), (200_000, 5, 1), (400_000, 3, 6)])
+def test_few_dimensional_counts(n, dim, max_h):
+    rows = G.gmm_rows(n, dim, 64, 0.2, seed=dim)
+    with gts.Index(rows, 2, max_h=max_h) as a, gts.Index(rows, 2, max_h=max_h) as b:
+        b.set_plain_threads(1, 256)
+        for frac in (1e-4, 0.1):
+            r = float(np.float32(G.quantile_radius(2, frac, 20000, 3, rows=rows)))
+            for nq in (1, 8, 100, 443, 445, 1183, 1185, 2000):   # 296 CTAs are resident on a B200
+                q = G.query_ids(n, nq, nq)
+                np.testing.assert_array_equal(a.range(q, r), b.range(q, r))
+                if nq <= 100:
+                    _not_slower(_median_s(lambda: a.range(q, r)), _median_s(lambda: b.range(q, r)))
