@@ -243,30 +243,34 @@ __global__ void k_permute(int n, int dim, int metric, const int *id_list, const 
     }
 }
 
-// The nodes as records, and the batched sweep's cut nodes and their ancestors
-// (index.cuh); a CTA
-// appends its nodes in order, so lists stay nearly in position order.  Also
-// the number of childless nodes, counts[2].
+// The nodes as records, and the batched sweep's cut nodes, in pieces of at most
+// kCutSize objects, and their ancestors (index.cuh); a CTA appends its nodes
+// in order, so lists stay nearly in position order.  Also the number of
+// childless nodes, counts[2].
 __global__ void __launch_bounds__(256) k_cut_lists(int mnn, int order, const uint8_t *flags, const int *size,
-                                                   const int *pivot, const int *lid, const float *min_dis, int *cut,
+                                                   const int *pivot, const int *lid, const float *min_dis, int2 *cut,
                                                    int *anc, int *anc_idx, int *counts, int4 *rec)
 {
     __shared__ int base[2], woff[2][8];
     const int i = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    bool is[2] = {false, false};
+    bool inner = false;
+    int pieces = 0;
     const int leaves = __syncthreads_count(i < mnn && (flags[i] & kExists) && size[i] > 0 && pivot[i] < 0);
     if (threadIdx.x == 0 && leaves) atomicAdd(&counts[2], leaves);
     // a child that does not exist still bounds its neighbour's ring by its min_dis (0)
     if (i < mnn) rec[i] = make_int4(__float_as_int(min_dis[i]), (flags[i] & kExists) ? size[i] : 0, lid[i], pivot[i]);
     if (i < mnn && (flags[i] & kExists) && size[i] > 0) {
-        is[1] = pivot[i] >= 0 && size[i] > kCutSize;
-        is[0] = !is[1] && (i == 0 || size[(i - 1) / order] > kCutSize);
+        inner = pivot[i] >= 0 && size[i] > kCutSize;
+        if (!inner && (i == 0 || size[(i - 1) / order] > kCutSize)) pieces = (size[i] + kCutSize - 1) / kCutSize;
     }
-    unsigned m[2];
-    for (int u = 0; u < 2; u++) {
-        m[u] = __ballot_sync(0xffffffffu, is[u]);
-        if (lane == 0) woff[u][warp] = __popc(m[u]);
+    const unsigned m = __ballot_sync(0xffffffffu, inner);
+    int incl = pieces;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
     }
+    if (lane == 31) woff[0][warp] = incl;
+    if (lane == 0) woff[1][warp] = __popc(m);
     __syncthreads();
     if (threadIdx.x < 2) {
         const int u = threadIdx.x;
@@ -279,12 +283,18 @@ __global__ void __launch_bounds__(256) k_cut_lists(int mnn, int order, const uin
         base[u] = run ? atomicAdd(&counts[u], run) : 0;
     }
     __syncthreads();
-    for (int u = 0; u < 2; u++)
-        if (is[u]) {
-            const int at = base[u] + woff[u][warp] + __popc(m[u] & ((1u << lane) - 1u));
-            (u == 0 ? cut : anc)[at] = i;
-            if (u == 1) anc_idx[i] = at;
-        }
+    if (inner) {
+        const int at = base[1] + woff[1][warp] + __popc(m & ((1u << lane) - 1u));
+        anc[at] = i;
+        anc_idx[i] = at;
+    }
+    const int at = base[0] + woff[0][warp] + incl - pieces;
+    if (pieces == 1) cut[at] = make_int2(i, 0);
+    for (unsigned todo = __ballot_sync(0xffffffffu, pieces > 1); todo; todo &= todo - 1) {   // a large leaf: the warp together
+        const int from = __ffs(todo) - 1, node = __shfl_sync(0xffffffffu, i, from);
+        const int n = __shfl_sync(0xffffffffu, pieces, from), o = __shfl_sync(0xffffffffu, at, from);
+        for (int j = lane; j < n; j += 32) cut[o + j] = make_int2(node, j * kCutSize);
+    }
 }
 
 // Norms of the rows in tree order, in the angle metric's own arithmetic
@@ -433,7 +443,7 @@ static int build_tree_impl(gts_index *idx, cudaStream_t s)
     ALLOC(idx->node_pivot, mnn);
     ALLOC(idx->node_min_dis, mnn);
     ALLOC(idx->node_flags, mnn);
-    ALLOC(idx->cut_node, mnn);
+    ALLOC(idx->cut_node, (size_t)mnn + n / kCutSize + 1);   // a node's pieces: its share of the objects, rounded up
     ALLOC(idx->cut_anc, mnn);
     ALLOC(idx->cut_anc_idx, mnn);
     ALLOC(idx->node_rec, mnn);

@@ -20,10 +20,12 @@ struct gts_index {
     float *node_min_dis = nullptr;
     uint8_t *node_flags = nullptr;
     // the batched sweep's view of the tree (sweep.cu): its cut nodes (the
-    // topmost nodes of at most kCutSize objects, and larger childless ones),
-    // their ancestors with a node -> ancestor map, and for the angle metric
-    // the norms of the rows in tree order
-    int *cut_node = nullptr, *cut_anc = nullptr, *cut_anc_idx = nullptr;
+    // topmost nodes of at most kCutSize objects, and larger childless ones in
+    // pieces of that size) as (node, the piece's first object), their
+    // ancestors with a node -> ancestor map, and for the angle metric the norms
+    // of the rows in tree order
+    int2 *cut_node = nullptr;
+    int *cut_anc = nullptr, *cut_anc_idx = nullptr;
     int ncut = 0, ncut_anc = 0;
     int nleaf = 0;              // childless nodes with objects
     float *tnorm = nullptr;
@@ -124,7 +126,7 @@ namespace gts {
 //   [7] fast: (query tile, block) pairs tested by the block bound
 constexpr int kStatsN = 8;
 constexpr int kPackChars = 32;
-constexpr int kCutSize = 128;   // objects of a cut node at most, unless it has no children
+constexpr int kCutSize = 128;   // objects of a cut node (or a piece of one) at most
 
 // Build the tree for the data already placed in idx->rows / strs / lens.
 int build_tree(gts_index *idx, cudaStream_t s);

@@ -308,7 +308,8 @@ __global__ void __launch_bounds__(256) k_sw_query(SweepArgs s)
 // ---------------------------------------------------------------- ring bounds
 
 // The cut nodes that some query of tile blockIdx.y can reach: one thread per
-// cut node keeps a mask of the tile's (at most 128) queries and walks its ancestors, as
+// cut node (or piece of one: a warp went over a childless node of 20,000 strings
+// by itself for 1.8 ms) keeps a mask of the tile's (at most 128) queries and walks its ancestors, as
 // the traversal does from above.  The rows of the kept nodes of a CTA's 256
 // are appended to the tile's row list.
 __global__ void __launch_bounds__(256) k_sw_cut(SweepArgs s)
@@ -325,9 +326,10 @@ __global__ void __launch_bounds__(256) k_sw_cut(SweepArgs s)
     const int i = blockIdx.x * 256 + tid;
     int size = 0, lid = 0;
     if (i < s.ncut) {
-        const int node = s.cut[i];
-        size = t.node_size[node];
-        lid = t.node_lid[node];
+        const int2 piece = s.cut[i];
+        const int node = piece.x;
+        size = min(t.node_size[node] - piece.y, kCutSize);
+        lid = t.node_lid[node] + piece.y;
         uint32_t m[4];
 #pragma unroll
         for (int w = 0; w < 4; w++) {
@@ -380,7 +382,7 @@ __global__ void __launch_bounds__(256) k_sw_cut(SweepArgs s)
     };
     const unsigned mine = __ballot_sync(0xffffffffu, size > 0);
     int kept = size;
-    unsigned kb[4] = {0, 0, 0, 0};   // the lane's node: which of its first 128 strings stay
+    unsigned kb[4] = {0, 0, 0, 0};   // the lane's node: which of its strings stay
     if (s.lens_ok)
         for (unsigned todo = mine; todo; todo &= todo - 1) {
             const int from = __ffs(todo) - 1;
@@ -388,11 +390,8 @@ __global__ void __launch_bounds__(256) k_sw_cut(SweepArgs s)
             unsigned b[4];
 #pragma unroll
             for (int u = 0; u < 4; u++) b[u] = __ballot_sync(0xffffffffu, u * 32 + lane < n && fits(l + u * 32 + lane));
-            int c = 0;
-            for (int j = 128 + lane; j < n; j += 32) c += fits(l + j) ? 1 : 0;
-            if (n > 128) c = __reduce_add_sync(0xffffffffu, c);
             if (lane == from) {
-                kept = c;
+                kept = 0;
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
                     kb[u] = b[u];
@@ -433,12 +432,6 @@ __global__ void __launch_bounds__(256) k_sw_cut(SweepArgs s)
         for (int u = 0; u < 4; u++) {
             const unsigned b = __shfl_sync(0xffffffffu, kb[u], from);
             if ((b >> lane) & 1u) dst[o + __popc(b & below)] = l + u * 32 + lane;
-            o += __popc(b);
-        }
-        for (int j0 = 128; j0 < n; j0 += 32) {
-            const bool ok = j0 + lane < n && fits(l + j0 + lane);
-            const unsigned b = __ballot_sync(0xffffffffu, ok);
-            if (ok) dst[o + __popc(b & below)] = l + j0 + lane;
             o += __popc(b);
         }
     }

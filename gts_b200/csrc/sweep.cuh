@@ -15,7 +15,8 @@ struct SweepArgs {
     int q0, nq, ntiles, Qp, ld;         // the run's queries a.qids[q0 ..], padded count, query row stride
     int tq;                             // queries per tile (row lists, ring bounds)
     int ncut, nanc;
-    const int *cut, *anc, *anc_idx;
+    const int2 *cut;                    // (node, first object): pieces of at most kCutSize objects
+    const int *anc, *anc_idx;
     const float *tnorm;                 // angle: norms of the rows in tree order
     int *key, *order;                   // tree position of the query; sorted order -> query of the run
     int *bq;                            // sorted slot -> query of the batch (-1: padding)

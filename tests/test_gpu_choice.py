@@ -41,3 +41,20 @@ def test_few_dimensional_counts(n, dim, max_h):
                 np.testing.assert_array_equal(a.range(q, r), b.range(q, r))
                 if nq <= 100:
                     _not_slower(_median_s(lambda: a.range(q, r)), _median_s(lambda: b.range(q, r)))
+
+
+@pytest.mark.parametrize("n,max_h", [(200_000, 2), (40_000, 1)])   # leaves of 20,000 and 40,000 words
+def test_words_in_large_leaves(n, max_h):
+    strs, lens = G.word_strings(n, 7)
+    with gts.Index(None, 6, strs=strs, lens=lens, max_h=max_h) as a, \
+            gts.Index(None, 6, strs=strs, lens=lens, max_h=max_h) as b:
+        for mode in (0, 1):
+            b.set_plain_threads(mode, 256)
+        for nq in (8, 100):
+            q = G.query_ids(n, nq, nq)
+            for r in (1.0, 3.0):
+                np.testing.assert_array_equal(a.range(q, r), b.range(q, r))
+                _not_slower(_median_s(lambda: a.range(q, r)), _median_s(lambda: b.range(q, r)))
+            for x, y in zip(a.knn(q, 8, return_ids=True), b.knn(q, 8, return_ids=True)):
+                np.testing.assert_array_equal(x, y)
+            _not_slower(_median_s(lambda: a.knn(q, 8)), _median_s(lambda: b.knn(q, 8)))
