@@ -62,6 +62,11 @@ struct SearchArgs {
     int *n_items_out;
     int items_cap;
     int split_objs;   // 0: no hand-over
+    // count_objs > 0: answers nothing; query w * count_step walks the inner
+    // nodes only and adds the objects of the leaves it reaches, at most
+    // count_objs, to *reached
+    int count_objs, count_step;
+    unsigned long long *reached;
     float rel_eps;   // relative pruning slack
     float abs_eps;   // absolute pruning slack
 };
@@ -73,6 +78,9 @@ void fill_search_args(gts_index *idx, SearchArgs &a);
 // (search_warp.cu).
 bool warp_search_takes(const gts_index *idx, const SearchArgs &a);
 int launch_search_warp(gts_index *idx, const SearchArgs &a, cudaStream_t st);
+
+// Whether the batched sweep of rows is one for this batch, by its sizes alone.
+bool sweep_takes(const gts_index *idx, const SearchArgs &a);
 
 // The batched sweep (sweep.cu).  *done = 1: it answered every query of the
 // batch except those it lists (query, 0, 0, 0) in items[0 .. *n_left), which

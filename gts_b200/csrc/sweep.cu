@@ -45,6 +45,7 @@ constexpr int kSwLd = kSwK + 4;        // row stride in shared memory (16-byte r
 constexpr int kSwList = 2048;          // pairs a tile may finish one by one
 constexpr int kSwWindow = 1024;        // objects around a query's place that bound its k-th distance
 constexpr int kSwMaxTiles = 32;        // query tiles per run
+constexpr int kSwFew = 32;             // up to so many queries take the small tile
 constexpr int kSwSample = 16;          // the sample pass looks at every 16th row
 constexpr int kSwSampleMin = 1 << 16;  // objects from which on it pays
 constexpr int kSwRounds = 3;           // further passes over kNN queries whose lists overflowed
@@ -209,6 +210,7 @@ __global__ void __launch_bounds__(kSwThreads) k_sw_seed(SweepArgs s, int window)
     }
 }
 
+// The order to be sorted.
 __global__ void k_sw_iota(int n, int *v)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -249,14 +251,19 @@ __device__ __forceinline__ void sw_thresholds(const DevTree &t, float R, bool ok
 
 // One warp per sorted query slot: its row (zero padded), radius, thresholds
 // on the filter value, and an empty candidate list (the query object itself
-// first: its distance is 0 by definition, search_v2.cuh:338-340).
+// first: its distance is 0 by definition, search_v2.cuh:338-340).  The pass's
+// counters are cleared here too.
 __global__ void __launch_bounds__(256) k_sw_query(SweepArgs s)
 {
     const DevTree &t = s.a.t;
     const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (blockIdx.x == 0) {
+        for (int j = threadIdx.x; j < s.ntiles; j += 256) s.nrows[j] = 0;
+        if (threadIdx.x == 0) s.ctr[0] = 0;
+    }
     if (i >= s.Qp) return;
     const bool have = i < s.nq;
-    const int q = !have ? -1 : (s.again ? s.again[s.q0 + i].x : s.q0 + s.order[i]);   // in the batch
+    const int q = !have ? -1 : (s.again ? s.again[s.q0 + i].x : s.q0 + (s.nq > 128 ? s.order[i] : i));   // in the batch
     if (lane == 0) s.bq[i] = q;
     const int qid = have && !s.a.qrows ? s.a.qids[q] : -1;
     const bool ok = have && (s.a.qrows || (qid >= 0 && qid < t.num));
@@ -266,6 +273,7 @@ __global__ void __launch_bounds__(256) k_sw_query(SweepArgs s)
         float R = -1.f;
         if (ok) R = s.a.mode != kModeKnn ? s.a.r : (s.again ? s.again_R[s.q0 + i] : s.seed[q - s.q0]);
         float vthr, vlow, qn = 0.f;
+        if (have && !ok) atomicMax(s.a.status, (int)kKsBadQuery);
         if (ok && t.metric == kAngle) {
             float sa = 0.f;
             for (int j = 0; j < t.dim; j++) sa = fmaf(src[j], src[j], sa);
@@ -539,26 +547,38 @@ __global__ void __launch_bounds__(kSwThreads) k_sw_pivots(SweepArgs s)
         sw_add<M, QI>(sm.a[ch & 1], sm.b[ch & 1], tq, to, acc);
         __syncthreads();
     }
+    // the bounds, half of the pivots at a time through shared memory: written
+    // out per accumulator they made the single CTA of a small batch take 35 us
+    // at 64 dimensions, in a loop 17
+    constexpr int kQ = 16 * QI, kLd = kQ + 1;
+    float *v = &sm.a[0][0];
+    static_assert(sizeof(sm.a) + sizeof(sm.b) >= sizeof(float) * 64 * kLd, "half a tile of values");
 #pragma unroll
-    for (int i = 0; i < QI; i++) {
-        const int q = q0 + tq + 16 * i;
-        const int self = s.self[q];
+    for (int h = 0; h < 2; h++) {
+#pragma unroll
+        for (int i = 0; i < QI; i++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) v[(to + 16 * c) * kLd + tq + 16 * i] = acc[i][4 * h + c];
+        __syncthreads();
+        const int q = q0 + tid % kQ, self = s.self[q];
         const float qn = s.qnorm[q];
-#pragma unroll
-        for (int c = 0; c < 8; c++) {
-            const int r = to + 16 * c;
-            if (a0 + r >= s.nanc) continue;
+#pragma unroll 1
+        for (int r = tid / kQ; r < 64; r += kSwThreads / kQ) {
+            const int p = 64 * h + r;
+            if (a0 + p >= s.nanc) break;
+            const float x = v[r * kLd + tid % kQ];
             float lo, hi;
             if (M == kAngle) {
-                lo = hi = (float)angle_of_cos_f64(acc[i][c] / (s.tnorm[sm.pos[r]] * qn));
+                lo = hi = (float)angle_of_cos_f64(x / (s.tnorm[sm.pos[p]] * qn));
             } else {
-                lo = sw_lo(M, t.dim, acc[i][c]);
-                hi = sw_hi(M, t.dim, acc[i][c]);
+                lo = sw_lo(M, t.dim, x);
+                hi = sw_hi(M, t.dim, x);
             }
-            if (sm.pos[r] == self) lo = hi = 0.f;
-            s.dlo[(size_t)(a0 + r) * s.Qp + q] = lo;
-            s.dhi[(size_t)(a0 + r) * s.Qp + q] = hi;
+            if (sm.pos[p] == self) lo = hi = 0.f;
+            s.dlo[(size_t)(a0 + p) * s.Qp + q] = lo;
+            s.dhi[(size_t)(a0 + p) * s.Qp + q] = hi;
         }
+        __syncthreads();
     }
 }
 
@@ -1121,21 +1141,46 @@ void sweep_cut_launch(const SweepArgs &s, int ntiles, cudaStream_t st)
     k_sw_cut<<<dim3((s.ncut + 255) / 256, ntiles), 256, 0, st>>>(s);
 }
 
+// The sizes from which on the sweep is the sooner one.  A batch of one tile
+// waits for a chain of stages of 16 dimensions, 2.9 us each for the pivots and
+// 5.2 for the rows (1.1 and 2.2 with the tile of 32 queries).  A CTA of the traversal
+// waits for its query's objects, some 18 ns each, and for a second wave from
+// about 256 queries on; L2 kNN values and angles cost it more per dimension.
+// Traversal and sweep, us, a batch of 100 where not given:
+//   L1 range  1,000 x 1,000  177  775    4,000 x 128  143  183    5,000 x 64  241  159
+//     2,000 x 33, 1,000 queries  275  155    2,000 x 300, 30 queries  131  178
+//   L1 kNN    2,000 x 300    213  348    4,000 x 300  299  345    4,000 x 128, 300 queries  497  252
+//   L2 range  2,000 x 300    249  317    4,000 x 300  318  342    60,000 x 300  2,649  223
+//   L2 kNN      500 x 1,000 1,795 827
+//   angle     2,000 x 33     101  132    1,000 x 300  191  251    4,000 x 64  251  183
+// Objects exactly equal to the query lie in a leaf or two of a deep tree: 0.43 ms
+// for 10,000 queries over 1,000,000 x 128, 0.88 by the sweep.
+static bool sweep_pays(const gts_index *idx, const SearchArgs &a)
+{
+    const long long n = idx->num, d = idx->dim, q = a.qnum;
+    if (n * d < 1 << 16 && n * q < 1 << 20) return false;
+    const bool knn = a.mode == kModeKnn, few = q <= kSwFew;
+    const long long waves = n * std::max(q, 256ll) / 256;   // objects in the traversal's way
+    if (knn && idx->metric == kL2) return true;
+    if (a.mode == kModeRangeIds) return n >= 4 * d;         // two traversals and a sort on the host
+    if (!knn && a.r == 0.f && n <= 32ll * idx->nleaf) return false;
+    if (idx->metric == kAngle) return few ? n * d >= 1 << 17 : waves >= 4096 || (waves >= 2000 && n * d >= 250000);
+    if (idx->metric == kL2) return few ? n >= 2 * d : waves >= 2048 && waves >= 8 * d;
+    return few ? n >= 2048 && (knn || n >= 16 * d) : waves >= 4096 && waves >= (knn ? 8 : 48) * d;
+}
+
 // Batches the sweep takes: row metrics of more dimensions than a lane filters
 // alone, without deletions, learned seeds, or a caller's choice of the
 // traversal (pinned threads, a set hand-over threshold); radii whose squares
 // stay finite.
-static bool sweep_takes(const gts_index *idx, const SearchArgs &a)
+bool sweep_takes(const gts_index *idx, const SearchArgs &a)
 {
     if (idx->metric == kEdit || idx->dim <= kLaneRowDim || idx->dim > 2048 || idx->ncut < 1) return false;
     if (a.deleted || a.seed_r2_bits || a.items_in || a.qstrs) return false;
     const int slot = a.mode == kModeRangeTimed ? kModeRangeCount : a.mode;
     if (idx->plain_pinned[slot] || (a.mode != kModeKnn && idx->plain_split_set)) return false;
     if (a.mode == kModeKnn ? a.k > 128 : !(a.r >= 0.f && a.r <= 1e15f)) return false;
-    // below these sizes the traversal's one launch is as fast (2,000 x 24: 94 us
-    // for a range batch either way; 5,000 x 128 kNN: 640 us for one query
-    // against 130 here)
-    return (long long)idx->num * idx->dim >= 1 << 16 || (long long)idx->num * a.qnum >= 1 << 20;
+    return sweep_pays(idx, a);
 }
 
 namespace {
@@ -1179,13 +1224,11 @@ bool sweep_begin(gts_index *idx, const SearchArgs &a, SweepBatch *b)
 // bounds are known.
 int sweep_pass(gts_index *idx, SweepArgs &s, cudaStream_t st)
 {
-    GTS_CUDA_TRY(cudaMemsetAsync(s.ctr, 0, sizeof(int), st));
-    GTS_CUDA_TRY(cudaMemsetAsync(s.nrows, 0, sizeof(int) * s.ntiles, st));
     k_sw_query<<<(s.Qp + 7) / 8, 256, 0, st>>>(s);
     // 32 queries per tile when there are no more of them: the 128-wide tile
     // would multiply padding
     const bool sampled = s.a.mode == kModeKnn && !s.again && idx->num >= kSwSampleMin;
-    int rc = s.nq <= 32 ? launch_metric<2>(idx, s, sampled, st) : launch_metric<8>(idx, s, sampled, st);
+    int rc = s.nq <= kSwFew ? launch_metric<2>(idx, s, sampled, st) : launch_metric<8>(idx, s, sampled, st);
     if (rc) return rc;
     idx->kernel_launches++;
     return GTS_OK;
@@ -1210,12 +1253,16 @@ int sweep_enqueue(gts_index *idx, SweepBatch &b, int q0, cudaStream_t st)
     s.nq = std::min(b.run, s.a.qnum - q0);
     s.ntiles = (s.nq + 127) / 128;
     int *skey = s.key + s.Qp, *iota = skey + s.Qp;
-    k_sw_seed<<<s.nq, kSwThreads, sizeof(float) * (size_t)idx->dim, st>>>(s, kSwWindow);
-    k_sw_iota<<<(s.nq + 255) / 256, 256, 0, st>>>(s.nq, s.nq > 128 ? iota : s.order);
-    idx->kernel_launches += 2;
-    if (s.nq > 128)   // queries of one tile should be neighbours in the tree order
+    if (s.nq > 128 || s.a.mode == kModeKnn) {   // a tile of range queries needs neither places nor seeds
+        k_sw_seed<<<s.nq, kSwThreads, sizeof(float) * (size_t)idx->dim, st>>>(s, kSwWindow);
+        idx->kernel_launches++;
+    }
+    if (s.nq > 128) {   // queries of one tile should be neighbours in the tree order
+        k_sw_iota<<<(s.nq + 255) / 256, 256, 0, st>>>(s.nq, iota);
+        idx->kernel_launches++;
         GTS_CUDA_TRY(cub::DeviceRadixSort::SortPairs(b.cub, b.cub_bytes, s.key, skey, iota, s.order, s.nq, 0, key_bits,
                                                      st));
+    }
     return sweep_pass(idx, s, st);
 }
 

@@ -58,3 +58,41 @@ def test_words_in_large_leaves(n, max_h):
             for x, y in zip(a.knn(q, 8, return_ids=True), b.knn(q, 8, return_ids=True)):
                 np.testing.assert_array_equal(x, y)
             _not_slower(_median_s(lambda: a.knn(q, 8)), _median_s(lambda: b.knn(q, 8)))
+
+
+@pytest.mark.parametrize("metric,n,dim,nq", [
+    (1, 1000, 1000, 100), (0, 1000, 300, 60), (2, 1000, 300, 100), (5, 1000, 300, 100), (1, 2000, 33, 100),
+    (1, 1000, 1000, 20), (2, 8000, 9, 100), (1, 5000, 64, 100), (5, 4000, 64, 40), (2, 2100, 128, 30)])
+def test_small_indexes(metric, n, dim, nq):
+    rows = G.gmm_rows(n, dim, 16, 0.3, seed=n + dim) + np.float32(0.5)
+    q = G.query_ids(n, nq, nq)
+    with gts.Index(rows, metric, max_h=3) as a, gts.Index(rows, metric, max_h=3) as b:
+        for mode in (0, 1, 2):
+            b.set_plain_threads(mode, 256)
+        for k in (1, 16):
+            for x, y in zip(a.knn(q, k, return_ids=True), b.knn(q, k, return_ids=True)):
+                np.testing.assert_array_equal(x, y)
+            _not_slower(_median_s(lambda: a.knn(q, k)), _median_s(lambda: b.knn(q, k)))
+        r = float(np.median(a.knn(q, 16)))
+        np.testing.assert_array_equal(a.range(q, r), b.range(q, r))
+        for x, y in zip(a.range_ids(q, r), b.range_ids(q, r)):
+            np.testing.assert_array_equal(x, y)
+        _not_slower(_median_s(lambda: a.range(q, r)), _median_s(lambda: b.range(q, r)))
+
+
+@pytest.mark.parametrize("n,dim", [(1_000_000, 9), (1_000_000, 16), (500_000, 64)])
+def test_selective_counts(n, dim):
+    """Radii of no, few and many hits; the batch is asked from 1,024 queries on."""
+    rng = np.random.default_rng(dim)
+    rows = rng.standard_normal((n, dim), dtype=np.float32) * np.float32(0.15)
+    rows += (rng.random((1024, dim), dtype=np.float32) * 4)[rng.integers(0, 1024, n)]
+    rows[:500] = rows[500:1000]
+    with gts.Index(rows, 2, max_h=6) as a, gts.Index(rows, 2, max_h=6) as b:
+        b.set_plain_threads(1, 256)
+        near = float(np.median(a.knn(G.query_ids(n, 64, 1), 2)))
+        for nq in (33, 1023, 1024, 6000):
+            q = np.concatenate([np.arange(20), G.query_ids(n, nq - 20, nq)]).astype(np.int32)
+            for r in (0.0, 1e-3, near / 4, near, 1.5 * near):
+                np.testing.assert_array_equal(a.range(q, r), b.range(q, r))
+                if nq >= 1024:
+                    _not_slower(_median_s(lambda: a.range(q, r), 3), _median_s(lambda: b.range(q, r), 3))
