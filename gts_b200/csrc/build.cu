@@ -199,12 +199,17 @@ __global__ void k_clear_level(int start, int nb, uint8_t *split)
 // Tree-order copies of the data so that a leaf's objects are contiguous.
 // Character-class signatures of the strings in tree order (edit lower bounds)
 // and their first kPackChars characters (zeros past the end) as two 16-byte words.
-__global__ void k_str_sig(int n, const char *tstrs, const int *tlens, uint4 *tsig, uint4 *tpack)
+// In lens: characters altogether, strings of more than 32 and of more than 64.
+__global__ void k_str_sig(int n, const char *tstrs, const int *tlens, uint4 *tsig, uint4 *tpack, unsigned long long *lens)
 {
+    unsigned chars = 0, over32 = 0, over64 = 0;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < (size_t)n; i += (size_t)gridDim.x * blockDim.x) {
         const char *s = tstrs + i * kStrStride;
         const int len = tlens[i];
         tsig[i] = str_sig(s, len);
+        chars += max(len, 0);
+        over32 += len > 32;
+        over64 += len > 64;
         uint32_t w[kPackChars / 4];
 #pragma unroll
         for (int k = 0; k < kPackChars / 4; k++) {
@@ -216,6 +221,14 @@ __global__ void k_str_sig(int n, const char *tstrs, const int *tlens, uint4 *tsi
         }
         tpack[2 * i] = make_uint4(w[0], w[1], w[2], w[3]);
         tpack[2 * i + 1] = make_uint4(w[4], w[5], w[6], w[7]);
+    }
+    chars = __reduce_add_sync(0xffffffffu, chars);
+    over32 = __reduce_add_sync(0xffffffffu, over32);
+    over64 = __reduce_add_sync(0xffffffffu, over64);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&lens[0], (unsigned long long)chars);
+        atomicAdd(&lens[1], (unsigned long long)over32);
+        atomicAdd(&lens[2], (unsigned long long)over64);
     }
 }
 
@@ -409,10 +422,11 @@ struct BuildScratch {
     int *node_of_pos = nullptr, *ids_alt = nullptr, *posv = nullptr, *posv_alt = nullptr, *nsplit = nullptr;
     double *key = nullptr, *key_alt = nullptr;
     uint8_t *split = nullptr;
+    unsigned long long *lens = nullptr;
     void *temp = nullptr;
     ~BuildScratch()
     {
-        void *ps[] = {node_of_pos, ids_alt, posv, posv_alt, nsplit, key, key_alt, split, temp};
+        void *ps[] = {node_of_pos, ids_alt, posv, posv_alt, nsplit, key, key_alt, split, lens, temp};
         for (void *p : ps)
             if (p) dev_free(p);
     }
@@ -466,6 +480,7 @@ static int build_tree_impl(gts_index *idx, cudaStream_t s)
     ALLOC(sc.split, mnn);
     ALLOC(sc.posv, n);
     ALLOC(sc.posv_alt, n);
+    ALLOC(sc.lens, 3);
     ALLOC(sc.nsplit, 4);   // nodes still to split; cut nodes, their ancestors, childless nodes
 #undef ALLOC
     int lid_bits = 1;
@@ -528,20 +543,24 @@ static int build_tree_impl(gts_index *idx, cudaStream_t s)
     k_permute<<<grid_for(work, 256), 256, 0, s>>>(n, idx->dim, idx->metric, idx->id_list, idx->rows,
                                                   idx->trows, idx->strs, idx->tstrs, idx->lens,
                                                   idx->tlens, idx->pos_of_id);
+    GTS_CUDA_TRY(cudaMemsetAsync(sc.lens, 0, 3 * sizeof(*sc.lens), s));
     if (idx->metric == kEdit) k_str_sig<<<grid_for((size_t)n, 256), 256, 0, s>>>(n, idx->tstrs, idx->tlens, idx->tsig,
-                                                                             idx->tpack);
+                                                                             idx->tpack, sc.lens);
     if (idx->metric == kAngle) k_row_norms<<<grid_for((size_t)n, 256), 256, 0, s>>>(n, idx->dim, idx->trows, idx->tnorm);
     GTS_CUDA_TRY(cudaMemsetAsync(sc.nsplit + 1, 0, 3 * sizeof(int), s));
     k_cut_lists<<<(mnn + 255) / 256, 256, 0, s>>>(mnn, O, idx->node_flags, idx->node_size, idx->node_pivot, idx->node_lid,
                                                   idx->node_min_dis, idx->cut_node, idx->cut_anc, idx->cut_anc_idx,
                                                   sc.nsplit + 1, idx->node_rec);
     int ncuts[3] = {0, 0, 0};
+    unsigned long long lens[3] = {0, 0, 0};
     GTS_CUDA_TRY(cudaMemcpyAsync(ncuts, sc.nsplit + 1, sizeof(ncuts), cudaMemcpyDeviceToHost, s));
+    if (idx->metric == kEdit) GTS_CUDA_TRY(cudaMemcpyAsync(lens, sc.lens, sizeof(lens), cudaMemcpyDeviceToHost, s));
     GTS_CUDA_TRY(cudaStreamSynchronize(s));
     GTS_CUDA_TRY(cudaGetLastError());
     idx->ncut = ncuts[0];
     idx->ncut_anc = ncuts[1];
     idx->nleaf = ncuts[2];
+    for (int i = 0; i < 3; i++) idx->str_lens[i] = (long long)lens[i];
     return GTS_OK;
 }
 

@@ -28,6 +28,7 @@ struct gts_index {
     int *cut_anc = nullptr, *cut_anc_idx = nullptr;
     int ncut = 0, ncut_anc = 0;
     int nleaf = 0;              // childless nodes with objects
+    long long str_lens[3] = {}; // strings: characters, strings of more than 32 and of more than 64
     float *tnorm = nullptr;
     int4 *node_rec = nullptr;   // per node: (min_dis bits, size, first position, pivot or -1), size 0 where none exists
 

@@ -29,7 +29,7 @@ struct SweepArgs {
     int *ccnt, *cpos;                   // candidate lists [Qp][cap]
     float *cv;
     int *cnt, *cnt2;                    // range: certain counts per sorted query
-    int *ctr;                           // [0] item counter, [1] queries left over
+    int *ctr;                           // [0] item counter, [1] queries left over, [2] of them (strings) for a full list
     int4 *left;                         // queries whose list overflowed: (query, 0, 0, 0) for the traversal
     float *left_R;                      // kNN: and a bound on their k-th distance, from the list
     const int4 *again;                  // kNN, a later round: the run's queries and bounds come from

@@ -21,8 +21,9 @@
 // exact k-th distance.  Queries are taken in the order of their lengths, then
 // of their places in the tree: a tile then needs few lengths of strings, and
 // leaves out the rest when it lists its rows.  Queries of 33 to 64 characters
-// get a pass of their own in 64-bit words; longer ones, and queries whose list
-// cannot hold their candidates, go to the traversal.
+// get a pass of their own in 64-bit words, or take the others along where many
+// strings are that long; longer ones, and queries whose list cannot hold their
+// candidates, go to the traversal.
 #include <cub/device/device_radix_sort.cuh>
 #include <algorithm>
 #include <climits>
@@ -40,7 +41,7 @@ constexpr int kSeChunk = 8;            // row tiles per work item
 constexpr int kSeWindow = 1024;        // objects around a query's place that bound its k-th distance
 constexpr int kSeCap = 2048;           // candidates listed per query
 constexpr int kSeHist = 128;           // distances are at most 108
-constexpr int kSeRounds = 1;           // further passes, in 64-bit words
+constexpr int kSeRounds = 2;           // further passes, in 64-bit words
 constexpr int kSeTextLd = kPackChars / 4 + 1;   // words per row's characters in shared memory (odd: no bank conflicts)
 
 struct EditArgs {
@@ -234,6 +235,10 @@ __global__ void __launch_bounds__(128) k_se_query(EditArgs e)
     const SweepArgs &s = e.s;
     const DevTree &t = s.a.t;
     const int i = blockIdx.x * 128 + threadIdx.x;
+    if (blockIdx.x == 0) {   // the pass's counters
+        for (int j = threadIdx.x; j < s.ntiles; j += 128) s.nrows[j] = 0;
+        if (threadIdx.x == 0) s.ctr[0] = 0;
+    }
     if (i >= s.Qp) return;
     const bool have = i < s.nq;
     const int q = !have ? -1 : (s.again ? s.again[s.q0 + i].x : s.order[s.q0 + i]);
@@ -511,6 +516,7 @@ __global__ void __launch_bounds__(128) k_se_knn(EditArgs e)
     if (m > s.cap) {
         if (tid == 0) {
             const int at = atomicAdd(&s.ctr[1], 1);
+            atomicAdd(&s.ctr[2], 1);
             s.left[at] = make_int4(q, 0, 0, 0);
             s.left_R[at] = (float)R;   // the exact k-th distance: another pass starts from it
         }
@@ -606,8 +612,6 @@ int edit_pass_words(gts_index *idx, EditArgs &e, cudaStream_t st)
     GTS_CUDA_TRY(cudaFuncSetAttribute(k_se_tile<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(EditSmem<W>)));
     GTS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_se_tile<W>, kSeThreads, sizeof(EditSmem<W>)));
     s.ntiles = (s.nq + kSeTq - 1) / kSeTq;
-    GTS_CUDA_TRY(cudaMemsetAsync(s.ctr, 0, sizeof(int), st));
-    GTS_CUDA_TRY(cudaMemsetAsync(s.nrows, 0, sizeof(int) * s.ntiles, st));
     k_se_query<<<(s.Qp + 127) / 128, 128, 0, st>>>(e);
     if (s.nanc > 0) {
         // a CTA per query leaves the chip idle for few of them: split the pivots
@@ -630,6 +634,27 @@ int edit_pass(gts_index *idx, EditArgs &e, cudaStream_t st)
 
 }  // namespace
 
+// The sizes from which on the sweep is the sooner one.  Its launches take some
+// 130 us for a tile and 220 for several, which a CTA of the traversal spends
+// on 16,000 to 64,000 words, the fewer the smaller their leaves; only large
+// batches of less pay.  Traversal and sweep, us, radius 2 where not given:
+//   8,000 words, 1,000 queries  178  277    32,768, leaves of 3,300, 100 queries  174  217
+//   16,384, 100 queries  138  204           32,768, small leaves, 100 queries     832  210
+//   32,768, 8 queries    155  137           100,000, leaves of 10,000, 100 queries  441  207
+// Radii far below the strings' lengths reach a leaf or two of a deep tree: words
+// at radius 0, 200,000 of them, 1,000 queries: 204 and 294; strings of 20 to 50
+// characters at radius 1, 60,000 of them, 100 queries: 114 and 307.  Strings of
+// more than 64 characters are left to the traversal anyway.
+static bool edit_sweep_pays(const gts_index *idx, const SearchArgs &a)
+{
+    const long long n = idx->num, q = a.qnum;
+    const bool deep = n <= 32ll * idx->nleaf;
+    if (2 * idx->str_lens[2] > n) return false;
+    if (a.mode != kModeKnn && deep && floorf(std::min(a.r, 1e6f)) * 16.f * (float)n < (float)idx->str_lens[0]) return false;
+    if (n * q >= 1 << 24) return true;
+    return n >= (q <= kSeTq ? (deep ? 1 << 14 : 1 << 15) : (deep ? 1 << 15 : 1 << 16));
+}
+
 int run_sweep_edit(gts_index *idx, const SearchArgs &a, cudaStream_t st, int *done, const int4 **items, int *n_left)
 {
     *done = 0;
@@ -637,8 +662,7 @@ int run_sweep_edit(gts_index *idx, const SearchArgs &a, cudaStream_t st, int *do
     const int slot = a.mode == kModeRangeTimed ? kModeRangeCount : a.mode;
     const bool knn = a.mode == kModeKnn;
     if (a.deleted || a.items_in || a.seed_r2_bits || idx->ncut < 1 || idx->plain_pinned[slot] ||
-        (!knn && idx->plain_split_set) || (knn ? a.k > 128 : !(a.r >= 0.f)) ||
-        ((long long)idx->num < 1 << 14 && (long long)idx->num * a.qnum < 1 << 20))
+        (!knn && idx->plain_split_set) || (knn ? a.k > 128 : !(a.r >= 0.f)) || !edit_sweep_pays(idx, a))
         return GTS_OK;
     const size_t budget = search_budget(idx);
     void *cub = nullptr;
@@ -663,6 +687,7 @@ int run_sweep_edit(gts_index *idx, const SearchArgs &a, cudaStream_t st, int *do
     int pos_bits = 1, rc;
     while (pos_bits < 31 && (1 << pos_bits) < idx->num) pos_bits++;
     const int run = tiles * kSeTq;
+    e.wide = 8 * idx->str_lens[1] > idx->num;   // many strings of more than 32 characters: one pass for all up to 64
     GTS_CUDA_TRY(cudaMemsetAsync(s.ctr, 0, 64, st));
     int *skey = s.key + a.qnum, *iota = skey + a.qnum;
     k_se_seed<<<a.qnum, kSeThreads, 0, st>>>(e, pos_bits);
@@ -675,22 +700,24 @@ int run_sweep_edit(gts_index *idx, const SearchArgs &a, cudaStream_t st, int *do
         s.nq = std::min(run, a.qnum - q0);
         if ((rc = edit_pass(idx, e, st))) return rc;
     }
-    auto outcome = [&](int *left, bool *ok) {
-        int h[2] = {0, 0}, status = 0;
+    auto outcome = [&](int *left, int *full, bool *ok) {
+        int h[3] = {0, 0, 0}, status = 0;
         GTS_CUDA_TRY(cudaMemcpyAsync(h, s.ctr, sizeof(h), cudaMemcpyDeviceToHost, st));
         GTS_CUDA_TRY(cudaMemcpyAsync(&status, idx->d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
         GTS_CUDA_TRY(cudaStreamSynchronize(st));
         *left = h[1];
+        *full = h[2];
         *ok = status == 0;
         return GTS_OK;
     };
     bool ok = false;
-    if ((rc = outcome(n_left, &ok))) return rc;
+    int full = 0;   // queries left because their list was
+    if ((rc = outcome(n_left, &full, &ok))) return rc;
     // once more: queries of 33 to 64 characters, and kNN queries whose lists
     // filled before their bound settled, from the exact k-th distance
     int4 *const lists[2] = {s.left, s.left + a.qnum};
     float *const bounds[2] = {s.left_R, s.left_R + a.qnum};
-    for (int round = 0; round < kSeRounds && ok && *n_left > 0; round++) {
+    for (int round = 0; round < kSeRounds && ok && (e.wide ? full : *n_left) > 0; round++) {
         const int n = *n_left;
         e.wide = 1;
         s.again = lists[round & 1];
@@ -703,7 +730,7 @@ int run_sweep_edit(gts_index *idx, const SearchArgs &a, cudaStream_t st, int *do
             s.nq = std::min(run, n - q0);
             if ((rc = edit_pass(idx, e, st))) return rc;
         }
-        if ((rc = outcome(n_left, &ok))) return rc;
+        if ((rc = outcome(n_left, &full, &ok))) return rc;
     }
     if (!ok) {   // a query id out of range: the traversal reports it
         GTS_CUDA_TRY(cudaMemsetAsync(idx->d_status, 0, sizeof(int), st));

@@ -13,20 +13,24 @@ from gts_b200 import datagen as G
 pytestmark = pytest.mark.gpu
 
 
-def _median_s(call, reps=7):
-    call()
+def _best_s(call, reps):
     t = []
     for _ in range(reps):
         t0 = time.perf_counter()
         call()
         t.append(time.perf_counter() - t0)
-    return float(np.median(t))
+    return min(t)
 
 
-def _not_slower(auto, pinned):
+def _not_slower(auto, pinned, reps=6):
     """Up to 1.5 times and 40 us more pass: launches are a few us each, and
-    the faults this looks for were 2 to 20 times."""
-    assert auto <= 1.5 * pinned + 40e-6, f"{auto * 1e6:.0f} us against {pinned * 1e6:.0f} us"
+    the faults this looks for were 2 to 20 times.  The best of several calls,
+    asked again where the machine was busy."""
+    for _ in range(4):
+        a, b = _best_s(auto, reps), _best_s(pinned, reps)
+        if a <= 1.5 * b + 40e-6:
+            return
+    pytest.fail(f"{a * 1e6:.0f} us against {b * 1e6:.0f} us")
 
 
 @pytest.mark.parametrize("n,dim,max_h", [(400_000, 2, 4), (400_000, 8, 4), (200_000, 5, 1), (400_000, 3, 6)])
@@ -40,7 +44,7 @@ def test_few_dimensional_counts(n, dim, max_h):
                 q = G.query_ids(n, nq, nq)
                 np.testing.assert_array_equal(a.range(q, r), b.range(q, r))
                 if nq <= 100:
-                    _not_slower(_median_s(lambda: a.range(q, r)), _median_s(lambda: b.range(q, r)))
+                    _not_slower(lambda: a.range(q, r), lambda: b.range(q, r))
 
 
 @pytest.mark.parametrize("n,max_h", [(200_000, 2), (40_000, 1)])   # leaves of 20,000 and 40,000 words
@@ -54,10 +58,10 @@ def test_words_in_large_leaves(n, max_h):
             q = G.query_ids(n, nq, nq)
             for r in (1.0, 3.0):
                 np.testing.assert_array_equal(a.range(q, r), b.range(q, r))
-                _not_slower(_median_s(lambda: a.range(q, r)), _median_s(lambda: b.range(q, r)))
+                _not_slower(lambda: a.range(q, r), lambda: b.range(q, r))
             for x, y in zip(a.knn(q, 8, return_ids=True), b.knn(q, 8, return_ids=True)):
                 np.testing.assert_array_equal(x, y)
-            _not_slower(_median_s(lambda: a.knn(q, 8)), _median_s(lambda: b.knn(q, 8)))
+            _not_slower(lambda: a.knn(q, 8), lambda: b.knn(q, 8))
 
 
 @pytest.mark.parametrize("metric,n,dim,nq", [
@@ -72,12 +76,12 @@ def test_small_indexes(metric, n, dim, nq):
         for k in (1, 16):
             for x, y in zip(a.knn(q, k, return_ids=True), b.knn(q, k, return_ids=True)):
                 np.testing.assert_array_equal(x, y)
-            _not_slower(_median_s(lambda: a.knn(q, k)), _median_s(lambda: b.knn(q, k)))
+            _not_slower(lambda: a.knn(q, k), lambda: b.knn(q, k))
         r = float(np.median(a.knn(q, 16)))
         np.testing.assert_array_equal(a.range(q, r), b.range(q, r))
         for x, y in zip(a.range_ids(q, r), b.range_ids(q, r)):
             np.testing.assert_array_equal(x, y)
-        _not_slower(_median_s(lambda: a.range(q, r)), _median_s(lambda: b.range(q, r)))
+        _not_slower(lambda: a.range(q, r), lambda: b.range(q, r))
 
 
 @pytest.mark.parametrize("n,dim", [(1_000_000, 9), (1_000_000, 16), (500_000, 64)])
@@ -95,4 +99,24 @@ def test_selective_counts(n, dim):
             for r in (0.0, 1e-3, near / 4, near, 1.5 * near):
                 np.testing.assert_array_equal(a.range(q, r), b.range(q, r))
                 if nq >= 1024:
-                    _not_slower(_median_s(lambda: a.range(q, r), 3), _median_s(lambda: b.range(q, r), 3))
+                    _not_slower(lambda: a.range(q, r), lambda: b.range(q, r), 3)
+
+
+@pytest.mark.parametrize("n,max_h,lo,hi", [(8000, 2, 3, 16), (32768, 5, 3, 16), (30000, 4, 20, 50), (20000, 4, 70, 108)])
+def test_words_few_short_and_long(n, max_h, lo, hi):
+    """Small word lists, radii far below the lengths, strings past the sweep's words."""
+    rng = np.random.default_rng(n)
+    lens = rng.integers(lo, hi + 1, n).astype(np.int32)
+    strs = np.where(np.arange(109)[None, :] < lens[:, None], rng.integers(97, 107, (n, 109)), 0).astype(np.uint8)
+    with gts.Index(None, 6, strs=strs, lens=lens, max_h=max_h) as a, \
+            gts.Index(None, 6, strs=strs, lens=lens, max_h=max_h) as b:
+        for mode in (0, 1):
+            b.set_plain_threads(mode, 256)
+        for nq in (4, 100, 600):
+            q = G.query_ids(n, nq, nq)
+            for r in (0.0, 1.0, 8.0):
+                np.testing.assert_array_equal(a.range(q, r), b.range(q, r))
+                _not_slower(lambda: a.range(q, r), lambda: b.range(q, r), 3)
+        for x, y in zip(a.knn(q[:100], 8, return_ids=True), b.knn(q[:100], 8, return_ids=True)):
+            np.testing.assert_array_equal(x, y)
+        _not_slower(lambda: a.knn(q[:100], 8), lambda: b.knn(q[:100], 8), 3)
