@@ -828,7 +828,7 @@ extern "C" int gts_plain_split(gts_index *idx, int objects, long long *items_han
     }
     if (objects >= 0) {
         idx->plain_split = objects;
-        idx->plain_split_set = true;
+        idx->plain_split_set = objects != gts_index::kSplitDefault;
     }
     if (items_handed) *items_handed = idx->last_split_items;
     return GTS_OK;

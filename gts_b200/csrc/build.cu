@@ -391,6 +391,8 @@ void free_tree(gts_index *idx)
     for (int &c : idx->fast_cfg) c = 0;
     for (bool &b : idx->fast_pinned) b = false;
     for (int &c : idx->plain_nt) c = 0;
+    for (bool &b : idx->plain_pinned) b = false;
+    for (bool &b : idx->plain_passed) b = false;
     graph_invalidate(idx);
     idx->mlp_ready = false;   // its feature pivots belong to the old tree
     void *ps[] = {idx->trows, idx->tstrs, idx->tlens, idx->tsig, idx->tpack, idx->id_list, idx->pos_of_id, idx->node_pid,

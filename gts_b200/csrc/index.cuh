@@ -57,6 +57,7 @@ struct gts_index {
     int range_variant = 1;   // fast range counts: 0 the block-stationary filter where it fits, 1 the tile filter
     // autotuned threads per query CTA of the plain traversal per search mode
     // (kNN, range count, range ids; search.cu), 0 = not tuned
+    static constexpr int kSplitDefault = 32768;
     int plain_nt[3] = {};
     // its query CTAs of 128 / 256 / 512 threads resident at once (0: not asked yet)
     int cta_resident[3] = {};
@@ -64,10 +65,12 @@ struct gts_index {
     // traversal over the batched sweep
     bool plain_pinned[3] = {};
     bool plain_split_set = false;
+    // batches large enough to tune went to another search: no threads chosen yet
+    bool plain_passed[3] = {};
     // range counts: objects a query verifies in one CTA before it hands its
     // older stack entries over as (query, node) items (0: never); the item
     // lists, and the items handed over since the last reset
-    int plain_split = 32768;
+    int plain_split = kSplitDefault;
     void *split_buf = nullptr;
     size_t split_bytes = 0;
     long long last_split_items = 0;

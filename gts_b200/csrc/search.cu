@@ -685,7 +685,7 @@ extern "C" int gts_plain_threads(const gts_index *idx, int mode, int *threads)
         gts_set_error("gts_plain_threads: null index / output or mode outside 0..2");
         return GTS_ERR_INVALID;
     }
-    *threads = idx->plain_nt[mode];
+    *threads = idx->plain_nt[mode] ? idx->plain_nt[mode] : idx->plain_passed[mode] ? gts::kPlainDefaultThreads : 0;
     return GTS_OK;
 }
 
@@ -697,6 +697,7 @@ extern "C" int gts_plain_threads_set(gts_index *idx, int mode, int threads)
     }
     idx->plain_nt[mode] = threads;
     idx->plain_pinned[mode] = threads != 0;
+    idx->plain_passed[mode] = false;
     return GTS_OK;
 }
 
@@ -842,8 +843,7 @@ static int run_search(gts_index *idx, SearchArgs &a, cudaStream_t st)
         int rc = run_sweep(idx, a, st, &swept, &items, &n_left);
         if (rc) return rc;
         if (swept) {
-            // where the sweep answers the large batches the traversal keeps its default
-            if (!idx->plain_nt[slot] && a.qnum >= 2 * plain_tune_sample(idx)) idx->plain_nt[slot] = kPlainDefaultThreads;
+            if (a.qnum >= 2 * plain_tune_sample(idx)) idx->plain_passed[slot] = true;
             if (n_left == 0) return GTS_OK;
             a.items_in = items;
             a.qnum = n_left;
@@ -851,7 +851,7 @@ static int run_search(gts_index *idx, SearchArgs &a, cudaStream_t st)
     }
     int nt = idx->plain_nt[slot];
     const bool by_warp = warp_search_takes(idx, a);   // no threads to choose
-    if (by_warp && !nt && !idx->keep_stats && a.qnum >= 2 * plain_tune_sample(idx)) idx->plain_nt[slot] = kPlainDefaultThreads;
+    if (by_warp && !idx->keep_stats && a.qnum >= 2 * plain_tune_sample(idx)) idx->plain_passed[slot] = true;
     if (!nt && !idx->keep_stats && !swept && !by_warp) {
         int rc = plain_autotune(idx, a, st, &nt);
         if (rc) return rc;

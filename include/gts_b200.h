@@ -206,10 +206,12 @@ int gts_fast_autotune_reset(gts_index *idx);
  * least twice the tuning sample (four times the most query CTAs resident at
  * once, about 1,800 on a B200) times 128 / 256 / 512 on its leading sample
  * and keeps the fastest (the answers do not depend on it); range ids take
- * the range-count choice.  *threads = 0 means not tuned yet (256 is used).
- * Batches that the sweep or the warp-per-query range counts answer tune
- * nothing.  _set pins it (128, 256, 512; 0 = tune again) and with it the
- * traversal, for that mode. */
+ * the range-count choice.  *threads = 0 means that no batch was that large
+ * yet; 256 also that the sweep or the warp-per-query range counts answered
+ * those that were: they tune nothing, the traversal uses its default, and
+ * the first such batch that it answers is tuned.  _set pins it (128, 256, 512;
+ * 0 = tune again) and with it the traversal, for that mode, until the index
+ * is rebuilt. */
 int gts_plain_threads(const gts_index *idx, int mode, int *threads);
 int gts_plain_threads_set(gts_index *idx, int mode, int threads);
 
@@ -220,7 +222,8 @@ int gts_plain_threads_set(gts_index *idx, int mode, int threads);
  * (query, node) work items, which the next launch spreads over every CTA
  * (their counts add up), so a few heavy queries do not leave the GPU idle
  * behind them.  objects = 0 turns this off, < 0 leaves it (default 32768);
- * setting it pins range counts and ids to the traversal.
+ * any other value than the default pins range counts and ids to the
+ * traversal, the default gives the choice back.
  * *items_handed (nullable): items handed over since the index was built. */
 int gts_plain_split(gts_index *idx, int objects, long long *items_handed);
 

@@ -120,3 +120,47 @@ def test_words_few_short_and_long(n, max_h, lo, hi):
         for x, y in zip(a.knn(q[:100], 8, return_ids=True), b.knn(q[:100], 8, return_ids=True)):
             np.testing.assert_array_equal(x, y)
         _not_slower(lambda: a.knn(q[:100], 8), lambda: b.knn(q[:100], 8), 3)
+
+
+def _swept(idx, call):
+    call()
+    return idx.search_stats()["pivots"] == 0   # the sweep counts none
+
+
+def test_large_batches_of_the_sweep_tune_nothing():
+    rows = G.gmm_rows(20000, 24, 16, 0.3, seed=9)
+    q = G.query_ids(20000, 8000, 10)
+    with gts.Index(rows, 2, max_h=4) as idx:
+        assert _swept(idx, lambda: idx.knn(q, 8))
+        assert idx.plain_threads(0) == 256           # the traversal's default
+        want = idx.knn(q[:100], 129, return_ids=True)
+        n0 = idx.kernel_launches()
+        first = idx.knn(q, 129, return_ids=True)     # past the sweep's k: the traversal's, and tuned now
+        n1 = idx.kernel_launches()
+        again = idx.knn(q, 129, return_ids=True)
+        assert n1 - n0 > idx.kernel_launches() - n1
+        assert idx.plain_threads(0) in (128, 256, 512)
+        for x, y, z in zip(first, again, want):
+            np.testing.assert_array_equal(x, y)
+            np.testing.assert_array_equal(x[:100], z)
+
+
+def test_a_pin_ends_with_the_index_or_the_default():
+    n = 12000
+    rows = G.gmm_rows(n, 24, 16, 0.3, seed=11)
+    q = G.query_ids(n, 700, 12)
+    r = float(np.float32(G.quantile_radius(2, 0.02, 20000, 13, rows=rows)))
+    flags, ids = G.update_stream(n, 400, 14, max_in_size=10)
+    with gts.Index(rows, 2, max_h=4) as idx:
+        assert _swept(idx, lambda: idx.range(q, r))
+        for mode in (0, 1):
+            idx.set_plain_threads(mode, 128)
+        assert not _swept(idx, lambda: idx.range(q, r)) and not _swept(idx, lambda: idx.knn(q, 8))
+        idx.update_run(flags, ids, r)                 # rebuilds: a new tree, untuned
+        assert idx.plain_threads(0) == 0 and idx.plain_threads(1) == 0
+        q2 = (q % idx.info["num"]).astype(np.int32)
+        assert _swept(idx, lambda: idx.range(q2, r)) and _swept(idx, lambda: idx.knn(q2, 8))
+        idx.plain_split(64)
+        assert not _swept(idx, lambda: idx.range(q2, r))
+        idx.plain_split(32768)                        # the default
+        assert _swept(idx, lambda: idx.range(q2, r))
