@@ -615,7 +615,8 @@ def run_gts(args):
                 learned = c["learned_seed"] if not pin_seed else args.learned_seed == "on"
                 blk = c["by_block"] if args.fast_filter == "auto" else args.fast_filter == "block"
                 streamed = c["streamed"] and not blk
-                idx.set_fast_config(int(g["p"]), learned, c["col_groups"], c["item_blocks"], streamed, blk)
+                idx.set_fast_config(int(g["p"]), learned, c["col_groups"], c["item_blocks"], streamed, blk,
+                                    c["keeps_start"] and not blk)
     clocks = ClockSampler(local).__enter__()
     for _ in range(args.warmup):
         flush_l2(torch, dev, flush)

@@ -283,7 +283,8 @@ class Index:
         v = [C.c_int() for _ in range(5)]
         _check(self._lib.gts_fast_config(self._h, k, *[C.byref(x) for x in v]))
         return {"tuned": bool(v[0].value), "learned_seed": bool(v[1].value), "col_groups": v[2].value,
-                "item_blocks": v[3].value, "streamed": v[4].value == 1, "by_block": v[4].value == 2}
+                "item_blocks": v[3].value, "streamed": v[4].value in (1, 4), "by_block": v[4].value == 2,
+                "keeps_start": v[4].value in (3, 4)}
 
     def fast_seeds(self, qids, k: int) -> np.ndarray:
         """The fast form's starting bound on each query's squared k-th
@@ -301,12 +302,13 @@ class Index:
         return n.value
 
     def set_fast_config(self, k: int, learned_seed: bool, col_groups: int, item_blocks: int = 16,
-                        streamed: bool = False, by_block: bool = False):
+                        streamed: bool = False, by_block: bool = False, keeps_start: bool = False):
         """Pin the fast-form configuration for k instead of tuning it
         (by_block: the block-stationary filter; col_groups and item_blocks
-        are then unused)."""
+        are then unused; keeps_start: the tile filter in which each query
+        keeps the bound it starts with, col_groups 4)."""
         _check(self._lib.gts_fast_config_set(self._h, k, int(bool(learned_seed)), col_groups, item_blocks,
-                                             2 if by_block else int(bool(streamed))))
+                                             2 if by_block else (3 if keeps_start else 0) + int(bool(streamed))))
 
     def fast_range_variant(self, variant=None) -> int:
         """Filter of the fast range counts: 0 the block-stationary one where

@@ -1714,7 +1714,7 @@ static FastCfg cfg_unpack(int v)
 }
 
 // Filter variant of a configuration as the ABI reports it.
-static int cfg_variant(const FastCfg &c) { return c.blk ? 2 : (c.stream ? 1 : 0); }
+static int cfg_variant(const FastCfg &c) { return c.blk ? 2 : (c.flat ? 3 : 0) + (c.stream ? 1 : 0); }
 
 static bool fast_tile_fits(const FastShape &fs, int cg, int k, bool stream);
 
@@ -2976,10 +2976,10 @@ extern "C" int gts_fast_config(const gts_index *idx, int k, int *tuned, int *lea
 extern "C" int gts_fast_config_set(gts_index *idx, int k, int learned, int col_groups, int item_blocks, int variant)
 {
     if (!idx || k < 1 || k > gts::kFMaxK || (col_groups != 1 && col_groups != 2 && col_groups != 4) ||
-        col_groups * k > 128 || (item_blocks != 8 && item_blocks != 16 && item_blocks != 32) || variant < 0 ||
-        variant > 2) {
-        gts_set_error("gts_fast_config_set: k in [1, 64], column groups 1/2/4 with groups * k <= 128, "
-                      "8/16/32 blocks per item, filter variant 0/1/2");
+        (variant < 3 && col_groups * k > 128) || (variant > 2 && col_groups != 4) ||
+        (item_blocks != 8 && item_blocks != 16 && item_blocks != 32) || variant < 0 || variant > 4) {
+        gts_set_error("gts_fast_config_set: k in [1, 64], column groups 1/2/4 with groups * k <= 128 (variants 3 and "
+                      "4: 4, any k), 8/16/32 blocks per item, filter variant 0 to 4");
         return GTS_ERR_INVALID;
     }
     const gts::FastShape fs = gts::fast_shape(idx->dim);
@@ -2990,13 +2990,14 @@ extern "C" int gts_fast_config_set(gts_index *idx, int k, int learned, int col_g
                       idx->dim);
         return GTS_ERR_INVALID;
     }
-    const bool stream = !blk && (variant == 1 || fs.kp > gts::kFResKp);
-    if (!blk && l2 && !gts::fast_tile_fits(fs, col_groups, k, stream)) {
+    const bool flat = variant > 2;
+    const bool stream = !blk && (variant == 1 || variant == 4 || fs.kp > gts::kFResKp);
+    if (!blk && l2 && !gts::fast_tile_fits(fs, col_groups, flat ? 1 : k, stream)) {
         gts_set_error("gts_fast_config_set: %d column groups at k %d do not fit the shared memory at dim %d",
                       col_groups, k, idx->dim);
         return GTS_ERR_INVALID;
     }
-    idx->fast_cfg[k] = gts::cfg_pack(gts::FastCfg{learned != 0, col_groups, item_blocks, stream, blk});
+    idx->fast_cfg[k] = gts::cfg_pack(gts::FastCfg{learned != 0, col_groups, item_blocks, stream, blk, false, flat});
     idx->fast_pinned[k] = true;
     return GTS_OK;
 }

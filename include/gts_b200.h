@@ -172,7 +172,8 @@ int gts_kernel_launches(const gts_index *idx, long long *count);
  * fastest that fits the shared memory is kept (every candidate returns the
  * same exact answers).  *variant: 0 tile filter, resident records; 1 tile
  * filter, streamed records; 2 block-stationary filter (*col_groups and
- * *item_blocks then unused).  *tuned = 0 reports the default that smaller
+ * *item_blocks then unused); 3 and 4 as 0 and 1, but each query keeps the
+ * bound it starts with (*col_groups 4, no heaps).  *tuned = 0 reports the default that smaller
  * batches use.  Any output pointer may be NULL. */
 int gts_fast_config(const gts_index *idx, int k, int *tuned, int *learned, int *col_groups, int *item_blocks,
                     int *variant);
@@ -187,8 +188,9 @@ int gts_fast_config(const gts_index *idx, int k, int *tuned, int *learned, int *
 int gts_fast_seeds(gts_index *idx, const int *qids, int qnum, int k, float *seeds_out);
 
 /* Pin the configuration for k (learned seed 0/1, 1/2/4 column groups with
- * groups * k <= 128, 8/16/32 blocks per item, filter variant 0/1/2 as
- * gts_fast_config reports it) instead of tuning it; GTS_ERR_INVALID when it
+ * groups * k <= 128, 8/16/32 blocks per item, filter variant 0 to 4 as
+ * gts_fast_config reports it; variants 3 and 4 take 4 column groups at any k)
+ * instead of tuning it; GTS_ERR_INVALID when it
  * does not fit this index's shared memory plan. */
 int gts_fast_config_set(gts_index *idx, int k, int learned, int col_groups, int item_blocks, int variant);
 

@@ -1,0 +1,50 @@
+"""The fast form's configurations as the ABI reports and takes them: every one
+that can be chosen can be read, written back and read again, and answers as the
+others do."""
+import numpy as np
+import pytest
+
+import gts_b200 as gts
+from gts_b200 import datagen as G
+
+pytestmark = pytest.mark.gpu
+
+KEYS = ("learned_seed", "col_groups", "item_blocks", "streamed", "by_block", "keeps_start")
+
+
+def _write(idx, k, c):
+    idx.set_fast_config(k, c["learned_seed"], c["col_groups"], c["item_blocks"], c["streamed"], c["by_block"],
+                        c["keeps_start"])
+
+
+@pytest.mark.parametrize("n,dim", [(12000, 64), (12000, 128), (9000, 200)])
+def test_a_tuned_configuration_can_be_written_back(oracle, n, dim):
+    rows = G.gmm_rows(n, dim, 24, 0.25, seed=dim)
+    ds = oracle.Dataset(2, rows)
+    q = G.query_ids(n, 2200, seed=22)
+    with gts.Index(rows, 2, max_h=4) as idx, gts.Index(rows, 2, max_h=4) as other:
+        for k in (1, 8, 64):
+            want = idx.knn(q, k, form=gts.FORM_FAST, return_ids=True)
+            tuned = idx.fast_config(k)
+            assert tuned["tuned"]
+            _write(other, k, tuned)
+            assert {x: other.fast_config(k)[x] for x in KEYS} == {x: tuned[x] for x in KEYS}
+            for x, y in zip(other.knn(q, k, form=gts.FORM_FAST, return_ids=True), want):
+                np.testing.assert_array_equal(x, y)
+            for x, y in zip(want, oracle.knn_brute(ds, q[:60], k)):
+                np.testing.assert_array_equal(x[:60], y)
+
+
+@pytest.mark.parametrize("streamed", [False, True])
+@pytest.mark.parametrize("k", [1, 16, 33, 64])
+def test_keeping_the_start_answers_as_the_heaps(oracle, k, streamed):
+    rows = np.concatenate([G.gmm_rows(9000, 96, 24, 0.25, seed=3), np.tile(G.gmm_rows(2, 96, 1, 0.2, 4), (800, 1))])
+    q = np.concatenate([G.query_ids(9000, 300, seed=5), [9000, 9001, 10599]]).astype(np.int32)   # the last ones overflow
+    with gts.Index(rows, 2, max_h=4) as idx:
+        idx.set_fast_config(k, False, 4, 8, streamed=streamed, keeps_start=True)
+        c = idx.fast_config(k)
+        assert c["keeps_start"] and c["streamed"] == streamed and c["col_groups"] == 4
+        for x, y in zip(idx.knn(q, k, form=gts.FORM_FAST, return_ids=True), oracle.knn_brute(oracle.Dataset(2, rows), q, k)):
+            np.testing.assert_array_equal(x, y)
+        with pytest.raises(gts.GtsError):
+            idx.set_fast_config(k, False, 2, 8, keeps_start=True)
