@@ -363,13 +363,13 @@ int ensure_io(gts_index *idx, size_t bytes)
     return GTS_OK;
 }
 
-int ensure_hits(gts_index *idx, size_t bytes, void **out)
+int ensure_hits(gts_index *idx, size_t bytes, size_t room, void **out)
 {
     if (bytes > idx->hits_bytes) {
         if (idx->hits) dev_free(idx->hits);
         idx->hits = nullptr;
         idx->hits_bytes = 0;
-        const size_t want = bytes + bytes / 4;
+        const size_t want = std::max(bytes, std::min(bytes + bytes / 4, room));
         if (dev_malloc(&idx->hits, want) != cudaSuccess) {
             cudaGetLastError();
             idx->hits = nullptr;

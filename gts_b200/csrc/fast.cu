@@ -2281,6 +2281,7 @@ static size_t plan_book(int qnum, int k, unsigned char *base, Book *b)
 struct FastCall {
     unsigned char *region;
     size_t region_bytes;
+    bool small_fits;   // the small batches' buffers fit the call's budget beside the region
     Book book[3];   // stage 0: filter on table seeds (no learned radius), 1: filter from the bound reached,
                     // 2: plain traversal
 };
@@ -2313,7 +2314,7 @@ static int rerun_failed(gts_index *idx, FastCall &fc, const FastCfg &cfg, int st
         idx->kernel_launches++;
     }
     int rc, n_small = n;
-    if (stage == 1 && fast_small_takes(idx, n)) {
+    if (stage == 1 && fc.small_fits && fast_small_takes(idx, n)) {
         // a few queries of a large batch: a tile pass of their own would cost
         // as much as a fifth of the batch's
         int *fail = nullptr;
@@ -2604,19 +2605,20 @@ static int search_knn_tiles(gts_index *idx, const int *d_qids, int qnum, int k, 
     int qc = 0;
     if ((rc = run_queries_for_budget(idx, qnum, [&](int q) { return rbytes_of(q) + 3 * bbytes_of(q); }, &qc)))
         return rc;
+    const size_t rbytes = rbytes_of(qc);
+    const size_t bbytes = bbytes_of(qc);
+    FastCall fc;
+    fc.small_fits = rbytes + 3 * bbytes + fast_small_bytes(idx) <= search_budget(idx);
     // a few queries do without tiles; those it leaves (rare) take the tiles
     // with the rest
-    if (fast_small_takes(idx, qnum) && !idx->fast_pinned[k] && !idx->time_filter) {
+    if (fc.small_fits && fast_small_takes(idx, qnum) && !idx->fast_pinned[k] && !idx->time_filter) {
         int *fail = nullptr, n_fail = 0;
         if ((rc = fast_small_run(idx, d_qids, qnum, k, nullptr, d_kth, d_ids, d_dists, &fail, &n_fail, true, st)))
             return rc;
         idx->last_fast_overflow = n_fail;
         if (n_fail == 0) return GTS_OK;
     }
-    const size_t rbytes = rbytes_of(qc);
-    const size_t bbytes = bbytes_of(qc);
     if ((rc = ensure_scratch(idx, rbytes + 3 * bbytes))) return rc;
-    FastCall fc;
     fc.region = (unsigned char *)idx->scratch;
     fc.region_bytes = rbytes;
     for (int s = 0; s < 3; s++) plan_book(qc, k, fc.region + rbytes + s * bbytes, &fc.book[s]);

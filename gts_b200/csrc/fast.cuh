@@ -187,6 +187,7 @@ int prune_blocks(const unsigned char *arec, const FastShape &fs, const FastSumma
 // those it can, lists the others' positions at *d_fail (valid until the next
 // call).  reset: clears the statistics first.
 constexpr int kSmallMax = 64;
+size_t fast_small_bytes(const gts_index *idx);   // its buffers, kept with the handle
 bool fast_small_takes(const gts_index *idx, int qnum);
 int fast_small_run(gts_index *idx, const int *d_qids, int qnum, int k, const int *d_carry, float *d_kth, int *d_ids,
                    float *d_dists, int **d_fail, int *n_fail, bool reset, cudaStream_t st);

@@ -213,9 +213,14 @@ __global__ void __launch_bounds__(128) k_small_final(SmallArgs a)
 
 // The handle's buffers for small batches: device lists, and the result word
 // in host memory.
+size_t fast_small_bytes(const gts_index *idx)
+{
+    return 1024 + 4 * (size_t)kSmallMax * ((size_t)idx->fast_nb + 1 + 2 * kSwCap + 2);
+}
+
 static int small_buffers(gts_index *idx, cudaStream_t st)
 {
-    const size_t need = 1024 + 4 * (size_t)kSmallMax * ((size_t)idx->fast_nb + 1 + 2 * kSwCap + 2);
+    const size_t need = fast_small_bytes(idx);
     if (!idx->small_result && cudaHostAlloc((void **)&idx->small_result, 64, cudaHostAllocMapped) != cudaSuccess) {
         cudaGetLastError();
         idx->small_result = nullptr;

@@ -91,6 +91,8 @@ struct gts_index {
     // hits of a range-ids run on their way to the host
     void *hits = nullptr;
     size_t hits_bytes = 0;
+    // scratch of the running call outside `scratch` (search_budget)
+    size_t held_bytes = 0;
     // CUDA graph of the fast form's filter pass (fast.cu), launched on the
     // handle's own stream and replayed while the batch shape stays the same
     cudaStream_t graph_stream = nullptr;
@@ -174,20 +176,22 @@ template <typename T>
 int dev_alloc(T **p, size_t n, size_t *acct);
 
 // Device scratch one search call may hold (gts_params.mem_budget_gb; 0 means
-// 8 GiB).  The fast form sizes its runs of queries, the seeded plain form its
-// chunks and the update path its query batches to fit it.
+// 8 GiB), less what the call holds already around a search of its own.  The
+// fast form and the sweeps size their runs of queries, the seeded plain form
+// its chunks and the update path its query batches to fit it.
 inline size_t search_budget(const gts_index *idx)
 {
     const double gb = idx->params.mem_budget_gb;
-    return gb > 0 ? (size_t)(gb * 1073741824.0) : ((size_t)8 << 30);
+    const size_t b = gb > 0 ? (size_t)(gb * 1073741824.0) : ((size_t)8 << 30);
+    return b > idx->held_bytes ? b - idx->held_bytes : 0;
 }
 
 // Grow idx->scratch to at least `bytes`.
 int ensure_scratch(gts_index *idx, size_t bytes);
 // Grow idx->io to at least `bytes`.
 int ensure_io(gts_index *idx, size_t bytes);
-// idx->hits of at least `bytes`.
-int ensure_hits(gts_index *idx, size_t bytes, void **out);
+// idx->hits of at least `bytes`, at most `room` where it grows.
+int ensure_hits(gts_index *idx, size_t bytes, size_t room, void **out);
 
 bool fast_supported(const gts_index *idx, int k);
 int mlp_seed(gts_index *idx, const int *d_qids, int qnum, int k, int *d_r2_bits, cudaStream_t st);

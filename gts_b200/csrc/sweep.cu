@@ -1122,12 +1122,14 @@ int launch_metric(gts_index *idx, const SweepArgs &s, bool sampled, cudaStream_t
     }
 }
 
-// The run's ordered hits into call order; offsets of the run's queries, of
-// which the run's first hit is number `base`.
-__global__ void k_sw_copy_hits(SweepArgs s, int base)
+// The ordered hits of the run's queries [q0, q1) into call order; offsets of
+// the run's queries, of which q0's first hit is number `base`.
+__global__ void k_sw_copy_hits(SweepArgs s, int q0, int q1, int base)
 {
     const int i = blockIdx.x;
-    const int q = s.bq[i], n = s.a.counts[q], o = s.a.offsets[q - s.q0] - base;
+    const int q = s.bq[i];
+    if (q < q0 || q >= q1) return;
+    const int n = s.a.counts[q], o = s.a.offsets[q - s.q0] - base;
     for (int c = threadIdx.x; c < n; c += blockDim.x) {
         s.a.rids[o + c] = s.cpos[(size_t)i * s.cap + c];
         s.a.rdists[o + c] = s.cv[(size_t)i * s.cap + c];
@@ -1386,22 +1388,36 @@ int sweep_range_ids(gts_index *idx, const int *d_qids, int qnum, float r, int *d
             *total += (size_t)counts_out[i];
         }
         if (*total > capacity || *total > 0x7fffffff || *total == base) continue;
-        // the run's hits, from the lists into call order and out
-        const size_t n = *total - base, ob = (sizeof(int) * (size_t)nq + 255) & ~(size_t)255, nb = (4 * n + 255) & ~(size_t)255;
-        void *buf = nullptr;
-        if ((rc = ensure_hits(idx, ob + 2 * nb, &buf))) return rc;
-        int *d_off = (int *)buf, *d_hid = (int *)((unsigned char *)buf + ob);
-        float *d_hd = (float *)((unsigned char *)buf + ob + nb);
-        GTS_CUDA_TRY(cudaMemcpyAsync(d_off, offsets_out + q0, sizeof(int) * nq, cudaMemcpyHostToDevice, st));
-        b.s.a.offsets = d_off;
-        b.s.a.rids = d_hid;
-        b.s.a.rdists = d_hd;
-        k_sw_copy_hits<<<nq, 64, 0, st>>>(b.s, (int)base);
-        idx->kernel_launches++;
-        GTS_CUDA_TRY(cudaGetLastError());
-        if (ids_out) GTS_CUDA_TRY(cudaMemcpyAsync(ids_out + base, d_hid, 4 * n, cudaMemcpyDeviceToHost, st));
-        if (dists_out) GTS_CUDA_TRY(cudaMemcpyAsync(dists_out + base, d_hd, 4 * n, cudaMemcpyDeviceToHost, st));
-        GTS_CUDA_TRY(cudaStreamSynchronize(st));
+        // the run's hits, from the lists into call order and out, as many
+        // queries at a time as the call's budget has room for
+        const size_t used = b.bytes + (lists.p ? 2 * sizeof(int) * (size_t)b.s.Qp * b.s.cap : 0);
+        const size_t room = search_budget(idx) > used ? search_budget(idx) - used : 0;
+        const size_t ob = (sizeof(int) * (size_t)nq + 255) & ~(size_t)255;
+        for (int i0 = q0, i1; i0 < q0 + nq; i0 = i1) {
+            auto bytes_to = [&](int i) {   // of the hits of queries i0 .. i
+                const size_t n = (size_t)offsets_out[i] + counts_out[i] - offsets_out[i0];
+                return ob + 2 * ((4 * n + 255) & ~(size_t)255);
+            };
+            if (bytes_to(i0) > room) return GTS_OK;
+            for (i1 = i0 + 1; i1 < q0 + nq && bytes_to(i1) <= room; i1++) {}
+            const size_t need = bytes_to(i1 - 1), nb = (need - ob) / 2;
+            const size_t first = (size_t)offsets_out[i0], n = (size_t)offsets_out[i1 - 1] + counts_out[i1 - 1] - first;
+            if (n == 0) continue;
+            void *buf = nullptr;
+            if ((rc = ensure_hits(idx, need, room, &buf))) return rc;
+            int *d_off = (int *)buf, *d_hid = (int *)((unsigned char *)buf + ob);
+            float *d_hd = (float *)((unsigned char *)buf + ob + nb);
+            GTS_CUDA_TRY(cudaMemcpyAsync(d_off, offsets_out + q0, sizeof(int) * nq, cudaMemcpyHostToDevice, st));
+            b.s.a.offsets = d_off;
+            b.s.a.rids = d_hid;
+            b.s.a.rdists = d_hd;
+            k_sw_copy_hits<<<nq, 64, 0, st>>>(b.s, i0, i1, (int)first);
+            idx->kernel_launches++;
+            GTS_CUDA_TRY(cudaGetLastError());
+            if (ids_out) GTS_CUDA_TRY(cudaMemcpyAsync(ids_out + first, d_hid, 4 * n, cudaMemcpyDeviceToHost, st));
+            if (dists_out) GTS_CUDA_TRY(cudaMemcpyAsync(dists_out + first, d_hd, 4 * n, cudaMemcpyDeviceToHost, st));
+            GTS_CUDA_TRY(cudaStreamSynchronize(st));
+        }
     }
     *done = 1;
     return GTS_OK;

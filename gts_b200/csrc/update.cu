@@ -339,7 +339,10 @@ int update_run(gts_index *idx, const int *flags, const int *ids, int nops, float
             const int n = std::min(qc, nq - q0);
             GTS_CUDA_TRY(cudaMemcpyAsync(d_q, P.q_obj.data() + q0, sizeof(int) * n, cudaMemcpyHostToDevice, s));
             GTS_CUDA_TRY(cudaMemcpyAsync(d_t, P.q_time.data() + q0, sizeof(int) * n, cudaMemcpyHostToDevice, s));
-            if ((rc = search_range_timed(idx, d_q, d_t, n, r, d_off, d_ents, d_ct, d_cc, s))) return rc;
+            idx->held_bytes = fixed + 16 * (size_t)qc;
+            rc = search_range_timed(idx, d_q, d_t, n, r, d_off, d_ents, d_ct, d_cc, s);
+            idx->held_bytes = 0;
+            if (rc) return rc;
             GTS_CUDA_TRY(cudaMemcpyAsync(ct.data() + q0, d_ct, sizeof(int) * n, cudaMemcpyDeviceToHost, s));
             GTS_CUDA_TRY(cudaMemcpyAsync(cc.data() + q0, d_cc, sizeof(int) * n, cudaMemcpyDeviceToHost, s));
         }

@@ -62,7 +62,8 @@ typedef struct {
                             fit one tile / query returns GTS_ERR_NOMEM.  The plain form's
                             sweep sizes its runs to it and leaves a batch of which not one
                             tile fits to the traversal, which holds no per-query device
-                            memory.  Negative: invalid. */
+                            memory; range hits leave in pieces that fit.  Not counted:
+                            argument and answer buffers.  Negative: invalid. */
 } gts_params;
 
 typedef struct {
