@@ -2611,7 +2611,7 @@ static int search_knn_tiles(gts_index *idx, const int *d_qids, int qnum, int k, 
     fc.small_fits = rbytes + 3 * bbytes + fast_small_bytes(idx) <= search_budget(idx);
     // a few queries do without tiles; those it leaves (rare) take the tiles
     // with the rest
-    if (fc.small_fits && fast_small_takes(idx, qnum) && !idx->fast_pinned[k] && !idx->time_filter) {
+    if (fc.small_fits && fast_small_takes(idx, qnum) && !idx->fast_pinned[k]) {
         int *fail = nullptr, n_fail = 0;
         if ((rc = fast_small_run(idx, d_qids, qnum, k, nullptr, d_kth, d_ids, d_dists, &fail, &n_fail, true, st)))
             return rc;

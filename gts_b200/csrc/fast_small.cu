@@ -282,15 +282,24 @@ int fast_small_run(gts_index *idx, const int *d_qids, int qnum, int k, const int
     a.reset = reset ? 1 : 0;
     const int groups = (qnum + kSmGroup - 1) / kSmGroup;
     const dim3 pg(std::max(1, std::min((a.nb + 7) / 8, 8 * 148 / groups)), groups);
+    const bool timed = idx->time_filter && idx->fev[0];   // the filter: everything before the exact values
+    if (timed) GTS_CUDA_TRY(cudaEventRecord(idx->fev[0], st));
     if (fs.kp <= 64) k_small_prune<2><<<pg, 256, 0, st>>>(a);
     else if (fs.kp <= 128) k_small_prune<4><<<pg, 256, 0, st>>>(a);
     else k_small_prune<10><<<pg, 256, 0, st>>>(a);
     k_small_rows<<<dim3(std::max(8, 4 * 148 / qnum), qnum), 256, sizeof(float) * fs.kp, st>>>(a);
+    if (timed) GTS_CUDA_TRY(cudaEventRecord(idx->fev[1], st));
     GTS_CUDA_TRY(cudaFuncSetAttribute(k_small_final, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FinalSmem)));
     k_small_final<<<qnum, 128, sizeof(FinalSmem), st>>>(a);
     idx->kernel_launches += 3;
     GTS_CUDA_TRY(cudaGetLastError());
     GTS_CUDA_TRY(cudaStreamSynchronize(st));
+    if (timed) {
+        float ms = 0.f;
+        GTS_CUDA_TRY(cudaEventElapsedTime(&ms, idx->fev[0], idx->fev[1]));
+        idx->filter_ms += ms;
+        idx->filter_launches++;
+    }
     *n_fail = *(volatile int *)idx->small_result;
     *d_fail = a.fail;
     return GTS_OK;

@@ -152,7 +152,8 @@ int gts_index_set_stream(gts_index *idx, void *stream);
 int gts_search_stats(const gts_index *idx, unsigned long long *out8);
 
 /* No counterpart in the reference.  Device time of the fast form's filter
- * kernel, from CUDA events around each launch on the index's stream.
+ * kernel (small batches: of the two kernels before the exact values), from
+ * CUDA events around each launch on the index's stream.
  * reset != 0 zeroes the totals and turns timing on (creating the events);
  * *ms / *launches (nullable) receive the totals since the last reset. */
 int gts_filter_timing(gts_index *idx, int reset, double *ms, long long *launches);

@@ -48,3 +48,22 @@ def test_keeping_the_start_answers_as_the_heaps(oracle, k, streamed):
             np.testing.assert_array_equal(x, y)
         with pytest.raises(gts.GtsError):
             idx.set_fast_config(k, False, 2, 8, keeps_start=True)
+
+
+@pytest.mark.parametrize("nq", [1, 64, 65])
+def test_timing_does_not_change_what_runs(nq):
+    rows = G.gmm_rows(9000, 64, 8, 0.3, seed=7)
+    q = G.query_ids(9000, nq, 8)
+    with gts.Index(rows, 2, max_h=4) as idx:
+        idx.fast_graphs(False)
+        counts = []
+        for timed in (False, True):
+            if timed:
+                idx.filter_timing(reset=True)
+            idx.knn(q, 8, form=gts.FORM_FAST)
+            n0 = idx.kernel_launches()
+            kth = idx.knn(q, 8, form=gts.FORM_FAST)
+            counts.append((idx.kernel_launches() - n0, kth))
+        ms, launches = idx.filter_timing()
+        assert counts[0][0] == counts[1][0] and launches == 2 and 0 < ms < 1000
+        np.testing.assert_array_equal(counts[0][1], counts[1][1])
