@@ -1556,10 +1556,11 @@ __global__ void __launch_bounds__(32 * kFinWarps) k_fast_final_warp(
 // queries of each block (a few per block) put in index order by insertion
 // sort.  A block with more than kOrderSortMax queries keeps their arrival
 // order: the order only groups the queries into tiles, the answers do not
-// depend on it.
+// depend on it (62 queries a block: 105 us, most of them one thread's
+// insertions).
 constexpr int kOrderThreads = 1024;
 constexpr int kOrderMaxNb = 24576;   // 2 x 4 bytes per block of shared memory
-constexpr int kOrderSortMax = 64;
+constexpr int kOrderSortMax = 16;
 __global__ void __launch_bounds__(kOrderThreads) k_fast_order(const int *__restrict__ keys, int qnum, int nb,
                                                               int *__restrict__ order)
 {
