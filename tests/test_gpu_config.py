@@ -67,3 +67,16 @@ def test_timing_does_not_change_what_runs(nq):
         ms, launches = idx.filter_timing()
         assert counts[0][0] == counts[1][0] and launches == 2 and 0 < ms < 1000
         np.testing.assert_array_equal(counts[0][1], counts[1][1])
+
+
+@pytest.mark.parametrize("dim,nq,tiles", [(300, 51, False), (300, 52, True), (128, 64, False), (128, 65, True), (64, 64, False)])
+def test_small_batches_by_width(oracle, dim, nq, tiles):
+    rows = G.gmm_rows(6000, dim, 8, 0.3, seed=dim)
+    q = G.query_ids(6000, nq, 9)
+    with gts.Index(rows, 2, max_h=4) as idx:
+        idx.prepare()
+        n0 = idx.kernel_launches()
+        got = idx.knn(q, 8, form=gts.FORM_FAST, return_ids=True)
+        assert (idx.kernel_launches() - n0 > 3) == tiles
+        for x, y in zip(got, oracle.knn_brute(oracle.Dataset(2, rows), q, 8)):
+            np.testing.assert_array_equal(x, y)
