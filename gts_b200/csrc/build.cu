@@ -12,9 +12,12 @@
 //      every node's range keeps its place and an unsplit node its order (eight
 //      plus a few radix passes over the whole chip; a segmented sort gave each
 //      of the few huge segments near the root one CTA: 19.2 ms against 1.9 for
-//      the five levels of 1,000,000 objects).  The reference sorts all N keys globally (tree.cuh:372); node codes keep
-//      the segments apart and the sort is stable, so for every tree in which
-//      each level's objects all sit in split nodes the order is identical;
+//      the five levels of 1,000,000 objects; small indexes keep it, done
+//      before a radix sort's dozen passes: building 5,000 x 8 takes 1.00 ms by
+//      segments and 1.30 by radix, 12,000 x 32 1.8 and 1.3).  The reference
+//      sorts all N keys globally (tree.cuh:372); node codes keep the segments
+//      apart and the sort is stable, so for every tree in which each level's
+//      objects all sit in split nodes the order is identical;
 //   4. k_split: O children per split node with the equal-count split, the
 //      last child taking the remainder, min_dis = dist(first object of the
 //      child, pivot) in F32-accumulated arithmetic, is_leaf = size <= MAX_SIZE
@@ -24,6 +27,7 @@
 // One 4-byte device->host read per level (the number of nodes still to
 // split) decides whether to continue, as the reference's reduce does.
 #include <cub/device/device_radix_sort.cuh>
+#include <cub/device/device_segmented_sort.cuh>
 #include <cstdio>
 #include <vector>
 #include "index.cuh"
@@ -103,12 +107,17 @@ __global__ void k_init(int n, int mnn, int *id_list, int *node_of_pos, int *node
     }
 }
 
+// seg (nullable): [2][nb] the nodes' ranges as sort segments, empty for those not split.
 __global__ void k_select_pivots(int start, int nb, const int *id_list, const int *node_size,
-                                const int *node_lid, const uint8_t *split, int *node_pivot)
+                                const int *node_lid, const uint8_t *split, int *node_pivot, int *seg)
 {
     int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nb) return;
     int nid = start + b;
+    if (seg) {
+        seg[b] = split[nid] ? node_lid[nid] : 0;
+        seg[nb + b] = split[nid] ? node_lid[nid] + node_size[nid] : 0;
+    }
     if (split[nid]) {
         int lid = node_lid[nid], size = node_size[nid];
         int rid = lid + size - 1;
@@ -330,6 +339,8 @@ static inline unsigned grid_for(size_t n, int block, unsigned cap = 148u * 32u)
     return (unsigned)(g > cap ? cap : g);
 }
 
+constexpr int kSegSortMax = 8192;   // objects up to which a level is sorted by segments
+
 int ensure_scratch(gts_index *idx, size_t bytes)
 {
     if (idx->scratch_bytes >= bytes) return GTS_OK;
@@ -421,14 +432,14 @@ void free_data(gts_index *idx)
 namespace {
 // Build-time scratch, released on every exit path.
 struct BuildScratch {
-    int *node_of_pos = nullptr, *ids_alt = nullptr, *posv = nullptr, *posv_alt = nullptr, *nsplit = nullptr;
+    int *node_of_pos = nullptr, *ids_alt = nullptr, *posv = nullptr, *posv_alt = nullptr, *nsplit = nullptr, *seg = nullptr;
     double *key = nullptr, *key_alt = nullptr;
     uint8_t *split = nullptr;
     unsigned long long *lens = nullptr;
     void *temp = nullptr;
     ~BuildScratch()
     {
-        void *ps[] = {node_of_pos, ids_alt, posv, posv_alt, nsplit, key, key_alt, split, lens, temp};
+        void *ps[] = {node_of_pos, ids_alt, posv, posv_alt, nsplit, seg, key, key_alt, split, lens, temp};
         for (void *p : ps)
             if (p) dev_free(p);
     }
@@ -484,6 +495,11 @@ static int build_tree_impl(gts_index *idx, cudaStream_t s)
     ALLOC(sc.posv_alt, n);
     ALLOC(sc.lens, 3);
     ALLOC(sc.nsplit, 4);   // nodes still to split; cut nodes, their ancestors, childless nodes
+    double maxnb_d = 1;   // nodes at the deepest level that can split: O^(H-2)
+    for (int l = 0; l + 2 < H; l++) maxnb_d *= O;
+    const bool by_segment = n <= kSegSortMax && maxnb_d <= n;
+    const int maxnb = by_segment ? (int)maxnb_d : 0;
+    if (by_segment) ALLOC(sc.seg, 2 * (size_t)maxnb);
 #undef ALLOC
     int lid_bits = 1;
     while (lid_bits < 31 && (1 << lid_bits) < n) lid_bits++;
@@ -493,6 +509,11 @@ static int build_tree_impl(gts_index *idx, cudaStream_t s)
     GTS_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, temp_lid, (uint32_t *)nullptr, (uint32_t *)nullptr,
                                                  sc.posv_alt, sc.posv, n, 0, lid_bits, s));
     temp_bytes = std::max(temp_bytes, temp_lid);
+    if (by_segment) {
+        GTS_CUDA_TRY(cub::DeviceSegmentedSort::StableSortPairs(nullptr, temp_lid, sc.key, sc.key_alt, idx->id_list,
+                                                               sc.ids_alt, n, maxnb, sc.seg, sc.seg, s));
+        temp_bytes = std::max(temp_bytes, temp_lid);
+    }
     if (dev_malloc(&sc.temp, temp_bytes ? temp_bytes : 1) != cudaSuccess) {
         cudaGetLastError();
         gts_set_error("cudaMalloc of sort scratch (%zu bytes) failed", temp_bytes);
@@ -508,15 +529,21 @@ static int build_tree_impl(gts_index *idx, cudaStream_t s)
         int nb = 1;
         for (int l = 0; l < cur_level; l++) nb *= O;
         k_select_pivots<<<(nb + 255) / 256, 256, 0, s>>>(start, nb, idx->id_list, idx->node_size,
-                                                         idx->node_lid, sc.split, idx->node_pivot);
+                                                         idx->node_lid, sc.split, idx->node_pivot, sc.seg);
         k_keys<<<grid_for(n, 256), 256, 0, s>>>(dd, n, start, nb, p.dis_code, p.infi_dis,
                                                  idx->id_list, sc.node_of_pos, sc.split,
                                                  idx->node_pivot, sc.key, sc.posv);
         size_t tb = temp_bytes;
-        GTS_CUDA_TRY(cub::DeviceRadixSort::SortPairs(sc.temp, tb, sc.key, sc.key_alt, sc.posv, sc.posv_alt, n, 0, 64,
-                                                     s));
         int *order = sc.posv_alt;
-        if (cur_level > 0) {   // the key buffers serve the second pass
+        if (by_segment) {
+            GTS_CUDA_TRY(cudaMemcpyAsync(sc.ids_alt, idx->id_list, sizeof(int) * (size_t)n, cudaMemcpyDeviceToDevice, s));
+            GTS_CUDA_TRY(cub::DeviceSegmentedSort::StableSortPairs(sc.temp, tb, sc.key, sc.key_alt, idx->id_list,
+                                                                   sc.ids_alt, n, nb, sc.seg, sc.seg + nb, s));
+        } else {
+            GTS_CUDA_TRY(cub::DeviceRadixSort::SortPairs(sc.temp, tb, sc.key, sc.key_alt, sc.posv, sc.posv_alt, n, 0,
+                                                         64, s));
+        }
+        if (!by_segment && cur_level > 0) {   // the key buffers serve the second pass
             uint32_t *lid = (uint32_t *)sc.key, *lid_alt = (uint32_t *)sc.key_alt;
             k_node_lids<<<(n + 255) / 256, 256, 0, s>>>(n, sc.posv_alt, sc.node_of_pos, idx->node_lid, lid);
             tb = temp_bytes;
@@ -524,7 +551,7 @@ static int build_tree_impl(gts_index *idx, cudaStream_t s)
                                                          lid_bits, s));
             order = sc.posv;
         }
-        k_apply_order<<<(n + 255) / 256, 256, 0, s>>>(n, order, idx->id_list, sc.ids_alt);
+        if (!by_segment) k_apply_order<<<(n + 255) / 256, 256, 0, s>>>(n, order, idx->id_list, sc.ids_alt);
         std::swap(idx->id_list, sc.ids_alt);
         GTS_CUDA_TRY(cudaMemsetAsync(sc.nsplit, 0, sizeof(int), s));
         long nthreads = (long)nb * O;
