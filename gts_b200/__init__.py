@@ -27,7 +27,7 @@ import os
 
 import numpy as np
 
-__all__ = ["GtsError", "Params", "Index", "load", "load_queries", "load_updates",
+__all__ = ["GtsError", "Params", "Index", "memory_release", "load", "load_queries", "load_updates",
            "indexConstru", "searchIndexKnnV2", "searchIndexRnnV2", "updateIndexRnn",
            "saveK", "saveR", "lib_path", "FORM_PLAIN", "FORM_FAST", "FORM_PLAIN_LEARNED"]
 
@@ -110,6 +110,16 @@ def _fp(a):
 
 
 # --------------------------------------------------------------------- I/O
+
+def memory_release() -> int:
+    """Give the device memory of freed indexes that waits for the next one (up
+    to 4 GiB per process) back to the driver; returns how many bytes.  Call it
+    when something else in the process needs the memory: the library itself
+    does when an allocation of its own fails."""
+    n = C.c_size_t()
+    _check(_load_lib().gts_memory_release(C.byref(n)))
+    return n.value
+
 
 def load(path: str):
     """Reference text data file -> (dim, num, metric, rows | (strs, lens))."""

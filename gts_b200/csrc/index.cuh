@@ -168,7 +168,7 @@ int sweep_range_ids(gts_index *idx, const int *d_qids, int qnum, float r, int *d
                     cudaStream_t s);
 
 // Device memory (memory.cu): as cudaMalloc / cudaFree, with freed blocks of
-// 1 MiB and more kept for the next request, up to a bound.
+// 64 KiB and more kept for the next request, up to a bound.
 cudaError_t dev_malloc(void **p, size_t bytes);
 void dev_free(void *p);
 

@@ -3,8 +3,11 @@
 // On a B200 host cudaMalloc of a block of 1 MiB or more takes 0.4 to 0.8 ms
 // and cudaFree 0.3 to 1 ms (single calls up to 10 ms), and building an index
 // takes some two dozen blocks: 9 of the 13 ms of building an index over
-// 200,000 words and asking it once.  Freed blocks of that size therefore wait,
-// up to kPoolCap bytes per process, for the next request they fit.
+// 200,000 words and asking it once.  Smaller blocks lie together in chunks of
+// 2 MiB, which cost as much whenever their sum passes another one: 0.6 ms more
+// for each index of 5,000 x 32 or 16,000 x 8.  Freed blocks of 64 KiB on
+// therefore wait, up to kPoolCap bytes and kPoolBlocks of them per process, for
+// the next request they fit.
 //
 //   * A block is handed out again only on its own device, and only after the
 //     device has been synchronised, as cudaFree would: a waiting block has no
@@ -23,9 +26,10 @@ namespace gts {
 
 namespace {
 
-constexpr size_t kPoolMin = (size_t)1 << 20;   // smaller blocks share the driver's own chunks and cost little
+constexpr size_t kPoolMin = (size_t)64 << 10;
 constexpr size_t kPoolCap = (size_t)4 << 30;
-constexpr size_t kPoolRound = (size_t)2 << 20;
+constexpr size_t kPoolBlocks = 1024;           // a request looks at each
+constexpr size_t kPoolLarge = (size_t)1 << 20, kPoolRound = (size_t)2 << 20;
 
 struct Block {
     void *p;
@@ -100,7 +104,8 @@ cudaError_t dev_malloc(void **p, size_t bytes)
 {
     *p = nullptr;
     if (bytes < kPoolMin) return cudaMalloc(p, bytes ? bytes : 1);
-    const size_t want = (bytes + kPoolRound - 1) / kPoolRound * kPoolRound;
+    const size_t unit = bytes < kPoolLarge ? kPoolMin : kPoolRound;
+    const size_t want = (bytes + unit - 1) / unit * unit;
     Block b{nullptr, want, 0, 0};
     where(&b.dev, &b.ctx);
     Pool &P = pool();
@@ -178,7 +183,7 @@ void dev_free(void *p)
         std::lock_guard<std::mutex> lock(P.m);
         P.idle.push_back(b);
         P.idle_bytes += b.bytes;
-        while (P.idle_bytes > kPoolCap) {
+        while (P.idle_bytes > kPoolCap || P.idle.size() > kPoolBlocks) {
             out.push_back(P.idle.front());
             P.idle_bytes -= P.idle.front().bytes;
             P.idle.erase(P.idle.begin());

@@ -118,7 +118,7 @@ int gts_index_export(const gts_index *idx, int *id_list, int *pid, float *min_di
 
 void gts_index_free(gts_index *idx);
 
-/* No counterpart in the reference.  Blocks of device memory of 1 MiB and more
+/* No counterpart in the reference.  Blocks of device memory of 64 KiB and more
  * that freed indexes (and grown work areas) no longer use are kept for the
  * next index, up to 4 GiB per process, because the driver takes about a
  * millisecond per block.  The library gives them back when one of its own

@@ -152,3 +152,10 @@ def test_small_batches_leave_their_buffers_out_of_a_tight_budget():
     tight, got = launches(hi)
     assert tight > 3
     np.testing.assert_array_equal(got, want)
+
+
+def test_memory_release_from_python():
+    with gts.Index(G.gmm_rows(100_000, 64, 16, 0.3, seed=11), 2, max_h=4):
+        pass
+    assert gts.memory_release() >= 50_000_000
+    assert gts.memory_release() == 0
