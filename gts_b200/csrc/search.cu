@@ -352,7 +352,13 @@ __global__ void __launch_bounds__(NT, 1) k_search(SearchArgs a)
             const int nint = s.nint, nleaf = s.nleaf;
             if (nint == 0 && nleaf == 0) break;
             const int nobj = s.leaf_pre[nleaf];
-            if (a.count_objs > 0 && s.n_obj >= (unsigned long long)a.count_objs) break;
+            if (a.count_objs > 0) {
+                // a step of leaves alone has no other barrier here between
+                // these reads and warp 0's next step
+                const bool enough = s.n_obj >= (unsigned long long)a.count_objs;
+                __syncthreads();
+                if (enough) break;
+            }
 
             // ---- leaves: filter every object, collect those needing exact values
             if (nleaf > 0 && a.count_objs <= 0) {
