@@ -777,11 +777,13 @@ def make_roofline(args, w, groups, stats, per_step_ms, total_ms, filter_ms, filt
         # sweep counts (query, kept row) pairs and reads a row once per tile
         # of 128 queries (strings: 32)
         row = 4 * d if w["metric"] != 6 else 113
-        swept = args.form == "plain" and (w["metric"] == 6 or d > 8)
+        # (the traversal counts a query's pivots, the sweep none)
+        plain = args.form != "plain-learned"   # strings and other metrics take the plain form whatever was asked
+        swept = plain and (w["metric"] == 6 or d > 8) and stats["pivots"] < sum(len(g["sel"]) for g in groups)
         share = (32 if w["metric"] == 6 else 128) if swept else 1
         ranges = all(g["op"] == "range" for g in groups)
         kernel = ("k_se_tile" if w["metric"] == 6 else "k_sw_tile") if swept else (
-            "k_search_warp" if args.form == "plain" and ranges else "k_search")
+            "k_search_warp" if plain and ranges and d <= 8 and w["metric"] != 6 else "k_search")
         alg_bytes = row * (stats["objects"] / share + stats["pivots"]) + sum(
             len(g["sel"]) * (row + (4 if g["op"] == "range" else 8 * int(g["p"]))) for g in groups)
         achieved = alg_bytes / (step_ms / 1e3) / 1e9

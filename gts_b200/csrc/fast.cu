@@ -16,8 +16,9 @@
 //    Block and superblock summaries (centre in FP32, |c|^2, radius max
 //    |o - c|) sit beside the records.
 //  * seeds: every query's k-th distance is bounded before any filtering by
-//    the k-th smallest distance inside its own block (the query is a data
-//    object), and by the learned radius model when one is trained.
+//    the k-th smallest distance over the objects of its own block and the 31
+//    nearest ones, from a table made with the records (fast_seed.cu; the query
+//    is a data object), and by the learned radius model when one is trained.
 //  * pruning: queries are sorted by block order into tiles of 128; the
 //    triangle inequality |q - c| - radius gives a lower bound per query and
 //    ball, first for superblocks, then for the blocks of the superblocks
@@ -30,8 +31,8 @@
 //    bulk copies, an MMA warp issues a 128 x 144 x K chain per block into one
 //    of three TMEM accumulators; 4 x CG epilogue warps turn each TMEM row into
 //    certified bounds lb <= d^2 <= ub for the 128 objects, keep the k
-//    smallest ub (a running k-th bound shared through global memory) and
-//    append every object with lb <= bound to the query's candidate list.
+//    smallest ub (a running k-th bound shared through global memory) or the
+//    bound the query came with, and append every object with lb <= bound to the query's candidate list.
 //    They meet only on mbarriers.
 //  * recheck: the final bound is the k-th smallest candidate ub; candidates
 //    with lb <= bound get their reference-arithmetic distance (one warp per
@@ -647,9 +648,9 @@ __device__ __forceinline__ bool fast_wait(uint64_t *bar, uint32_t parity, const 
 //              of block gi-3 has freed both.
 //   MMAs:      wait the operand and the accumulator gi%3, MMA chain, commit.
 //   epilogue:  wait the MMA of block gi, bound the 128 x 128 pairs, arrive
-//              on efree[gi%3].  Passing objects are staged in shared memory
-//              (shared-memory atomics only) and written to the queries'
-//              candidate lists once per item, one global atomic per thread.
+//              on efree[gi%3].  Passing objects are staged in the thread's
+//              slice of shared memory and written to the queries' candidate
+//              lists once per item, one global atomic per thread.
 // The warps meet only on mbarriers, across items too: the scheduling warp
 // writes an item's blocks while the one before is in work.
 //
@@ -1721,9 +1722,11 @@ static bool fast_tile_fits(const FastShape &fs, int cg, int k, bool stream);
 
 static FastCfg fast_default_cfg(const gts_index *idx, int k)
 {
-    // measured on clustered data: the own-block seed is tight for small k,
-    // the learned radius pays for its re-answers from k = 16 on; the column
-    // groups are the most whose shared memory fits this dimension
+    // batches too small to tune: the filter with bound heaps, which also serves
+    // seeds that leave something to tighten (the tuner measures it against the
+    // one without, larger batches only); the learned radius pays for its
+    // re-answers from k = 16 on; the column groups are the most whose shared
+    // memory fits this dimension
     const FastShape fs = fast_shape(idx->dim);
     const bool stream = fs.kp > kFResKp;
     int cg = fast_cg(k);

@@ -191,10 +191,9 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int m, int n)
 }
 
 // One lane of a converged warp, the same at every call.  MMAs are issued from
-// warp-uniform control flow under it: the compiler then keeps the operands in
-// uniform registers.  In a branch on the thread's index it moves each of them
-// there at every MMA: 107-135 cycles between 128 x 144 x 16 products that take
-// the tensor core 72.
+// warp-uniform control flow under it: 72 cycles between 128 x 144 x 16 products,
+// the tensor core's own time.  Issued in a branch on the thread's index they
+// followed each other in 107 to 135.
 __device__ __forceinline__ bool elect_one()
 {
     uint32_t r;

@@ -44,6 +44,8 @@ def run(scale: float = 0.1, seed: int = 11) -> None:
     qids = G.query_ids(n, q, seed=seed + 1)
     with _t("build", gts.Index, rows, 2, max_h=6 if n >= 400_000 else 5) as idx:
         fast = _t("fast kNN k=8 (first call: block order, records, autotune)", idx.knn, qids, 8, form=gts.FORM_FAST)
+        few = _t("fast kNN k=8, one query", idx.knn, qids[:1], 8, form=gts.FORM_FAST)
+        assert np.array_equal(fast[:1], few), "one query and a batch differ"
         plain = _t("plain kNN k=8", idx.knn, qids[: max(64, q // 10)], 8, form=gts.FORM_PLAIN)
         assert np.array_equal(fast[: len(plain)], plain), "fast and plain kNN differ"
         _t("learn radius", idx.learn_radius, n_train=max(2000, q * 4), k_max=64, epochs=4, seed=seed)

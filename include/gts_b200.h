@@ -38,7 +38,7 @@ extern "C" {
 
 /* Search forms. */
 #define GTS_FORM_PLAIN 0     /* ring bounds + FP32 filter + exact recheck, batched over row tiles
-                                (the pivot-tree traversal below its sizes and for what it leaves) */
+                                (the pivot-tree traversal where that is the sooner one) */
 #define GTS_FORM_FAST 1      /* learned radius + BF16 tensor-core filter + exact recheck (L2) */
 #define GTS_FORM_PLAIN_LEARNED 2  /* plain traversal seeded by the learned radius (L2, after
                                      gts_learn_radius; otherwise the plain form) */
