@@ -449,7 +449,9 @@ __global__ void __launch_bounds__(NT, 1) k_search(SearchArgs a)
                 // exact values for the collected positions
                 const int ncpos = s.ncpos;
                 if (tid == 0) s.n_exact += ncpos;
-                if (knn && s.ncand + ncpos > kCandCap) compact_candidates<NT>(s, a.k);
+                // the buffer holds them: every step leaves at most kCandCap -
+                // kLeafObjCap candidates behind (s.ncand may only be read
+                // between barriers: the others are adding to it already)
                 for (int c = tid; c < ncpos; c += NT) {
                     int pos = s.cpos[c];
                     int id = t.id_list[pos];
