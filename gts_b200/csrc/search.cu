@@ -350,7 +350,13 @@ __global__ void __launch_bounds__(NT, 1) k_search(SearchArgs a)
             }
             __syncthreads();
             const int nint = s.nint, nleaf = s.nleaf;
-            if (nint == 0 && nleaf == 0) break;
+            if (nint == 0 && nleaf == 0) {
+                // nothing left, or the bound has overtaken all entries of the
+                // step (kNN) and others lie below them
+                if (s.top == 0) break;
+                __syncthreads();
+                continue;
+            }
             const int nobj = s.leaf_pre[nleaf];
             if (a.count_objs > 0) {
                 // a step of leaves alone has no other barrier here between
