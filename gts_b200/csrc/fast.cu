@@ -2543,8 +2543,8 @@ static int fast_autotune(gts_index *idx, FastCall &fc, int qc, const int *d_qids
             best_ms = ms;
             best = c;
         }
-        // after the filter configurations, the best one with the other light recheck
-        if (ci + 1 == cands.size() && k <= kFinWarpK && !best.wfin) {
+        // after the filter configurations, the best one with the other light recheck, once
+        if (ci + 1 == cands.size() && k <= kFinWarpK && !c.wfin) {
             FastCfg w = best;
             w.wfin = true;
             cands.push_back(w);

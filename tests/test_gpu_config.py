@@ -80,3 +80,19 @@ def test_small_batches_by_width(oracle, dim, nq, tiles):
         assert (idx.kernel_launches() - n0 > 3) == tiles
         for x, y in zip(got, oracle.knn_brute(oracle.Dataset(2, rows), q, 8)):
             np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("dim", [130, 192, 250, 64])
+def test_tuning_ends(oracle, dim):
+    """Each configuration runs once, also where the recheck that is tried last
+    is the slower one."""
+    rows = G.gmm_rows(6000, dim, 1, 1.0, seed=dim)
+    q = G.query_ids(6000, 2100, 9)
+    with gts.Index(rows, 2, max_h=3) as idx:
+        idx.prepare()
+        for k in (1, 8):
+            n0 = idx.kernel_launches()
+            got = idx.knn(q, k, form=gts.FORM_FAST, return_ids=True)
+            assert idx.fast_config(k)["tuned"] and idx.kernel_launches() - n0 < 60 * 30   # 60 configurations at most
+            for x, y in zip(got, oracle.knn_brute(oracle.Dataset(2, rows), q[:50], k)):
+                np.testing.assert_array_equal(x[:50], y)
