@@ -2526,29 +2526,36 @@ static int fast_autotune(gts_index *idx, FastCall &fc, int qc, const int *d_qids
                         cands.push_back(FastCfg{learned != 0, cg, item, stream != 0, false});
         }
     }
-    for (size_t ci = 0; ci < cands.size(); ci++) {
-        const FastCfg c = cands[ci];
-        if (cudaEventRecord(e0, st) != cudaSuccess) {
-            rc = GTS_ERR_CUDA;
-            break;
-        }
-        if ((rc = fast_search_cfg(idx, fc, qc, c, d_qids, qnum, k, d_kth, d_ids, d_dists, st))) break;
-        float ms = 0.f;
+    auto timed_run = [&](const FastCfg &c, float *ms) -> int {
+        if (cudaEventRecord(e0, st) != cudaSuccess) return GTS_ERR_CUDA;
+        const int e = fast_search_cfg(idx, fc, qc, c, d_qids, qnum, k, d_kth, d_ids, d_dists, st);
+        if (e) return e;
         if (cudaEventRecord(e1, st) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
-            cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) {
-            rc = GTS_ERR_CUDA;
-            break;
-        }
+            cudaEventElapsedTime(ms, e0, e1) != cudaSuccess)
+            return GTS_ERR_CUDA;
+        return GTS_OK;
+    };
+    for (const FastCfg &c : cands) {
+        float ms = 0.f;
+        if ((rc = timed_run(c, &ms))) break;
         if (ms < best_ms) {
             best_ms = ms;
             best = c;
         }
-        // after the filter configurations, the best one with the other light recheck, once
-        if (ci + 1 == cands.size() && k <= kFinWarpK && !c.wfin) {
-            FastCfg w = best;
-            w.wfin = true;
-            cands.push_back(w);
+    }
+    // The best filter configuration with the other light recheck: two runs of
+    // each in turn, the faster one counts, since a first run captures its
+    // graph and every later one replays it.
+    if (!rc && k <= kFinWarpK) {
+        FastCfg two[2] = {best, best};
+        two[1].wfin = true;
+        float t[2] = {3.0e38f, 3.0e38f};
+        for (int i = 0; i < 4 && !rc; i++) {
+            float ms = 0.f;
+            rc = timed_run(two[i & 1], &ms);
+            t[i & 1] = std::min(t[i & 1], ms);
         }
+        best = two[t[1] < t[0] ? 1 : 0];
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
