@@ -2493,8 +2493,8 @@ static int fast_search_cfg(gts_index *idx, FastCall &fc, int qc, const FastCfg &
 // Autotuner.  The first batch of at least kTuneMinQueries queries with a
 // given k runs once per candidate configuration (learned seed on / off when
 // a model is trained, 4 / 2 / 1 epilogue column groups as the heap fits, 8 /
-// 16 / 32 blocks per work item), timed with CUDA events; every candidate
-// returns the same exact answers, so the fastest is kept for this k and
+// 16 / 32 blocks per work item), then the best one with both light rechecks,
+// timed with CUDA events; every candidate returns the same exact answers, so the fastest is kept for this k and
 // index (until the index is rebuilt or the model retrained).  Smaller batches
 // use the default configuration without tuning.
 constexpr int kTuneMinQueries = 2048;

@@ -84,8 +84,8 @@ def test_small_batches_by_width(oracle, dim, nq, tiles):
 
 @pytest.mark.parametrize("dim", [130, 192, 250, 64])
 def test_tuning_ends(oracle, dim):
-    """Each configuration runs once, also where the recheck that is tried last
-    is the slower one."""
+    """The runs are bounded, also where the recheck that is tried last is the
+    slower one."""
     rows = G.gmm_rows(6000, dim, 1, 1.0, seed=dim)
     q = G.query_ids(6000, 2100, 9)
     with gts.Index(rows, 2, max_h=3) as idx:
